@@ -110,3 +110,33 @@ def test_concat_matches_oracle(name):
     ref = dict(y=y, y_eval=y, dX=dX, dW=dW, dPE=dPE, idx=st["idx"], min_k=st["min_k"], min_delta=st["min_delta"],
                pidx=st["pidx"], pmin=st["pmin"], pmin_k=st["pmin_k"])
     compare(cfg, run_gpu(cfg, x, anchors, W, pe, dY), ref)
+
+
+# edges of the pair kernels: rows of one to several lane groups and ragged ones, two and three tokens, odd and even
+# lengths around a warp of pairs, and a sequence whose dX cells do not fit the block's shared memory
+PAIR_CASES = {
+    "two_tokens": dict(seed=820, B=3, S=2, E=12, Nt=3, Nc=2, Npe=2, O=4),
+    "three_tokens": dict(seed=821, B=2, S=3, E=12, Nt=3, Nc=2, Npe=0, O=8),
+    "odd_length": dict(seed=822, B=2, S=33, E=16, Nt=4, Nc=3, Npe=2, O=12, policy="internal", ext_lr=0.03125),
+    "full_warp": dict(seed=823, B=2, S=34, E=16, Nt=3, Nc=2, Npe=1, O=64),
+    "two_steps": dict(seed=824, B=2, S=9, E=16, Nt=3, Nc=2, Npe=2, O=132, policy="internal", ext_lr=0.03125),
+    "ragged": dict(seed=825, B=2, S=40, E=16, Nt=3, Nc=2, Npe=2, O=5),
+    "ragged_wide": dict(seed=826, B=2, S=7, E=16, Nt=3, Nc=2, Npe=2, O=45),
+    "long": dict(seed=827, B=1, S=1400, E=16, Nt=1, Nc=3, Npe=2, O=4),
+}
+
+
+@pytest.mark.parametrize("name", sorted(PAIR_CASES))
+def test_concat_pair_kernel_edges(name):
+    cfg = PAIR_CASES[name]
+    x, anchors, W, pe, dY = inputs_for(cfg)
+    pe3 = expand_pe(cfg, pe)
+    y, st = orc.concat_forward(W, x, pe3, anchors, cfg["Nt"], cfg["Nc"], cfg["O"], cfg["Npe"])
+    dX, dW, dPE = orc.concat_backward(W, dY, anchors, st, cfg["E"], cfg["Nc"], cfg["Npe"], forward_group_size=32)
+    ref = dict(y=y, y_eval=y, dX=dX, dPE=dPE, idx=st["idx"], min_k=st["min_k"], min_delta=st["min_delta"],
+               pidx=st["pidx"], pmin=st["pmin"], pmin_k=st["pmin_k"])
+    if cfg.get("policy") == "internal":
+        ref["W_after"] = W - np.float32(cfg["ext_lr"]) * dW.reshape(W.shape)
+    else:
+        ref["dW"] = dW
+    compare(cfg, run_gpu(cfg, x, anchors, W, pe, dY), ref)
