@@ -2,6 +2,8 @@
 //
 // Reference semantics: fill_outputs_product_cpu_logic (lut_runtime_kernels_logic.proto:2148-2264),
 // propagate_backward_product_cpu_logic (:2396-2628), gather_w_gradients_internal_product_cpu_logic (:2630-2744).
+#include <type_traits>
+
 #include "product_hist.cuh"
 #include "fp32_gemm_sm100.cuh"
 #include "product_pairs.cuh"
@@ -9,212 +11,599 @@
 namespace lutb {
 
 // --------------------------------------------------------------------------------------------
-// Row-selection histogram.  Block = (detector, sequence of the chunk); a warp owns a query j, counts the
-// rows its j keys select in a per-warp shared-memory histogram and writes it out as T uint16 counters.
-// H layout: [detector][row of the chunk = local sequence * S + j][T].
+// What the histogram and the routing kernel share: the detector's anchors sorted by what they compare.  An anchor pair
+// reads two elements of [x_i | x_j | pe(j - i - 1)], key token i and query token j.
 // --------------------------------------------------------------------------------------------
-// F32_ROWS: the counters are written as fp32 in the layout [row of the chunk][detector][T], the operand layout of the
-// tensor-core contractions (one plain GEMM over all detectors per pass).
-template <bool F32_ROWS>
-__global__ void __launch_bounds__(512) product_hist_kernel(const float *__restrict__ x1, const float *__restrict__ x2,
-                                                          const float *__restrict__ pe,
-                                                          const int32_t *__restrict__ anchors, void *__restrict__ Hout,
-                                                          int64_t b0, int64_t chunk_rows, int S, int e1, int e2, int npe,
-                                                          int n_detectors, int n_anchors, int sliced, float cmp_eps) {
-    extern __shared__ __align__(16) float smem[];
-    const int t = blockIdx.x;
-    const int64_t bl = blockIdx.y, b = b0 + bl;
-    PairStage st;
-    stage_pairs(st, smem, x1 + b * S * e1, x2 + b * S * e2, pe, anchors + (size_t)t * n_anchors * 2, S, e1, e2, npe,
-                n_anchors, n_detectors, t, sliced != 0, cmp_eps);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int T = 1 << n_anchors;
-    uint32_t *hist = reinterpret_cast<uint32_t *>(st.scratch) + warp * T;
-    for (int r = lane; r < T; r += 32) hist[r] = 0u;
-    __syncwarp();
-    for (int j = warp; j < S; j += nwarps) {
-        for (int i0 = 0; i0 < j; i0 += 32) {
-            const int i = i0 + lane;
-            int km; float dm;
-            if (i < j) atomicAdd(hist + eval_pair<false>(st, n_anchors, i, j, cmp_eps, km, dm), 1u);
+constexpr int kHistAnchors = 12;   // anchors per detector on the histogram path (tables of at most 4096 rows)
+
+struct AnchorLists {
+    int comp[2 * kHistAnchors], elem[2 * kHistAnchors];
+    int kq_pos[kHistAnchors];      // slot of a key-query anchor, -1: another kind
+    int pe_k[kHistAnchors];        // anchors with a positional end
+    int n_kq, n_pe;
+    uint32_t query_only, key_only, pe_mask;   // bit k set: anchor k is of that kind
+    // staged operands of the positional anchors: end e of anchor m is smem[at.x + i * at.y + q * at.z] for key i and query
+    // q as the kernel counts them, or (at.w) the query's staged end at.x
+    int4 pe_at[2 * kHistAnchors];
+};
+
+__device__ __forceinline__ void list_anchors(AnchorLists &al, const int32_t *__restrict__ anchors_t, int n_anchors, bool sliced,
+                                             int e1, int e2) {
+    if (threadIdx.x < 32) {   // lane k: anchor k
+        const int k = threadIdx.x;
+        int c[2] = {3, 3}, e[2] = {0, 0};
+        if (k < n_anchors) {
+            decode_anchor(__ldg(anchors_t + 2 * k), sliced, e1, e2, c[0], e[0]);
+            decode_anchor(__ldg(anchors_t + 2 * k + 1), sliced, e1, e2, c[1], e[1]);
         }
-        __syncwarp();
-        if (F32_ROWS) {
-            float *out = static_cast<float *>(Hout) + ((size_t)(bl * S + j) * n_detectors + t) * T;
-            for (int r = lane * 4; r < T; r += 128) {
-                const uint4 c = *reinterpret_cast<const uint4 *>(hist + r);
-                *reinterpret_cast<float4 *>(out + r) = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
-                *reinterpret_cast<uint4 *>(hist + r) = make_uint4(0u, 0u, 0u, 0u);
+        const bool used = c[0] != 3 && c[1] != 3, pe = used && (c[0] == 2 || c[1] == 2);
+        const bool kq = used && !pe && c[0] != c[1];
+        const unsigned pe_m = __ballot_sync(0xffffffffu, pe), kq_m = __ballot_sync(0xffffffffu, kq);
+        const unsigned ko_m = __ballot_sync(0xffffffffu, used && !pe && !kq && c[0] == 0);
+        const unsigned qo_m = __ballot_sync(0xffffffffu, used && !pe && !kq && c[0] == 1);
+        const unsigned below = (1u << k) - 1u;
+        if (k < kHistAnchors) {
+            al.comp[2 * k] = c[0]; al.comp[2 * k + 1] = c[1];
+            al.elem[2 * k] = e[0]; al.elem[2 * k + 1] = e[1];
+            al.kq_pos[k] = kq ? __popc(kq_m & below) : -1;
+            if (pe) al.pe_k[__popc(pe_m & below)] = k;
+        }
+        if (k == 0) {
+            al.n_kq = __popc(kq_m);
+            al.n_pe = __popc(pe_m);
+            al.pe_mask = pe_m; al.key_only = ko_m; al.query_only = qo_m;
+        }
+    }
+    __syncthreads();
+}
+
+// key > query with the dead band.  Without one the comparison of the operands is the comparison of their difference with
+// zero (subnormals are kept; equal infinities and NaN give false both ways).
+template <bool EPS>
+__device__ __forceinline__ bool above(float a, float b, float cmp_eps) {
+    return EPS ? greater_than_zero(__fsub_rn(a, b), cmp_eps) : a > b;
+}
+
+// Operands of query j0 + q, anchor k (each thread takes some (q, k)): the query end of key-query anchors (negated where
+// it comes first: every delta is then key minus query) with the anchor's bit, the whole delta of query-only ones, the
+// query end of positional ones.
+__device__ __forceinline__ void stage_query(const AnchorLists &al, float2 *qv, float *qd, const float *__restrict__ xq, int q, int k) {
+    const int slot = al.kq_pos[k];
+    const int c0 = al.comp[2 * k], c1 = al.comp[2 * k + 1];
+    if (c0 != 1 && c1 != 1) return;
+    const float v0 = c0 == 1 ? __ldg(xq + al.elem[2 * k]) : 0.f, v1 = c1 == 1 ? __ldg(xq + al.elem[2 * k + 1]) : 0.f;
+    if (slot >= 0) qv[q * kHistAnchors + slot] = make_float2(c0 == 1 ? -v0 : v1, __uint_as_float(1u << k));
+    else if ((al.query_only >> k) & 1u) qd[q * kHistAnchors + k] = __fsub_rn(v0, v1);
+    else qd[q * kHistAnchors + k] = c0 == 1 ? v0 : v1;
+}
+
+// The two ends of positional anchor m: staged, or (anchors past the staged ones) from global memory.  i, q: key and query
+// as the kernel counts them for its staged operands; qd_row: the query's staged ends.
+__device__ __forceinline__ void positional_ends(const AnchorLists &al, const float *smem, const float *qd_row, int m, bool staged,
+                                                int i, int q, const float *__restrict__ xk, const float *__restrict__ xq,
+                                                const float *__restrict__ pe_d, float &v0, float &v1) {
+    if (staged) {
+        const int4 a = al.pe_at[2 * m], b = al.pe_at[2 * m + 1];
+        v0 = (a.w ? qd_row : smem)[a.x + i * a.y + q * a.z];
+        v1 = (b.w ? qd_row : smem)[b.x + i * b.y + q * b.z];
+        return;
+    }
+    const int k = al.pe_k[m];
+    const int c0 = al.comp[2 * k], c1 = al.comp[2 * k + 1];
+    v0 = __ldg((c0 == 0 ? xk : c0 == 1 ? xq : pe_d) + al.elem[2 * k]);
+    v1 = __ldg((c1 == 0 ? xk : c1 == 1 ? xq : pe_d) + al.elem[2 * k + 1]);
+}
+
+// --------------------------------------------------------------------------------------------
+// Row-selection histogram: for every query (b, j) and detector t, how many of the j keys select each of the T rows.
+// Block = (detector, 128 queries, sequence); what the pairs need of the keys is staged once, then the warps work on their
+// own: a warp takes four queries at a time, counts in a private shared-memory array and writes it out.  LANE = KEY: the
+// key ends of 32 keys are in registers while the warp walks its queries, whose operands (two anchors' query ends and
+// bits per 16-byte load) are the same for all lanes; a key-query anchor then costs a compare and a predicated OR.  The
+// loop over the anchors is unrolled for their number (NKQ), so that the four queries overlap.
+// F32_ROWS: the counters are written as fp32 in the layout [row of the chunk = local sequence * S + j][detector][T], the
+// operand layout of the tensor-core contractions (one plain GEMM over all detectors per pass); otherwise as uint16 in
+// the layout [detector][row of the chunk][T].
+// PACKED: two 16-bit counters per word (a count is at most S - 1 < 65536), which keeps 16 warps per block up to
+// 1024-row tables.
+// Bound: instruction issue, and at 256-row tables the 537 MB of counters it writes.  Measured (before: lanes over the keys
+// of one query, the anchors' operands read from shared memory for every pair): 64 sequences x 128 tokens, 64 detectors of
+// 256 rows 271 -> 182 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 187 us.
+// --------------------------------------------------------------------------------------------
+constexpr int kHistQueries = 128, kHistTile = 4;
+
+struct HistArgs {
+    const float *x1, *x2, *pe;
+    const int32_t *anchors;
+    void *H;
+    int64_t b0, chunk_rows;
+    int S, e1, e2, npe, n_detectors, n_anchors, sliced;
+    float cmp_eps;
+    int pe_cap;      // anchors with a positional end whose operands are staged in shared memory
+};
+
+// dynamic shared memory of one block, in floats: per warp counters and query operands | key ends | key bits | positional operands
+__host__ __device__ inline size_t hist_warp_floats(int T, bool packed) {
+    return (size_t)kHistTile * T / (packed ? 2 : 1) + kHistTile * kHistAnchors * 3;
+}
+__host__ __device__ inline size_t hist_floats(int T, bool packed, int warps, int n_anchors, int pe_cap, int S) {
+    const int Sp = (S + 31) & ~31;
+    return warps * hist_warp_floats(T, packed) + (size_t)(n_anchors + 1 + 3 * pe_cap) * Sp;
+}
+
+template <bool PACKED>
+__device__ __forceinline__ void count_row(uint32_t *hist, uint32_t li) {
+    if (PACKED) atomicAdd(hist + (li >> 1), 1u << ((li & 1u) * 16u));
+    else atomicAdd(hist + li, 1u);
+}
+
+struct HistTile {
+    const float *smem, *ks, *qd, *x1b, *x2b, *pe_t;   // pe_t: embeddings of the block's detector
+    const uint32_t *kb_s;
+    uint32_t *hist;
+    const float2 *qv;
+    int Sp, j0, nq, n_kq, n_pe, pe_stride;
+};
+
+// counts the keys of queries j0 .. j0 + nq - 1
+template <int NKQ, bool PE, bool EPS, bool PACKED>
+__device__ __forceinline__ void count_tile(const HistArgs &p, const AnchorLists &al, const HistTile &h, uint32_t qbits) {
+    const int lane = threadIdx.x & 31;
+    const int T = 1 << p.n_anchors, words = PACKED ? T / 2 : T;
+    for (int i0 = 0; i0 < h.j0 + h.nq - 1; i0 += 32) {
+        const int i = i0 + lane;
+        float kv[NKQ > 0 ? NKQ : 1];
+#pragma unroll
+        for (int m = 0; m < NKQ; m++) kv[m] = m < h.n_kq ? h.ks[m * h.Sp + i] : 0.f;
+        const uint32_t kbits = h.kb_s[i];
+#pragma unroll
+        for (int q = 0; q < kHistTile; q++) {
+            const int j = h.j0 + q;
+            uint32_t li = kbits | __shfl_sync(0xffffffffu, qbits, q);
+            const float4 *qv4 = reinterpret_cast<const float4 *>(h.qv + q * kHistAnchors);
+#pragma unroll
+            for (int m = 0; m < NKQ; m += 2) {
+                const float4 f = qv4[m / 2];
+                if (above<EPS>(kv[m], f.x, p.cmp_eps)) li |= __float_as_uint(f.y);
+                if (above<EPS>(kv[m + 1], f.z, p.cmp_eps)) li |= __float_as_uint(f.w);
             }
-            __syncwarp();
+            if (i < j && q < h.nq) {
+                if (PE) {
+                    for (int m = 0; m < h.n_pe; m++) {
+                        float v0, v1;
+                        positional_ends(al, h.smem, h.qd + q * kHistAnchors, m, m < p.pe_cap, i, j, h.x1b + (size_t)i * p.e1, h.x2b + (size_t)j * p.e2,
+                                        h.pe_t + (size_t)(j - i - 1) * h.pe_stride, v0, v1);
+                        if (above<EPS>(v0, v1, p.cmp_eps)) li |= 1u << al.pe_k[m];
+                    }
+                }
+                count_row<PACKED>(h.hist + q * words, li);
+            }
+        }
+    }
+}
+
+template <int MAXKQ, bool EPS, bool F32_ROWS, bool PACKED>
+__global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ AnchorLists al;
+    const int t = blockIdx.x;
+    const int j_begin = (gridDim.y - 1 - blockIdx.y) * kHistQueries;   // the ranges with the most keys first
+    const int64_t bl = blockIdx.z, b = p.b0 + bl;
+    const int S = p.S, Nc = p.n_anchors, T = 1 << Nc, Sp = (S + 31) & ~31;
+    const int j_end = min(S, j_begin + kHistQueries);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int words = PACKED ? T / 2 : T;
+    const size_t per_warp = hist_warp_floats(T, PACKED);
+    uint32_t *hist = reinterpret_cast<uint32_t *>(smem + warp * per_warp);          // [kHistTile][words]
+    float2 *qv = reinterpret_cast<float2 *>(hist + kHistTile * words);             // [kHistTile][kHistAnchors] (query end, bit)
+    float *qd = reinterpret_cast<float *>(qv + kHistTile * kHistAnchors);          // [kHistTile][kHistAnchors]
+    float *ks = smem + nwarps * per_warp;                                          // [Nc][Sp] key ends of the key-query anchors
+    uint32_t *kb_s = reinterpret_cast<uint32_t *>(ks + Nc * Sp);                   // [Sp] bits of the key-only anchors
+    float *kpe = reinterpret_cast<float *>(kb_s + Sp);                             // [pe_cap][Sp] key ends of the positional anchors
+    float *pes = kpe + p.pe_cap * Sp;                                              // [2 * pe_cap][Sp] positional ends by distance
+    list_anchors(al, p.anchors + (size_t)t * Nc * 2, Nc, p.sliced != 0, p.e1, p.e2);
+    const int n_kq = al.n_kq, n_pe = al.n_pe;
+
+    for (int w = lane; w < kHistTile * words; w += 32) hist[w] = 0u;
+    // slots past the last key-query anchor: a NaN compares false everywhere
+    for (int w = lane; w < kHistTile * kHistAnchors; w += 32) qv[w] = make_float2(__int_as_float(0x7fffffff), 0.f);
+    const float *x1b = p.x1 + (size_t)b * S * p.e1, *x2b = p.x2 + (size_t)b * S * p.e2;
+    for (int k = warp; k <= Nc; k += nwarps) {   // one warp per anchor; the key bits last
+        if (k == Nc) {
+            for (int i = lane; i < j_end; i += 32) {
+                uint32_t bits = 0u;
+                for (uint32_t left = al.key_only; left; left &= left - 1) {
+                    const int a = __ffs(left) - 1;
+                    if (above<EPS>(__ldg(x1b + (size_t)i * p.e1 + al.elem[2 * a]), __ldg(x1b + (size_t)i * p.e1 + al.elem[2 * a + 1]), p.cmp_eps)) bits |= 1u << a;
+                }
+                kb_s[i] = bits;
+            }
             continue;
         }
-        uint16_t *out = static_cast<uint16_t *>(Hout) + ((size_t)t * chunk_rows + bl * S + j) * T;
-        for (int r = lane * 8; r < T; r += 256) {
-            const uint4 lo = *reinterpret_cast<const uint4 *>(hist + r);
-            const uint4 hi = *reinterpret_cast<const uint4 *>(hist + r + 4);
-            uint4 packed;
-            packed.x = lo.x | (lo.y << 16);
-            packed.y = lo.z | (lo.w << 16);
-            packed.z = hi.x | (hi.y << 16);
-            packed.w = hi.z | (hi.w << 16);
-            *reinterpret_cast<uint4 *>(out + r) = packed;
-            *reinterpret_cast<uint4 *>(hist + r) = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4 *>(hist + r + 4) = make_uint4(0u, 0u, 0u, 0u);
+        const int slot = al.kq_pos[k], c0 = al.comp[2 * k];
+        if (slot < 0) continue;
+        const float *src = x1b + al.elem[2 * k + (c0 == 0 ? 0 : 1)];
+#pragma unroll 4
+        for (int i = lane; i < j_end; i += 32) {
+            const float v = __ldg(src + (size_t)i * p.e1);
+            ks[slot * Sp + i] = c0 == 0 ? v : -v;
+        }
+    }
+    for (int m = 0; m < min(n_pe, p.pe_cap); m++) {
+        const int k = al.pe_k[m];
+        for (int e = 0; e < 2; e++) {
+            const int c = al.comp[2 * k + e], el = al.elem[2 * k + e];
+            if (c == 0)
+                for (int i = threadIdx.x; i < j_end; i += blockDim.x) kpe[m * Sp + i] = __ldg(x1b + (size_t)i * p.e1 + el);
+            else if (c == 2)
+                for (int d = threadIdx.x; d < j_end - 1; d += blockDim.x)
+                    pes[(2 * m + e) * Sp + d] = __ldg(p.pe + ((size_t)d * p.n_detectors + t) * p.npe + el);
+            // (keys and queries are counted from the start of the sequence here: distance j - i - 1)
+            if (threadIdx.x == 0)
+                al.pe_at[2 * m + e] = c == 0 ? make_int4((int)(kpe + m * Sp - smem), 1, 0, 0)
+                                    : c == 2 ? make_int4((int)(pes + (2 * m + e) * Sp - smem) - 1, -1, 1, 0)
+                                             : make_int4(k, 0, 0, 1);
+        }
+    }
+    __syncthreads();
+
+    HistTile h;
+    h.smem = smem; h.ks = ks; h.kb_s = kb_s; h.x1b = x1b; h.x2b = x2b;
+    h.pe_t = p.pe + (size_t)t * p.npe;
+    h.pe_stride = p.n_detectors * p.npe;
+    h.hist = hist; h.qv = qv; h.qd = qd; h.Sp = Sp; h.n_kq = n_kq; h.n_pe = n_pe;
+    const int tiles = (j_end - j_begin + kHistTile - 1) / kHistTile;
+    for (int n = 0; n * nwarps < tiles; n++) {
+        // back and forth over the warps: later tiles have more keys
+        const int tile = n * nwarps + ((n & 1) ? nwarps - 1 - warp : warp);
+        if (tile >= tiles) continue;
+        const int j0 = j_begin + tile * kHistTile, nq = min(kHistTile, j_end - j0);
+        {
+            const int q = lane & (kHistTile - 1);
+            if (q < nq)
+                for (int k = lane / kHistTile; k < Nc; k += 32 / kHistTile) stage_query(al, qv, qd, x2b + (size_t)(j0 + q) * p.e2, q, k);
+        }
+        __syncwarp();
+        uint32_t qbits = 0u;   // lane q: the query-only anchors of query j0 + q
+        if (lane < kHistTile) {
+            for (uint32_t left = al.query_only; left; left &= left - 1) {
+                const int k = __ffs(left) - 1;
+                if (above<EPS>(qd[lane * kHistAnchors + k], 0.f, p.cmp_eps)) qbits |= 1u << k;
+            }
+        }
+        h.j0 = j0; h.nq = nq;
+        if (EPS || n_pe > 0) count_tile<MAXKQ, true, EPS, PACKED>(p, al, h, qbits);
+        else if (n_kq <= 2) count_tile<2, false, EPS, PACKED>(p, al, h, qbits);
+        else if (n_kq <= 4) count_tile<4, false, EPS, PACKED>(p, al, h, qbits);
+        else if (n_kq <= 6) count_tile<6, false, EPS, PACKED>(p, al, h, qbits);
+        else if (MAXKQ == 8 || n_kq <= 8) count_tile<8, false, EPS, PACKED>(p, al, h, qbits);
+        else count_tile<MAXKQ, false, EPS, PACKED>(p, al, h, qbits);
+        __syncwarp();
+        // write out and clear
+        float *out_f = static_cast<float *>(p.H) + ((size_t)(bl * S + j0) * p.n_detectors + t) * T;
+        uint16_t *out_h = static_cast<uint16_t *>(p.H) + ((size_t)t * p.chunk_rows + bl * S + j0) * T;
+        for (int w = lane; w < nq * (T / 4); w += 32) {
+            const int q = w >> (Nc - 2), r = w & (T / 4 - 1);
+            uint4 c;
+            if (PACKED) {
+                uint2 *cell = reinterpret_cast<uint2 *>(hist) + w;
+                const uint2 v = *cell;
+                *cell = make_uint2(0u, 0u);
+                c = make_uint4(v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16);
+            } else {
+                uint4 *cell = reinterpret_cast<uint4 *>(hist) + w;
+                c = *cell;
+                *cell = make_uint4(0u, 0u, 0u, 0u);
+            }
+            if (F32_ROWS) *reinterpret_cast<float4 *>(out_f + (size_t)q * p.n_detectors * T + r * 4) = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
+            else *reinterpret_cast<uint2 *>(out_h + (size_t)w * 4) = make_uint2(c.x | (c.y << 16), c.z | (c.w << 16));
         }
         __syncwarp();
     }
 }
 
 // --------------------------------------------------------------------------------------------
-// Input-gradient routing.  Same block / warp layout; the warp stages Q_t[(b,j), :] (the dot product of
-// dY[b,j,:] with every row of table t) and each pair reads its two entries: g = Q[idx] - Q[idx ^ 2^kmin],
-// du = up(min_delta) * g, +du / -du to the sources of the flipped anchor's two ends.
-// SMEM_ACC: the block first sums its contributions per (token, anchor end) and per (distance, element) in shared
-// memory and issues one global atomic per touched cell at the end (the global atomics of a block drop from one
-// or two per pair to at most S * 2 * Nc + (S-1) * Npe); without it only the query token's cells are pre-reduced
-// per warp.
+// Input-gradient routing: every pair (i, j) reads two entries of Q_t[(b,j), :] (the dot products of dY[b,j,:] with the
+// rows of table t): g = Q[idx] - Q[idx ^ 2^kmin], du = up(min_delta) * g, +du / -du to the sources of the flipped
+// anchor's two ends.
+//
+// Bound by instruction issue, so the pairs are laid out for the fewest instructions per pair.  Block = (detector, 128
+// keys, sequence), four warps; LANE = KEY: a lane keeps what a pair needs of its key in registers for the whole block
+// (the key ends of the anchors that compare a key with a query, the bits and smallest delta of the anchors that read
+// the key alone), and the warps walk the queries above it, eight at a time.  What a pair needs of the query is the same
+// for all lanes: one 16-byte shared load brings two anchors' query ends and their bits.  Values whose query end comes
+// first are negated on both sides, so that every delta is key minus query.  Key-range blocks also give a single long
+// sequence S / 128 times the blocks (64 detectors alone leave more than half of the SMs idle).
+//
+// Sums: the key's cells are a private shared-memory column per lane (plain read-modify-write), flushed once per block.
+// The query's cells would collide (32 lanes, a few anchors), so a pair's (du, anchor) is parked in an 8 x 32 tile that
+// the warp reads back with the lanes over queries, again into private columns; the block adds the columns up once per
+// eight queries.
+// Measured (before: a warp per query, about 600 instructions per 32 pairs): 64 sequences x 128 tokens, 64 detectors of 256
+// rows 862 -> 478 us; 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 922 us.
 // --------------------------------------------------------------------------------------------
-// MAXM > 0: the pair loop keeps the address plan of the detector's mixed anchors (at most MAXM) in registers
-// (product_pairs.cuh, MixedPlan); 0: plain eval_pair.  The plan costs about 5 registers per anchor: it pays where the
-// block's shared memory already limits an SM to one block (tables of 1024 rows and more: 257 against 286 ms per step on
-// the 1024-token, 1024-row configuration) and loses where it takes the second block away (256-row tables: 5.1 against 3.5 ms).
-// HIST: the kernel evaluates every pair anyway, so it can count the selected rows on the way and write the histogram
-// the table-gradient contraction needs (1: uint16 [detector][row of the chunk][T], 2: fp32 [row of the chunk][detector][T],
-// the layouts of product_hist_kernel); the backward pass then launches no histogram kernel of its own.  Used where the
-// extra T counters per warp do not cost the block its occupancy.
-// QG: the two entries of Q a pair needs are read from global memory (through L1) instead of from a staged copy of the
-// query's row: T floats less scratch per warp, on long sequences the difference between 8 and 16 warps per block.
-template <bool SMEM_ACC, int MAXM, int HIST, bool QG>
-__global__ void __launch_bounds__(512) product_route_kernel(const float *__restrict__ x1, const float *__restrict__ x2,
-                                                           const float *__restrict__ pe,
-                                                           const int32_t *__restrict__ anchors,
-                                                           const float *__restrict__ Q, float *__restrict__ dX1,
-                                                           float *__restrict__ dX2, float *__restrict__ dPE, int64_t b0,
-                                                           int64_t q_row_stride, int64_t q_det_stride, int S, int e1,
-                                                           int e2, int npe, int n_detectors, int n_anchors, int sliced,
-                                                           float cmp_eps, void *__restrict__ Hout, int64_t chunk_rows) {
-    extern __shared__ __align__(16) float smem[];
-    const int t = blockIdx.x;
-    const int64_t bl = blockIdx.y, b = b0 + bl;
-    PairStage st;
-    stage_pairs(st, smem, x1 + b * S * e1, x2 + b * S * e2, pe, anchors + (size_t)t * n_anchors * 2, S, e1, e2, npe,
-                n_anchors, n_detectors, t, sliced != 0, cmp_eps);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int T = 1 << n_anchors;
-    const int ends = 2 * n_anchors;
-    const int q_floats = QG ? 0 : T;
-    const int per_warp = q_floats + 32 * ends + (HIST ? T : 0);
-    float *q_s = st.scratch + warp * per_warp;
-    uint32_t *hist = reinterpret_cast<uint32_t *>(q_s + q_floats + 32 * ends);
-    if (HIST) {
-        for (int r = lane; r < T; r += 32) hist[r] = 0u;
-        __syncwarp();
-    }
-    // contributions to the query token j: a private column per lane ([end][lane], plain read-modify-write; every
-    // lane of a pair batch would otherwise hit the same few cells), summed over the lanes once per query
-    float *jacc = q_s + q_floats;
-    float *tacc = st.scratch + nwarps * per_warp;  // [S][ends]
-    float *pacc = tacc + S * ends;                            // [S-1][npe]
-    if (SMEM_ACC) {
-        for (int w = threadIdx.x; w < S * ends + (S - 1) * npe; w += blockDim.x) tacc[w] = 0.f;
-        __syncthreads();
-    }
-    MixedPlan<MAXM == 0 ? 1 : MAXM> mp;
-    if (MAXM > 0) mp.load(st);
-    for (int j = (HIST ? 0 : 1) + warp; j < S; j += nwarps) {   // (query 0 has no pair: only its empty histogram row)
-        QueryPart qp{0u, 0.f};
-        if (MAXM > 0) {
-            mp.set_query(st, j);
-            qp = query_part(st, j);
-        }
-        const float *qrow = Q + (size_t)t * q_det_stride + (size_t)(bl * S + j) * q_row_stride;
-        if (!QG)
-            for (int r = lane * 4; r < T; r += 128)
-                *reinterpret_cast<float4 *>(q_s + r) = __ldcs(reinterpret_cast<const float4 *>(qrow + r));
-        for (int q = 0; q < ends; q++) jacc[q * 32 + lane] = 0.f;
-        __syncwarp();
-        for (int i0 = 0; i0 < j; i0 += 32) {
-            const int i = i0 + lane;
-            if (i >= j) continue;
-            int k; float d;
-            const int32_t li = MAXM > 0 ? eval_pair_planned<true, (MAXM == 0 ? 1 : MAXM)>(st, mp, qp, i, j, cmp_eps, k, d)
-                                        : eval_pair<true>(st, n_anchors, i, j, cmp_eps, k, d);
-            if (HIST) atomicAdd(hist + li, 1u);
-            if (k < 0) continue;
-            // up(d) * (Q[row] - Q[flipped row]) in fp32: Q is an fp32 contraction already, and the double-precision
-            // reciprocal of the reference's formula was the most expensive part of a pair (the direct kernels and the
-            // fixed-point mode keep it)
-            const float rcp = __frcp_rn(1.0f + fabsf(d));
-            const float q_sel = QG ? __ldg(qrow + li) : q_s[li];
-            const float q_alt = QG ? __ldg(qrow + (li ^ (1 << k))) : q_s[li ^ (1 << k)];
-            const float du = (d > 0.f ? 0.5f : -0.5f) * rcp * rcp * (q_sel - q_alt);
-            if (!(fabsf(du) > kEpsF)) continue;
+constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
+constexpr int kExLd = 33;          // leading dimension of the (query, key) exchange tile
+
+struct RouteArgs {
+    const float *x1, *x2, *pe;
+    const int32_t *anchors;
+    const float *Q;
+    float *dX1, *dX2, *dPE;
+    int64_t b0, q_row_stride, q_det_stride;
+    int S, e1, e2, npe, n_detectors, n_anchors, sliced;
+    float cmp_eps;
+    int pe_cap;      // anchors with a positional end whose operands are staged in shared memory
+    int pe_cells;    // 1: the block sums dPE in shared memory
+};
+
+// dynamic shared memory of one block, in floats: Q rows | query operands | per-warp columns and exchange tile | staged
+// positional operands | dPE cells
+__host__ __device__ inline size_t route_floats(int T, int n_anchors, int pe_cap, int pe_cells, int S, int npe) {
+    return (size_t)kTileQ * T + kTileQ * kHistAnchors * 3 + (size_t)kRouteWarps * (64 * n_anchors + 2 * kTileQ * kExLd) +
+           (size_t)pe_cap * (kRouteKeys + 2 * kRouteWindow) + (pe_cells ? (size_t)(S - 1) * npe : 0);
+}
+
+// The running first minimum of |delta| as one ordered integer: |delta| above, the anchor below, so that "smaller, or equal
+// with a smaller anchor number" is a 64-bit comparison.  It starts at FLT_MAX without an anchor; a delta that is no smaller
+// (or NaN) never replaces it.  low: the anchor's bit; with a dead band, twice that plus "delta > 0" (without one, that is
+// what the anchor's bit of the table index says).
+__device__ __forceinline__ unsigned long long margin_key(float abs_d, uint32_t low) {
+    return ((unsigned long long)__float_as_uint(abs_d) << 32) | low;
+}
+template <bool EPS>
+__device__ __forceinline__ uint32_t margin_low(uint32_t bit, float d) {
+    return EPS ? 2u * bit + (d > 0.f ? 1u : 0u) : bit;
+}
+
+struct RouteTile {
+    const float *smem, *Qs, *qd, *xk, *x2b, *pe_t;
+    const float4 *qstate;   // [kTileQ] {bits, |delta|, low of the query-only anchors}
+    const float2 *qv;
+    float *kcol, *pacc;
+    float2 *ex;
+    int j0, i, ikey, n_pe, pe_stride, t;
+    uint32_t pe_mask, kbits;
+    unsigned long long kmin;
+};
+
+template <int NKQ, bool PE, bool EPS, int MAXKQ>
+__device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists &al, const RouteTile &r, const float (&kv)[MAXKQ]) {
+    const int lane = threadIdx.x & 31, T = 1 << p.n_anchors;
+#pragma unroll 4
+    for (int q = 0; q < kTileQ; q++) {
+        const int j = r.j0 + q;
+        const float4 qs = r.qstate[q];
+        uint32_t li = r.kbits | __float_as_uint(qs.x);
+        unsigned long long best = margin_key(qs.y, __float_as_uint(qs.z));
+        best = r.kmin < best ? r.kmin : best;
+        if (NKQ > 0) {
+            // anchor numbers ascend: strictly smaller is enough inside this group
+            float md = kFltMax;
+            uint32_t low = 0u;
+            const float4 *qv4 = reinterpret_cast<const float4 *>(r.qv + q * kHistAnchors);
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int comp = st.comp[2 * k + e], elem = st.elem[2 * k + e];
-                const float val = e == 0 ? du : -du;
-                if (comp == 0) {
-                    if (SMEM_ACC) atomicAdd(tacc + i * ends + 2 * k + e, val);
-                    else atomicAdd(dX1 + ((size_t)b * S + i) * e1 + elem, val);
-                } else if (comp == 1) {
-                    jacc[(2 * k + e) * 32 + lane] += val;
-                } else if (comp == 2) {
-                    if (SMEM_ACC) atomicAdd(pacc + (j - i - 1) * npe + elem, val);
-                    else atomicAdd(dPE + ((size_t)(j - i - 1) * n_detectors + t) * npe + elem, val);
+            for (int m = 0; m < NKQ; m += 2) {
+                const float4 f = qv4[m / 2];
+                const float da = __fsub_rn(kv[m], f.x), db = __fsub_rn(kv[m + 1], f.z);
+                const uint32_t ba = __float_as_uint(f.y), bb = __float_as_uint(f.w);
+                if (EPS ? greater_than_zero(da, p.cmp_eps) : da > 0.f) li |= ba;
+                if (fabsf(da) < md) { md = fabsf(da); low = margin_low<EPS>(ba, da); }
+                if (EPS ? greater_than_zero(db, p.cmp_eps) : db > 0.f) li |= bb;
+                if (fabsf(db) < md) { md = fabsf(db); low = margin_low<EPS>(bb, db); }
+            }
+            const unsigned long long mixed = margin_key(md, low);
+            best = mixed < best ? mixed : best;
+        }
+        const bool pair = r.i < j && j < p.S;
+        const int dist = max(0, min(j, p.S - 1) - r.i - 1);
+        if (PE) {
+            for (int m = 0; m < r.n_pe; m++) {
+                float v0, v1;
+                positional_ends(al, r.smem, r.qd + q * kHistAnchors, m, m < p.pe_cap, r.ikey, q, r.xk,
+                                r.x2b + (size_t)min(j, p.S - 1) * p.e2, r.pe_t + (size_t)dist * r.pe_stride, v0, v1);
+                const uint32_t bit = 1u << al.pe_k[m];
+                const float d = __fsub_rn(v0, v1);
+                if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= bit;
+                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(bit, d));
+                best = c < best ? c : best;
+            }
+        }
+        const float md = __uint_as_float((uint32_t)(best >> 32));
+        const uint32_t low = (uint32_t)best, bit = EPS ? low >> 1 : low;
+        const bool positive = EPS ? (low & 1u) != 0u : (li & bit) != 0u;
+        // up(d) * (Q[row] - Q[flipped row]) in fp32: Q is an fp32 contraction already (the direct kernels and the
+        // fixed-point mode keep the double-precision reciprocal of the reference's formula).  One Newton step on the
+        // hardware's reciprocal is as close as the rounded one and needs no branch.
+        const float a = 1.0f + md;
+        float rc;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(a));
+        rc = fmaf(rc, fmaf(-a, rc, 1.0f), rc);
+        const float *qrow = r.Qs + q * T;
+        float du = (positive ? 0.5f : -0.5f) * rc * rc * (qrow[li] - qrow[li ^ bit]);
+        du = pair && bit != 0u && fabsf(du) > kEpsF ? du : 0.f;
+        const int off = bit ? (31 - __clz(bit)) * 32 : 0;
+        r.kcol[off + lane] += du;
+        r.ex[q * kExLd + lane] = make_float2(du, __int_as_float(off));
+        if (PE) {
+            if ((bit & r.pe_mask) && du != 0.f) {
+                const int k = off / 32;
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    if (al.comp[2 * k + e] != 2) continue;
+                    const float v = e == 0 ? du : -du;
+                    if (p.pe_cells) atomicAdd(r.pacc + dist * p.npe + al.elem[2 * k + e], v);
+                    else atomicAdd(p.dPE + ((size_t)dist * p.n_detectors + r.t) * p.npe + al.elem[2 * k + e], v);
                 }
             }
         }
-        __syncwarp();
-        if (lane < ends && st.comp[lane] == 1) {
-            float sum = 0.f;
-#pragma unroll 8
-            for (int m = 0; m < 32; m++) sum += jacc[lane * 32 + ((m + lane) & 31)];
-            if (sum != 0.f) {
-                if (SMEM_ACC) atomicAdd(tacc + j * ends + lane, sum);
-                else atomicAdd(dX2 + ((size_t)b * S + j) * e2 + st.elem[lane], sum);
-            }
-        }
-        __syncwarp();
-        if (HIST == 2) {
-            float *out = static_cast<float *>(Hout) + ((size_t)(bl * S + j) * n_detectors + t) * T;
-            for (int r = lane * 4; r < T; r += 128) {
-                const uint4 c = *reinterpret_cast<const uint4 *>(hist + r);
-                *reinterpret_cast<float4 *>(out + r) = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
-                *reinterpret_cast<uint4 *>(hist + r) = make_uint4(0u, 0u, 0u, 0u);
-            }
-            __syncwarp();
-        } else if (HIST == 1) {
-            uint16_t *out = static_cast<uint16_t *>(Hout) + ((size_t)t * chunk_rows + bl * S + j) * T;
-            for (int r = lane * 8; r < T; r += 256) {
-                const uint4 lo = *reinterpret_cast<const uint4 *>(hist + r);
-                const uint4 hi = *reinterpret_cast<const uint4 *>(hist + r + 4);
-                uint4 packed;
-                packed.x = lo.x | (lo.y << 16);
-                packed.y = lo.z | (lo.w << 16);
-                packed.z = hi.x | (hi.y << 16);
-                packed.w = hi.z | (hi.w << 16);
-                *reinterpret_cast<uint4 *>(out + r) = packed;
-                *reinterpret_cast<uint4 *>(hist + r) = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(hist + r + 4) = make_uint4(0u, 0u, 0u, 0u);
-            }
-            __syncwarp();
+    }
+}
+
+template <int MAXKQ, bool EPS>
+__global__ void __launch_bounds__(32 * kRouteWarps) product_route_kernel(const RouteArgs p) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ AnchorLists al;
+    __shared__ float4 qstate[kTileQ];
+    const int t = blockIdx.x;
+    const int k0 = blockIdx.y * kRouteKeys;
+    const int64_t bl = blockIdx.z, b = p.b0 + bl;
+    const int S = p.S, Nc = p.n_anchors, T = 1 << Nc;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float *Qs = smem;                                             // [kTileQ][T]
+    float2 *qv = reinterpret_cast<float2 *>(Qs + kTileQ * T);     // [kTileQ][kHistAnchors] (query end, anchor bit)
+    float *qd = reinterpret_cast<float *>(qv + kTileQ * kHistAnchors);   // [kTileQ][kHistAnchors] see stage_query
+    float *cols = qd + kTileQ * kHistAnchors;                     // per warp: [Nc][32] key cells, [Nc][32] query cells
+    float *kcol = cols + warp * 64 * Nc, *qcol = kcol + 32 * Nc;
+    float *rest = cols + kRouteWarps * 64 * Nc;
+    float2 *ex = reinterpret_cast<float2 *>(rest) + warp * kTileQ * kExLd;   // [kTileQ][kExLd] (du, column offset)
+    float *kpe = rest + kRouteWarps * 2 * kTileQ * kExLd;         // [pe_cap][kRouteKeys] key ends of the positional anchors
+    float *pew = kpe + p.pe_cap * kRouteKeys;                     // [2 * pe_cap][kRouteWindow] their positional ends
+    float *pacc = pew + 2 * p.pe_cap * kRouteWindow;              // [S-1][npe]
+    list_anchors(al, p.anchors + (size_t)t * Nc * 2, Nc, p.sliced != 0, p.e1, p.e2);
+    const int n_kq = al.n_kq, n_pe = al.n_pe, n_staged = min(n_pe, p.pe_cap);
+
+    for (int w = lane; w < 64 * Nc; w += 32) kcol[w] = 0.f;
+    if (p.pe_cells)
+        for (int w = threadIdx.x; w < (S - 1) * p.npe; w += blockDim.x) pacc[w] = 0.f;
+    // query slots past the last key-query anchor: a NaN compares false everywhere
+    for (int w = threadIdx.x; w < kTileQ * kHistAnchors; w += blockDim.x) qv[w] = make_float2(__int_as_float(0x7fffffff), 0.f);
+
+    // this lane's key
+    const int ikey = threadIdx.x, i = k0 + ikey;
+    const float *xk = p.x1 + ((size_t)b * S + min(i, S - 1)) * p.e1;
+    float kv[MAXKQ];
+#pragma unroll
+    for (int m = 0; m < MAXKQ; m++) kv[m] = 0.f;
+    uint32_t kbits = 0u;
+    unsigned long long kmin = margin_key(kFltMax, 0u);
+    for (int k = 0; k < Nc; k++) {
+        const int c0 = al.comp[2 * k];
+        const int slot = al.kq_pos[k];
+        if (slot >= 0) {
+            const float v = c0 == 0 ? __ldg(xk + al.elem[2 * k]) : -__ldg(xk + al.elem[2 * k + 1]);
+#pragma unroll
+            for (int m = 0; m < MAXKQ; m++)
+                if (m == slot) kv[m] = v;
+        } else if ((al.key_only >> k) & 1u) {
+            const float d = __fsub_rn(__ldg(xk + al.elem[2 * k]), __ldg(xk + al.elem[2 * k + 1]));
+            if (greater_than_zero(d, p.cmp_eps)) kbits |= 1u << k;
+            const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(1u << k, d));
+            kmin = c < kmin ? c : kmin;
         }
     }
-    if (SMEM_ACC) {
-        __syncthreads();
-        for (int w = threadIdx.x; w < S * ends; w += blockDim.x) {
-            const float v = tacc[w];
-            if (v == 0.f) continue;
-            const int s = w / ends, q = w - s * ends;
-            if (st.comp[q] == 0) atomicAdd(dX1 + ((size_t)b * S + s) * e1 + st.elem[q], v);
-            else if (st.comp[q] == 1) atomicAdd(dX2 + ((size_t)b * S + s) * e2 + st.elem[q], v);
+    for (int m = 0; m < n_staged; m++) {
+        const int k = al.pe_k[m];
+        for (int e = 0; e < 2; e++) {
+            const int c = al.comp[2 * k + e];
+            if (c == 0) kpe[m * kRouteKeys + ikey] = __ldg(xk + al.elem[2 * k + e]);
+            // (keys are counted from the block's first, queries from the tile's: window entry q - i + kRouteKeys - 1)
+            if (threadIdx.x == 0)
+                al.pe_at[2 * m + e] = c == 0 ? make_int4((int)(kpe + m * kRouteKeys - smem), 1, 0, 0)
+                                    : c == 2 ? make_int4((int)(pew + (2 * m + e) * kRouteWindow - smem) + kRouteKeys - 1, -1, 1, 0)
+                                             : make_int4(k, 0, 0, 1);
         }
-        for (int w = threadIdx.x; w < (S - 1) * npe; w += blockDim.x) {
+    }
+
+    RouteTile r;
+    r.smem = smem; r.Qs = Qs; r.qd = qd; r.xk = xk; r.qv = qv; r.qstate = qstate;
+    r.x2b = p.x2 + (size_t)b * S * p.e2;
+    r.pe_t = p.pe + (size_t)t * p.npe;
+    r.pe_stride = p.n_detectors * p.npe;
+    r.kcol = kcol; r.pacc = pacc; r.ex = ex;
+    r.i = i; r.ikey = ikey; r.n_pe = n_pe; r.t = t;
+    r.pe_mask = al.pe_mask; r.kbits = kbits; r.kmin = kmin;
+    const float *Qt = p.Q + (size_t)t * p.q_det_stride + (size_t)bl * S * p.q_row_stride;
+    for (int j0 = k0 + 1; j0 < S; j0 += kTileQ) {
+        const int nq = min(kTileQ, S - j0);
+        __syncthreads();   // the previous eight queries' tiles are free
+        for (int w = threadIdx.x; w < nq * (T / 4); w += blockDim.x) {
+            const int q = w >> (Nc - 2), c = w & (T / 4 - 1);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Qs + w * 4);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(Qt + (size_t)(j0 + q) * p.q_row_stride + c * 4) : "memory");
+        }
+        {
+            const int q = threadIdx.x & (kTileQ - 1), k = threadIdx.x / kTileQ;
+            if (k < Nc && q < nq) stage_query(al, qv, qd, r.x2b + (size_t)(j0 + q) * p.e2, q, k);
+        }
+        // positional ends of the distances between the tile's queries and the block's keys: entry w holds distance
+        // j0 - k0 - kRouteKeys + w
+        for (int m = 0; m < 2 * n_staged; m++) {
+            const int end = 2 * al.pe_k[m >> 1] + (m & 1);
+            if (al.comp[end] != 2) continue;
+            for (int w = threadIdx.x; w < kRouteWindow; w += blockDim.x) {
+                const int dist = j0 - k0 - kRouteKeys + w;
+                if (dist >= 0 && dist < S - 1) pew[m * kRouteWindow + w] = __ldg(r.pe_t + (size_t)dist * r.pe_stride + al.elem[end]);
+            }
+        }
+        __syncthreads();   // the staged deltas are there
+        if (threadIdx.x < kTileQ) {
+            const int q = threadIdx.x;
+            uint32_t bits = 0u;
+            unsigned long long best = margin_key(kFltMax, 0u);
+            for (uint32_t left = al.query_only; left; left &= left - 1) {
+                const int k = __ffs(left) - 1;
+                const float d = qd[q * kHistAnchors + k];
+                if (greater_than_zero(d, p.cmp_eps)) bits |= 1u << k;
+                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(1u << k, d));
+                best = c < best ? c : best;
+            }
+            qstate[q] = make_float4(__uint_as_float(bits), __uint_as_float((uint32_t)(best >> 32)), __uint_as_float((uint32_t)best), 0.f);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (k0 + warp * 32 < j0 + nq - 1) {   // (otherwise no key of this warp lies below any of the queries)
+            r.j0 = j0;
+            if (EPS || n_pe > 0) route_tile<MAXKQ, true, EPS, MAXKQ>(p, al, r, kv);
+            else if (n_kq <= 2) route_tile<2, false, EPS, MAXKQ>(p, al, r, kv);
+            else if (n_kq <= 4) route_tile<4, false, EPS, MAXKQ>(p, al, r, kv);
+            else if (n_kq <= 6) route_tile<6, false, EPS, MAXKQ>(p, al, r, kv);
+            else route_tile<MAXKQ, false, EPS, MAXKQ>(p, al, r, kv);
+            __syncwarp();
+            // lanes over (query, quarter of the keys)
+            const float2 *mine = ex + (lane & (kTileQ - 1)) * kExLd + (lane / kTileQ) * kTileQ;
+#pragma unroll
+            for (int n = 0; n < 8; n++) {
+                const float2 v = mine[n];
+                qcol[__float_as_int(v.y) + lane] += v.x;
+            }
+        }
+        __syncthreads();
+        // add up the query cells: 4 warps x 4 quarters per (query, anchor)
+        const int q = threadIdx.x & (kTileQ - 1);
+        for (int k = threadIdx.x / kTileQ; k < Nc; k += 4 * kRouteWarps) {
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < kRouteWarps; w++)
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    float *c = cols + w * 64 * Nc + 32 * Nc + k * 32 + q + 8 * ((h + k) & 3);
+                    s += *c;
+                    *c = 0.f;
+                }
+            if (j0 + q < S && s != 0.f) {
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    if (al.comp[2 * k + e] == 1) atomicAdd(p.dX2 + ((size_t)b * S + j0 + q) * p.e2 + al.elem[2 * k + e], e == 0 ? s : -s);
+            }
+        }
+    }
+    if (i < S) {
+        for (int k = 0; k < Nc; k++) {
+            const float s = kcol[k * 32 + lane];
+            if (s == 0.f) continue;
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                if (al.comp[2 * k + e] == 0) atomicAdd(p.dX1 + ((size_t)b * S + i) * p.e1 + al.elem[2 * k + e], e == 0 ? s : -s);
+        }
+    }
+    if (p.pe_cells) {
+        __syncthreads();
+        for (int w = threadIdx.x; w < (S - 1) * p.npe; w += blockDim.x) {
             const float v = pacc[w];
             if (v == 0.f) continue;
-            const int d = w / npe, c = w - d * npe;
-            atomicAdd(dPE + ((size_t)d * n_detectors + t) * npe + c, v);
+            const int d = w / p.npe, c = w - d * p.npe;
+            atomicAdd(p.dPE + ((size_t)d * p.n_detectors + t) * p.npe + c, v);
         }
     }
 }
@@ -415,14 +804,17 @@ static int launch_contract(KernelId id, GemmArgs g, int batches, cudaStream_t st
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-static size_t stage_bytes(const ProductCall &c, size_t per_warp_floats, int warps = 8) {
-    return (pair_stage_floats(c.S, c.cfg->n_anchors, c.cfg->pos_dim) + (size_t)warps * per_warp_floats) * 4;
+// Shared memory the routing kernel of the direct staging (product_pairs.cuh) would take: the bound on the sequence length
+// of this path.
+static size_t stage_bytes(const ProductCall &c, size_t per_warp_floats) {
+    return (pair_stage_floats(c.S, c.cfg->n_anchors, c.cfg->pos_dim) + (size_t)8 * per_warp_floats) * 4;
 }
 
-// Long sequences leave room for only one block per SM (the staged tokens alone are 130 KB at 1024 tokens): give that
-// block 16 warps when its per-warp scratch still fits.
-static int pair_block_warps(const ProductCall &c, size_t per_warp_floats) {
-    return (c.S >= 512 && stage_bytes(c, per_warp_floats, 16) <= (size_t)kMaxSmemPerBlock - 1024) ? 16 : 8;
+// Anchors with a positional end whose operands the kernels stage: all of them in sliced mode (a third of the anchor ends
+// are positional there), two otherwise.
+static int staged_pe_anchors(const lutb_layer_cfg *cfg) {
+    if (cfg->pos_dim == 0) return 0;
+    return cfg->sliced_product || cfg->n_anchors < 2 ? cfg->n_anchors : 2;
 }
 
 bool product_hist_supported(const ProductCall &c, const void *weights, const void *io_rows, const void *dW) {
@@ -509,17 +901,43 @@ static int plan(const ProductCall &c, bool backward, bool allow_tc, void *worksp
 static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int64_t n, cudaStream_t stream) {
     const lutb_layer_cfg *cfg = c.cfg;
     const size_t T = (size_t)1 << cfg->n_anchors;
-    const int warps = pair_block_warps(c, T);
-    const size_t smem = stage_bytes(c, T, warps);
-    dim3 grid((unsigned)cfg->n_detectors, (unsigned)n);
+    HistArgs h;
+    h.x1 = c.x1; h.x2 = c.x2; h.pe = c.pe; h.anchors = c.anchors; h.H = p.H;
+    h.b0 = b0; h.chunk_rows = n * c.S;
+    h.S = c.S; h.e1 = c.e1; h.e2 = c.e2; h.npe = cfg->pos_dim;
+    h.n_detectors = cfg->n_detectors; h.n_anchors = cfg->n_anchors; h.sliced = cfg->sliced_product; h.cmp_eps = cfg->cmp_eps;
+    const bool packed = T > 512;
+    // warps per block: what puts the most warps on an SM (a wide table's counters leave room for one block only, which then
+    // has to bring them all); very long sequences leave the positional operands in global memory
+    const int tiles = ((c.S < kHistQueries ? c.S : kHistQueries) + kHistTile - 1) / kHistTile;
+    int warps = 0;
+    for (int cap = staged_pe_anchors(cfg);; cap = 0) {
+        int most = 0;
+        for (int w = 16; w >= 1; w /= 2) {
+            const size_t need = hist_floats(T, packed, w, cfg->n_anchors, cap, c.S) * 4 + 1024;
+            const int resident = w * (int)((size_t)kMaxSmemPerBlock / need);
+            if (resident > most && (w <= tiles || w == 1)) { most = resident; warps = w; }
+        }
+        h.pe_cap = cap;
+        if (most >= 4 || cap == 0) break;
+    }
+    LUTB_REQUIRE(warps > 0, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
+    const size_t smem = hist_floats(T, packed, warps, cfg->n_anchors, h.pe_cap, c.S) * 4;
+    dim3 grid((unsigned)cfg->n_detectors, (unsigned)((c.S + kHistQueries - 1) / kHistQueries), (unsigned)n);
     KernelScope scope(K_PRODUCT_HIST, stream);
     auto launch = [&](auto kern) -> int {
         if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, warps * 32, smem, stream>>>(c.x1, c.x2, c.pe, c.anchors, p.H, b0, n * c.S, c.S, c.e1, c.e2, cfg->pos_dim,
-                                                 cfg->n_detectors, cfg->n_anchors, cfg->sliced_product, cfg->cmp_eps);
+        kern<<<grid, warps * 32, smem, stream>>>(h);
         return LUTB_OK;
     };
-    const int rc = p.tc ? launch(product_hist_kernel<true>) : launch(product_hist_kernel<false>);
+    const bool eps = cfg->cmp_eps != 0.f;
+    auto pick = [&](auto f32) -> int {
+        constexpr bool F = decltype(f32)::value;
+        if (cfg->n_anchors <= 8) return eps ? launch(product_hist_kernel<8, true, F, false>) : launch(product_hist_kernel<8, false, F, false>);
+        if (!packed) return eps ? launch(product_hist_kernel<12, true, F, false>) : launch(product_hist_kernel<12, false, F, false>);
+        return eps ? launch(product_hist_kernel<12, true, F, true>) : launch(product_hist_kernel<12, false, F, true>);
+    };
+    const int rc = p.tc ? pick(std::true_type{}) : pick(std::false_type{});
     if (rc) return rc;
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
@@ -578,22 +996,13 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
     const bool have_hist = reuse && p.chunk == c.batch;
     const lutb_layer_cfg *cfg = c.cfg;
     const int T = 1 << cfg->n_anchors, O = cfg->n_outputs, Nt = cfg->n_detectors;
-    int route_warps = pair_block_warps(c, (size_t)T + 64 * cfg->n_anchors);
-    // long sequences: Q read from global memory when that is what gives the block 16 warps
-    const bool q_global = route_warps < 16 && pair_block_warps(c, (size_t)64 * cfg->n_anchors) == 16;
-    if (q_global) route_warps = 16;
-    size_t route_smem = stage_bytes(c, (q_global ? 0 : (size_t)T) + 64 * cfg->n_anchors, route_warps);
-    const size_t acc_bytes = ((size_t)c.S * 2 * cfg->n_anchors + (size_t)(c.S - 1) * cfg->pos_dim) * 4;
-    // block-level accumulators only while two blocks still fit an SM
-    const bool smem_acc = !q_global && route_smem + acc_bytes <= 100 * 1024;
-    if (smem_acc) route_smem += acc_bytes;
+    const int pe_cap = staged_pe_anchors(cfg);
+    // dPE cells in shared memory while they are few
+    const int pe_cells = cfg->pos_dim > 0 && (size_t)(c.S - 1) * cfg->pos_dim * 4 <= 8 * 1024;
+    const size_t route_smem = route_floats(T, cfg->n_anchors, pe_cap, pe_cells, c.S, cfg->pos_dim) * 4;
     // In-place SGD reads unmodified tables for every input gradient: with more than one chunk the table update
     // runs as a second sweep over the chunks.
     const bool second_sweep = in_place && p.chunk < c.batch;
-    // the routing kernel counts the rows itself where T more counters per warp still leave room for two blocks per SM
-    const bool fuse_hist = !have_hist && !second_sweep && smem_acc && !q_global && cfg->n_anchors <= 8 &&
-                           route_smem + (size_t)route_warps * T * 4 <= 100 * 1024;
-    if (fuse_hist) route_smem += (size_t)route_warps * T * 4;
     auto table_gradient = [&](int64_t b0, int64_t rows) -> int {
         if (p.tc) {
             // target[Nt*T, O] += lr * H^T . dY  (H stored [rows, Nt*T])
@@ -618,7 +1027,7 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
     for (int64_t b0 = 0; b0 < c.batch; b0 += p.chunk) {
         const int64_t n = (c.batch - b0 < p.chunk) ? c.batch - b0 : p.chunk;
         const int64_t rows = n * c.S;
-        if (!fuse_hist && !have_hist) {
+        if (!have_hist) {
             rc = launch_hist(c, p, b0, n, stream);
             if (rc) return rc;
         }
@@ -640,26 +1049,27 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             if (rc) return rc;
         }
         {
-            const int64_t q_row_stride = p.tc ? (int64_t)Nt * T : T, q_det_stride = p.tc ? T : rows * T;
-            dim3 grid((unsigned)Nt, (unsigned)n);
+            RouteArgs ra;
+            ra.x1 = c.x1; ra.x2 = c.x2; ra.pe = c.pe; ra.anchors = c.anchors; ra.Q = p.Q;
+            ra.dX1 = dX1; ra.dX2 = dX2; ra.dPE = dPE;
+            ra.b0 = b0;
+            ra.q_row_stride = p.tc ? (int64_t)Nt * T : T;
+            ra.q_det_stride = p.tc ? T : rows * T;
+            ra.S = c.S; ra.e1 = c.e1; ra.e2 = c.e2; ra.npe = cfg->pos_dim;
+            ra.n_detectors = Nt; ra.n_anchors = cfg->n_anchors; ra.sliced = cfg->sliced_product; ra.cmp_eps = cfg->cmp_eps;
+            ra.pe_cap = pe_cap; ra.pe_cells = pe_cells;
+            // (no block for the last key range when its first key is the last token: it has no query)
+            dim3 grid((unsigned)Nt, (unsigned)((c.S - 1 + kRouteKeys - 1) / kRouteKeys), (unsigned)n);
             KernelScope scope(K_PRODUCT_ROUTE, stream);
             auto launch = [&](auto kern) -> int {
                 if (route_smem > 48 * 1024)
                     LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_smem));
-                kern<<<grid, route_warps * 32, route_smem, stream>>>(c.x1, c.x2, c.pe, c.anchors, p.Q, dX1, dX2, dPE, b0, q_row_stride,
-                                                                     q_det_stride, c.S, c.e1, c.e2, cfg->pos_dim, Nt, cfg->n_anchors,
-                                                                     cfg->sliced_product, cfg->cmp_eps, p.H, n * c.S);
+                kern<<<grid, 32 * kRouteWarps, route_smem, stream>>>(ra);
                 return LUTB_OK;
             };
-            const int na = cfg->n_anchors;
-            if (fuse_hist) rc = p.tc ? launch(product_route_kernel<true, 0, 2, false>) : launch(product_route_kernel<true, 0, 1, false>);
-            else if (q_global)
-                rc = na <= 8 ? launch(product_route_kernel<false, 0, 0, true>) : na <= 12 ? launch(product_route_kernel<false, 12, 0, true>)
-                                                                                          : launch(product_route_kernel<false, 16, 0, true>);
-            else if (smem_acc) rc = na <= 8 ? launch(product_route_kernel<true, 0, 0, false>) : na <= 12 ? launch(product_route_kernel<true, 12, 0, false>)
-                                                                                                         : launch(product_route_kernel<true, 16, 0, false>);
-            else rc = na <= 8 ? launch(product_route_kernel<false, 0, 0, false>) : na <= 12 ? launch(product_route_kernel<false, 12, 0, false>)
-                                                                                             : launch(product_route_kernel<false, 16, 0, false>);
+            const bool eps = cfg->cmp_eps != 0.f;
+            if (cfg->n_anchors <= 8) rc = eps ? launch(product_route_kernel<8, true>) : launch(product_route_kernel<8, false>);
+            else rc = eps ? launch(product_route_kernel<12, true>) : launch(product_route_kernel<12, false>);
             if (rc) return rc;
             LUTB_LAUNCH_CHECK();
         }

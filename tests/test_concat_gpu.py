@@ -139,4 +139,11 @@ def test_concat_pair_kernel_edges(name):
         ref["W_after"] = W - np.float32(cfg["ext_lr"]) * dW.reshape(W.shape)
     else:
         ref["dW"] = dW
-    compare(cfg, run_gpu(cfg, x, anchors, W, pe, dY), ref)
+    got = run_gpu(cfg, x, anchors, W, pe, dY)
+    if name == "long":
+        # a table cell sums up to n = S (S - 1) / 2 fp32 terms here, on both sides and in different orders: about
+        # sqrt(n) * 2^-24 of the sum for each
+        n = cfg["S"] * (cfg["S"] - 1) / 2
+        golden_util.assert_close(got["dW"], ref["dW"], 2 * n ** 0.5 * 2.0 ** -24, "dW")
+        ref["dW"] = got["dW"]
+    compare(cfg, got, ref)

@@ -99,7 +99,7 @@ def hist_capable(cfg):
     return not cfg.get("int_mode") and 4 <= cfg["Nc"] <= 12 and cfg["O"] % 4 == 0 and cfg["S"] >= 2
 
 
-# more than 512 tokens: the histogram and routing kernels switch to 16-warp blocks.  A table cell here sums up to ~1e5
+# more than 512 tokens.  A table cell here sums up to ~1e5
 # fp32 terms in the oracle and on the GPU alike, in different orders: the order-dependent rounding of such a sum is a
 # few 1e-5 of its size, so this case is checked at 1e-4
 ORACLE_CASES["long_sequence"] = dict(seed=707, B=1, S=520, E=8, Nt=3, Nc=6, Npe=2, O=8, n_virtual=18, rel=1e-4)
@@ -110,6 +110,17 @@ ORACLE_CASES["hist_big_table"] = dict(seed=722, B=1, S=260, E=16, Nt=2, Nc=10, N
 ORACLE_CASES["hist_odd_shapes"] = dict(seed=723, B=3, S=67, E=7, Nt=37, Nc=4, Npe=1, O=20, n_virtual=15)
 ORACLE_CASES["internal_sgd"] = dict(seed=706, B=3, S=24, E=16, Nt=5, Nc=5, Npe=3, O=12, policy="internal", ext_lr=0.25,
                                     lr_meta=0.5, n_virtual=35)
+# edges of the histogram and routing kernels: sequences that end inside, at and just behind a block of 32 keys, eight
+# queries and 128 keys; anchors that mostly read the positional embedding (more of them than are staged, and dPE cells that
+# do not fit shared memory); the smallest and largest tables; a dead band
+ORACLE_CASES["route_one_warp"] = dict(seed=730, B=2, S=33, E=5, Nt=6, Nc=8, Npe=3, O=8, n_virtual=13)
+ORACLE_CASES["route_key_ranges"] = dict(seed=731, B=1, S=129, E=6, Nt=5, Nc=4, Npe=2, O=8, n_virtual=14)
+ORACLE_CASES["route_two_ranges"] = dict(seed=732, B=2, S=137, E=6, Nt=4, Nc=9, Npe=0, O=4, n_virtual=12)
+ORACLE_CASES["route_positional"] = dict(seed=733, B=2, S=140, E=3, Nt=4, Nc=7, Npe=20, O=8, n_virtual=26)
+ORACLE_CASES["route_largest_table"] = dict(seed=734, B=1, S=40, E=9, Nt=2, Nc=12, Npe=1, O=4, n_virtual=19)
+ORACLE_CASES["route_dead_band"] = dict(seed=735, B=2, S=66, E=9, Nt=4, Nc=10, Npe=2, O=4, n_virtual=20, cmp_eps=0.3,
+                                       quantized_input=True)
+ORACLE_CASES["route_ties"] = dict(seed=736, B=2, S=64, E=6, Nt=6, Nc=8, Npe=0, O=4, n_virtual=12, quantized_input=True)
 # 1 direct gathers, 2 histogram + contraction (tensor cores when the library has them), 3 histogram + fp32 FMA contraction
 VARIANT_CASES = [(n, v) for n in sorted(ORACLE_CASES) for v in (1, 2, 3) if v == 1 or hist_capable(ORACLE_CASES[n])]
 
