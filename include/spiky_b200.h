@@ -402,6 +402,19 @@ int lutb_concat_sparse_backward(const lutb_layer_cfg *cfg, const lutb_sparse_ind
 int lutb_infer_int8_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const int8_t *q_tables, const float *scales,
                                const float *x, const int32_t *anchors, int32_t *acc, int32_t *idx, int dequant,
                                void *stream);
+/*
+ * The same with a workspace, and the fp32 counterpart (lutb_nonseq_fc_forward in its evaluation form): large layers
+ * gather from tables staged in shared memory.  The workspace functions return the bytes a call can use, 0 where the
+ * plain gather is the better one (workspace NULL selects it); alignment 256 bytes.  y / acc are accumulated into.
+ */
+size_t lutb_infer_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch, int dequant);
+int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t batch, const int8_t *q_tables, const float *scales,
+                                  const float *x, const int32_t *anchors, int32_t *acc, int32_t *idx, int dequant,
+                                  void *workspace, size_t workspace_bytes, void *stream);
+size_t lutb_infer_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch);
+int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const float *x,
+                               const int32_t *anchors, float *y, int32_t *idx, void *workspace, size_t workspace_bytes,
+                               void *stream);
 int lutb_fixed_to_float(float *buffer, int64_t n, double int_rescaler, void *stream);
 
 /*

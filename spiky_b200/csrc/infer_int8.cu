@@ -14,6 +14,7 @@
 //                            conversion and one fp64 FMA per entry (the scale is converted once per detector);
 //                            building the double from integer operations instead measured the same within 3 %
 #include "lutb_common.cuh"
+#include "infer_staged.cuh"
 #include "nonseq_fc.cuh"
 
 namespace lutb {
@@ -145,6 +146,44 @@ extern "C" int lutb_infer_int8_accumulate(const lutb_layer_cfg *cfg, int64_t bat
     LUTB_LAUNCH_CHECK();
     }
 #undef LUTB_INT8
+    return LUTB_OK;
+}
+
+extern "C" size_t lutb_infer_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch, int dequant) {
+    if (validate_cfg(cfg) != LUTB_OK || batch <= 0 || dequant != LUTB_INT8_DEQUANT_EXACT) return 0;
+    if (!infer_staged_int8_applies(cfg, reinterpret_cast<const void *>((uintptr_t)256))) return 0;
+    return infer_staged_int8_workspace(cfg, batch);
+}
+
+extern "C" int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t batch, const int8_t *q_tables,
+                                             const float *scales, const float *x, const int32_t *anchors, int32_t *acc,
+                                             int32_t *idx, int dequant, void *workspace, size_t workspace_bytes,
+                                             void *stream) {
+    int rc = validate_cfg(cfg);
+    if (rc) return rc;
+    const bool staged = workspace != nullptr && batch > 0 && dequant == LUTB_INT8_DEQUANT_EXACT &&
+                        infer_staged_int8_applies(cfg, q_tables);
+    if (!staged) return lutb_infer_int8_accumulate(cfg, batch, q_tables, scales, x, anchors, acc, idx, dequant, stream);
+    LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "int8 inference is defined for non-sequence layers");
+    LUTB_REQUIRE(q_tables && scales && x && anchors && acc && idx, LUTB_ERR_NULL, "a required tensor pointer is NULL");
+    LUTB_REQUIRE(cfg->int_rescaler > 0.0, LUTB_ERR_MODE, "int_rescaler must be positive");
+    const size_t need = infer_staged_int8_workspace(cfg, batch);
+    LUTB_REQUIRE(workspace_bytes >= need, LUTB_ERR_WORKSPACE, "the staged gather needs %zu bytes of workspace", need);
+    LUTB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, LUTB_ERR_ALIGN, "workspace must be 256-byte aligned");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t pass = infer_staged_pass(batch);
+    uint8_t *packed = static_cast<uint8_t *>(workspace);
+    void *plan = packed + packed_index_bytes(cfg, batch);
+    rc = launch_int8_scale_plan(cfg, scales, plan, st);
+    if (rc) return rc;
+    for (int64_t b0 = 0; b0 < batch; b0 += pass) {
+        const int64_t n = batch - b0 < pass ? batch - b0 : pass;
+        rc = launch_check_detectors(x + b0 * cfg->n_inputs, n, cfg->n_inputs, anchors, cfg->n_detectors, cfg->n_anchors, cfg->cmp_eps,
+                                    idx + b0 * cfg->n_detectors, nullptr, nullptr, st, packed, packed_index_pitch(n));
+        if (rc) return rc;
+        rc = launch_infer_staged_int8(cfg, n, q_tables, scales, plan, packed, acc + b0 * cfg->n_outputs, st);
+        if (rc) return rc;
+    }
     return LUTB_OK;
 }
 

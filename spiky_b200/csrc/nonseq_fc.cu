@@ -4,6 +4,7 @@
 #include "lutb_common.cuh"
 #include "nonseq_fc.cuh"
 #include "fc_dw_sorted.cuh"
+#include "infer_staged.cuh"
 
 namespace lutb {
 
@@ -76,7 +77,8 @@ __global__ void __launch_bounds__(256) check_detectors_kernel(const float *__res
                                                              int n_anchors, float cmp_eps, int threads_per_group,
                                                              int32_t *__restrict__ idx,
                                                              float *__restrict__ min_delta,
-                                                             int32_t *__restrict__ min_k) {
+                                                             int32_t *__restrict__ min_k,
+                                                             uint8_t *__restrict__ packed, size_t packed_pitch) {
     extern __shared__ __align__(16) float xs_all[];
     const int groups = blockDim.x / threads_per_group;
     const int g = threadIdx.x / threads_per_group;
@@ -141,6 +143,18 @@ __global__ void __launch_bounds__(256) check_detectors_kernel(const float *__res
                 if (TRAIN) { min_delta[o] = md[r]; min_k[o] = mk[r]; }
             }
         }
+        if (!TRAIN && packed != nullptr) {
+            // (the bytes of rows past the end lie in the row's padding)
+            uint8_t *dst = packed + (size_t)t * packed_pitch + row0;
+            if constexpr (R % 4 == 0) {
+#pragma unroll
+                for (int r4 = 0; r4 < R; r4 += 4)
+                    *reinterpret_cast<uint32_t *>(dst + r4) = (uint32_t)li[r4] | (uint32_t)li[r4 + 1] << 8 | (uint32_t)li[r4 + 2] << 16 | (uint32_t)li[r4 + 3] << 24;
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; r++) dst[r] = (uint8_t)li[r];
+            }
+        }
     }
 }
 
@@ -149,7 +163,7 @@ template <bool TRAIN>
 __global__ void check_detectors_global_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
                                               const int2 *__restrict__ anchors, int n_detectors, int n_anchors,
                                               float cmp_eps, int32_t *__restrict__ idx, float *__restrict__ min_delta,
-                                              int32_t *__restrict__ min_k) {
+                                              int32_t *__restrict__ min_k, uint8_t *__restrict__ packed, size_t packed_pitch) {
     const int64_t total = rows * n_detectors;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / n_detectors;
@@ -168,13 +182,15 @@ __global__ void check_detectors_global_kernel(const float *__restrict__ x, int64
         }
         idx[i] = li;
         if (TRAIN) { min_delta[i] = md; min_k[i] = mk; }
+        else if (packed != nullptr) packed[(size_t)t * packed_pitch + r] = (uint8_t)li;
     }
 }
 
 template <int R>
 static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, const int32_t *anchors,
                                     int n_detectors, int n_anchors, float cmp_eps, int32_t *idx, float *min_delta,
-                                    int32_t *min_k, int tpg, int groups, int64_t blocks, cudaStream_t stream) {
+                                    int32_t *min_k, int tpg, int groups, int64_t blocks, cudaStream_t stream,
+                                    uint8_t *packed, size_t packed_pitch) {
     const size_t smem = (size_t)groups * staged_floats<R>(n_inputs) * sizeof(float);
     LUTB_REQUIRE(blocks <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "batch too large for one launch");
     const bool train = min_delta != nullptr;
@@ -182,14 +198,14 @@ static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, 
     if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KernelScope scope(K_CHECK_DETECTORS, stream);
     kern<<<(unsigned)blocks, tpg * groups, smem, stream>>>(x, rows, n_inputs, reinterpret_cast<const int2 *>(anchors),
-                                                          n_detectors, n_anchors, cmp_eps, tpg, idx, min_delta, min_k);
+                                                          n_detectors, n_anchors, cmp_eps, tpg, idx, min_delta, min_k, packed, packed_pitch);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
 }
 
 int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int32_t *anchors, int n_detectors,
                            int n_anchors, float cmp_eps, int32_t *idx, float *min_delta, int32_t *min_k,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, uint8_t *packed, size_t packed_pitch) {
     const int sm = device_info().sm_count;
     // threads per row group: one per detector, rounded to warps, at most 256
     int tpg = ((min(n_detectors, 256) + 31) / 32) * 32;
@@ -206,11 +222,11 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
         if (train)
             check_detectors_global_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(
                 x, rows, n_inputs, reinterpret_cast<const int2 *>(anchors), n_detectors, n_anchors, cmp_eps, idx,
-                min_delta, min_k);
+                min_delta, min_k, packed, packed_pitch);
         else
             check_detectors_global_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(
                 x, rows, n_inputs, reinterpret_cast<const int2 *>(anchors), n_detectors, n_anchors, cmp_eps, idx,
-                min_delta, min_k);
+                min_delta, min_k, packed, packed_pitch);
         LUTB_LAUNCH_CHECK();
         return LUTB_OK;
     }
@@ -222,10 +238,10 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
     const int64_t items = row_tiles * ((n_detectors + tpg - 1) / tpg);
     const int64_t blocks = row_tiles >= (int64_t)2 * sm ? row_tiles : min(items, (int64_t)2 * sm);
     switch (R) {
-        case 8: return launch_check_detectors_r<8>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream);
-        case 4: return launch_check_detectors_r<4>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream);
-        case 2: return launch_check_detectors_r<2>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream);
-        default: return launch_check_detectors_r<1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream);
+        case 8: return launch_check_detectors_r<8>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        case 4: return launch_check_detectors_r<4>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        case 2: return launch_check_detectors_r<2>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        default: return launch_check_detectors_r<1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
     }
 }
 
@@ -767,6 +783,39 @@ extern "C" int lutb_nonseq_fc_forward(const lutb_layer_cfg *cfg, int64_t batch, 
                                   cfg->backward_group, cfg->int_mode != 0, cfg->int_rescaler, st);
     if (rc) return rc;
     if (cfg->int_mode) return launch_fixed_to_float(y, batch * (int64_t)cfg->n_outputs, cfg->int_rescaler, st);
+    return LUTB_OK;
+}
+
+extern "C" size_t lutb_infer_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
+    const void *aligned = reinterpret_cast<const void *>((uintptr_t)256);
+    if (validate_cfg(cfg) != LUTB_OK || batch <= 0 || !infer_staged_fp32_applies(cfg, aligned, aligned)) return 0;
+    return infer_staged_fp32_workspace(cfg, batch);
+}
+
+extern "C" int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const float *x,
+                                          const int32_t *anchors, float *y, int32_t *idx, void *workspace,
+                                          size_t workspace_bytes, void *stream) {
+    int rc = validate_cfg(cfg);
+    if (rc) return rc;
+    const bool staged = workspace != nullptr && batch > 0 && infer_staged_fp32_applies(cfg, weights, y);
+    if (!staged) return lutb_nonseq_fc_forward(cfg, batch, weights, x, anchors, y, idx, nullptr, nullptr, stream);
+    LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "inference is defined for non-sequence layers");
+    LUTB_REQUIRE(weights && x && anchors && y && idx, LUTB_ERR_NULL, "a required tensor pointer is NULL");
+    const size_t need = infer_staged_fp32_workspace(cfg, batch);
+    LUTB_REQUIRE(workspace_bytes >= need, LUTB_ERR_WORKSPACE, "the staged gather needs %zu bytes of workspace", need);
+    LUTB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, LUTB_ERR_ALIGN, "workspace must be 256-byte aligned");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t pass = infer_staged_pass(batch);
+    uint8_t *packed = static_cast<uint8_t *>(workspace);
+    float *partial = reinterpret_cast<float *>(packed + packed_index_bytes(cfg, batch));
+    for (int64_t b0 = 0; b0 < batch; b0 += pass) {
+        const int64_t n = batch - b0 < pass ? batch - b0 : pass;
+        rc = launch_check_detectors(x + b0 * cfg->n_inputs, n, cfg->n_inputs, anchors, cfg->n_detectors, cfg->n_anchors, cfg->cmp_eps,
+                                    idx + b0 * cfg->n_detectors, nullptr, nullptr, st, packed, packed_index_pitch(n));
+        if (rc) return rc;
+        rc = launch_infer_staged_fp32(cfg, n, weights, packed, partial, y + b0 * cfg->n_outputs, st);
+        if (rc) return rc;
+    }
     return LUTB_OK;
 }
 

@@ -80,16 +80,19 @@ class LUTInference:
         L = _native.lib()
         stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
         idx = torch.empty(B * self.Nt, dtype=torch.int32, device=self.device)
+        cfg = ctypes.byref(self.cfg)
         with torch.cuda.device(self.device):
+            need = L.lutb_infer_int8_workspace(cfg, B, self.dequant) if self.int8 else L.lutb_infer_fp32_workspace(cfg, B)
+            ws = torch.empty(need, dtype=torch.uint8, device=self.device) if need else None
             if self.int8:
                 acc = torch.zeros(B * self.O, dtype=torch.int32, device=self.device)
-                rc = L.lutb_infer_int8_accumulate(ctypes.byref(self.cfg), B, _ptr(self.tables), _ptr(self.scales),
-                                                  _ptr(x.view(-1)), _ptr(self.anchors), _ptr(acc), _ptr(idx), self.dequant,
-                                                  stream)
+                rc = L.lutb_infer_int8_accumulate_ws(cfg, B, _ptr(self.tables), _ptr(self.scales), _ptr(x.view(-1)),
+                                                     _ptr(self.anchors), _ptr(acc), _ptr(idx), self.dequant, _ptr(ws),
+                                                     need, stream)
             else:
                 acc = torch.zeros(B * self.O, dtype=torch.float32, device=self.device)
-                rc = L.lutb_nonseq_fc_forward(ctypes.byref(self.cfg), B, _ptr(self.tables), _ptr(x.view(-1)),
-                                              _ptr(self.anchors), _ptr(acc), _ptr(idx), None, None, stream)
+                rc = L.lutb_infer_fp32_accumulate(cfg, B, _ptr(self.tables), _ptr(x.view(-1)), _ptr(self.anchors),
+                                                  _ptr(acc), _ptr(idx), _ptr(ws), need, stream)
         _native.check(rc)
         self.last_indices = idx.view(B, self.Nt)
         return acc.view(B, self.O)

@@ -100,3 +100,43 @@ def test_detector_shards_combine_exactly_int8_and_within_tolerance_fp32(world):
     golden_util.assert_close(got32, want32, 1e-5, "sharded fp32")
     ref32, _, _, _ = orc.nonseq_fc_forward(W.numpy(), x, anchors, Nt, Nc, O, train=False)
     golden_util.assert_close(want32, ref32, 1e-5, "fp32 vs oracle")
+
+
+# the staged gathers at the edges of their tiles (1024 / 256 samples), column slices (32 / 64 outputs), detector runs and
+# batch passes (16384 samples)
+@pytest.mark.parametrize("shape", [(1, 50, 512, 8, 36), (1023, 64, 521, 6, 64), (1025, 33, 513, 7, 68), (300, 40, 700, 8, 100),
+                                   (16400, 20, 512, 4, 36)])
+def test_staged_fp32_inference_matches_oracle(shape):
+    from spiky_b200.inference import LUTInference
+
+    B, I, Nt, Nc, O = shape
+    x = synth.normal(941, (B, I))
+    anchors = synth.anchor_pairs(942, Nt, Nc, I)
+    W = synth.normal(943, (Nt * (1 << Nc) * O,), 0.0, 0.02)
+    layer = LUTInference(I, O, Nt, Nc, torch.from_numpy(anchors), torch.from_numpy(W))
+    y = layer(torch.from_numpy(x).cuda()).cpu().numpy()
+    ref, ridx, _, _ = orc.nonseq_fc_forward(W, x, anchors, Nt, Nc, O, train=False)
+    assert np.array_equal(layer.last_indices.cpu().numpy(), ridx)
+    golden_util.assert_close(y, ref, 1e-5, "y")
+
+
+@pytest.mark.parametrize("shape", [(1, 50, 1024, 8, 40, 32), (255, 33, 1030, 5, 64, 32), (257, 64, 1027, 7, 72, 7),
+                                   (70, 40, 1024, 8, 136, 300), (16400, 20, 1024, 4, 48, 32)])
+def test_staged_int8_inference_is_bit_exact(shape):
+    """Blocks whose scales have one exponent, spread over many (the fp64 route), are zero, negative or subnormal."""
+    from spiky_b200.inference import LUTInference
+
+    B, I, Nt, Nc, O, blk = shape
+    x, anchors, q, s = make_problem(950, B, I, Nt, Nc, O)
+    s[64:128] = 0.0
+    s[130] = 0.0
+    s[200] = np.float32(1e-12)          # spread beyond 2^7: fp64
+    s[260:290] *= -1.0
+    s[330:340] = np.float32(1e-42)      # subnormal beside normal scales
+    s[384:448] = np.float32(3e-5)
+    layer = LUTInference(I, O, Nt, Nc, torch.from_numpy(anchors), torch.from_numpy(q), torch.from_numpy(s),
+                         int_rescaler=0.05, backward_group_size=blk)
+    acc = layer.partial(torch.from_numpy(x).cuda()).cpu().numpy()
+    want, ridx = orc.infer_int8(q, s, x, anchors, Nt, Nc, O, backward_group_size=blk, int_rescaler=0.05, exact=True)
+    assert np.array_equal(layer.last_indices.cpu().numpy(), ridx)
+    assert np.array_equal(acc, want)
