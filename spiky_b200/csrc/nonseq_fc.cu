@@ -26,6 +26,10 @@ __host__ __device__ constexpr size_t staged_floats(int n_inputs) {
     return R % 4 == 0 ? ((((size_t)n_inputs * (R / 4)) + 7) & ~(size_t)7) * 4 : (size_t)R * n_inputs;
 }
 
+static size_t staged_bytes(int R, int n_inputs) {
+    return 4 * (R == 8 ? staged_floats<8>(n_inputs) : R == 4 ? staged_floats<4>(n_inputs) : (size_t)R * n_inputs);
+}
+
 // Stages the R rows [row0, row0 + nrows) of one row group: coalesced global reads, transposed shared writes.
 template <int R>
 __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ x, int64_t row0, int nrows, int n_inputs,
@@ -66,13 +70,20 @@ __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ 
     }
 }
 
-// Work items: (row tile of GROUPS * R rows, chunk of threads_per_group detectors), row tile major.  Block b takes the
+// Work items: (row tile of GROUPS * R rows, chunk of threads_per_group / D detectors), row tile major.  Block b takes the
 // items [n * b / grid, n * (b + 1) / grid): with a grid of one block per row tile that is the tile's own chunks; small
 // batches launch a multiple of the SM count instead and a block's range may cross into the next tile, which it then
 // stages as well.  (Splitting the detectors into a fixed number of slices per tile left 320 blocks on 148 SMs: the SMs
 // with three blocks set the kernel's time, max / avg active cycles 1.3.)
+//
+// Bound by the wavefronts of the load/store unit: the anchors' inputs are random, so the 8 lanes that share a wavefront of
+// 16-byte reads fall into the same banks 2.65 times over, and an anchor list read 8 bytes at a time touches 16 lines per
+// load.  With 8 rows, D = 2 neighbouring lanes share a detector (4 rows each): a wavefront then holds 4 random 32-byte
+// pieces, which collide 2.1 times, and the lists are read two anchors at a time.  Measured (one thread a detector before):
+// 16384 rows x 4096 inputs, 4096 detectors of 8 anchors 625 -> 444 us (8 rows in one block of 1024 threads an SM against 4);
+// 65536 x 784, 64 detectors of 6 anchors 83 -> 70 us.
 template <int R, bool TRAIN>
-__global__ void __launch_bounds__(256) check_detectors_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
+__global__ void __launch_bounds__(R == 8 ? 1024 : 256) check_detectors_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
                                                              const int2 *__restrict__ anchors, int n_detectors,
                                                              int n_anchors, float cmp_eps, int threads_per_group,
                                                              int32_t *__restrict__ idx,
@@ -80,12 +91,15 @@ __global__ void __launch_bounds__(256) check_detectors_kernel(const float *__res
                                                              int32_t *__restrict__ min_k,
                                                              uint8_t *__restrict__ packed, size_t packed_pitch) {
     extern __shared__ __align__(16) float xs_all[];
+    constexpr int D = R == 8 ? 2 : 1, RT = R / D;   // threads per detector, rows per thread
     const int groups = blockDim.x / threads_per_group;
     const int g = threadIdx.x / threads_per_group;
     const int lt = threadIdx.x - g * threads_per_group;
+    const int half = lt % D, per_chunk = threads_per_group / D;
     float *xs = xs_all + (size_t)g * staged_floats<R>(n_inputs);
     const bool vec_ok = (n_inputs % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    const int chunks = (n_detectors + threads_per_group - 1) / threads_per_group;
+    const bool pairs_ok = (n_anchors % 2 == 0) && ((reinterpret_cast<uintptr_t>(anchors) & 15) == 0);
+    const int chunks = (n_detectors + per_chunk - 1) / per_chunk;
     const int64_t rows_per_tile = (int64_t)groups * R;
     const int64_t n_items = ((rows + rows_per_tile - 1) / rows_per_tile) * chunks;
     const int64_t item0 = n_items * blockIdx.x / gridDim.x, item1 = n_items * (blockIdx.x + 1) / gridDim.x;
@@ -101,58 +115,65 @@ __global__ void __launch_bounds__(256) check_detectors_kernel(const float *__res
             __syncthreads();
             staged = tile;
         }
-        const int t = chunk * threads_per_group + lt;
+        const int t = chunk * per_chunk + lt / D;
         if (nrows <= 0 || t >= n_detectors) continue;
-        int32_t li[R];
-        float md[R];
-        int32_t mk[R];
+        int32_t li[RT];
+        float md[RT];
+        int32_t mk[RT];
 #pragma unroll
-        for (int r = 0; r < R; r++) { li[r] = 0; md[r] = 0.f; mk[r] = -1; }
-        const int2 *ap = anchors + (size_t)t * n_anchors;
-#pragma unroll 4
-        for (int k = 0; k < n_anchors; k++) {
-            const int2 p = __ldg(ap + k);
-            if (p.x == kNoAnchor || p.y == kNoAnchor) continue;
-            float a[R], b[R];
-            if constexpr (R % 4 == 0) {
-#pragma unroll
-                for (int r4 = 0; r4 < R / 4; r4++) {
-                    const float4 qa = reinterpret_cast<const float4 *>(xs)[swizzle_slot(p.x * (R / 4) + r4)];
-                    const float4 qb = reinterpret_cast<const float4 *>(xs)[swizzle_slot(p.y * (R / 4) + r4)];
-                    a[4 * r4] = qa.x; a[4 * r4 + 1] = qa.y; a[4 * r4 + 2] = qa.z; a[4 * r4 + 3] = qa.w;
-                    b[4 * r4] = qb.x; b[4 * r4 + 1] = qb.y; b[4 * r4 + 2] = qb.z; b[4 * r4 + 3] = qb.w;
-                }
+        for (int r = 0; r < RT; r++) { li[r] = 0; md[r] = 0.f; mk[r] = -1; }
+        auto one_anchor = [&](int k, int px, int py) {
+            if (px == kNoAnchor || py == kNoAnchor) return;
+            float a[RT], b[RT];
+            if constexpr (RT == 4) {
+                const float4 qa = reinterpret_cast<const float4 *>(xs)[swizzle_slot(px * D + half)];
+                const float4 qb = reinterpret_cast<const float4 *>(xs)[swizzle_slot(py * D + half)];
+                a[0] = qa.x; a[1] = qa.y; a[2] = qa.z; a[3] = qa.w;
+                b[0] = qb.x; b[1] = qb.y; b[2] = qb.z; b[3] = qb.w;
             } else {
 #pragma unroll
-                for (int r = 0; r < R; r++) { a[r] = xs[(size_t)p.x * R + r]; b[r] = xs[(size_t)p.y * R + r]; }
+                for (int r = 0; r < RT; r++) { a[r] = xs[(size_t)px * R + r]; b[r] = xs[(size_t)py * R + r]; }
             }
 #pragma unroll
-            for (int r = 0; r < R; r++) {
+            for (int r = 0; r < RT; r++) {
                 const float d = __fsub_rn(a[r], b[r]);
                 if (greater_than_zero(d, cmp_eps)) li[r] |= (1 << k);
                 if (TRAIN) {
                     if (mk[r] == -1 || fabsf(d) < fabsf(md[r])) { md[r] = d; mk[r] = k; }
                 }
             }
+        };
+        const int2 *ap = anchors + (size_t)t * n_anchors;
+        if (pairs_ok) {
+#pragma unroll 2
+            for (int k = 0; k < n_anchors; k += 2) {
+                const int4 p = __ldg(reinterpret_cast<const int4 *>(ap + k));
+                one_anchor(k, p.x, p.y);
+                one_anchor(k + 1, p.z, p.w);
+            }
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < n_anchors; k++) {
+                const int2 p = __ldg(ap + k);
+                one_anchor(k, p.x, p.y);
+            }
         }
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            if (r < nrows) {
-                const int64_t o = (row0 + r) * n_detectors + t;
+        for (int r = 0; r < RT; r++) {
+            const int row = half * RT + r;
+            if (row < nrows) {
+                const int64_t o = (row0 + row) * n_detectors + t;
                 idx[o] = li[r];
                 if (TRAIN) { min_delta[o] = md[r]; min_k[o] = mk[r]; }
             }
         }
         if (!TRAIN && packed != nullptr) {
             // (the bytes of rows past the end lie in the row's padding)
-            uint8_t *dst = packed + (size_t)t * packed_pitch + row0;
-            if constexpr (R % 4 == 0) {
+            uint8_t *dst = packed + (size_t)t * packed_pitch + row0 + half * RT;
+            if constexpr (RT == 4) *reinterpret_cast<uint32_t *>(dst) = (uint32_t)li[0] | (uint32_t)li[1] << 8 | (uint32_t)li[2] << 16 | (uint32_t)li[3] << 24;
+            else {
 #pragma unroll
-                for (int r4 = 0; r4 < R; r4 += 4)
-                    *reinterpret_cast<uint32_t *>(dst + r4) = (uint32_t)li[r4] | (uint32_t)li[r4 + 1] << 8 | (uint32_t)li[r4 + 2] << 16 | (uint32_t)li[r4 + 3] << 24;
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; r++) dst[r] = (uint8_t)li[r];
+                for (int r = 0; r < RT; r++) dst[r] = (uint8_t)li[r];
             }
         }
     }
@@ -207,13 +228,15 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
                            int n_anchors, float cmp_eps, int32_t *idx, float *min_delta, int32_t *min_k,
                            cudaStream_t stream, uint8_t *packed, size_t packed_pitch) {
     const int sm = device_info().sm_count;
-    // threads per row group: one per detector, rounded to warps, at most 256
-    int tpg = ((min(n_detectors, 256) + 31) / 32) * 32;
-    // rows per group: up to 8 (each anchor pair is fetched once per 8 rows), fewer when rows are long
+    // rows per group: 8 while they fit a block (each anchor pair is fetched once per 8 rows), fewer for few or longer rows
     const size_t row_bytes = (size_t)n_inputs * sizeof(float);
     const size_t budget = 100 * 1024;  // two resident blocks per SM
     int R = 8;
-    while (R > 1 && ((size_t)R * row_bytes > budget || rows < R)) R >>= 1;
+    while (R > 1 && (staged_bytes(R, n_inputs) > (R == 8 ? (size_t)kMaxSmemPerBlock - 1024 : budget) || rows < R)) R >>= 1;
+    // threads per row group: one per detector (two with 8 rows), rounded to warps; at most 256 detectors, or 512 where the rows
+    // leave room for one block only
+    const int per_det = R == 8 ? 2 : 1, widest = R != 8 ? 256 : staged_bytes(R, n_inputs) > budget ? 1024 : 512;
+    int tpg = ((min(n_detectors * per_det, widest) + 31) / 32) * 32;
     if ((size_t)R * row_bytes > (size_t)kMaxSmemPerBlock - 1024) {
         const bool train = min_delta != nullptr;
         const int64_t total = rows * n_detectors;
@@ -230,13 +253,14 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
         LUTB_LAUNCH_CHECK();
         return LUTB_OK;
     }
-    int groups = 256 / tpg;
+    int groups = tpg >= 256 ? 1 : 256 / tpg;
     while (groups > 1 && ((size_t)groups * R * row_bytes > budget || rows < (int64_t)groups * R * 2 * sm)) groups >>= 1;
-    // one block per row tile; small batches: two blocks per SM, each with an equal share of the (tile, detector chunk)
-    // work items
+    // one block per row tile; small batches: as many blocks as are resident (two per SM, one where the rows take more than
+    // half of it), each with an equal share of the (tile, detector chunk) work items
+    const int64_t resident = (int64_t)sm * (groups * staged_bytes(R, n_inputs) > budget ? 1 : 2);
     const int64_t row_tiles = (rows + (int64_t)groups * R - 1) / ((int64_t)groups * R);
-    const int64_t items = row_tiles * ((n_detectors + tpg - 1) / tpg);
-    const int64_t blocks = row_tiles >= (int64_t)2 * sm ? row_tiles : min(items, (int64_t)2 * sm);
+    const int64_t items = row_tiles * ((n_detectors + tpg / per_det - 1) / (tpg / per_det));
+    const int64_t blocks = row_tiles >= resident ? row_tiles : min(items, resident);
     switch (R) {
         case 8: return launch_check_detectors_r<8>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
         case 4: return launch_check_detectors_r<4>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);

@@ -200,3 +200,37 @@ def test_sorted_variant_rejects_missing_workspace():
     rc = L.lutb_nonseq_fc_backward(ctypes.byref(cfg), 16, p(t(64)), p(t(64)), p(t(16, torch.int32)), p(t(64, torch.int32)),
                                    p(t(64)), p(t(64, torch.int32)), p(t(128)), p(t(64)), -1.0, 3, None, 0, None)
     assert rc == -4 and b"workspace" in L.lutb_last_error()
+
+
+@pytest.mark.parametrize("rows,I,Nt,Nc", [(1, 5, 1, 1), (8, 64, 33, 6), (9, 63, 257, 7), (19, 4096, 600, 8), (8, 5801, 40, 4),
+                                          (17, 5900, 40, 5), (5, 9000, 31, 8), (700, 100, 300, 2), (2500, 40, 24, 3)])
+def test_check_detectors_row_and_detector_splits(rows, I, Nt, Nc):
+    """Eight rows with two threads a detector (one or two blocks per SM), fewer rows for longer inputs, anchor lists read
+    two at a time or one by one, unused anchor pairs, an input that is not 16-byte aligned."""
+    import ctypes
+    from spiky_b200 import _native
+
+    x = synth.normal(960, (rows, I))
+    anchors = synth.anchor_pairs(961, Nt, Nc, max(I, 2)).reshape(Nt, Nc, 2).copy()
+    if Nc > 2:
+        anchors[::3, 1] = -1
+    cfg = _native.LayerCfg(n_inputs=I, n_outputs=4, n_detectors=Nt, n_anchors=Nc, seq_len=1, pos_dim=0, forward_group=32,
+                           backward_group=32, int_mode=0, sliced_product=0, cmp_eps=0.0, reserved0=0.0, int_rescaler=1.0,
+                           lr_meta=1.0)
+    ridx, rmd, rmk = orc.check_detectors(x, anchors.reshape(-1), Nt, Nc, 0.0, True)
+    ta = torch.from_numpy(anchors.reshape(-1)).cuda()
+    for shift in (0, 1):
+        store = torch.zeros(rows * I + shift, device="cuda")
+        tx = store[shift:]
+        tx.copy_(torch.from_numpy(x).reshape(-1))
+        idx = torch.empty(rows * Nt, dtype=torch.int32, device="cuda")
+        md, mk = torch.empty(rows * Nt, device="cuda"), torch.empty_like(idx)
+        p = [ctypes.c_void_p(t.data_ptr()) for t in (tx, ta, idx, md, mk)]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        L = _native.lib()
+        _native.check(L.lutb_check_detectors(ctypes.byref(cfg), rows, p[0], p[1], p[2], p[3], p[4], stream))
+        assert np.array_equal(idx.cpu().numpy(), ridx.reshape(-1)) and np.array_equal(mk.cpu().numpy(), rmk.reshape(-1))
+        assert np.array_equal(md.cpu().numpy().view(np.int32), rmd.reshape(-1).view(np.int32))
+        idx.fill_(-7)
+        _native.check(L.lutb_check_detectors(ctypes.byref(cfg), rows, p[0], p[1], p[2], None, None, stream))
+        assert np.array_equal(idx.cpu().numpy(), ridx.reshape(-1))
