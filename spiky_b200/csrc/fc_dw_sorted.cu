@@ -135,13 +135,17 @@ int launch_fc_dw_sorted(const float *dY, const int32_t *idx, float *target, int6
 
 // ------------------------------------------------------------------------------------------
 // Table gradient as a list of touched rows (Sparse gradient policy): after the counting sort a segment
-// (detector, row) with at least one sample is a touched row.  A block of 1024 threads looks at 1024 consecutive
-// segments: the touched ones are counted (block totals -> exclusive scan by one block -> base of every block), each
-// gets its position in the list from a block-wide scan of the flags, and the block's 32 warps reduce the touched
-// segments one by one, writing the row number and the row of sums at that position.  Rows come out in ascending
-// (detector, row) order; every cell is summed in ascending sample order like the dense sorted variant.
+// (detector, row) with at least one sample is a touched row.  A block looks at kRowsBlock consecutive segments: the
+// touched ones are counted (block totals -> exclusive scan by one block -> base of every block), each gets its position
+// in the list from a scan of the flags, and the block's warps reduce the touched segments one by one, writing the row
+// number and the row of sums at that position.  Rows come out in ascending (detector, row) order; every cell is summed
+// in ascending sample order like the dense sorted variant.
+// The reduction is a chain of dependent loads (sample number, then its gradient), so it wants many warps with few
+// segments each and several samples' loads in flight: blocks of 1024 segments gave a 6400-row layer 7 blocks and 32
+// segments a warp; 64 segments and 8 warps, four samples and two columns at a time, measured 90 -> 28 us there (1111
+// samples, 33 outputs).
 // ------------------------------------------------------------------------------------------
-constexpr int kRowsBlock = 1024;
+constexpr int kRowsBlock = 64, kRowsThreads = 256;   // (two warps of segments: the scan in the emit kernel counts on it)
 
 __device__ __forceinline__ bool segment_touched(const int32_t *offsets, int64_t seg, int table_rows, int nblk, int64_t batch,
                                                 int32_t *begin, int32_t *end) {
@@ -186,27 +190,28 @@ __global__ void __launch_bounds__(1024) dw_rows_scan_kernel(int32_t *__restrict_
     if (threadIdx.x == 0) *count_out = carry;
 }
 
-__global__ void __launch_bounds__(kRowsBlock) dw_rows_emit_kernel(const float *__restrict__ dY, const int32_t *__restrict__ offsets,
+__global__ void __launch_bounds__(kRowsThreads) dw_rows_emit_kernel(const float *__restrict__ dY, const int32_t *__restrict__ offsets,
                                                                  const int32_t *__restrict__ perm,
                                                                  const int32_t *__restrict__ block_base, int64_t n_seg,
                                                                  int64_t batch, int n_outputs, int table_rows, int nblk,
                                                                  double lr, int64_t capacity, int64_t *__restrict__ row_ids,
                                                                  float *__restrict__ values) {
-    __shared__ int32_t warp_sums[32];
     __shared__ int32_t position[kRowsBlock];   // list position of a touched segment, -1 otherwise
+    __shared__ int32_t first_sum;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t seg0 = (int64_t)blockIdx.x * kRowsBlock;
-    const int64_t seg = seg0 + threadIdx.x;
     int32_t b, e;
-    const bool touched = seg < n_seg && segment_touched(offsets, seg, table_rows, nblk, batch, &b, &e);
+    const bool mine = threadIdx.x < kRowsBlock;   // two warps look, all of them reduce
+    const bool touched = mine && seg0 + threadIdx.x < n_seg && segment_touched(offsets, seg0 + threadIdx.x, table_rows, nblk, batch, &b, &e);
     const unsigned mask = __ballot_sync(0xffffffffu, touched);
-    if (lane == 0) warp_sums[warp] = __popc(mask);
+    if (threadIdx.x == 0) first_sum = __popc(mask);
     __syncthreads();
-    int32_t before = __ldg(block_base + blockIdx.x);
-    for (int w = 0; w < warp; w++) before += warp_sums[w];
-    position[threadIdx.x] = touched ? before + __popc(mask & ((1u << lane) - 1u)) : -1;
+    if (mine) {
+        const int32_t before = __ldg(block_base + blockIdx.x) + (warp == 1 ? first_sum : 0);
+        position[threadIdx.x] = touched ? before + __popc(mask & ((1u << lane) - 1u)) : -1;
+    }
     __syncthreads();
-    for (int i = warp; i < kRowsBlock; i += 32) {
+    for (int i = warp; i < kRowsBlock; i += kRowsThreads / 32) {
         const int32_t pos = position[i];
         if (pos < 0 || pos >= capacity) continue;   // warp-uniform
         const int64_t sg = seg0 + i;
@@ -215,13 +220,26 @@ __global__ void __launch_bounds__(kRowsBlock) dw_rows_emit_kernel(const float *_
         const int32_t *list = perm + (size_t)(sg / table_rows) * batch;
         if (lane == 0) row_ids[pos] = sg;
         float *row = values + (size_t)pos * n_outputs;
-        for (int o = lane; o < n_outputs; o += 32) {
-            float acc = 0.f;
-            for (int32_t s = begin; s < end; s++) {
-                const double g = (double)__ldg(dY + (size_t)__ldg(list + s) * n_outputs + o);
-                if (fabs(g) > kEps) acc += (float)(g * lr);
+        for (int o = lane; o < n_outputs; o += 64) {
+            const bool second = o + 32 < n_outputs;
+            float acc0 = 0.f, acc1 = 0.f;
+            for (int32_t s = begin; s < end; s += 4) {
+                float g0[4], g1[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const bool on = s + u < end;
+                    const float *src = dY + (on ? (size_t)__ldg(list + s + u) * n_outputs : 0) + o;
+                    g0[u] = on ? __ldg(src) : 0.f;
+                    g1[u] = on && second ? __ldg(src + 32) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (fabs((double)g0[u]) > kEps) acc0 += (float)((double)g0[u] * lr);
+                    if (fabs((double)g1[u]) > kEps) acc1 += (float)((double)g1[u] * lr);
+                }
             }
-            row[o] = acc;
+            row[o] = acc0;
+            if (second) row[o + 32] = acc1;
         }
     }
 }
@@ -261,7 +279,7 @@ int launch_fc_dw_rows(const float *dY, const int32_t *idx, int64_t batch, int n_
     LUTB_LAUNCH_CHECK();
     dw_rows_scan_kernel<<<1, 1024, 0, stream>>>(block_sums, n_blocks, count_out);
     LUTB_LAUNCH_CHECK();
-    dw_rows_emit_kernel<<<(unsigned)n_blocks, kRowsBlock, 0, stream>>>(dY, counts, perm, block_sums, n_seg, batch, n_outputs,
+    dw_rows_emit_kernel<<<(unsigned)n_blocks, kRowsThreads, 0, stream>>>(dY, counts, perm, block_sums, n_seg, batch, n_outputs,
                                                                     table_rows, nblk, lr, capacity, row_ids, values);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
