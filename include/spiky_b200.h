@@ -415,6 +415,8 @@ size_t lutb_infer_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch);
 int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const float *x,
                                const int32_t *anchors, float *y, int32_t *idx, void *workspace, size_t workspace_bytes,
                                void *stream);
+/* Clears up to three buffers in one launch (sizes in bytes, multiples of 4; 4-byte aligned; size 0: none). */
+int lutb_zero_buffers(void *a, int64_t a_bytes, void *b, int64_t b_bytes, void *c, int64_t c_bytes, void *stream);
 int lutb_fixed_to_float(float *buffer, int64_t n, double int_rescaler, void *stream);
 
 /*

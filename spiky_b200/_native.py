@@ -105,6 +105,7 @@ SIGNATURES = {
     "lutb_infer_int8_accumulate_ws": (_int, [_cfgp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _int, _vp, _size, _vp]),
     "lutb_infer_fp32_workspace": (_size, [_cfgp, _i64]),
     "lutb_infer_fp32_accumulate": (_int, [_cfgp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _size, _vp]),
+    "lutb_zero_buffers": (_int, [_vp, _i64, _vp, _i64, _vp, _i64, _vp]),
     "lutb_fixed_to_float": (_int, [_vp, _i64, _dbl, _vp]),
     "lutb_dense_to_sparse_workspace": (_size, [_i64]),
     "lutb_count_nonzero_32": (_int, [_vp, _i64, _vp, _vp, _size, _vp]),

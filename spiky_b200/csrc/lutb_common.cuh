@@ -93,6 +93,7 @@ enum KernelId {
     K_PEER_SGD_UPDATE,
     K_PEER_BARRIER,
     K_PEER_BROADCAST,
+    K_ZERO_BUFFERS,
     K_COUNT
 };
 

@@ -27,6 +27,10 @@ _MAX_GROUP = 1024  # forward_group_size upper bound of the reference's launch co
 
 
 def _check_tensor(t, name, real, device_index, int_bytes=4):
+    # (the common case first: one expression, about a third of the time of the checks that say what is wrong)
+    if (int_bytes == 4 and isinstance(t, torch.Tensor) and t.dtype is (torch.float32 if real else torch.int32)
+            and t.dim() == 1 and t.is_contiguous() and t.get_device() == device_index and t.is_cuda):
+        return
     if not isinstance(t, torch.Tensor):
         raise RuntimeError(f"{name} must be a tensor")
     if not t.is_contiguous():
@@ -47,7 +51,7 @@ def _check_tensor(t, name, real, device_index, int_bytes=4):
 
 
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()   # (the argument types of the library are declared: an int will do)
 
 
 class _LUTDataManager:
@@ -231,23 +235,38 @@ class _LUTDataManager:
     # ------------------------------------------------------------------ runtime helpers
     def _lr_meta(self):
         # the reference stores the rate as fp32 (BaseSynapseMeta.lr) and widens it to double
-        return float(torch.tensor(self._metas[0][0], dtype=torch.float32).item())
+        return ctypes.c_float(self._metas[0][0]).value
 
     def _cfg(self, cmp_eps=0.0, sliced=False, seq_len=None):
-        return LayerCfg(
-            n_inputs=self._n_inputs, n_outputs=self._n_outputs, n_detectors=self._n_detectors,
-            n_anchors=self._n_anchors, seq_len=self._seq_len if seq_len is None else seq_len, pos_dim=self._pos_dim,
-            forward_group=self._fwd_group, backward_group=self._bwd_group, int_mode=int(self._INT_MODE),
-            sliced_product=int(bool(sliced)), cmp_eps=float(cmp_eps), reserved0=0.0,
-            int_rescaler=self._int_rescaler, lr_meta=self._lr_meta(),
-        )
+        """The library's description of the layer (a copy of the one kept for these arguments)."""
+        seq_len = self._seq_len if seq_len is None else seq_len
+        key = (float(cmp_eps), bool(sliced), seq_len, self._metas[0][0] if self._metas else None)
+        cfgs = self.__dict__.setdefault("_cfgs", {})
+        cfg = cfgs.get(key)
+        if cfg is None:
+            cfg = LayerCfg(
+                n_inputs=self._n_inputs, n_outputs=self._n_outputs, n_detectors=self._n_detectors,
+                n_anchors=self._n_anchors, seq_len=seq_len, pos_dim=self._pos_dim,
+                forward_group=self._fwd_group, backward_group=self._bwd_group, int_mode=int(self._INT_MODE),
+                sliced_product=int(bool(sliced)), cmp_eps=float(cmp_eps), reserved0=0.0,
+                int_rescaler=self._int_rescaler, lr_meta=self._lr_meta(),
+            )
+            if len(cfgs) >= 16:   # (a caller that varies the dead band: keep the latest few)
+                cfgs.clear()
+            cfgs[key] = cfg
+        return LayerCfg.from_buffer_copy(cfg)
+
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        state.pop("_cfgs", None)
+        return state
 
     def _require_cuda(self):
         if self._device < 0:
             raise RuntimeError("spiky_b200 has no CPU execution path: move the layer to a CUDA device first")
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self._device).cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(self._device)   # torch.cuda.current_stream(...).cuda_stream without the object
 
     # ------------------------------------------------------------------ non-sequence runtime
     def forward_step(self, r_weights, batch_size, r_input, r_detector_anchors, w_output, w_lookup_indices,

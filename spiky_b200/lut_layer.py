@@ -21,6 +21,7 @@ from typing import List
 import torch
 import torch.nn as nn
 
+from . import _native
 from .lut_data_manager import LUTDataManagerF, LUTDataManagerI
 from . import structure as _structure
 from .structure import PointSamplingPolicy, PointSamplingType  # noqa: F401  (part of the public surface)
@@ -111,6 +112,19 @@ def _normalise_device(device):
     if dev.type == "cuda" and dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
     return dev
+
+
+def _zeros(device, a, b=0, c=0):
+    """Up to three zeroed flat fp32 tensors of the given sizes (None for a size of zero); on a CUDA device one launch on
+    the current stream clears them all."""
+    if device.type != "cuda":
+        return [torch.zeros(n, dtype=torch.float32, device=device) if n else None for n in (a, b, c)]
+    out = [torch.empty(n, dtype=torch.float32, device=device) if n else None for n in (a, b, c)]
+    p = [None if t is None else t.data_ptr() for t in out]
+    with torch.cuda.device(device):
+        _native.check(_native.lib().lutb_zero_buffers(p[0], 4 * a, p[1], 4 * b, p[2], 4 * c,
+                                                      torch._C._cuda_getCurrentRawStream(device.index)))
+    return out
 
 
 class _LUTFunction(torch.autograd.Function):
@@ -457,6 +471,18 @@ class LUTLayerBasic(nn.Module):
             return self._shared_context.get_weight_gradients_buffer(numel, self.device, self._multi_id)
         return torch.zeros_like(self._weights, requires_grad=False)
 
+    def _fresh_gradients(self, x_numel, pe_numel=0, table=True):
+        """(input gradient, table gradient, embedding gradient) a backward pass accumulates into, all zero; a count of zero
+        or table=False: None in its place."""
+        dense = table and self._weights_gradient_policy.type == GradientType.Dense
+        weights = self._weights
+        dx, dw, dpe = _zeros(self.device, x_numel, weights.numel() if dense else 0, pe_numel)
+        if dense:
+            dw = dw.view(weights.shape)
+        elif table:
+            dw = self._weight_grad_target()
+        return dx, dw, dpe
+
     def _external_lr(self):
         if self._weights_gradient_policy.type != GradientType.Internal:
             return -1.0
@@ -532,13 +558,17 @@ class LUTLayerBasic(nn.Module):
         assert min_anchor_delta_indices.shape == shape
         assert grad_output.shape == (B, 1) + tuple(self.output_shape())
         external = x_grad is not None
-        if not external and need_input_grad:
-            x_grad = torch.zeros(x.numel(), dtype=torch.float32, device=self.device)
-        if (not external and self._weights_gradient_policy.type == GradientType.Sparse and self._is_fully_connected
-                and self._lut_dm.get_summations_data_type() == "float32" and self._sparse_rows_direct):
+        sparse_rows = (not external and self._weights_gradient_policy.type == GradientType.Sparse and self._is_fully_connected
+                       and self._lut_dm.get_summations_data_type() == "float32" and self._sparse_rows_direct)
+        hook = getattr(self, "_table_update_hook", None)
+        sink = None if external else getattr(self, "_table_gradient_sink", None)
+        w_grad = None
+        if not external:
+            x_grad, w_grad, _ = self._fresh_gradients(x.numel() if need_input_grad else 0,
+                                                      table=not sparse_rows and hook is None and sink is None)
+        if sparse_rows:
             return self._backward_step_sparse_rows(x, grad_output, lookup_indices, min_anchor_deltas,
                                                    min_anchor_delta_indices, x_grad, B)
-        hook = getattr(self, "_table_update_hook", None)
         if hook is not None and not external:
             # data-parallel sharded table update: only the input gradient is computed here; the hook gathers the
             # (index, output gradient) pairs of all ranks and updates this rank's share of the tables in place
@@ -551,10 +581,12 @@ class LUTLayerBasic(nn.Module):
                     SKIP_TABLE_GRADIENT, None, None)
             hook(self, lookup_indices.reshape(-1), grad_flat, B)
             return (None if x_grad is None else x_grad.view(x.shape)), None
-        sink = None if external else getattr(self, "_table_gradient_sink", None)
         # data-parallel update over peer memory: the dense table gradient goes into the sink's shared buffer and the
         # sink reduces it over the ranks and updates the tables; the parameter gets no .grad
-        w_grad = self._weight_grad_target() if sink is None else sink.gradient_buffer(self)
+        if sink is not None:
+            w_grad = sink.gradient_buffer(self)
+        elif external:
+            w_grad = self._weight_grad_target()
         self._lut_dm.backward_backprop(
             self._weights.detach(), B, grad_output.contiguous().view(-1), self._detector_anchors,
             lookup_indices.reshape(-1), min_anchor_deltas.reshape(-1), min_anchor_delta_indices.reshape(-1),
@@ -620,12 +652,10 @@ class LUTLayerBasic(nn.Module):
         else:
             assert positional_lookup_indices is None and positional_min_deltas is None
         external = x_grad is not None
+        pe_numel = (S - 1) * Nt * self._positional_dim
+        dx, w_grad, pe_grad = self._fresh_gradients(0 if external else x.numel(), pe_numel)
         if not external:
-            x_grad = torch.zeros(x.numel(), dtype=torch.float32, device=self.device)
-        w_grad = self._weight_grad_target()
-        pe_grad = None
-        if self._positional_dim > 0:
-            pe_grad = torch.zeros((S - 1) * Nt * self._positional_dim, dtype=torch.float32, device=self.device)
+            x_grad = dx
 
         def flat(t):
             return None if t is None else t.reshape(-1)
@@ -665,13 +695,12 @@ class LUTLayerBasic(nn.Module):
         B, S = x.shape[0], x.shape[1]
         assert grad_output.shape == (B, S) + tuple(self.output_shape())
         external = x_grad is not None
-        if not external:
-            x_grad = torch.zeros(x.numel(), dtype=torch.float32, device=self.device)
-        w_grad = self._weight_grad_target()
-        pe = pe_grad = None
+        pe = None
         if self._positional_dim > 0:
             pe = pos_embeddings.detach().contiguous().view(-1)
-            pe_grad = torch.zeros_like(pe)
+        dx, w_grad, pe_grad = self._fresh_gradients(0 if external else x.numel(), 0 if pe is None else pe.numel())
+        if not external:
+            x_grad = dx
         xf, gf = x.view(-1), x_grad.view(-1)
         self._lut_dm.backward_backprop_product(
             self._weights.detach(), B, S, xf, xf, self._detector_anchors, grad_output.contiguous().view(-1), gf, gf,

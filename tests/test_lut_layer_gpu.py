@@ -87,3 +87,18 @@ def test_state_dict_round_trip():
     x = torch.rand(3, 1, 32, device="cuda:0")
     a.eval(); b.eval()
     assert torch.equal(a(x), b(x))
+
+
+@pytest.mark.parametrize("sizes", [(1, 0, 0), (0, 5, 1023), (1024, 1025, 0), (3, 300001, 7), (0, 0, 0)])
+def test_zeroed_buffers(sizes):
+    """One launch clears up to three buffers: pieces of 4 KB, ragged ends, sizes of zero, unaligned starts."""
+    from spiky_b200 import _native
+    from spiky_b200.lut_layer import _zeros
+
+    for n, t in zip(sizes, _zeros(torch.device("cuda", 0), *sizes)):
+        assert (t is None) if n == 0 else (t.numel() == n and not t.any())
+    keep = [torch.ones(n + 2, device="cuda") for n in sizes]
+    args = [a for k, n in zip(keep, sizes) for a in (k.data_ptr() + 4, 4 * n)]
+    _native.check(_native.lib().lutb_zero_buffers(*args, torch.cuda.current_stream().cuda_stream))
+    for k, n in zip(keep, sizes):
+        assert not k[1:n + 1].any() and float(k[0]) == 1.0 and float(k[n + 1]) == 1.0
