@@ -35,6 +35,7 @@ extern "C" {
                                point of the sweep (0.06 to 4096 samples per table row, 2.3x to 10x), so AUTO is ATOMIC */
 #define LUTB_DW_ATOMIC 1    /* row-coalesced global reductions (red.global.add.v4.f32 into L2) */
 #define LUTB_DW_SORTED 3    /* counting sort of the batch by row + segmented reduce; deterministic order; needs workspace */
+#define LUTB_DX_WRITE 0x100 /* or'ed into dw_variant: the input gradient is written, not added to, and need not be cleared */
 
 /*
  * Geometry and numeric mode of one LUT layer; mirrors the constructor arguments of

@@ -11,6 +11,7 @@ LIB_PATH = os.path.join(_HERE, "lib", "libspiky_b200.so")
 
 # dW kernel variants (include/spiky_b200.h)
 DW_AUTO, DW_ATOMIC, DW_SORTED = 0, 1, 3
+DX_WRITE = 0x100            # or'ed into dw_variant: the input gradient is written, not added to
 SKIP_TABLE_GRADIENT = -2.0  # external_lr value: input gradient only (lutb_nonseq_sparse_backward)
 # product-mode kernel variants (include/spiky_b200.h)
 PRODUCT_AUTO, PRODUCT_DIRECT, PRODUCT_HIST, PRODUCT_HIST_FMA = 0, 1, 2, 3

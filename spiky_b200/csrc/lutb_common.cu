@@ -69,16 +69,17 @@ int launch_fixed_to_float(float *buf, int64_t n, double rescaler, cudaStream_t s
     return LUTB_OK;
 }
 
-// Zero fill of a few buffers in one launch: what a backward pass clears (input gradient, table gradient, embedding
-// gradient) are one small and one large buffer as a rule, and for a small layer their separate fills were a third of its
-// launches.  Blocks take 4 KB pieces of the buffers laid end to end; 16-byte stores where a buffer is aligned.
+// Zero fill of a few small buffers in one launch: what a backward pass clears (input gradient, table gradient, embedding
+// gradient) were a third of a small layer's launches as separate fills.  Blocks take 4 KB pieces of the buffers laid end to
+// end; 16-byte stores where a buffer is aligned.  Buffers of 1 MB and more go to the driver's memset, which fills at
+// the rate of the memory (28 us for 205 MB; this kernel took 40, and 66 with one block per piece).
 constexpr int kZeroBuffers = 3;
 struct ZeroList {
     unsigned char *ptr[kZeroBuffers];
     int64_t bytes[kZeroBuffers];
     int64_t first_piece[kZeroBuffers + 1];
 };
-constexpr int64_t kZeroPiece = 4096;
+constexpr int64_t kZeroPiece = 4096, kZeroMemset = 1 << 20;
 __global__ void __launch_bounds__(256) zero_buffers_kernel(const ZeroList z) {
     for (int64_t piece = blockIdx.x; piece < z.first_piece[kZeroBuffers]; piece += gridDim.x) {
         int k = 0;
@@ -206,14 +207,14 @@ extern "C" int lutb_zero_buffers(void *a, int64_t a_bytes, void *b, int64_t b_by
         LUTB_REQUIRE(buffers[k] != nullptr || bytes[k] == 0, LUTB_ERR_NULL, "a buffer is NULL");
         LUTB_REQUIRE((reinterpret_cast<uintptr_t>(buffers[k]) & 3) == 0, LUTB_ERR_ALIGN, "buffers must be 4-byte aligned");
         z.ptr[k] = static_cast<unsigned char *>(buffers[k]);
-        z.bytes[k] = bytes[k];
-        z.first_piece[k + 1] = z.first_piece[k] + (bytes[k] + kZeroPiece - 1) / kZeroPiece;
+        if (bytes[k] >= kZeroMemset) LUTB_CUDA(cudaMemsetAsync(buffers[k], 0, (size_t)bytes[k], static_cast<cudaStream_t>(stream)));
+        z.bytes[k] = bytes[k] >= kZeroMemset ? 0 : bytes[k];
+        z.first_piece[k + 1] = z.first_piece[k] + (z.bytes[k] + kZeroPiece - 1) / kZeroPiece;
     }
     const int64_t pieces = z.first_piece[kZeroBuffers];
     if (pieces == 0) return LUTB_OK;
-    const int64_t cap = (int64_t)device_info().sm_count * 16;
     KernelScope scope(K_ZERO_BUFFERS, static_cast<cudaStream_t>(stream));
-    zero_buffers_kernel<<<(unsigned)(pieces < cap ? pieces : cap), 256, 0, static_cast<cudaStream_t>(stream)>>>(z);
+    zero_buffers_kernel<<<(unsigned)pieces, 256, 0, static_cast<cudaStream_t>(stream)>>>(z);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
 }

@@ -537,77 +537,148 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
 // Kernel 3: surrogate input gradient (reference: propagate_through_detectors_non_seq_fc_logic,
 // proto:1421-1499).  Per (sample, detector): g = sum_o dY[o] * (W[t, j, o] - W[t, j ^ 2^k, o]),
 // du = up(min_delta) * g, then +du / -du on the two inputs of the flipped anchor pair.
-// Same warp layout as the forward gather; both rows are read with coalesced vector loads.  The products of one
-// vector are summed in fp32 and added to a double per lane (converting every operand to double kept the
-// conversion unit busy: three conversions per element), the lane groups are reduced in double, and the dot
-// products of 32 detectors are parked in shared memory so that the surrogate derivative (a double division) and
-// the two reductions into dX run once per detector on 32 lanes instead of once per lane group on one lane in LG.
+// A warp owns a sample; its lane groups of LG lanes read the two rows of a detector with coalesced vector loads, two or four
+// detectors a group in flight, up to eight before they are reduced.  The products of one vector are summed in fp32 and added
+// to a double per lane; the lanes of a group transpose-reduce their detectors' sums in double (one shuffle step per halving
+// of the detectors instead of a full reduction each), so that every lane ends with one detector's dot product and the
+// surrogate derivative (a double division) and the two reductions into dX run on 32 lanes.
+// Bound: load/store wavefronts (75 % of their peak at 65536 samples x 64 detectors of 64 rows x 32 outputs), latency where
+// samples are few.  Measured (one detector a group in flight, a full reduction per detector before), with the clearing of dX:
+// 256 samples 10.9 -> 8.6 us; 1111 samples, 50 detectors, 33 outputs 32.0 -> 14.8 us; 512 samples, 64 detectors, 10 outputs
+// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.9 us; 65536 samples 187 -> 187 us.
+// (Walking groups of detectors whose tables fit L1 measured 220 us there: the groups leave lanes idle.)
 // --------------------------------------------------------------------------------------------
-template <int VEC>
-__global__ void __launch_bounds__(256) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
+// WRITE: dX is written instead of added to (and need not be cleared): the warp sums its sample's row in shared memory and
+// writes it out once.
+template <int LG, int VEC, bool WRITE>
+__global__ void __launch_bounds__(256, LG >= 16 ? 2 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                            const int2 *__restrict__ anchors,
                                                            const int32_t *__restrict__ idx,
                                                            const float *__restrict__ min_delta,
                                                            const int32_t *__restrict__ min_k, float *__restrict__ dX,
                                                            int64_t batch, int n_inputs, int n_outputs, int n_detectors,
-                                                           int n_anchors, int table_rows, int lanes_per_row) {
-    __shared__ double dots[8][32];
-    const int lane = threadIdx.x & 31;
-    const int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (b >= batch) return;
-    double *my_dots = dots[(threadIdx.x >> 5) & 7];
-    const int LG = lanes_per_row;
-    const int NG = 32 / LG;
-    const int g = lane / LG;
-    const int j = lane - g * LG;
-    const float *dy = dY + b * n_outputs;
-    float *dx = dX + b * n_inputs;
-    const int64_t base = b * n_detectors;
-    const int step = LG * VEC;
-
-    for (int tb = 0; tb < n_detectors; tb += 32) {
-        const int nvalid = min(32, n_detectors - tb);
-        int32_t my_idx = 0, my_k = -1;
-        float my_m = 0.f;
-        if (lane < nvalid) {
-            my_idx = __ldg(idx + base + tb + lane);
-            my_k = __ldg(min_k + base + tb + lane);
-            my_m = __ldg(min_delta + base + tb + lane);
-        }
-        for (int sb = 0; sb < nvalid; sb += NG) {   // uniform trip count: every lane runs every shuffle
-            const int s = sb + g;
-            const int32_t li = __shfl_sync(0xffffffffu, my_idx, s & 31);
-            const int32_t k = __shfl_sync(0xffffffffu, my_k, s & 31);
-            double acc = 0.0;
-            const bool valid = s < nvalid && k >= 0;
-            if (valid) {
-                const int t = tb + s;
-                const float *row = W + ((size_t)t * table_rows + li) * n_outputs;
-                const float *alt = W + ((size_t)t * table_rows + (li ^ (1 << k))) * n_outputs;
-                for (int col = j * VEC; col < n_outputs; col += step) {
-                    float a[VEC], c[VEC], d[VEC];
-                    Vec<VEC>::load(row + col, a);
-                    Vec<VEC>::load(alt + col, c);
-                    Vec<VEC>::load(dy + col, d);
-                    float part = 0.f;
+                                                           int n_anchors, int table_rows, int group_dets, int block_samples) {
+    constexpr int NG = 32 / LG, CH = LG < 8 ? LG : 8, U = CH < (LG >= 16 ? 4 : 2) ? CH : (LG >= 16 ? 4 : 2);   // CH detectors a group at a time
+    const int lane = threadIdx.x & 31, g = lane / LG, j = lane - g * LG;
+    const int my_s = j * NG + g;   // this lane's detector of every 32: iteration i of group g takes detector i * NG + g
+    const int t_begin = blockIdx.y * group_dets, t_end = min(n_detectors, t_begin + group_dets);
+    const int64_t b_end = min(batch, ((int64_t)blockIdx.x + 1) * block_samples);
+    extern __shared__ __align__(16) float dx_rows[];
+    const int row_floats = (n_inputs + 3) & ~3;
+    float *dx_s = dx_rows + (threadIdx.x >> 5) * row_floats;
+    if (WRITE) {
+        for (int i = lane; i < row_floats; i += 32) dx_s[i] = 0.f;
+        __syncwarp();
+    }
+    for (int64_t b = (int64_t)blockIdx.x * block_samples + (threadIdx.x >> 5); b < b_end; b += blockDim.x >> 5) {
+        const float *dy = dY + b * n_outputs;
+        float *dx = dX + b * n_inputs;
+        const int64_t base = b * n_detectors;
+        float d0[VEC];   // this lane's columns of dY where a row is one step
+        if (j * VEC < n_outputs) Vec<VEC>::load(dy + j * VEC, d0);
+        else {
 #pragma unroll
-                    for (int e = 0; e < VEC; e++) part = fmaf(d[e], a[e] - c[e], part);
-                    acc += (double)part;
+            for (int e = 0; e < VEC; e++) d0[e] = 0.f;
+        }
+        for (int tb = t_begin; tb < t_end; tb += 32) {
+            const int nvalid = min(32, t_end - tb);
+            int32_t my_idx = 0, my_k = -1;
+            float my_m = 0.f;
+            if (my_s < nvalid) {
+                my_idx = __ldg(idx + base + tb + my_s);
+                my_k = __ldg(min_k + base + tb + my_s);
+                my_m = __ldg(min_delta + base + tb + my_s);
+            }
+            double dot = 0.0;
+#pragma unroll 1
+            for (int ch = 0; ch < LG && ch * NG < nvalid; ch += CH) {
+                double v[CH];
+#pragma unroll
+                for (int i0 = 0; i0 < CH; i0 += U) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) v[i0 + u] = 0.0;
+                    if ((ch + i0) * NG >= nvalid) continue;   // warp uniform
+                    const float *row[U], *alt[U];
+                    bool on[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int i = ch + i0 + u, s = i * NG + g;
+                        const int32_t li = __shfl_sync(0xffffffffu, my_idx, g * LG + i);
+                        const int32_t k = __shfl_sync(0xffffffffu, my_k, g * LG + i);
+                        on[u] = s < nvalid && k >= 0;
+                        const float *tab = W + (size_t)(tb + (on[u] ? s : 0)) * table_rows * n_outputs;
+                        row[u] = tab + (size_t)li * n_outputs;
+                        alt[u] = tab + (size_t)(on[u] ? li ^ (1 << k) : 0) * n_outputs;
+                    }
+                    for (int c0 = 0; c0 < n_outputs; c0 += LG * VEC) {
+                        const int col = c0 + j * VEC;
+                        float d[VEC], a[U][VEC], c[U][VEC];
+                        if (c0 == 0) {
+#pragma unroll
+                            for (int e = 0; e < VEC; e++) d[e] = d0[e];
+                        } else if (col < n_outputs) {
+                            Vec<VEC>::load(dy + col, d);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+#pragma unroll
+                            for (int e = 0; e < VEC; e++) a[u][e] = c[u][e] = 0.f;
+                            if (on[u] && col < n_outputs) {
+                                Vec<VEC>::load(row[u] + col, a[u]);
+                                Vec<VEC>::load(alt[u] + col, c[u]);
+                            }
+                        }
+                        if (col < n_outputs) {
+#pragma unroll
+                            for (int u = 0; u < U; u++) {
+                                float part = 0.f;
+#pragma unroll
+                                for (int e = 0; e < VEC; e++) part = fmaf(d[e], a[u][e] - c[u][e], part);
+                                v[i0 + u] += (double)part;
+                            }
+                        }
+                    }
+                }
+                // lane j ends with the chunk's detector j % CH: halving steps over the detectors, then plain ones
+#pragma unroll
+                for (int o = CH / 2; o >= 1; o >>= 1) {
+                    const bool upper = (j & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < o; i++) {
+                        const double send = upper ? v[i] : v[i + o];
+                        const double keep = upper ? v[i + o] : v[i];
+                        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+#pragma unroll
+                for (int o = CH; o < LG; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                if (j / CH == ch / CH) dot = v[0];
+            }
+            if (my_s < nvalid && my_k >= 0) {
+                const double du = surrogate_up(my_m) * dot;
+                if (fabs(du) > kEps) {
+                    const int2 p = __ldg(anchors + (size_t)(tb + my_s) * n_anchors + my_k);
+                    float *cells = WRITE ? dx_s : dx;
+                    atomicAdd(cells + p.x, (float)du);
+                    atomicAdd(cells + p.y, -(float)du);
                 }
             }
-            for (int off = 1; off < LG; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if (s < nvalid && j == 0) my_dots[s] = acc;
         }
-        __syncwarp();
-        if (lane < nvalid && my_k >= 0) {
-            const double du = surrogate_up(my_m) * my_dots[lane];
-            if (fabs(du) > kEps) {
-                const int2 p = __ldg(anchors + (size_t)(tb + lane) * n_anchors + my_k);
-                atomicAdd(dx + p.x, (float)du);
-                atomicAdd(dx + p.y, -(float)du);
+        if (WRITE) {
+            __syncwarp();
+            if (row_floats == n_inputs && (reinterpret_cast<uintptr_t>(dX) & 15) == 0) {
+                for (int i = lane * 4; i < n_inputs; i += 128) {
+                    __stcs(reinterpret_cast<float4 *>(dx + i), *reinterpret_cast<const float4 *>(dx_s + i));
+                    *reinterpret_cast<float4 *>(dx_s + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            } else {
+                for (int i = lane; i < n_inputs; i += 32) {
+                    dx[i] = dx_s[i];
+                    dx_s[i] = 0.f;
+                }
             }
+            __syncwarp();
         }
-        __syncwarp();
     }
 }
 
@@ -728,7 +799,7 @@ __global__ void __launch_bounds__(256) fc_weight_grad_atomic_kernel(const float 
 
 int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const float *dY, const int32_t *anchors,
                        const int32_t *idx, const float *min_delta, const int32_t *min_k, float *dX, float *target,
-                       double lr, cudaStream_t stream, bool skip_table_gradient = false) {
+                       double lr, cudaStream_t stream, bool skip_table_gradient = false, bool write_dx = false) {
     const int O = cfg->n_outputs, Nt = cfg->n_detectors, T = 1 << cfg->n_anchors;
     const bool int_mode = cfg->int_mode != 0;
     const bool vec4 = (O % 4 == 0) && ((reinterpret_cast<uintptr_t>(W) & 15) == 0) &&
@@ -741,6 +812,18 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
     LUTB_REQUIRE(blocks <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "batch too large for one launch");
     const int sm = device_info().sm_count;
 
+    // rows of dX in shared memory: while at least three blocks of eight warps fit an SM
+    const size_t row_bytes = (size_t)((cfg->n_inputs + 3) & ~3) * 4;
+    const bool rows = write_dx && dX != nullptr && !int_mode && 8 * row_bytes <= 64 * 1024;
+    // few samples: small blocks, or (a sample's row has one owner where it is written) 32 detectors a block, so that more SMs
+    // share the work
+    const bool few = blocks < 2 * sm;
+    const int group_dets = few && !rows ? min(Nt, 32) : Nt, dx_warps = few && rows ? 2 : warps;
+    if (write_dx && dX != nullptr && !rows) {
+        const int rc = lutb_zero_buffers(dX, batch * (int64_t)cfg->n_inputs * 4, nullptr, 0, nullptr, 0, stream);
+        if (rc) return rc;
+    }
+
     // input gradient (dX == nullptr: the caller does not want it)
     if (dX != nullptr) {
     KernelScope scope(K_FC_INPUT_GRAD, stream);
@@ -750,14 +833,40 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
         fc_input_grad_fixed_kernel<<<(unsigned)gblocks, 128, 0, stream>>>(
             W, dY, reinterpret_cast<const int2 *>(anchors), idx, min_delta, min_k, dX, batch, cfg->n_inputs, O, Nt,
             cfg->n_anchors, T, cfg->forward_group, cfg->int_rescaler);
-    } else if (vec4) {
-        fc_input_grad_kernel<4><<<(unsigned)blocks, warps * 32, 0, stream>>>(
-            W, dY, reinterpret_cast<const int2 *>(anchors), idx, min_delta, min_k, dX, batch, cfg->n_inputs, O, Nt,
-            cfg->n_anchors, T, lanes);
     } else {
-        fc_input_grad_kernel<1><<<(unsigned)blocks, warps * 32, 0, stream>>>(
-            W, dY, reinterpret_cast<const int2 *>(anchors), idx, min_delta, min_k, dX, batch, cfg->n_inputs, O, Nt,
-            cfg->n_anchors, T, lanes);
+        const int groups = (Nt + group_dets - 1) / group_dets;
+        int64_t per_block = (batch * groups / ((int64_t)sm * 16) + dx_warps - 1) / dx_warps * dx_warps;
+        if (per_block < dx_warps) per_block = dx_warps;
+        if (per_block > 4096) per_block = 4096;
+        const dim3 grid((unsigned)((batch + per_block - 1) / per_block), (unsigned)groups);
+        LUTB_REQUIRE(groups <= 65535, LUTB_ERR_SHAPE, "too many detectors for one launch");
+        int launch_rc = LUTB_OK;
+        auto launch = [&](auto add, auto write) -> int {
+            const size_t smem = rows ? dx_warps * row_bytes : 0;
+            auto kern = rows ? write : add;
+            if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<grid, dx_warps * 32, smem, stream>>>(W, dY, reinterpret_cast<const int2 *>(anchors), idx, min_delta, min_k, dX, batch,
+                                                  cfg->n_inputs, O, Nt, cfg->n_anchors, T, group_dets, (int)per_block);
+            return LUTB_OK;
+        };
+        if (vec4) {
+            switch (lanes) {
+                case 32: launch_rc = launch(fc_input_grad_kernel<32, 4, false>, fc_input_grad_kernel<32, 4, true>); break;
+                case 16: launch_rc = launch(fc_input_grad_kernel<16, 4, false>, fc_input_grad_kernel<16, 4, true>); break;
+                case 8: launch_rc = launch(fc_input_grad_kernel<8, 4, false>, fc_input_grad_kernel<8, 4, true>); break;
+                case 4: launch_rc = launch(fc_input_grad_kernel<4, 4, false>, fc_input_grad_kernel<4, 4, true>); break;
+                case 2: launch_rc = launch(fc_input_grad_kernel<2, 4, false>, fc_input_grad_kernel<2, 4, true>); break;
+                default: launch_rc = launch(fc_input_grad_kernel<1, 4, false>, fc_input_grad_kernel<1, 4, true>); break;
+            }
+        } else {
+            switch (lanes) {
+                case 32: launch_rc = launch(fc_input_grad_kernel<32, 1, false>, fc_input_grad_kernel<32, 1, true>); break;
+                case 16: launch_rc = launch(fc_input_grad_kernel<16, 1, false>, fc_input_grad_kernel<16, 1, true>); break;
+                case 8: launch_rc = launch(fc_input_grad_kernel<8, 1, false>, fc_input_grad_kernel<8, 1, true>); break;
+                default: launch_rc = launch(fc_input_grad_kernel<4, 1, false>, fc_input_grad_kernel<4, 1, true>); break;
+            }
+        }
+        if (launch_rc) return launch_rc;
     }
     }
     LUTB_LAUNCH_CHECK();
@@ -844,6 +953,7 @@ extern "C" int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t bat
 }
 
 extern "C" size_t lutb_nonseq_fc_backward_workspace(const lutb_layer_cfg *cfg, int64_t batch, int dw_variant) {
+    dw_variant &= ~LUTB_DX_WRITE;
     if (cfg == nullptr || batch <= 0 || dw_variant != LUTB_DW_SORTED || cfg->int_mode) return 0;
     return fc_dw_sorted_workspace(batch, cfg->n_detectors, 1 << cfg->n_anchors);
 }
@@ -855,6 +965,8 @@ extern "C" int lutb_nonseq_fc_backward(const lutb_layer_cfg *cfg, int64_t batch,
     int rc = validate_cfg(cfg);
     if (rc) return rc;
     LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "backward_backprop should only be called when sequence_length == 1");
+    const bool write_dx = (dw_variant & LUTB_DX_WRITE) != 0;
+    dw_variant &= ~LUTB_DX_WRITE;
     LUTB_REQUIRE(dw_variant == LUTB_DW_AUTO || dw_variant == LUTB_DW_ATOMIC || dw_variant == LUTB_DW_SORTED, LUTB_ERR_MODE,
                  "unknown dw_variant %d", dw_variant);
     // fixed-point sums are order independent already: the sorted variant only applies to fp32 accumulators
@@ -878,7 +990,7 @@ extern "C" int lutb_nonseq_fc_backward(const lutb_layer_cfg *cfg, int64_t batch,
     // the reference narrows external_lr to fp32 before use (lut.cu:1076)
     if (external_lr >= 0.0) lr *= -(double)(float)external_lr;
     float *target = external_lr >= 0.0 ? weights : dW;
-    rc = launch_fc_backward(cfg, batch, weights, dY, anchors, idx, min_delta, min_k, dX, target, lr, st, sorted || skip_table);
+    rc = launch_fc_backward(cfg, batch, weights, dY, anchors, idx, min_delta, min_k, dX, target, lr, st, sorted || skip_table, write_dx);
     if (rc) return rc;
     if (sorted && !skip_table) {
         rc = launch_fc_dw_sorted(dY, idx, target, batch, cfg->n_outputs, cfg->n_detectors, 1 << cfg->n_anchors, lr,

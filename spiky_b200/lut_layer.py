@@ -115,7 +115,7 @@ def _normalise_device(device):
 
 
 def _zeros(device, a, b=0, c=0):
-    """Up to three zeroed flat fp32 tensors of the given sizes (None for a size of zero); on a CUDA device one launch on
+    """Up to three zeroed flat fp32 tensors of the given sizes (None for a size of zero); on a CUDA device one call on
     the current stream clears them all."""
     if device.type != "cuda":
         return [torch.zeros(n, dtype=torch.float32, device=device) if n else None for n in (a, b, c)]
@@ -496,7 +496,7 @@ class LUTLayerBasic(nn.Module):
     _sparse_rows_direct = True
 
     def _backward_step_sparse_rows(self, x, grad_output, lookup_indices, min_anchor_deltas, min_anchor_delta_indices,
-                                   x_grad, batch_size):
+                                   x_grad, batch_size, dw_variant=0):
         """Input gradient by the usual kernels, table gradient as a list of touched rows; the result is the sparse
         tensor ``_process_gradients`` builds from the dense gradient: cell indices ascending, zero cells dropped."""
         from ._native import SKIP_TABLE_GRADIENT
@@ -506,7 +506,7 @@ class LUTLayerBasic(nn.Module):
         if x_grad is not None:
             dm.backward_backprop(self._weights.detach(), batch_size, grad_flat, self._detector_anchors, idx_flat,
                                  min_anchor_deltas.reshape(-1), min_anchor_delta_indices.reshape(-1), x_grad.view(-1),
-                                 SKIP_TABLE_GRADIENT, None, None)
+                                 SKIP_TABLE_GRADIENT, None, None, dw_variant=dw_variant)
         dx = None if x_grad is None else x_grad.view(x.shape)
         rows, values = dm.table_gradient_rows(batch_size, grad_flat, idx_flat)
         if rows.numel() == 0:
@@ -563,12 +563,18 @@ class LUTLayerBasic(nn.Module):
         hook = getattr(self, "_table_update_hook", None)
         sink = None if external else getattr(self, "_table_gradient_sink", None)
         w_grad = None
+        dw_variant = self._dw_variant
         if not external:
-            x_grad, w_grad, _ = self._fresh_gradients(x.numel() if need_input_grad else 0,
+            # the fully connected kernels write the input gradient; the others add to a cleared one
+            writes = need_input_grad and self._is_fully_connected and self.device.type == "cuda"
+            x_grad, w_grad, _ = self._fresh_gradients(x.numel() if need_input_grad and not writes else 0,
                                                       table=not sparse_rows and hook is None and sink is None)
+            if writes:
+                x_grad = torch.empty(x.numel(), dtype=torch.float32, device=self.device)
+                dw_variant |= _native.DX_WRITE
         if sparse_rows:
             return self._backward_step_sparse_rows(x, grad_output, lookup_indices, min_anchor_deltas,
-                                                   min_anchor_delta_indices, x_grad, B)
+                                                   min_anchor_delta_indices, x_grad, B, dw_variant)
         if hook is not None and not external:
             # data-parallel sharded table update: only the input gradient is computed here; the hook gathers the
             # (index, output gradient) pairs of all ranks and updates this rank's share of the tables in place
@@ -578,7 +584,7 @@ class LUTLayerBasic(nn.Module):
                 self._lut_dm.backward_backprop(
                     self._weights.detach(), B, grad_flat, self._detector_anchors, lookup_indices.reshape(-1),
                     min_anchor_deltas.reshape(-1), min_anchor_delta_indices.reshape(-1), x_grad.view(-1),
-                    SKIP_TABLE_GRADIENT, None, None)
+                    SKIP_TABLE_GRADIENT, None, None, dw_variant=dw_variant)
             hook(self, lookup_indices.reshape(-1), grad_flat, B)
             return (None if x_grad is None else x_grad.view(x.shape)), None
         # data-parallel update over peer memory: the dense table gradient goes into the sink's shared buffer and the
@@ -590,7 +596,7 @@ class LUTLayerBasic(nn.Module):
         self._lut_dm.backward_backprop(
             self._weights.detach(), B, grad_output.contiguous().view(-1), self._detector_anchors,
             lookup_indices.reshape(-1), min_anchor_deltas.reshape(-1), min_anchor_delta_indices.reshape(-1),
-            None if x_grad is None else x_grad.view(-1), self._external_lr(), w_grad, None, dw_variant=self._dw_variant)
+            None if x_grad is None else x_grad.view(-1), self._external_lr(), w_grad, None, dw_variant=dw_variant)
         if sink is not None:
             sink.gradient_ready(self)
             return (None if x_grad is None else x_grad.view(x.shape)), None

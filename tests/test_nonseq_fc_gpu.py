@@ -234,3 +234,38 @@ def test_check_detectors_row_and_detector_splits(rows, I, Nt, Nc):
         idx.fill_(-7)
         _native.check(L.lutb_check_detectors(ctypes.byref(cfg), rows, p[0], p[1], p[2], None, None, stream))
         assert np.array_equal(idx.cpu().numpy(), ridx.reshape(-1))
+
+
+@pytest.mark.parametrize("B,I,Nt,Nc,O", [(1, 7, 1, 1, 1), (9, 33, 5, 4, 4), (70, 100, 33, 6, 12), (600, 50, 70, 5, 33),
+                                         (2400, 64, 64, 6, 32), (2403, 37, 16, 8, 64), (2500, 2052, 20, 3, 132),
+                                         (2400, 63, 40, 4, 5), (19000, 24, 9, 4, 8)])
+def test_input_gradient_kernel_splits(B, I, Nt, Nc, O):
+    """Lane groups of every width, rows of several steps, few samples (32 detectors a block) and many; the input gradient
+    added to what is there and written over what is there (with rows that fit shared memory and longer ones)."""
+    import ctypes
+    from spiky_b200 import _native
+
+    x = synth.normal(970, (B, I))
+    anchors = synth.anchor_pairs(971, Nt, Nc, I)
+    W = synth.normal(972, (Nt * (1 << Nc) * O,), 0.0, 0.05)
+    dY = synth.normal(973, (B, O))
+    _, idx, md, mk = orc.nonseq_fc_forward(W, x, anchors, Nt, Nc, O)
+    want, dW = orc.nonseq_fc_backward(W, dY, anchors, idx, md, mk, I, Nc)
+    cfg = _native.LayerCfg(n_inputs=I, n_outputs=O, n_detectors=Nt, n_anchors=Nc, seq_len=1, pos_dim=0, forward_group=32,
+                           backward_group=32, int_mode=0, sliced_product=0, cmp_eps=0.0, reserved0=0.0, int_rescaler=1.0,
+                           lr_meta=1.0)
+    tW, tdY, ta, ti, tm, tk = [torch.from_numpy(np.ascontiguousarray(v)).reshape(-1).cuda() for v in (W, dY, anchors, idx, md, mk)]
+    L, stream = _native.lib(), torch.cuda.current_stream().cuda_stream
+    for variant, start in ((0, 1.0), (_native.DX_WRITE, float("nan"))):
+        dX, gW = torch.full((B * I,), start, device="cuda"), torch.zeros_like(tW)
+        _native.check(L.lutb_nonseq_fc_backward(ctypes.byref(cfg), B, tW.data_ptr(), tdY.data_ptr(), ta.data_ptr(), ti.data_ptr(),
+                                                tm.data_ptr(), tk.data_ptr(), dX.data_ptr(), gW.data_ptr(), -1.0, variant, None, 0,
+                                                stream))
+        got = dX.cpu().numpy().reshape(B, I)
+        if variant == 0:
+            # (adding to 1 rounds every partial sum at 2^-24)
+            assert np.abs(got - 1.0 - want).max() <= 1e-5 * np.abs(want).max() + 2.0 ** -24 * 4 * Nt
+        else:
+            golden_util.assert_close(got, want, 1e-5, "dX")
+        if B < 10000:
+            golden_util.assert_close(gW.cpu().numpy(), dW.reshape(-1), 1e-5, "dW")
