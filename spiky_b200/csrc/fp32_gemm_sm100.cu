@@ -2,7 +2,7 @@
 //
 // The contractions (product_hist.cuh) multiply exact small integers (row counts) or fp32 tables / gradients and must
 // keep fp32 accuracy (parity bar 1e-5), so plain TF32 or BF16 inputs are not an option.  Two routes, both CUTLASS 3
-// collectives instantiated for sm_100a (operands arrive in shared memory by TMA - cluster 1x1x1: plain copies of this
+// collectives instantiated for sm_100a (operands arrive in shared memory by TMA - a cluster of one block or one pair: plain copies of this
 // GPU's own memory -, tcgen05.mma accumulates in fp32 in tensor memory, the epilogue reads the accumulators back with
 // tcgen05.ld and applies alpha / beta):
 //
@@ -72,13 +72,15 @@ struct FastF32Gemm {
     using StrideD = typename Kernel::StrideD;
 };
 
-template <class LayoutA, class LayoutB>
+// PAIR: two SMs share a 256 x 256 tile (cta_group::2): each loads its half of both operands, so that an operand byte from
+// shared memory feeds twice the multiply-adds.  The loads are plain (a cluster of exactly one pair has nobody to multicast to).
+template <class LayoutA, class LayoutB, bool PAIR = false>
 struct Tf32Gemm {
     using Element = cutlass::tfloat32_t;   // fp32 storage; the MMA reads sign, exponent and the top 10 mantissa bits
     using LayoutC = cutlass::layout::RowMajor;
     static constexpr int kAlign = 4;
-    using MmaTile = Shape<_128, _128, _32>;
-    using Cluster = Shape<_1, _1, _1>;
+    using MmaTile = cute::conditional_t<PAIR, Shape<_256, _256, _32>, Shape<_128, _128, _32>>;
+    using Cluster = cute::conditional_t<PAIR, Shape<_2, _1, _1>, Shape<_1, _1, _1>>;
     using Epilogue = typename cutlass::epilogue::collective::CollectiveBuilder<
         cutlass::arch::Sm100, cutlass::arch::OpClassTensorOp, MmaTile, Cluster,
         cutlass::epilogue::collective::EpilogueTileAuto, float, float, float, LayoutC, kAlign, float, LayoutC, kAlign,
@@ -146,6 +148,12 @@ using FastTT = FastF32Gemm<cutlass::layout::ColumnMajor, cutlass::layout::RowMaj
 using Tf32TN = Tf32Gemm<cutlass::layout::RowMajor, cutlass::layout::ColumnMajor>;
 using Tf32NN = Tf32Gemm<cutlass::layout::RowMajor, cutlass::layout::RowMajor>;
 using Tf32TT = Tf32Gemm<cutlass::layout::ColumnMajor, cutlass::layout::RowMajor>;
+template <class Cfg>
+struct PairOf;
+template <class LayoutA, class LayoutB>
+struct PairOf<Tf32Gemm<LayoutA, LayoutB, false>> {
+    using type = Tf32Gemm<LayoutA, LayoutB, true>;
+};
 
 bool tc_gemm_available() { return true; }
 
@@ -217,9 +225,25 @@ __global__ void combine_halves_kernel(const float *__restrict__ P, float *__rest
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-template <class T3>
-static size_t gemm_ws3(int M, int N, int K) {
-    return workspace_of<T3>(M, N, K);
+// A pair of SMs per 256 x 256 tile where there are tiles for most of the SMs, one SM per 128 x 128 tile below.  Measured
+// on the contractions of the histogram path, one SM / pair: 8192 x 512 x 16384 214 / 176 us, 16384 x 512 x 8192 (A^T . B)
+// 214 / 166, 8192 x 16384 x 768 318 / 258; 1024 x 2048 x 65536 in 8 slices 423 / 341, 65536 x 2048 x 1024 384 / 337,
+// 1024 x 65536 x 3072 592 / 488.
+static bool pair_tiles(int M, int N, int batches) {
+    return (int64_t)((M + 255) / 256) * ((N + 255) / 256) * batches >= 64;
+}
+template <class Cfg>
+static int run_tiles(int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,
+                     float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream,
+                     Batches batches = Batches{}) {
+    if (pair_tiles(M, N, batches.count))
+        return run<typename PairOf<Cfg>::type>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream, batches);
+    return run<Cfg>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream, batches);
+}
+template <class Cfg>
+static size_t workspace_of_tiles(int M, int N, int K) {
+    const size_t a = workspace_of<Cfg>(M, N, K), b = workspace_of<typename PairOf<Cfg>::type>(M, N, K);
+    return a > b ? a : b;
 }
 
 // Plan of one call.  TN (both operands contraction-major): one GEMM of depth 3K on concatenated copies.  NN / TT with an
@@ -261,19 +285,19 @@ static SplitPlan split_plan(TcGemmKind kind, int M, int N, int K, bool a_exact) 
     SplitPlan p{};
     if (kind == TC_A_ROWS_B_ROWS_OF_N && !a_exact) {
         p.mode = 0;
-        p.gemm_ws = align256(workspace_of<Tf32TN>(M, N, 3 * K));
+        p.gemm_ws = align256(workspace_of_tiles<Tf32TN>(M, N, 3 * K));
         p.a_bytes = align256((size_t)M * 3 * K * 4);
         p.b_bytes = align256((size_t)N * 3 * K * 4);
     } else if (kind != TC_A_ROWS_B_ROWS_OF_N && a_exact && N % 4 == 0) {
         p.mode = 1;
         mode1_slices(kind, N, K, &p.slices, &p.kc);
-        p.gemm_ws = align256(kind == TC_A_ROWS_B_ROWS_OF_K ? workspace_of<Tf32NN>(M, 2 * N, K) : workspace_of<Tf32TT>(M, 2 * N, K));
+        p.gemm_ws = align256(kind == TC_A_ROWS_B_ROWS_OF_K ? workspace_of_tiles<Tf32NN>(M, 2 * N, K) : workspace_of_tiles<Tf32TT>(M, 2 * N, K));
         p.b_bytes = align256((size_t)K * 2 * N * 4);
         p.p_bytes = align256((size_t)M * 2 * N * 4 * (kind == TC_A_ROWS_B_ROWS_OF_K ? p.slices : 1));
     } else {
         p.mode = 2;
-        size_t w = workspace_of<Tf32TN>(M, N, K);
-        const size_t w2 = workspace_of<Tf32NN>(M, N, K), w3 = workspace_of<Tf32TT>(M, N, K);
+        size_t w = workspace_of_tiles<Tf32TN>(M, N, K);
+        const size_t w2 = workspace_of_tiles<Tf32NN>(M, N, K), w3 = workspace_of_tiles<Tf32TT>(M, N, K);
         w = w > w2 ? w : w2;
         p.gemm_ws = align256(w > w3 ? w : w3);
         p.a_bytes = a_exact ? 0 : align256((size_t)M * K * 4 * 2);
@@ -326,7 +350,7 @@ int tc_gemm(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, c
         if (rc) return rc;
         rc = split(B, N, K, ldb, Bs, 3, 0b001u, stream);
         if (rc) return rc;
-        return run<Tf32TN>(M, N, 3 * K, As, 3 * (int64_t)K, Bs, 3 * (int64_t)K, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
+        return run_tiles<Tf32TN>(M, N, 3 * K, As, 3 * (int64_t)K, Bs, 3 * (int64_t)K, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
     }
     if (plan.mode == 1) {
         // B' = [hi | lo] along the free index: one GEMM of width 2N into P, then C = alpha * (P_hi + P_lo) + beta * C
@@ -340,12 +364,12 @@ int tc_gemm(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, c
             bt.a = plan.kc;
             bt.b = (int64_t)plan.kc * 2 * N;
             bt.c = (int64_t)M * 2 * N;
-            rc = run<Tf32NN>(M, 2 * N, plan.kc, A, lda, Bs, 2 * (int64_t)N, P, 2 * (int64_t)N, 1.f, 0.f, gw, plan.gemm_ws, stream, bt);
+            rc = run_tiles<Tf32NN>(M, 2 * N, plan.kc, A, lda, Bs, 2 * (int64_t)N, P, 2 * (int64_t)N, 1.f, 0.f, gw, plan.gemm_ws, stream, bt);
             if (rc) return rc;
         } else {
             for (int k0 = 0; k0 < K; k0 += plan.kc) {
                 const int kn = K - k0 < plan.kc ? K - k0 : plan.kc;
-                rc = run<Tf32TT>(M, 2 * N, kn, A + (int64_t)k0 * lda, lda, Bs + (int64_t)k0 * 2 * N, 2 * (int64_t)N, P,
+                rc = run_tiles<Tf32TT>(M, 2 * N, kn, A + (int64_t)k0 * lda, lda, Bs + (int64_t)k0 * 2 * N, 2 * (int64_t)N, P,
                                  2 * (int64_t)N, 1.f, k0 == 0 ? 0.f : 1.f, gw, plan.gemm_ws, stream);
                 if (rc) return rc;
             }

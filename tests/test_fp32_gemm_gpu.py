@@ -61,6 +61,11 @@ def test_fp32_gemm_matches_fp64_product(kind, shape, fast):
     assert (C.double() - ref).abs().max().item() <= 1e-5 * ref.abs().max().item()
 
 
+def test_fp32_gemm_on_pairs_of_sms():
+    """More than 64 tiles of 256 x 256, ragged in both directions: two SMs a tile."""
+    test_fp32_gemm_matches_fp64_product(0, (2100, 2052, 96), False)
+
+
 def test_fp32_gemm_rejects_misaligned_leading_dimensions():
     from spiky_b200 import _native
     if not _native.lib().lutb_fp32_gemm_available():
