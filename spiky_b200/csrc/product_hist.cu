@@ -318,9 +318,11 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
 // Sums: the key's cells are a private shared-memory column per lane (plain read-modify-write), flushed once per block.
 // The query's cells would collide (32 lanes, a few anchors), so a pair's (du, anchor) is parked in an 8 x 32 tile that
 // the warp reads back with the lanes over queries, again into private columns; the block adds the columns up once per
-// eight queries.
+// eight queries. 
 // Measured (before: a warp per query, about 600 instructions per 32 pairs): 64 sequences x 128 tokens, 64 detectors of 256
-// rows 862 -> 478 us; 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 922 us.
+// rows 862 -> 440 us (323 without positional anchors); 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 832 us (590
+// without: the blocks of the few detectors with such an anchor end last).  Two barriers per eight queries instead of four
+// gave 8 % at 128 tokens; a per-warp window of distances for dPE instead of an add per pair cost 20 % there.
 // --------------------------------------------------------------------------------------------
 constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
 constexpr int kExLd = 33;          // leading dimension of the (query, key) exchange tile
@@ -358,24 +360,43 @@ __device__ __forceinline__ uint32_t margin_low(uint32_t bit, float d) {
 
 struct RouteTile {
     const float *smem, *Qs, *qd, *xk, *x2b, *pe_t;
-    const float4 *qstate;   // [kTileQ] {bits, |delta|, low of the query-only anchors}
     const float2 *qv;
     float *kcol, *pacc;
     float2 *ex;
     int j0, i, ikey, n_pe, pe_stride, t;
     uint32_t pe_mask, kbits;
     unsigned long long kmin;
+    // lane q < kTileQ: the query-only anchors of query j0 + q
+    uint32_t qbits;
+    float qmd;
+    uint32_t qlow;
 };
+
+__device__ __forceinline__ void add_positional(const RouteArgs &p, float *pacc, int dist, int t, int elem, float v) {
+    if (p.pe_cells) atomicAdd(pacc + dist * p.npe + elem, v);
+    else atomicAdd(p.dPE + ((size_t)dist * p.n_detectors + t) * p.npe + elem, v);
+}
 
 template <int NKQ, bool PE, bool EPS, int MAXKQ>
 __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists &al, const RouteTile &r, const float (&kv)[MAXKQ]) {
     const int lane = threadIdx.x & 31, T = 1 << p.n_anchors;
-#pragma unroll 4
+    // the first positional anchor's operands as two addresses and steps per query (it is always staged)
+    const float *end0 = nullptr, *end1 = nullptr;
+    int step0 = 0, step1 = 0;
+    uint32_t pe_bit = 0u;
+    if (PE && r.n_pe > 0) {
+        const int4 a = al.pe_at[0], b = al.pe_at[1];
+        end0 = a.w ? r.qd + a.x : r.smem + a.x + r.ikey * a.y;
+        end1 = b.w ? r.qd + b.x : r.smem + b.x + r.ikey * b.y;
+        step0 = a.w ? kHistAnchors : a.z;
+        step1 = b.w ? kHistAnchors : b.z;
+        pe_bit = 1u << al.pe_k[0];
+    }
+#pragma unroll 2
     for (int q = 0; q < kTileQ; q++) {
         const int j = r.j0 + q;
-        const float4 qs = r.qstate[q];
-        uint32_t li = r.kbits | __float_as_uint(qs.x);
-        unsigned long long best = margin_key(qs.y, __float_as_uint(qs.z));
+        uint32_t li = r.kbits | __shfl_sync(0xffffffffu, r.qbits, q);
+        unsigned long long best = margin_key(__shfl_sync(0xffffffffu, r.qmd, q), __shfl_sync(0xffffffffu, r.qlow, q));
         best = r.kmin < best ? r.kmin : best;
         if (NKQ > 0) {
             // anchor numbers ascend: strictly smaller is enough inside this group
@@ -397,8 +418,14 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
         }
         const bool pair = r.i < j && j < p.S;
         const int dist = max(0, min(j, p.S - 1) - r.i - 1);
-        if (PE) {
-            for (int m = 0; m < r.n_pe; m++) {
+        if (PE && r.n_pe > 0) {
+            {
+                const float d = __fsub_rn(end0[q * step0], end1[q * step1]);
+                if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= pe_bit;
+                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(pe_bit, d));
+                best = c < best ? c : best;
+            }
+            for (int m = 1; m < r.n_pe; m++) {
                 float v0, v1;
                 positional_ends(al, r.smem, r.qd + q * kHistAnchors, m, m < p.pe_cap, r.ikey, q, r.xk,
                                 r.x2b + (size_t)min(j, p.S - 1) * p.e2, r.pe_t + (size_t)dist * r.pe_stride, v0, v1);
@@ -425,15 +452,13 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
         const int off = bit ? (31 - __clz(bit)) * 32 : 0;
         r.kcol[off + lane] += du;
         r.ex[q * kExLd + lane] = make_float2(du, __int_as_float(off));
-        if (PE) {
+        if (PE && r.n_pe > 0) {
             if ((bit & r.pe_mask) && du != 0.f) {
                 const int k = off / 32;
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    if (al.comp[2 * k + e] != 2) continue;
-                    const float v = e == 0 ? du : -du;
-                    if (p.pe_cells) atomicAdd(r.pacc + dist * p.npe + al.elem[2 * k + e], v);
-                    else atomicAdd(p.dPE + ((size_t)dist * p.n_detectors + r.t) * p.npe + al.elem[2 * k + e], v);
+                    if (al.comp[2 * k + e] == 2)
+                        add_positional(p, r.pacc, dist, r.t, al.elem[2 * k + e], e == 0 ? du : -du);
                 }
             }
         }
@@ -441,10 +466,9 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
 }
 
 template <int MAXKQ, bool EPS>
-__global__ void __launch_bounds__(32 * kRouteWarps) product_route_kernel(const RouteArgs p) {
+__global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_route_kernel(const RouteArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
-    __shared__ float4 qstate[kTileQ];
     const int t = blockIdx.x;
     const int k0 = blockIdx.y * kRouteKeys;
     const int64_t bl = blockIdx.z, b = p.b0 + bl;
@@ -506,17 +530,19 @@ __global__ void __launch_bounds__(32 * kRouteWarps) product_route_kernel(const R
     }
 
     RouteTile r;
-    r.smem = smem; r.Qs = Qs; r.qd = qd; r.xk = xk; r.qv = qv; r.qstate = qstate;
+    r.smem = smem; r.Qs = Qs; r.qd = qd; r.xk = xk; r.qv = qv;
     r.x2b = p.x2 + (size_t)b * S * p.e2;
     r.pe_t = p.pe + (size_t)t * p.npe;
     r.pe_stride = p.n_detectors * p.npe;
     r.kcol = kcol; r.pacc = pacc; r.ex = ex;
     r.i = i; r.ikey = ikey; r.n_pe = n_pe; r.t = t;
-    r.pe_mask = al.pe_mask; r.kbits = kbits; r.kmin = kmin;
+    r.pe_mask = al.pe_mask;
+    r.kbits = kbits; r.kmin = kmin;
     const float *Qt = p.Q + (size_t)t * p.q_det_stride + (size_t)bl * S * p.q_row_stride;
+    __syncthreads();
     for (int j0 = k0 + 1; j0 < S; j0 += kTileQ) {
         const int nq = min(kTileQ, S - j0);
-        __syncthreads();   // the previous eight queries' tiles are free
+        // (every warp has passed the barrier behind the previous tile's pairs: its operands are free)
         for (int w = threadIdx.x; w < nq * (T / 4); w += blockDim.x) {
             const int q = w >> (Nc - 2), c = w & (T / 4 - 1);
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Qs + w * 4);
@@ -536,26 +562,27 @@ __global__ void __launch_bounds__(32 * kRouteWarps) product_route_kernel(const R
                 if (dist >= 0 && dist < S - 1) pew[m * kRouteWindow + w] = __ldg(r.pe_t + (size_t)dist * r.pe_stride + al.elem[end]);
             }
         }
-        __syncthreads();   // the staged deltas are there
-        if (threadIdx.x < kTileQ) {
-            const int q = threadIdx.x;
-            uint32_t bits = 0u;
-            unsigned long long best = margin_key(kFltMax, 0u);
-            for (uint32_t left = al.query_only; left; left &= left - 1) {
-                const int k = __ffs(left) - 1;
-                const float d = qd[q * kHistAnchors + k];
-                if (greater_than_zero(d, p.cmp_eps)) bits |= 1u << k;
-                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(1u << k, d));
-                best = c < best ? c : best;
-            }
-            qstate[q] = make_float4(__uint_as_float(bits), __uint_as_float((uint32_t)(best >> 32)), __uint_as_float((uint32_t)best), 0.f);
-        }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         if (k0 + warp * 32 < j0 + nq - 1) {   // (otherwise no key of this warp lies below any of the queries)
             r.j0 = j0;
-            if (EPS || n_pe > 0) route_tile<MAXKQ, true, EPS, MAXKQ>(p, al, r, kv);
-            else if (n_kq <= 2) route_tile<2, false, EPS, MAXKQ>(p, al, r, kv);
+            r.qbits = 0u;
+            unsigned long long best = margin_key(kFltMax, 0u);
+            if (lane < kTileQ) {
+                for (uint32_t left = al.query_only; left; left &= left - 1) {
+                    const int k = __ffs(left) - 1;
+                    const float d = qd[lane * kHistAnchors + k];
+                    if (greater_than_zero(d, p.cmp_eps)) r.qbits |= 1u << k;
+                    const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(1u << k, d));
+                    best = c < best ? c : best;
+                }
+            }
+            r.qmd = __uint_as_float((uint32_t)(best >> 32));
+            r.qlow = (uint32_t)best;
+            if (EPS || n_pe > 0) {
+                if (MAXKQ > 8 && !EPS && n_kq <= 6) route_tile<6, true, EPS, MAXKQ>(p, al, r, kv);
+                else route_tile<MAXKQ, true, EPS, MAXKQ>(p, al, r, kv);
+            } else if (n_kq <= 2) route_tile<2, false, EPS, MAXKQ>(p, al, r, kv);
             else if (n_kq <= 4) route_tile<4, false, EPS, MAXKQ>(p, al, r, kv);
             else if (n_kq <= 6) route_tile<6, false, EPS, MAXKQ>(p, al, r, kv);
             else route_tile<MAXKQ, false, EPS, MAXKQ>(p, al, r, kv);
