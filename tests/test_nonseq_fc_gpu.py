@@ -269,3 +269,26 @@ def test_input_gradient_kernel_splits(B, I, Nt, Nc, O):
             golden_util.assert_close(got, want, 1e-5, "dX")
         if B < 10000:
             golden_util.assert_close(gW.cpu().numpy(), dW.reshape(-1), 1e-5, "dW")
+
+
+@pytest.mark.parametrize("O", [1, 2, 3, 7, 10, 17, 31, 33, 45, 63, 65, 130, 4, 36, 132])
+def test_forward_gather_widths(O):
+    """Rows of every lane group, one and two columns a lane, several column chunks, aligned and not; detectors that end
+    inside a group of 32."""
+    from spiky_b200.lut_data_manager import LUTDataManagerF
+
+    B, I, Nt, Nc = 21, 40, 37, 4
+    x = synth.normal(980, (B, I))
+    anchors = synth.anchor_pairs(981, Nt, Nc, I)
+    W = synth.normal(982, (Nt * (1 << Nc) * O,), 0.0, 0.05)
+    want, idx, md, mk = orc.nonseq_fc_forward(W, x, anchors, Nt, Nc, O)
+    dm = LUTDataManagerF(I, O, Nt, Nc, 1, 0, 0, 32, 32)
+    dm.register_synapse_meta(1.0, -1.0, 1.0, 0.0, 0.0)
+    dm.initialize_neurons(True)
+    dm.to_device(0)
+    y = torch.zeros(B * O, device="cuda")
+    ti = torch.empty(B * Nt, dtype=torch.int32, device="cuda")
+    dm.forward_step(torch.from_numpy(W).cuda(), B, torch.from_numpy(x).reshape(-1).cuda(),
+                    torch.from_numpy(anchors).reshape(-1).cuda(), y, ti)
+    assert np.array_equal(ti.cpu().numpy(), idx.reshape(-1))
+    golden_util.assert_close(y.cpu().numpy().reshape(B, O), want, 1e-5, "y")
