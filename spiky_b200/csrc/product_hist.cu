@@ -325,6 +325,7 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
 // gave 8 % at 128 tokens; a per-warp window of distances for dPE instead of an add per pair cost 20 % there.
 // --------------------------------------------------------------------------------------------
 constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
+constexpr int kRouteQueries = 256; // queries of one block
 constexpr int kExLd = 33;          // leading dimension of the (query, key) exchange tile
 
 struct RouteArgs {
@@ -363,7 +364,7 @@ struct RouteTile {
     const float2 *qv;
     float *kcol, *pacc;
     float2 *ex;
-    int j0, i, ikey, n_pe, pe_stride, t;
+    int j0, j_end, i, ikey, n_pe, pe_stride, t;
     uint32_t pe_mask, kbits;
     unsigned long long kmin;
     // lane q < kTileQ: the query-only anchors of query j0 + q
@@ -416,7 +417,7 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
             const unsigned long long mixed = margin_key(md, low);
             best = mixed < best ? mixed : best;
         }
-        const bool pair = r.i < j && j < p.S;
+        const bool pair = r.i < j && j < r.j_end;
         const int dist = max(0, min(j, p.S - 1) - r.i - 1);
         if (PE && r.n_pe > 0) {
             {
@@ -470,7 +471,11 @@ __global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
     const int t = blockIdx.x;
-    const int k0 = blockIdx.y * kRouteKeys;
+    // blockIdx.y: (segment of kRouteQueries queries, key range); the later key ranges have fewer segments
+    const int n_ranges = (p.S - 1 + kRouteKeys - 1) / kRouteKeys;
+    const int seg = blockIdx.y / n_ranges, k0 = (blockIdx.y - seg * n_ranges) * kRouteKeys;
+    const int j_begin = k0 + 1 + seg * kRouteQueries, j_end = min(p.S, j_begin + kRouteQueries);
+    if (j_begin >= p.S) return;
     const int64_t bl = blockIdx.z, b = p.b0 + bl;
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,13 +540,14 @@ __global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_
     r.pe_t = p.pe + (size_t)t * p.npe;
     r.pe_stride = p.n_detectors * p.npe;
     r.kcol = kcol; r.pacc = pacc; r.ex = ex;
+    r.j_end = j_end;
     r.i = i; r.ikey = ikey; r.n_pe = n_pe; r.t = t;
     r.pe_mask = al.pe_mask;
     r.kbits = kbits; r.kmin = kmin;
     const float *Qt = p.Q + (size_t)t * p.q_det_stride + (size_t)bl * S * p.q_row_stride;
     __syncthreads();
-    for (int j0 = k0 + 1; j0 < S; j0 += kTileQ) {
-        const int nq = min(kTileQ, S - j0);
+    for (int j0 = j_begin; j0 < j_end; j0 += kTileQ) {
+        const int nq = min(kTileQ, j_end - j0);
         // (every warp has passed the barrier behind the previous tile's pairs: its operands are free)
         for (int w = threadIdx.x; w < nq * (T / 4); w += blockDim.x) {
             const int q = w >> (Nc - 2), c = w & (T / 4 - 1);
@@ -1086,7 +1092,9 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             ra.n_detectors = Nt; ra.n_anchors = cfg->n_anchors; ra.sliced = cfg->sliced_product; ra.cmp_eps = cfg->cmp_eps;
             ra.pe_cap = pe_cap; ra.pe_cells = pe_cells;
             // (no block for the last key range when its first key is the last token: it has no query)
-            dim3 grid((unsigned)Nt, (unsigned)((c.S - 1 + kRouteKeys - 1) / kRouteKeys), (unsigned)n);
+            const int ranges = (c.S - 1 + kRouteKeys - 1) / kRouteKeys, segs = (c.S - 1 + kRouteQueries - 1) / kRouteQueries;
+            LUTB_REQUIRE((int64_t)ranges * segs <= 65535, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
+            dim3 grid((unsigned)Nt, (unsigned)(ranges * segs), (unsigned)n);
             KernelScope scope(K_PRODUCT_ROUTE, stream);
             auto launch = [&](auto kern) -> int {
                 if (route_smem > 48 * 1024)
