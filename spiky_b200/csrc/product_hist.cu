@@ -96,7 +96,7 @@ __device__ __forceinline__ void positional_ends(const AnchorLists &al, const flo
 
 // --------------------------------------------------------------------------------------------
 // Row-selection histogram: for every query (b, j) and detector t, how many of the j keys select each of the T rows.
-// Block = (detector, 128 queries, sequence); what the pairs need of the keys is staged once, then the warps work on their
+// Block = (detector, 32 to 128 queries, sequence); what the pairs need of the keys is staged once, then the warps work on their
 // own: a warp takes four queries at a time, counts in a private shared-memory array and writes it out.  LANE = KEY: the
 // key ends of 32 keys are in registers while the warp walks its queries, whose operands (two anchors' query ends and
 // bits per 16-byte load) are the same for all lanes; a key-query anchor then costs a compare and a predicated OR.  The
@@ -110,7 +110,7 @@ __device__ __forceinline__ void positional_ends(const AnchorLists &al, const flo
 // of one query, the anchors' operands read from shared memory for every pair): 64 sequences x 128 tokens, 64 detectors of
 // 256 rows 271 -> 182 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 187 us.
 // --------------------------------------------------------------------------------------------
-constexpr int kHistQueries = 128, kHistTile = 4;
+constexpr int kHistTile = 4;
 
 struct HistArgs {
     const float *x1, *x2, *pe;
@@ -120,6 +120,7 @@ struct HistArgs {
     int S, e1, e2, npe, n_detectors, n_anchors, sliced;
     float cmp_eps;
     int pe_cap;      // anchors with a positional end whose operands are staged in shared memory
+    int queries;     // of one block
 };
 
 // dynamic shared memory of one block, in floats: per warp counters and query operands | key ends | key bits | positional operands
@@ -187,10 +188,10 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
     const int t = blockIdx.x;
-    const int j_begin = (gridDim.y - 1 - blockIdx.y) * kHistQueries;   // the ranges with the most keys first
+    const int j_begin = (gridDim.y - 1 - blockIdx.y) * p.queries;   // the ranges with the most keys first
     const int64_t bl = blockIdx.z, b = p.b0 + bl;
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc, Sp = (S + 31) & ~31;
-    const int j_end = min(S, j_begin + kHistQueries);
+    const int j_end = min(S, j_begin + p.queries);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int words = PACKED ? T / 2 : T;
     const size_t per_warp = hist_warp_floats(T, PACKED);
@@ -320,12 +321,11 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
 // the warp reads back with the lanes over queries, again into private columns; the block adds the columns up once per
 // eight queries. 
 // Measured (before: a warp per query, about 600 instructions per 32 pairs): 64 sequences x 128 tokens, 64 detectors of 256
-// rows 862 -> 440 us (323 without positional anchors); 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 832 us (590
-// without: the blocks of the few detectors with such an anchor end last).  Two barriers per eight queries instead of four
+// rows 862 -> 440 us (323 without positional anchors); 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 410 us (851 before a
+// block's queries were limited).  Two barriers per eight queries instead of four
 // gave 8 % at 128 tokens; a per-warp window of distances for dPE instead of an add per pair cost 20 % there.
 // --------------------------------------------------------------------------------------------
 constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
-constexpr int kRouteQueries = 256; // queries of one block
 constexpr int kExLd = 33;          // leading dimension of the (query, key) exchange tile
 
 struct RouteArgs {
@@ -338,6 +338,7 @@ struct RouteArgs {
     float cmp_eps;
     int pe_cap;      // anchors with a positional end whose operands are staged in shared memory
     int pe_cells;    // 1: the block sums dPE in shared memory
+    int queries;     // of one block
 };
 
 // dynamic shared memory of one block, in floats: Q rows | query operands | per-warp columns and exchange tile | staged
@@ -471,10 +472,10 @@ __global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
     const int t = blockIdx.x;
-    // blockIdx.y: (segment of kRouteQueries queries, key range); the later key ranges have fewer segments
+    // blockIdx.y: (segment of p.queries queries, key range); the later key ranges have fewer segments
     const int n_ranges = (p.S - 1 + kRouteKeys - 1) / kRouteKeys;
     const int seg = blockIdx.y / n_ranges, k0 = (blockIdx.y - seg * n_ranges) * kRouteKeys;
-    const int j_begin = k0 + 1 + seg * kRouteQueries, j_end = min(p.S, j_begin + kRouteQueries);
+    const int j_begin = k0 + 1 + seg * p.queries, j_end = min(p.S, j_begin + p.queries);
     if (j_begin >= p.S) return;
     const int64_t bl = blockIdx.z, b = p.b0 + bl;
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc;
@@ -931,6 +932,24 @@ static int plan(const ProductCall &c, bool backward, bool allow_tc, void *worksp
     return LUTB_OK;
 }
 
+// Queries of one block of the pair kernels: the most, up to 128, that still give every SM a dozen blocks, 32 at least.  Routing,
+// 64 detectors, 32 / 64 / 128 queries: 1 x 128 tokens 37 / 63 / 117 us, 8 x 128 86 / 91 / 136, 4 x 256 117 / 121 / 139, 64 x 128
+// 529 / 467 / 458, 1 x 1024 453 / 413 / 410 (with every query of a key range in one block 851).
+// key_range: keys of one block (a block has the queries above its first key); 0: all of them, as the histogram kernel has it: its
+// blocks stage every key below their queries first, so that long sequences keep 128 queries (1 x 1024 tokens 187 us with 128
+// queries, 352 with 32; 1 x 500 tokens 64 and 42 us; 1 x 128 tokens 26 and 14 us).
+static int queries_per_block(int S, int64_t detectors_times_sequences, int key_range) {
+    const int least = key_range == 0 && S > 512 ? 128 : 32;
+    for (int q = 128; q > least; q /= 2) {
+        int64_t blocks = 0;
+        if (key_range == 0) blocks = (S + q - 1) / q;
+        else
+            for (int k0 = 0; k0 < S - 1; k0 += key_range) blocks += (S - 1 - k0 + q - 1) / q;
+        if (blocks * detectors_times_sequences >= 12 * (int64_t)device_info().sm_count) return q;
+    }
+    return least;
+}
+
 static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int64_t n, cudaStream_t stream) {
     const lutb_layer_cfg *cfg = c.cfg;
     const size_t T = (size_t)1 << cfg->n_anchors;
@@ -942,7 +961,8 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     const bool packed = T > 512;
     // warps per block: what puts the most warps on an SM (a wide table's counters leave room for one block only, which then
     // has to bring them all); very long sequences leave the positional operands in global memory
-    const int tiles = ((c.S < kHistQueries ? c.S : kHistQueries) + kHistTile - 1) / kHistTile;
+    h.queries = queries_per_block(c.S, (int64_t)cfg->n_detectors * n, 0);
+    const int tiles = ((c.S < h.queries ? c.S : h.queries) + kHistTile - 1) / kHistTile;
     int warps = 0;
     for (int cap = staged_pe_anchors(cfg);; cap = 0) {
         int most = 0;
@@ -956,7 +976,7 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     }
     LUTB_REQUIRE(warps > 0, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
     const size_t smem = hist_floats(T, packed, warps, cfg->n_anchors, h.pe_cap, c.S) * 4;
-    dim3 grid((unsigned)cfg->n_detectors, (unsigned)((c.S + kHistQueries - 1) / kHistQueries), (unsigned)n);
+    dim3 grid((unsigned)cfg->n_detectors, (unsigned)((c.S + h.queries - 1) / h.queries), (unsigned)n);
     KernelScope scope(K_PRODUCT_HIST, stream);
     auto launch = [&](auto kern) -> int {
         if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1092,7 +1112,8 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             ra.n_detectors = Nt; ra.n_anchors = cfg->n_anchors; ra.sliced = cfg->sliced_product; ra.cmp_eps = cfg->cmp_eps;
             ra.pe_cap = pe_cap; ra.pe_cells = pe_cells;
             // (no block for the last key range when its first key is the last token: it has no query)
-            const int ranges = (c.S - 1 + kRouteKeys - 1) / kRouteKeys, segs = (c.S - 1 + kRouteQueries - 1) / kRouteQueries;
+            ra.queries = queries_per_block(c.S, (int64_t)Nt * n, kRouteKeys);
+            const int ranges = (c.S - 1 + kRouteKeys - 1) / kRouteKeys, segs = (c.S - 1 + ra.queries - 1) / ra.queries;
             LUTB_REQUIRE((int64_t)ranges * segs <= 65535, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
             dim3 grid((unsigned)Nt, (unsigned)(ranges * segs), (unsigned)n);
             KernelScope scope(K_PRODUCT_ROUTE, stream);
