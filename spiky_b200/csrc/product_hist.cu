@@ -319,10 +319,11 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
 // Sums: the key's cells are a private shared-memory column per lane (plain read-modify-write), flushed once per block.
 // The query's cells would collide (32 lanes, a few anchors), so a pair's (du, anchor) is parked in an 8 x 32 tile that
 // the warp reads back with the lanes over queries, again into private columns; the block adds the columns up once per
-// eight queries. 
+// eight queries.
 // Measured (before: a warp per query, about 600 instructions per 32 pairs): 64 sequences x 128 tokens, 64 detectors of 256
-// rows 862 -> 440 us (323 without positional anchors); 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 410 us (851 before a
-// block's queries were limited).  Two barriers per eight queries instead of four
+// rows 862 -> 490 us; 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 435 us (851 before a block's queries were limited).
+// The rounded reciprocal of the surrogate is 6 % of that (460 and 413 us with a refined hardware approximation, which gave
+// the same bits on what was tried).  Two barriers per eight queries instead of four
 // gave 8 % at 128 tokens; a per-warp window of distances for dPE instead of an add per pair cost 20 % there.
 // --------------------------------------------------------------------------------------------
 constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
@@ -442,12 +443,8 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
         const uint32_t low = (uint32_t)best, bit = EPS ? low >> 1 : low;
         const bool positive = EPS ? (low & 1u) != 0u : (li & bit) != 0u;
         // up(d) * (Q[row] - Q[flipped row]) in fp32: Q is an fp32 contraction already (the direct kernels and the
-        // fixed-point mode keep the double-precision reciprocal of the reference's formula).  One Newton step on the
-        // hardware's reciprocal is as close as the rounded one and needs no branch.
-        const float a = 1.0f + md;
-        float rc;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(a));
-        rc = fmaf(rc, fmaf(-a, rc, 1.0f), rc);
+        // fixed-point mode keep the double-precision reciprocal of the reference's formula)
+        const float rc = __frcp_rn(1.0f + md);
         const float *qrow = r.Qs + q * T;
         float du = (positive ? 0.5f : -0.5f) * rc * rc * (qrow[li] - qrow[li ^ bit]);
         du = pair && bit != 0u && fabsf(du) > kEpsF ? du : 0.f;

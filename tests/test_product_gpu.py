@@ -177,6 +177,29 @@ def test_product_contractions_on_pairs_of_sms():
         golden_util.assert_close(got[k], want[k], REL, k)
 
 
+def test_routing_surrogate_is_the_rounded_formula():
+    """One pair per sequence whose contraction is exact: the routed gradient is 0.5 * r * r with r the correctly rounded
+    fp32 reciprocal of 1 + |delta|, bit for bit, from the smallest margins to those whose reciprocal is subnormal."""
+    B = 4096
+    rng = np.random.default_rng(9)
+    d = np.exp2(rng.uniform(-24.0, 24.0, B)).astype(np.float32) * rng.choice([-1, 1], B).astype(np.float32)
+    d[:8] = [0.0, 1e-30, -1.0, 1.0, 3.0, -1e17, 2.0 ** 126, -3.3e38]
+    cfg = dict(E=2, Nt=1, Nc=4, O=4, S=2, Npe=0)
+    anchors = np.full((1, 4, 2), -1, np.int32)
+    anchors[0, 0] = (0, 2)          # key's element 0 against the query's
+    W = np.zeros((16, 4), np.float32)
+    W[1, 0] = 1.0
+    x, dY = np.zeros((B, 2, 2), np.float32), np.zeros((B, 2, 4), np.float32)
+    x[:, 0, 0] = d
+    dY[:, 1, 0] = 1.0
+    for variant in (2, 3):
+        got = run_gpu(cfg, x, anchors, W.reshape(-1), None, dY, variant)["dX"].reshape(B, 2, 2)
+        r = np.float32(1) / (np.float32(1) + np.abs(d))
+        want = np.float32(0.5) * r * r
+        want[want <= np.float32(1e-17)] = 0.0
+        assert np.array_equal(got[:, 0, 0], want) and np.array_equal(got[:, 1, 0], -want)
+
+
 def test_product_histogram_rejects_unsupported():
     cfg = dict(seed=711, B=1, S=4, E=6, Nt=2, Nc=3, Npe=2, O=4, n_virtual=14)
     x, anchors, W, pe, dY = inputs_for(cfg)
