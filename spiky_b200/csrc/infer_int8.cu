@@ -162,7 +162,7 @@ extern "C" int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t 
     int rc = validate_cfg(cfg);
     if (rc) return rc;
     const bool staged = workspace != nullptr && batch > 0 && dequant == LUTB_INT8_DEQUANT_EXACT &&
-                        infer_staged_int8_applies(cfg, q_tables);
+                        infer_staged_int8_applies(cfg, q_tables) && infer_staged_pass(cfg, batch, true) > 0;
     if (!staged) return lutb_infer_int8_accumulate(cfg, batch, q_tables, scales, x, anchors, acc, idx, dequant, stream);
     LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "int8 inference is defined for non-sequence layers");
     LUTB_REQUIRE(q_tables && scales && x && anchors && acc && idx, LUTB_ERR_NULL, "a required tensor pointer is NULL");
@@ -171,9 +171,9 @@ extern "C" int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t 
     LUTB_REQUIRE(workspace_bytes >= need, LUTB_ERR_WORKSPACE, "the staged gather needs %zu bytes of workspace", need);
     LUTB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, LUTB_ERR_ALIGN, "workspace must be 256-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t pass = infer_staged_pass(batch);
+    const int64_t pass = infer_staged_pass(cfg, batch, true);
     uint8_t *packed = static_cast<uint8_t *>(workspace);
-    void *plan = packed + packed_index_bytes(cfg, batch);
+    void *plan = packed + packed_index_bytes(cfg, pass);
     rc = launch_int8_scale_plan(cfg, scales, plan, st);
     if (rc) return rc;
     for (int64_t b0 = 0; b0 < batch; b0 += pass) {

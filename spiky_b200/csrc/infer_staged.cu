@@ -331,7 +331,10 @@ __global__ void __launch_bounds__(kStagedThreads, 1) infer_staged_int8_kernel(co
 // ------------------------------------------------------------------------------------------ rules and launches
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-constexpr int64_t kPassSamples = 16384;   // bounds the workspace; every pass reads the tables once more from DRAM
+// A pass takes as many samples as a workspace of kPassBytes (packed indices and partial sums) and kPassSamples allow, in whole
+// tiles; every pass reads the tables once more.  Where not even one tile fits, the plain gather runs.  The bound lets
+// the 16384 samples of 4096 detectors x 64 outputs (784 MB) through in one pass.
+constexpr int64_t kPassSamples = 16384, kPassBytes = 800ll << 20;
 
 // Where the staged gather is the better one (indices included; staged / plain, us).  Rows of 32 outputs or fewer leave lanes
 // idle here while the plain gather's chains get short, and more exact: they stay there.  fp32, from 512 detectors on, any
@@ -341,15 +344,25 @@ constexpr int64_t kPassSamples = 16384;   // bounds the workspace; every pass re
 constexpr int kMinOutputs = 33, kMinDetectorsFp32 = 512, kMinDetectorsInt8 = 1024;
 
 size_t packed_index_pitch(int64_t batch) { return (size_t)((batch + kTile - 1) / kTile * kTile); }
-int64_t infer_staged_pass(int64_t batch) { return batch < kPassSamples ? batch : kPassSamples; }
-size_t packed_index_bytes(const lutb_layer_cfg *cfg, int64_t batch) {
-    return align256(packed_index_pitch(infer_staged_pass(batch)) * cfg->n_detectors);
+
+static int det_blocks(int Nt) { return (Nt + kDetBlock - 1) / kDetBlock; }
+static int trunc_blocks(const lutb_layer_cfg *cfg) { return (cfg->n_detectors + cfg->backward_group - 1) / cfg->backward_group; }
+
+// bytes of the partial sums of one sample
+static int64_t partial_bytes(const lutb_layer_cfg *cfg, bool int8) { return int8 ? 0 : (int64_t)det_blocks(cfg->n_detectors) * cfg->n_outputs * 4; }
+
+// samples of one pass (batch or a multiple of kTile, the passes of one call nearly equal); 0: one tile is too much
+int64_t infer_staged_pass(const lutb_layer_cfg *cfg, int64_t batch, bool int8) {
+    int64_t most = kPassBytes / (cfg->n_detectors + partial_bytes(cfg, int8)) / kTile * kTile;
+    if (most > kPassSamples) most = kPassSamples;
+    if (most == 0 || batch <= most) return most == 0 ? 0 : batch;
+    const int64_t passes = (batch + most - 1) / most, each = (batch + passes - 1) / passes;
+    return (each + kTile - 1) / kTile * kTile;
 }
+size_t packed_index_bytes(const lutb_layer_cfg *cfg, int64_t pass) { return align256(packed_index_pitch(pass) * cfg->n_detectors); }
 
 static size_t smem_fp32(int T) { return (size_t)kStages * 2 * ((size_t)T * kRow * 4 + kTile); }
 static size_t smem_int8(int T) { return (size_t)kStages * kDets8 * ((size_t)T * kCols8 + kTile8 + 8); }
-static int det_blocks(int Nt) { return (Nt + kDetBlock - 1) / kDetBlock; }
-static int trunc_blocks(const lutb_layer_cfg *cfg) { return (cfg->n_detectors + cfg->backward_group - 1) / cfg->backward_group; }
 
 bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, const void *weights, const void *y) {
     const int O = cfg->n_outputs;
@@ -364,10 +377,12 @@ bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, const void *q_tables) 
 }
 
 size_t infer_staged_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
-    return packed_index_bytes(cfg, batch) + align256((size_t)det_blocks(cfg->n_detectors) * infer_staged_pass(batch) * cfg->n_outputs * 4) + 256;
+    const int64_t pass = infer_staged_pass(cfg, batch, false);
+    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256((size_t)(pass * partial_bytes(cfg, false))) + 256;
 }
 size_t infer_staged_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
-    return packed_index_bytes(cfg, batch) + align256(scale_plan_bytes(cfg->n_detectors, trunc_blocks(cfg))) + 256;
+    const int64_t pass = infer_staged_pass(cfg, batch, true);
+    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256(scale_plan_bytes(cfg->n_detectors, trunc_blocks(cfg))) + 256;
 }
 
 int launch_infer_staged_fp32(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const uint8_t *packed, float *partial,

@@ -910,7 +910,8 @@ extern "C" int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t bat
                                           size_t workspace_bytes, void *stream) {
     int rc = validate_cfg(cfg);
     if (rc) return rc;
-    const bool staged = workspace != nullptr && batch > 0 && infer_staged_fp32_applies(cfg, weights, y);
+    const bool staged = workspace != nullptr && batch > 0 && infer_staged_fp32_applies(cfg, weights, y) &&
+                        infer_staged_pass(cfg, batch, false) > 0;
     if (!staged) return lutb_nonseq_fc_forward(cfg, batch, weights, x, anchors, y, idx, nullptr, nullptr, stream);
     LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "inference is defined for non-sequence layers");
     LUTB_REQUIRE(weights && x && anchors && y && idx, LUTB_ERR_NULL, "a required tensor pointer is NULL");
@@ -918,9 +919,9 @@ extern "C" int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t bat
     LUTB_REQUIRE(workspace_bytes >= need, LUTB_ERR_WORKSPACE, "the staged gather needs %zu bytes of workspace", need);
     LUTB_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, LUTB_ERR_ALIGN, "workspace must be 256-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t pass = infer_staged_pass(batch);
+    const int64_t pass = infer_staged_pass(cfg, batch, false);
     uint8_t *packed = static_cast<uint8_t *>(workspace);
-    float *partial = reinterpret_cast<float *>(packed + packed_index_bytes(cfg, batch));
+    float *partial = reinterpret_cast<float *>(packed + packed_index_bytes(cfg, pass));
     for (int64_t b0 = 0; b0 < batch; b0 += pass) {
         const int64_t n = batch - b0 < pass ? batch - b0 : pass;
         rc = launch_check_detectors(x + b0 * cfg->n_inputs, n, cfg->n_inputs, anchors, cfg->n_detectors, cfg->n_anchors, cfg->cmp_eps,

@@ -83,7 +83,12 @@ class LUTInference:
         cfg = ctypes.byref(self.cfg)
         with torch.cuda.device(self.device):
             need = L.lutb_infer_int8_workspace(cfg, B, self.dequant) if self.int8 else L.lutb_infer_fp32_workspace(cfg, B)
-            ws = torch.empty(need, dtype=torch.uint8, device=self.device) if need else None
+            ws = None
+            if need:
+                try:
+                    ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+                except torch.OutOfMemoryError:
+                    need = 0   # the plain gather needs none
             if self.int8:
                 acc = torch.zeros(B * self.O, dtype=torch.int32, device=self.device)
                 rc = L.lutb_infer_int8_accumulate_ws(cfg, B, _ptr(self.tables), _ptr(self.scales), _ptr(x.view(-1)),

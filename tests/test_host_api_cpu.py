@@ -101,3 +101,24 @@ def test_quantize_tables_is_symmetric_per_table():
         LUTInference.shard_of(0, 3, 16, 4, 64, 3, anchors, tables)          # 64 detectors over 3 ranks
     with pytest.raises(AssertionError):
         LUTInference.shard_of(0, 4, 16, 4, 64, 3, anchors, tables)          # 16 per rank, blocks of 32
+
+
+def test_staged_inference_workspace_is_bounded():
+    """Any layer and batch: at most 800 MB and what a 1 GB layer's indices and scales round up to; none where not even one
+    tile of samples fits (the plain gather runs there)."""
+    import ctypes
+    from spiky_b200 import _native
+
+    L = _native.lib()
+    seen = set()
+    for Nt in (512, 1024, 4096, 16384, 1 << 20):
+        for O in (36, 64, 256, 1024, 4096, 16384):
+            for B in (1, 1000, 1024, 16384, 16385, 1 << 20):
+                cfg = _native.LayerCfg(n_inputs=64, n_outputs=O, n_detectors=Nt, n_anchors=4, seq_len=1, pos_dim=0,
+                                       forward_group=32, backward_group=32, int_mode=0, sliced_product=0, cmp_eps=0.0,
+                                       reserved0=0.0, int_rescaler=1.0, lr_meta=1.0)
+                for need in (L.lutb_infer_fp32_workspace(ctypes.byref(cfg), B),
+                             L.lutb_infer_int8_workspace(ctypes.byref(cfg), B, 1)):
+                    assert need <= (800 << 20) + 16 * Nt + 4096
+                    seen.add(need > 0)
+    assert seen == {False, True}

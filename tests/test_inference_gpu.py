@@ -140,3 +140,29 @@ def test_staged_int8_inference_is_bit_exact(shape):
     want, ridx = orc.infer_int8(q, s, x, anchors, Nt, Nc, O, backward_group_size=blk, int_rescaler=0.05, exact=True)
     assert np.array_equal(layer.last_indices.cpu().numpy(), ridx)
     assert np.array_equal(acc, want)
+
+
+def test_staged_fp32_inference_in_several_passes(monkeypatch):
+    """More partial sums than one pass may hold: passes of 1024 samples, the last one short; the plain gather (the way out
+    when the workspace cannot be had) agrees."""
+    import ctypes
+    from spiky_b200 import _native
+    from spiky_b200.inference import LUTInference
+
+    B, I, Nt, Nc, O = 2100, 20, 512, 1, 5000
+    x = torch.from_numpy(synth.normal(951, (B, I))).cuda()
+    W = torch.from_numpy(synth.normal(952, (Nt * 2 * O,), 0.0, 0.02))
+    layer = LUTInference(I, O, Nt, Nc, torch.from_numpy(synth.anchor_pairs(953, Nt, Nc, I)), W)
+    need = _native.lib().lutb_infer_fp32_workspace(ctypes.byref(layer.cfg), B)
+    assert need == _native.lib().lutb_infer_fp32_workspace(ctypes.byref(layer.cfg), 1024) > 0
+    staged, idx = layer(x), layer.last_indices
+    empty = torch.empty
+
+    def no_workspace(*a, **k):
+        if k.get("dtype") is torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*a, **k)
+    monkeypatch.setattr(torch, "empty", no_workspace)
+    plain = layer(x)
+    assert torch.equal(idx, layer.last_indices)
+    golden_util.assert_close(staged.cpu().numpy(), plain.cpu().numpy(), 1e-5, "y")
