@@ -151,7 +151,7 @@ extern "C" int lutb_infer_int8_accumulate(const lutb_layer_cfg *cfg, int64_t bat
 
 extern "C" size_t lutb_infer_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch, int dequant) {
     if (validate_cfg(cfg) != LUTB_OK || batch <= 0 || dequant != LUTB_INT8_DEQUANT_EXACT) return 0;
-    if (!infer_staged_int8_applies(cfg, reinterpret_cast<const void *>((uintptr_t)256))) return 0;
+    if (!infer_staged_int8_applies(cfg, batch, reinterpret_cast<const void *>((uintptr_t)256))) return 0;
     return infer_staged_int8_workspace(cfg, batch);
 }
 
@@ -162,7 +162,7 @@ extern "C" int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t 
     int rc = validate_cfg(cfg);
     if (rc) return rc;
     const bool staged = workspace != nullptr && batch > 0 && dequant == LUTB_INT8_DEQUANT_EXACT &&
-                        infer_staged_int8_applies(cfg, q_tables) && infer_staged_pass(cfg, batch, true) > 0;
+                        infer_staged_int8_applies(cfg, batch, q_tables) && infer_staged_pass(cfg, batch, true) > 0;
     if (!staged) return lutb_infer_int8_accumulate(cfg, batch, q_tables, scales, x, anchors, acc, idx, dequant, stream);
     LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "int8 inference is defined for non-sequence layers");
     LUTB_REQUIRE(q_tables && scales && x && anchors && acc && idx, LUTB_ERR_NULL, "a required tensor pointer is NULL");

@@ -336,12 +336,30 @@ static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 // the 16384 samples of 4096 detectors x 64 outputs (784 MB) through in one pass.
 constexpr int64_t kPassSamples = 16384, kPassBytes = 800ll << 20;
 
-// Where the staged gather is the better one (indices included; staged / plain, us).  Rows of 32 outputs or fewer leave lanes
-// idle here while the plain gather's chains get short, and more exact: they stay there.  fp32, from 512 detectors on, any
-// batch: 4096 detectors x 256 rows x 64 outputs 132 / 396 at 16 samples, 181 / 857 at 1024, 503 / 949 at 4096, 1650 / 2395 at
-// 16384; 512 detectors 42 / 56, 46 / 63, 89 / 87, 216 / 245.  int8, from 1024 detectors on: 4096 detectors 56 / 245, 183 / 318,
-// 540 / 812, 1857 / 2440; 1024 detectors 50 / 68, 67 / 81, 175 / 194, 499 / 585; 512 detectors 48 / 40, 60 / 44, 95 / 103, 300 / 298.
+// Where the staged gather is the better one (indices included; staged / plain, us).  A staged tile costs the same whether it
+// is full or holds one sample, and grows with detectors x outputs; the plain gather pays for each sample's rows, in more blocks
+// at once the wider they are, and for tables beyond L2.
+// fp32, from 512 detectors on: 4096 detectors x 256 rows x 64 outputs 132 / 396 at 16 samples, 181 / 857 at 1024, 503 / 949 at
+// 4096, 1650 / 2395 at 16384; 512 detectors 42 / 56, 46 / 63, 89 / 87, 216 / 245.  Rows of 32 outputs or fewer leave lanes idle
+// here while the plain gather's chains get short, and more exact: they stay there; 36 outputs (two slices, the second nearly
+// empty) 46 / 93 at 1 sample, 134 / 146 at 4096 with 1024 detectors.  Wide rows, few samples: 1024 detectors x 256 rows x 1024
+// outputs, 1 sample 245 / 204, 64 samples 254 / 338; 512 detectors x 4096 outputs 435 / 107 at 1 sample, 452 / 370 at 256;
+// 256 outputs 64 / 58 and 64 / 97 at 1 and 256 samples with 512 detectors, 93 / 107 at 1 sample with 1024.  Tables in L2: 512
+// detectors x 16 rows x 512 outputs 71 / 58 at 256 samples.  A little more than one wave of work items is as slow as two: 512
+// detectors x 36 outputs x 4096 samples 91 / 81.
+// int8, from 1024 detectors on: 4096 detectors x 64 outputs 56 / 245, 183 / 318, 540 / 812, 1857 / 2440; 1024 detectors 50 / 68,
+// 67 / 81, 175 / 194, 499 / 585; 512 detectors 48 / 40, 60 / 44, 95 / 103, 300 / 298.  1024 detectors x 1024 outputs 101 / 87 at
+// 1 sample, 108 / 114 at 8; x 4096 outputs 253 / 87 and 265 / 181 at 1 and 64.
 constexpr int kMinOutputs = 33, kMinDetectorsFp32 = 512, kMinDetectorsInt8 = 1024;
+
+static bool staged_fp32_pays(int64_t batch, int Nt, int T, int O) {
+    const int64_t sm = device_info().sm_count;
+    const int64_t items = (int64_t)((Nt + kDetBlock - 1) / kDetBlock) * ((batch + kTile - 1) / kTile) * ((O + kRow - 1) / kRow);
+    if (Nt < 1024 && batch > kTile && items > sm && 2 * items < 3 * sm) return false;
+    if (batch >= 512 || O <= (Nt < 1024 ? 128 : 256)) return true;
+    return O <= 1024 && batch >= (Nt < 1024 ? 128 : 32) && (int64_t)Nt * T >= 65536;
+}
+static bool staged_int8_pays(int64_t batch, int O) { return O <= 512 || batch >= 256 || (O <= 1024 && batch >= 8); }
 
 size_t packed_index_pitch(int64_t batch) { return (size_t)((batch + kTile - 1) / kTile * kTile); }
 
@@ -364,16 +382,16 @@ size_t packed_index_bytes(const lutb_layer_cfg *cfg, int64_t pass) { return alig
 static size_t smem_fp32(int T) { return (size_t)kStages * 2 * ((size_t)T * kRow * 4 + kTile); }
 static size_t smem_int8(int T) { return (size_t)kStages * kDets8 * ((size_t)T * kCols8 + kTile8 + 8); }
 
-bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, const void *weights, const void *y) {
+bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *weights, const void *y) {
     const int O = cfg->n_outputs;
     if (cfg->int_mode || cfg->n_anchors > 8 || O % 4 != 0 || O < kMinOutputs) return false;
     if (((reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(y)) & 15) != 0) return false;
-    return cfg->n_detectors >= kMinDetectorsFp32;
+    return cfg->n_detectors >= kMinDetectorsFp32 && staged_fp32_pays(batch, cfg->n_detectors, 1 << cfg->n_anchors, O);
 }
 
-bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, const void *q_tables) {
+bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *q_tables) {
     if (cfg->n_anchors > 8 || cfg->n_outputs % 8 != 0 || cfg->n_outputs < kMinOutputs || (reinterpret_cast<uintptr_t>(q_tables) & 7) != 0) return false;
-    return cfg->n_detectors >= kMinDetectorsInt8;
+    return cfg->n_detectors >= kMinDetectorsInt8 && staged_int8_pays(batch, cfg->n_outputs);
 }
 
 size_t infer_staged_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch) {

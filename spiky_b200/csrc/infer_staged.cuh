@@ -8,9 +8,9 @@ namespace lutb {
 // Row indices as the staged gathers read them: one byte per (detector, sample), detector-major, `pitch` bytes apart.
 size_t packed_index_pitch(int64_t batch);
 
-// Whether a layer takes the staged gather (the comments at the rules say where the lines lie).
-bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, const void *weights, const void *y);
-bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, const void *q_tables);
+// Whether a call takes the staged gather (the comments at the rules say where the lines lie).
+bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *weights, const void *y);
+bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *q_tables);
 
 // Samples of one pass (0: the staged gather does not run) and the workspace of a call: packed indices of a pass first
 // (packed_index_bytes), then the partial sums of the detector blocks (fp32) or the integer form of the scales (int8).

@@ -901,7 +901,7 @@ extern "C" int lutb_nonseq_fc_forward(const lutb_layer_cfg *cfg, int64_t batch, 
 
 extern "C" size_t lutb_infer_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
     const void *aligned = reinterpret_cast<const void *>((uintptr_t)256);
-    if (validate_cfg(cfg) != LUTB_OK || batch <= 0 || !infer_staged_fp32_applies(cfg, aligned, aligned)) return 0;
+    if (validate_cfg(cfg) != LUTB_OK || batch <= 0 || !infer_staged_fp32_applies(cfg, batch, aligned, aligned)) return 0;
     return infer_staged_fp32_workspace(cfg, batch);
 }
 
@@ -910,7 +910,7 @@ extern "C" int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t bat
                                           size_t workspace_bytes, void *stream) {
     int rc = validate_cfg(cfg);
     if (rc) return rc;
-    const bool staged = workspace != nullptr && batch > 0 && infer_staged_fp32_applies(cfg, weights, y) &&
+    const bool staged = workspace != nullptr && batch > 0 && infer_staged_fp32_applies(cfg, batch, weights, y) &&
                         infer_staged_pass(cfg, batch, false) > 0;
     if (!staged) return lutb_nonseq_fc_forward(cfg, batch, weights, x, anchors, y, idx, nullptr, nullptr, stream);
     LUTB_REQUIRE(cfg->seq_len == 1, LUTB_ERR_MODE, "inference is defined for non-sequence layers");

@@ -122,3 +122,27 @@ def test_staged_inference_workspace_is_bounded():
                     assert need <= (800 << 20) + 16 * Nt + 4096
                     seen.add(need > 0)
     assert seen == {False, True}
+
+
+def test_few_samples_of_a_wide_layer_take_the_plain_gather():
+    """A staged tile costs the same for one sample as for a full one: no workspace is asked for where the rows of the few
+    samples are the cheaper read; rows of the widths and batches the staged gather is for keep it."""
+    import ctypes
+    from spiky_b200 import _native
+
+    L = _native.lib()
+
+    def staged(kind, B, Nt, Nc, O):
+        cfg = _native.LayerCfg(n_inputs=64, n_outputs=O, n_detectors=Nt, n_anchors=Nc, seq_len=1, pos_dim=0,
+                               forward_group=32, backward_group=32, int_mode=0, sliced_product=0, cmp_eps=0.0,
+                               reserved0=0.0, int_rescaler=1.0, lr_meta=1.0)
+        need = (L.lutb_infer_fp32_workspace(ctypes.byref(cfg), B) if kind == "fp32"
+                else L.lutb_infer_int8_workspace(ctypes.byref(cfg), B, 1))
+        return need > 0
+
+    for args in (("fp32", 1, 512, 8, 4096), ("fp32", 256, 512, 8, 4096), ("fp32", 8, 1024, 8, 1024), ("fp32", 1, 512, 8, 256),
+                 ("fp32", 256, 512, 4, 512), ("int8", 1, 1024, 8, 1024), ("int8", 64, 1024, 8, 4096)):
+        assert not staged(*args), args
+    for args in (("fp32", 1, 4096, 8, 64), ("fp32", 16, 1024, 8, 256), ("fp32", 64, 1024, 8, 1024), ("fp32", 512, 512, 8, 4096),
+                 ("int8", 1, 4096, 8, 64), ("int8", 8, 1024, 8, 1024), ("int8", 256, 1024, 8, 4096)):
+        assert staged(*args), args
