@@ -37,10 +37,12 @@ __device__ __forceinline__ size_t concat_row(int32_t Q, int32_t K, int32_t PE, i
 }
 
 // --------------------------------------------------------------------------------------------
-// Pair order of the fp32 kernels.  Block = (detector, sample); a warp owns a "folded" query pair: queries
-// j = S - 1 - r and j = r have S - 1 keys together, so every unit of work has the same S - 1 pairs and 32 of them
-// fill a warp (walking one query at a time leaves half of the lanes without a key at 32 tokens).  A lane works out
-// one pair's table row; then the warp's lane groups of LG lanes (LG * VEC columns, a whole row where it fits) take the
+// Pair order of the fp32 kernels.  Block = (detector, sample); a warp owns a "folded" query pair: of the queries [j_begin,
+// j_end) (the whole sequence, or one rank's share when the queries are sharded) the r-th from the end and the r-th from the
+// start have j_begin + j_end - 1 keys together, so every unit of work has the same number of pairs, S - 1 for a whole
+// sequence, and 32 of them fill a warp (walking one query at a time leaves half of the lanes without a key at 32 tokens;
+// folding a share of the queries about the middle of the sequence leaves most units of a small share empty: 32 of 256 queries
+// of 4 sequences cost 117 us forward and 465 us backward).  A lane works out one pair's table row; then the warp's lane groups of LG lanes (LG * VEC columns, a whole row where it fits) take the
 // pairs of the 32 that belong to them, NG = 32 / LG pairs at a time, with the row loads of U pairs per group issued
 // before the first is used: the rows are random, so what bounds the kernel is how many of these reads are in flight.
 // Measured (32 sequences x 32 tokens, 64 detectors of 65536 rows x 32 outputs, 1.0 M pairs; lanes over the outputs of
@@ -49,18 +51,15 @@ __device__ __forceinline__ size_t concat_row(int32_t Q, int32_t K, int32_t PE, i
 // --------------------------------------------------------------------------------------------
 struct FoldedPair {
     int i, j;
-    bool first;   // belongs to query S - 1 - r (the longer of the two)
+    bool first;   // belongs to the longer query of the two
 };
-__device__ __forceinline__ FoldedPair folded_pair(int r, int p, int S) {
+__device__ __forceinline__ FoldedPair folded_pair(int ja, int jb, int p) {
     FoldedPair f;
-    const int ja = S - 1 - r;
     f.first = p < ja;
-    f.j = f.first ? ja : r;
+    f.j = f.first ? ja : jb;
     f.i = f.first ? p : p - ja;
     return f;
 }
-// number of pairs of folded query pair r: S - 1, or (the middle query of an odd length, alone) r
-__device__ __forceinline__ int folded_count(int r, int S) { return S - 1 - r == r ? r : S - 1; }
 
 template <int VEC>
 __device__ __forceinline__ void load_row(const float *p, bool on, float (&v)[VEC]) {
@@ -100,8 +99,9 @@ __global__ void __launch_bounds__(256) concat_forward_kernel(const float *__rest
     const int g = lane / LG, q = lane - g * LG;
     const size_t rows = (size_t)1 << (2 * nc + npe);
     const float *Wt = W + (size_t)t * rows * n_outputs;
-    for (int r = warp; 2 * r < S; r += nwarps) {
-        const int count = folded_count(r, S);
+    for (int r = warp; 2 * r < j_end - j_begin; r += nwarps) {
+        const int ja = j_end - 1 - r, jb = j_begin + r;
+        const int count = ja + (jb != ja ? jb : 0);   // (the middle query of an odd number is alone)
         for (int c0 = 0; c0 < n_outputs; c0 += LG * VEC) {
             const int col = c0 + q * VEC;
             const bool active = col < n_outputs;
@@ -112,9 +112,8 @@ __global__ void __launch_bounds__(256) concat_forward_kernel(const float *__rest
                 // bit 31: the pair belongs to the shorter query; bit 30: no pair
                 uint32_t mine = 0x40000000u;
                 if (p0 + lane < count) {
-                    const FoldedPair f = folded_pair(r, p0 + lane, S);
-                    if (f.j >= j_begin && f.j < j_end)
-                        mine = (uint32_t)concat_row(Ks[f.j], Ks[f.i], Ps[f.j - f.i - 1], nc, npe) | (f.first ? 0u : 0x80000000u);
+                    const FoldedPair f = folded_pair(ja, jb, p0 + lane);
+                    mine = (uint32_t)concat_row(Ks[f.j], Ks[f.i], Ps[f.j - f.i - 1], nc, npe) | (f.first ? 0u : 0x80000000u);
                 }
 #pragma unroll 1
                 for (int i0 = 0; i0 < LG && p0 + i0 < count; i0 += U) {
@@ -144,11 +143,10 @@ __global__ void __launch_bounds__(256) concat_forward_kernel(const float *__rest
                     acc_b[e] += __shfl_xor_sync(0xffffffffu, acc_b[e], m);
                 }
             }
-            const int ja = S - 1 - r;
             float *yb = y + (size_t)b * S * n_outputs + col;
             // one group adds the longer query's sum, the next (where there is one) the shorter's
-            if (active && g == 0 && ja > 0 && ja >= j_begin && ja < j_end) red_row<VEC>(yb + (size_t)ja * n_outputs, acc_a);
-            if (active && g == (NG > 1 ? 1 : 0) && r > 0 && r != ja && r >= j_begin && r < j_end) red_row<VEC>(yb + (size_t)r * n_outputs, acc_b);
+            if (active && g == 0 && ja > 0) red_row<VEC>(yb + (size_t)ja * n_outputs, acc_a);
+            if (active && g == (NG > 1 ? 1 : 0) && jb > 0 && jb != ja) red_row<VEC>(yb + (size_t)jb * n_outputs, acc_b);
         }
     }
 }
@@ -236,8 +234,9 @@ __global__ void __launch_bounds__(256) concat_backward_kernel(const float *__res
     const float *Wt = W + (size_t)t * rows * n_outputs;
     float *Tt = DO_DW ? target + (size_t)t * rows * n_outputs : nullptr;
     const float *dYb = dY + (size_t)b * S * n_outputs;
-    for (int r = warp; 2 * r < S; r += nwarps) {
-        const int count = folded_count(r, S);
+    for (int r = warp; 2 * r < j_end - j_begin; r += nwarps) {
+        const int ja = j_end - 1 - r, jb = j_begin + r;
+        const int count = ja + (jb != ja ? jb : 0);   // (the middle query of an odd number is alone)
         for (int p0 = 0; p0 < count; p0 += 32) {
             // this lane's pair; my_j < 0: none
             int my_j = -1, my_i = 0, my_flip = 0, my_pos = 0;
@@ -245,23 +244,21 @@ __global__ void __launch_bounds__(256) concat_backward_kernel(const float *__res
             float my_m = 0.f;
             bool my_pe = false;
             if (p0 + lane < count) {
-                const FoldedPair f = folded_pair(r, p0 + lane, S);
-                if (f.j >= j_begin && f.j < j_end) {
-                    my_j = f.j; my_i = f.i;
-                    const int32_t Q = Ks[f.j], K = Ks[f.i], PEi = Ps[f.j - f.i - 1];
-                    const float qm = Km[f.j], km = Km[f.i], pm = Pm[f.j - f.i - 1];
-                    const int qk = Kk[f.j], kk = Kk[f.i];
-                    my_row = (uint32_t)concat_row(Q, K, PEi, nc, npe);
-                    const bool flip_query = fabsf(qm) < fabsf(km);
-                    my_flip = flip_query ? qk : kk;
-                    my_m = flip_query ? qm : km;
-                    my_pos = flip_query ? f.j : f.i;
-                    // (a detector without a usable anchor pair has no bit to flip)
-                    my_alt = my_flip < 0 ? my_row : my_row ^ (1u << (my_flip + npe + (flip_query ? nc : 0)));
-                    if (npe > 0 && fabsf(pm) < fabsf(qm) && fabsf(pm) < fabsf(km)) {
-                        my_pe = true;
-                        my_palt = my_row ^ (1u << Pk[f.j - f.i - 1]);
-                    }
+                const FoldedPair f = folded_pair(ja, jb, p0 + lane);
+                my_j = f.j; my_i = f.i;
+                const int32_t Q = Ks[f.j], K = Ks[f.i], PEi = Ps[f.j - f.i - 1];
+                const float qm = Km[f.j], km = Km[f.i], pm = Pm[f.j - f.i - 1];
+                const int qk = Kk[f.j], kk = Kk[f.i];
+                my_row = (uint32_t)concat_row(Q, K, PEi, nc, npe);
+                const bool flip_query = fabsf(qm) < fabsf(km);
+                my_flip = flip_query ? qk : kk;
+                my_m = flip_query ? qm : km;
+                my_pos = flip_query ? f.j : f.i;
+                // (a detector without a usable anchor pair has no bit to flip)
+                my_alt = my_flip < 0 ? my_row : my_row ^ (1u << (my_flip + npe + (flip_query ? nc : 0)));
+                if (npe > 0 && fabsf(pm) < fabsf(qm) && fabsf(pm) < fabsf(km)) {
+                    my_pe = true;
+                    my_palt = my_row ^ (1u << Pk[f.j - f.i - 1]);
                 }
             }
             const unsigned pe_mask = DO_DX ? __ballot_sync(0xffffffffu, my_pe) : 0u;
@@ -647,7 +644,7 @@ static int launch_concat_pairs_forward(const lutb_layer_cfg *cfg, int64_t batch,
         return LUTB_OK;
     }
     const bool vec4 = O % 4 == 0 && aligned16(weights) && aligned16(y);
-    const int threads = 32 * min(8, (S + 1) / 2);
+    const int threads = 32 * min(8, (j_end - j_begin + 1) / 2);
     const int64_t per = samples_per_launch(Nt);
     for (int64_t b0 = 0; b0 < batch; b0 += per) {
         const int n = (int)min(per, batch - b0);
@@ -681,7 +678,7 @@ static int launch_concat_pairs_backward(const lutb_layer_cfg *cfg, int64_t batch
     // the (token, anchor pair) cells of dX join the token state while four blocks still fit an SM
     const size_t state = (size_t)6 * S * 4, cells = (size_t)S * Nc * 4;
     const int smem_dx = state + cells <= 48 * 1024;
-    const int threads = 32 * min(8, (S + 1) / 2);
+    const int threads = 32 * min(8, (j_end - j_begin + 1) / 2);
     auto pass = [&](auto dx_c, auto dw_c, float *target) -> int {
         constexpr bool DX = decltype(dx_c)::value, DWF = decltype(dw_c)::value;
         const bool vec4 = O % 4 == 0 && aligned16(weights) && aligned16(dY) && aligned16(target);

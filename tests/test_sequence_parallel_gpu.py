@@ -81,6 +81,47 @@ def test_query_ranges_add_up_to_the_unsharded_layer_and_the_oracle():
     assert y_parts[0][:, S // 2:].abs().sum() == 0
 
 
+@pytest.mark.parametrize("S,cuts", [(2, (0, 1, 2)), (5, (0, 2, 3, 5)), (33, (0, 1, 7, 16, 17, 30, 33)), (70, (0, 3, 34, 36, 69, 70)),
+                                    (9, (0, 9))])
+def test_query_ranges_that_cut_folded_pairs(S, cuts):
+    """Ranges before, across and behind the middle of even and odd lengths, down to single queries: each writes its own rows
+    and together they are the oracle's layer."""
+    from spiky_b200.lut_layer import LUTLayer, SynapseMeta
+
+    B, E, Nt, Nc, Npe, O = 2, 16, 3, 3, 2, 12
+    layer = LUTLayer(E, Nc, Nt, O, sequence_length=S, synapse_meta=SynapseMeta(min_weight=-1.0, max_weight=1.0),
+                     concatenation_product=True, positional_dim=Npe, random_seed=6, device="cuda:0")
+    g = torch.Generator().manual_seed(S)
+    with torch.no_grad():
+        layer._weights.copy_(torch.empty(layer._weights.shape).normal_(0.0, 0.05, generator=g))
+    x, dy = torch.rand(B, S, E, generator=g) * 2 - 1, torch.randn(B, S, O, generator=g)
+    W, anchors = layer._weights.detach().cpu().numpy(), layer._detector_anchors.cpu().numpy()
+    pe = layer._prepare_positional_embeddings().detach().contiguous().view(-1)
+    y_ref, st = orc.concat_forward(W, x.numpy(), pe.cpu().numpy().reshape(S - 1, Nt, Npe), anchors, Nt, Nc, O, Npe)
+    dX_ref, dW_ref, dPE_ref = orc.concat_backward(W, dy.numpy(), anchors, st, E, Nc, Npe)
+    dm, xt, dyt = layer._lut_dm, x.cuda().view(-1), dy.cuda().view(-1)
+    idx, mk = (torch.empty(B * S * Nt, dtype=torch.int32, device="cuda") for _ in range(2))
+    md = torch.empty(B * S * Nt, device="cuda")
+    pidx, pmk = (torch.empty((S - 1) * Nt, dtype=torch.int32, device="cuda") for _ in range(2))
+    pmd = torch.empty((S - 1) * Nt, device="cuda")
+    dm.check_detectors(B * S, xt, layer._detector_anchors, idx, 0.0, md, mk)
+    dm.check_positional(pe, pidx, 0.0, pmd, pmk)
+    dX, dW, dPE = torch.zeros(B * S * E, device="cuda"), torch.zeros_like(layer._weights), torch.zeros((S - 1) * Nt * Npe, device="cuda")
+    whole = torch.zeros(B, S, O, device="cuda")
+    for j0, j1 in zip(cuts, cuts[1:]):
+        y = torch.zeros(B * S * O, device="cuda")
+        dm.concat_pairs_forward(layer._weights.detach(), B, idx, pidx, y, j0, j1)
+        y = y.view(B, S, O)
+        assert not y[:, :j0].any() and not y[:, j1:].any()
+        whole += y
+        dm.concat_pairs_backward(layer._weights.detach(), B, dyt, layer._detector_anchors, idx, md, mk, dX, -1.0, pidx, pmd, pmk,
+                                 dPE, dW, j0, j1)
+    golden_util.assert_close(whole.cpu().numpy(), y_ref, REL, "y")
+    golden_util.assert_close(dX.cpu().numpy().reshape(B, S, E), dX_ref, REL, "dX")
+    golden_util.assert_close(dW.detach().cpu().numpy(), dW_ref, REL, "dW")
+    golden_util.assert_close(dPE.cpu().numpy(), dPE_ref, REL, "dPE")
+
+
 def test_query_range_is_validated():
     from spiky_b200.lut_layer import LUTLayer, SynapseMeta
 
