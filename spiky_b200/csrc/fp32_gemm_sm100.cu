@@ -225,12 +225,19 @@ __global__ void combine_halves_kernel(const float *__restrict__ P, float *__rest
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// A pair of SMs per 256 x 256 tile where there are tiles for most of the SMs, one SM per 128 x 128 tile below.  Measured
-// on the contractions of the histogram path, one SM / pair: 8192 x 512 x 16384 214 / 176 us, 16384 x 512 x 8192 (A^T . B)
-// 214 / 166, 8192 x 16384 x 768 318 / 258; 1024 x 2048 x 65536 in 8 slices 423 / 341, 65536 x 2048 x 1024 384 / 337,
-// 1024 x 65536 x 3072 592 / 488.
+// A pair of SMs per 256 x 256 tile or one SM per 128 x 128 tile: whichever takes less time by waves of tiles.  A wave is what
+// the SMs hold at once; a pair's tile is four times the work on twice the SMs and takes 1.6 times as long (a byte from shared
+// memory feeds twice the multiply-adds).  Padding counts: a half empty 256-row tile takes as long as a full one.  Measured on the
+// contractions of the histogram path with their operand copies, one SM / pair, us:
+// pair: 8192 x 512 x 16384 214 / 176, 16384 x 512 x 8192 (A^T . B) 214 / 166, 8192 x 16384 x 768 318 / 258; 1024 x 2048 x 65536
+//   in 8 slices 423 / 341, 65536 x 2048 x 1024 384 / 337, 1024 x 65536 x 3072 592 / 488; 512 x 16384 x 768 50 / 46
+// one SM: 128 x 16384 x 768 34 / 39, 384 x 16384 x 768 45 / 48; A^T . B 16384 x 128 x 128 20 / 22, 10240 x 320 x 800 35 / 40
+// even: 160 to 256 x 16384 x 768 38 / 38, 640 x 16384 x 768 55 / 55; 1024 x 4096 x 768 takes the pair at 30 / 33
 static bool pair_tiles(int M, int N, int batches) {
-    return (int64_t)((M + 255) / 256) * ((N + 255) / 256) * batches >= 64;
+    const int64_t sm = device_info().sm_count > 1 ? device_info().sm_count : 2;
+    const int64_t pairs = (int64_t)((M + 255) / 256) * ((N + 255) / 256) * batches, singles = (int64_t)((M + 127) / 128) * ((N + 127) / 128) * batches;
+    const int64_t pair_waves = (pairs + sm / 2 - 1) / (sm / 2), single_waves = (singles + sm - 1) / sm;
+    return 8 * pair_waves < 5 * single_waves;
 }
 template <class Cfg>
 static int run_tiles(int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,

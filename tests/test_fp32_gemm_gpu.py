@@ -62,8 +62,8 @@ def test_fp32_gemm_matches_fp64_product(kind, shape, fast):
 
 
 def test_fp32_gemm_on_pairs_of_sms():
-    """More than 64 tiles of 256 x 256, ragged in both directions: two SMs a tile."""
-    test_fp32_gemm_matches_fp64_product(0, (2100, 2052, 96), False)
+    """One wave of 256 x 256 tiles against two of 128 x 128, ragged in both directions: two SMs a tile."""
+    test_fp32_gemm_matches_fp64_product(0, (1800, 2052, 96), False)
 
 
 def test_fp32_gemm_rejects_misaligned_leading_dimensions():

@@ -167,10 +167,12 @@ def test_product_histogram_chunks_match_single_pass():
             golden_util.assert_close(chunked[k], full[k], REL, f"{name}.{k}")
 
 
-def test_product_contractions_on_pairs_of_sms():
-    """Enough rows and detectors that every contraction has 64 tiles of 256 x 256 (two SMs a tile) against the fp32 FMA
-    contractions, with rows that end inside a tile."""
-    cfg = dict(seed=760, B=33, S=127, E=32, Nt=33, Nc=8, Npe=2, O=256, n_virtual=66)
+@pytest.mark.parametrize("B", [33, 66])
+def test_product_contractions_on_pairs_of_sms(B):
+    """Enough rows and detectors that every contraction has its 256 x 256 tiles on two SMs each, against the fp32 FMA
+    contractions, with rows that end inside a tile; 8382 rows: the table gradient accumulates two slices of them (8192 and
+    the rest)."""
+    cfg = dict(seed=760, B=B, S=127, E=32, Nt=33, Nc=8, Npe=2, O=256, n_virtual=66)
     x, anchors, W, pe, dY = inputs_for(cfg)
     got, want = run_gpu(cfg, x, anchors, W, pe, dY, 2), run_gpu(cfg, x, anchors, W, pe, dY, 3)
     for k in want:
