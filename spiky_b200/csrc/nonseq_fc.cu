@@ -36,7 +36,7 @@ __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ 
                                            int lt, int threads_per_group, bool vec_ok) {
     if (vec_ok) {
         const int n4 = n_inputs >> 2;
-        for (int i4 = lt; i4 < n4; i4 += threads_per_group) {
+        auto four_inputs = [&](int i4) {
             float v[R][4];
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -57,6 +57,12 @@ __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ 
                     for (int r = 0; r < R; r++) dst[r] = v[r][j];
                 }
             }
+        };
+        if constexpr (R == 4) {   // (eight loads in flight, as with eight rows; the other counts are as fast as they come)
+#pragma unroll 2
+            for (int i4 = lt; i4 < n4; i4 += threads_per_group) four_inputs(i4);
+        } else {
+            for (int i4 = lt; i4 < n4; i4 += threads_per_group) four_inputs(i4);
         }
     } else {
         for (int i = lt; i < n_inputs; i += threads_per_group) {
@@ -76,14 +82,13 @@ __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ 
 // stages as well.  (Splitting the detectors into a fixed number of slices per tile left 320 blocks on 148 SMs: the SMs
 // with three blocks set the kernel's time, max / avg active cycles 1.3.)
 //
-// Bound by the wavefronts of the load/store unit: the anchors' inputs are random, so the 8 lanes that share a wavefront of
-// 16-byte reads fall into the same banks 2.65 times over, and an anchor list read 8 bytes at a time touches 16 lines per
-// load.  With 8 rows, D = 2 neighbouring lanes share a detector (4 rows each): a wavefront then holds 4 random 32-byte
-// pieces, which collide 2.1 times, and the lists are read two anchors at a time.  Measured (one thread a detector before):
-// 16384 rows x 4096 inputs, 4096 detectors of 8 anchors 625 -> 444 us (8 rows in one block of 1024 threads an SM against 4);
-// 65536 x 784, 64 detectors of 6 anchors 83 -> 70 us.
-template <int R, bool TRAIN>
-__global__ void __launch_bounds__(R == 8 ? 1024 : 256) check_detectors_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
+// Bound by the wavefronts of the load/store unit where anchors are many: their inputs are random, so the 8 lanes that share a
+// wavefront of 16-byte reads fall into the same banks 2.65 times over, and an anchor list read 8 bytes at a time touches 16
+// lines per load.  D = 2: of 8 rows, two neighbouring lanes share a detector (4 rows each): a wavefront then holds 4 random
+// 32-byte pieces, which collide 2.1 times; lists are read two anchors at a time.  Where anchors are few the stores count instead
+// (D = 2 writes 64-byte pieces) and blocks of 256 threads overlap staging better; two_lanes() draws the line.
+template <int R, int D, bool TRAIN>
+__global__ void __launch_bounds__(D == 2 ? 1024 : 256) check_detectors_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
                                                              const int2 *__restrict__ anchors, int n_detectors,
                                                              int n_anchors, float cmp_eps, int threads_per_group,
                                                              int32_t *__restrict__ idx,
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(R == 8 ? 1024 : 256) check_detectors_kernel(co
                                                              int32_t *__restrict__ min_k,
                                                              uint8_t *__restrict__ packed, size_t packed_pitch) {
     extern __shared__ __align__(16) float xs_all[];
-    constexpr int D = R == 8 ? 2 : 1, RT = R / D;   // threads per detector, rows per thread
+    constexpr int RT = R / D;   // rows of a thread (D threads per detector)
     const int groups = blockDim.x / threads_per_group;
     const int g = threadIdx.x / threads_per_group;
     const int lt = threadIdx.x - g * threads_per_group;
@@ -125,11 +130,14 @@ __global__ void __launch_bounds__(R == 8 ? 1024 : 256) check_detectors_kernel(co
         auto one_anchor = [&](int k, int px, int py) {
             if (px == kNoAnchor || py == kNoAnchor) return;
             float a[RT], b[RT];
-            if constexpr (RT == 4) {
-                const float4 qa = reinterpret_cast<const float4 *>(xs)[swizzle_slot(px * D + half)];
-                const float4 qb = reinterpret_cast<const float4 *>(xs)[swizzle_slot(py * D + half)];
-                a[0] = qa.x; a[1] = qa.y; a[2] = qa.z; a[3] = qa.w;
-                b[0] = qb.x; b[1] = qb.y; b[2] = qb.z; b[3] = qb.w;
+            if constexpr (R % 4 == 0) {
+#pragma unroll
+                for (int r4 = 0; r4 < RT / 4; r4++) {
+                    const float4 qa = reinterpret_cast<const float4 *>(xs)[swizzle_slot(px * (R / 4) + half * (RT / 4) + r4)];
+                    const float4 qb = reinterpret_cast<const float4 *>(xs)[swizzle_slot(py * (R / 4) + half * (RT / 4) + r4)];
+                    a[4 * r4] = qa.x; a[4 * r4 + 1] = qa.y; a[4 * r4 + 2] = qa.z; a[4 * r4 + 3] = qa.w;
+                    b[4 * r4] = qb.x; b[4 * r4 + 1] = qb.y; b[4 * r4 + 2] = qb.z; b[4 * r4 + 3] = qb.w;
+                }
             } else {
 #pragma unroll
                 for (int r = 0; r < RT; r++) { a[r] = xs[(size_t)px * R + r]; b[r] = xs[(size_t)py * R + r]; }
@@ -170,8 +178,11 @@ __global__ void __launch_bounds__(R == 8 ? 1024 : 256) check_detectors_kernel(co
         if (!TRAIN && packed != nullptr) {
             // (the bytes of rows past the end lie in the row's padding)
             uint8_t *dst = packed + (size_t)t * packed_pitch + row0 + half * RT;
-            if constexpr (RT == 4) *reinterpret_cast<uint32_t *>(dst) = (uint32_t)li[0] | (uint32_t)li[1] << 8 | (uint32_t)li[2] << 16 | (uint32_t)li[3] << 24;
-            else {
+            if constexpr (RT % 4 == 0) {
+#pragma unroll
+                for (int r = 0; r < RT; r += 4)
+                    *reinterpret_cast<uint32_t *>(dst + r) = (uint32_t)li[r] | (uint32_t)li[r + 1] << 8 | (uint32_t)li[r + 2] << 16 | (uint32_t)li[r + 3] << 24;
+            } else {
 #pragma unroll
                 for (int r = 0; r < RT; r++) dst[r] = (uint8_t)li[r];
             }
@@ -207,7 +218,7 @@ __global__ void check_detectors_global_kernel(const float *__restrict__ x, int64
     }
 }
 
-template <int R>
+template <int R, int D>
 static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, const int32_t *anchors,
                                     int n_detectors, int n_anchors, float cmp_eps, int32_t *idx, float *min_delta,
                                     int32_t *min_k, int tpg, int groups, int64_t blocks, cudaStream_t stream,
@@ -215,7 +226,7 @@ static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, 
     const size_t smem = (size_t)groups * staged_floats<R>(n_inputs) * sizeof(float);
     LUTB_REQUIRE(blocks <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "batch too large for one launch");
     const bool train = min_delta != nullptr;
-    auto kern = train ? check_detectors_kernel<R, true> : check_detectors_kernel<R, false>;
+    auto kern = train ? check_detectors_kernel<R, D, true> : check_detectors_kernel<R, D, false>;
     if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KernelScope scope(K_CHECK_DETECTORS, stream);
     kern<<<(unsigned)blocks, tpg * groups, smem, stream>>>(x, rows, n_inputs, reinterpret_cast<const int2 *>(anchors),
@@ -224,19 +235,48 @@ static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, 
     return LUTB_OK;
 }
 
+constexpr size_t kCheckBudget = 100 * 1024;   // staged rows of a block: two resident blocks per SM
+
+// Whether two lanes share a detector (8 rows a group).  Measured over 8 to 32768 rows, 32 to 6000 inputs, 16 to 4096
+// detectors, 2 to 13 anchors, training and evaluation; figures in us, two lanes / one lane a detector:
+//  - rows that leave room for one block of 1024 threads (the other side: 4 rows): many anchors and detectors, and row tiles for
+//    most of the SMs: 4096 rows x 4096 inputs, 4096 detectors of 8 anchors 0.78 of the time; 8192 x 4000, 16 detectors 291 / 109,
+//    1000 detectors of 2 anchors 60 / 56, 64 rows, 1000 of 8 10.4 / 6.3
+//  - few detectors: one lane each leaves an SM short of threads, the sooner the more shared memory their rows take: 32768 x 784,
+//    64 detectors 0.87, 32768 x 3000, 64 detectors 0.6, 128 detectors 0.74; 100000 x 32, 64 detectors of 4 47 / 39
+//  - long rows: 32768 x 3000, 256 detectors of 6 0.9; x 1500 to 2048 0.93 to 0.97, of 2 anchors in evaluation 1.1
+//  - a few row tiles per SM, which are all there is to fill it: 4096 x 300, 1024 detectors of 7 29 / 39; 32768 rows 1.1 to 1.2
+//  - many anchors and detectors: 32768 x 784, 768 detectors of 8 anchors 0.95; 100000 x 32, 300 of 3 222 / 149
+static bool two_lanes(int64_t rows, int n_inputs, int n_detectors, int n_anchors) {
+    const size_t staged = staged_bytes(8, n_inputs);
+    const int64_t tiles = (rows + 7) / 8;
+    const int sm = device_info().sm_count;
+    if (rows < 8 || staged > (size_t)kMaxSmemPerBlock - 1024) return false;
+    if (staged > kCheckBudget)
+        return n_anchors >= 6 && n_detectors >= 768 && tiles * ((n_detectors + 511) / 512) >= sm - sm / 8 &&
+               (rows <= 16384 || n_detectors >= 2048 || n_anchors >= 8);
+    if (n_detectors <= 32) return staged < 22 * 1024;
+    if (n_detectors <= 128 && staged >= 22 * 1024) return true;
+    if (n_detectors <= 64 && rows <= 8192) return true;
+    if (staged >= 80 * 1024) return n_detectors <= 192 || n_anchors >= 4;
+    if (staged >= 44 * 1024) return n_anchors >= 6 && n_detectors >= 256;
+    if (n_anchors >= 6 && n_detectors >= (n_anchors >= 10 ? 256 : 384) && tiles >= 2 * sm && tiles <= 5 * sm) return true;
+    return n_anchors >= 8 && n_detectors >= 768 && staged >= 6 * 1024;
+}
+
 int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int32_t *anchors, int n_detectors,
                            int n_anchors, float cmp_eps, int32_t *idx, float *min_delta, int32_t *min_k,
                            cudaStream_t stream, uint8_t *packed, size_t packed_pitch) {
     const int sm = device_info().sm_count;
-    // rows per group: 8 while they fit a block (each anchor pair is fetched once per 8 rows), fewer for few or longer rows
+    // rows per group: 8 while two blocks fit an SM (each anchor pair is fetched once per 8 rows), or one block of twice the threads
+    // where that pays; fewer for few or longer rows
     const size_t row_bytes = (size_t)n_inputs * sizeof(float);
-    const size_t budget = 100 * 1024;  // two resident blocks per SM
+    const int D = two_lanes(rows, n_inputs, n_detectors, n_anchors) ? 2 : 1;
     int R = 8;
-    while (R > 1 && (staged_bytes(R, n_inputs) > (R == 8 ? (size_t)kMaxSmemPerBlock - 1024 : budget) || rows < R)) R >>= 1;
-    // threads per row group: one per detector (two with 8 rows), rounded to warps; at most 256 detectors, or 512 where the rows
-    // leave room for one block only
-    const int per_det = R == 8 ? 2 : 1, widest = R != 8 ? 256 : staged_bytes(R, n_inputs) > budget ? 1024 : 512;
-    int tpg = ((min(n_detectors * per_det, widest) + 31) / 32) * 32;
+    while (R > 1 && (rows < R || (D == 1 && staged_bytes(R, n_inputs) > kCheckBudget))) R >>= 1;
+    // threads per row group: D per detector, rounded to warps; at most 256 detectors, or 512 where the rows leave room for one block
+    const int widest = D == 1 ? 256 : staged_bytes(R, n_inputs) > kCheckBudget ? 1024 : 512;
+    int tpg = ((min(n_detectors * D, widest) + 31) / 32) * 32;
     if ((size_t)R * row_bytes > (size_t)kMaxSmemPerBlock - 1024) {
         const bool train = min_delta != nullptr;
         const int64_t total = rows * n_detectors;
@@ -254,18 +294,20 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
         return LUTB_OK;
     }
     int groups = tpg >= 256 ? 1 : 256 / tpg;
-    while (groups > 1 && ((size_t)groups * R * row_bytes > budget || rows < (int64_t)groups * R * 2 * sm)) groups >>= 1;
+    while (groups > 1 && ((size_t)groups * R * row_bytes > kCheckBudget || rows < (int64_t)groups * R * 2 * sm)) groups >>= 1;
     // one block per row tile; small batches: as many blocks as are resident (two per SM, one where the rows take more than
     // half of it), each with an equal share of the (tile, detector chunk) work items
-    const int64_t resident = (int64_t)sm * (groups * staged_bytes(R, n_inputs) > budget ? 1 : 2);
+    const int64_t resident = (int64_t)sm * (groups * staged_bytes(R, n_inputs) > kCheckBudget ? 1 : 2);
     const int64_t row_tiles = (rows + (int64_t)groups * R - 1) / ((int64_t)groups * R);
-    const int64_t items = row_tiles * ((n_detectors + tpg / per_det - 1) / (tpg / per_det));
+    const int64_t items = row_tiles * ((n_detectors + tpg / D - 1) / (tpg / D));
     const int64_t blocks = row_tiles >= resident ? row_tiles : min(items, resident);
     switch (R) {
-        case 8: return launch_check_detectors_r<8>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
-        case 4: return launch_check_detectors_r<4>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
-        case 2: return launch_check_detectors_r<2>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
-        default: return launch_check_detectors_r<1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        case 8:
+            if (D == 2) return launch_check_detectors_r<8, 2>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+            return launch_check_detectors_r<8, 1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        case 4: return launch_check_detectors_r<4, 1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        case 2: return launch_check_detectors_r<2, 1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
+        default: return launch_check_detectors_r<1, 1>(x, rows, n_inputs, anchors, n_detectors, n_anchors, cmp_eps, idx, min_delta, min_k, tpg, groups, blocks, stream, packed, packed_pitch);
     }
 }
 
