@@ -398,93 +398,123 @@ __global__ void __launch_bounds__(256) fc_gather_forward_fixed_kernel(const floa
     }
 }
 
-// Forward gather for fp32 accumulators: one warp per (sample, chunk of LG * J columns of VEC floats); the row loads of up to
-// 16 / J detectors per lane are all issued before the first one is consumed, which is what hides the latency of the (random)
-// row reads.  VEC = 4 for 16-byte aligned rows (J = 1); VEC = 1 for the others, J = 2 where a row is a little wider than a warp.
-// Measured on rows that are not (a loop with a load per detector and lane in flight before): 1111 samples, 50 detectors, 33
-// outputs 18.4 -> 6.3 us; 512 samples, 64 detectors, 10 outputs 17.7 -> 5.7 us.
-template <int LG, int VEC, int J>
+// Forward gather for fp32 accumulators and 16-byte aligned rows: one warp per (sample, chunk of LG float4 columns); the row
+// loads of up to 16 detectors per lane are all issued before the first one is consumed, which is what hides the latency of the
+// (random) row reads.
+template <int LG>
 __global__ void __launch_bounds__(256) fc_gather_forward_vec_kernel(const float *__restrict__ W,
                                                                    const int32_t *__restrict__ idx,
                                                                    float *__restrict__ y, int64_t batch, int n_outputs,
                                                                    int n_detectors, int table_rows, int t0, int t1) {
     constexpr int NG = 32 / LG;
-    constexpr int IT = 32 / NG;                          // row loads per lane and 32 detectors
-    constexpr int BATCH = IT > 16 / J ? 16 / J : IT;     // loads in flight per lane
+    constexpr int IT = 32 / NG;                  // row loads per lane and 32 detectors
+    constexpr int BATCH = IT > 16 ? 16 : IT;     // loads in flight per lane
     const int lane = threadIdx.x & 31;
     const int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (b >= batch) return;
     const int g = lane / LG, j = lane - g * LG;
-    const int col = (blockIdx.y * (LG * J) + j) * VEC;   // further columns of the lane LG * VEC apart
-    bool active[J];
-#pragma unroll
-    for (int q = 0; q < J; q++) active[q] = col + q * LG * VEC < n_outputs;
+    const int col = (blockIdx.y * LG + j) * 4;
+    const bool active = col < n_outputs;
     const int32_t *idx_b = idx + b * n_detectors;
     const float *Wc = W + col;
-    double acc[J][VEC];
-#pragma unroll
-    for (int q = 0; q < J; q++)
-#pragma unroll
-        for (int e = 0; e < VEC; e++) acc[q][e] = 0.0;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int tb = t0; tb < t1; tb += 32) {
         const int nvalid = min(32, t1 - tb);
         const int32_t mine = (lane < nvalid) ? __ldg(idx_b + tb + lane) : 0;
-        float part[J][VEC];
-#pragma unroll
-        for (int q = 0; q < J; q++)
-#pragma unroll
-            for (int e = 0; e < VEC; e++) part[q][e] = 0.f;
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i0 = 0; i0 < IT; i0 += BATCH) {
-            float w[BATCH][J][VEC];
+            float4 w[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) {
+                const int d = (i0 + i) * NG + g;
+                const int32_t li = __shfl_sync(0xffffffffu, mine, d);
+                w[i] = (active && d < nvalid)
+                           ? __ldg(reinterpret_cast<const float4 *>(Wc + ((size_t)(tb + d) * table_rows + li) * n_outputs))
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) { part[0] += w[i].x; part[1] += w[i].y; part[2] += w[i].z; part[3] += w[i].w; }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[e] += (double)part[e];
+    }
+#pragma unroll
+    for (int m = LG; m < 32; m <<= 1) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], m);
+    }
+    if (active && g == 0) {
+        float4 *out = reinterpret_cast<float4 *>(y + b * n_outputs + col);
+        float4 cur = *out;
+        cur.x += (float)acc[0]; cur.y += (float)acc[1]; cur.z += (float)acc[2]; cur.w += (float)acc[3];
+        *out = cur;
+    }
+}
+
+// The same for rows that are not 16-byte aligned: chunks of LG * J columns, J columns a lane (LG apart), the row loads of up to
+// 16 / J detectors in flight.  J = 2 where a row is a little wider than a warp, J = 4 for wide rows (a chunk per 32 columns reads
+// the indices again for each of them).  (One template for both kernels cost the aligned rows 5 %: 60000 samples, 40 detectors,
+// 256 outputs 223 -> 235 us.)
+// Measured (a loop with a load per detector and lane in flight before): 1111 samples, 50 detectors, 33 outputs 18.4 -> 6.3 us;
+// 512 samples, 64 detectors, 10 outputs 17.7 -> 5.7 us.  J = 1 / 4, with the index comparison: 8192 samples, 16 detectors, 129
+// outputs 29 / 21, 1001 outputs 132 / 56; 60000 x 40, 65 outputs 227 / 106; few warps (32 samples, 65 outputs) 10.5 / 12.6.
+template <int LG, int J>
+__global__ void __launch_bounds__(256) fc_gather_forward_scalar_kernel(const float *__restrict__ W,
+                                                                      const int32_t *__restrict__ idx,
+                                                                      float *__restrict__ y, int64_t batch, int n_outputs,
+                                                                      int n_detectors, int table_rows, int t0, int t1) {
+    constexpr int NG = 32 / LG;
+    constexpr int IT = 32 / NG;                          // row loads per lane and 32 detectors
+    constexpr int BATCH = IT > 16 / J ? 16 / J : IT;     // detectors in flight per lane
+    const int lane = threadIdx.x & 31;
+    const int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (b >= batch) return;
+    const int g = lane / LG, j = lane - g * LG;
+    const int col = blockIdx.y * (LG * J) + j;   // further columns of the lane LG apart
+    bool active[J];
+#pragma unroll
+    for (int q = 0; q < J; q++) active[q] = col + q * LG < n_outputs;
+    const int32_t *idx_b = idx + b * n_detectors;
+    const float *Wc = W + col;
+    double acc[J];
+#pragma unroll
+    for (int q = 0; q < J; q++) acc[q] = 0.0;
+    for (int tb = t0; tb < t1; tb += 32) {
+        const int nvalid = min(32, t1 - tb);
+        const int32_t mine = (lane < nvalid) ? __ldg(idx_b + tb + lane) : 0;
+        float part[J];
+#pragma unroll
+        for (int q = 0; q < J; q++) part[q] = 0.f;
+#pragma unroll
+        for (int i0 = 0; i0 < IT; i0 += BATCH) {
+            if (J > 1 && i0 * NG >= nvalid) break;   // (warp uniform; J = 1 keeps the next batch's loads ahead of this one's sums)
+            float w[BATCH][J];
 #pragma unroll
             for (int i = 0; i < BATCH; i++) {
                 const int d = (i0 + i) * NG + g;
                 const int32_t li = __shfl_sync(0xffffffffu, mine, d);
 #pragma unroll
-                for (int q = 0; q < J; q++) {
-                    if constexpr (VEC == 4) {
-                        const float4 v = (active[q] && d < nvalid)
-                                             ? __ldg(reinterpret_cast<const float4 *>(Wc + ((size_t)(tb + d) * table_rows + li) * n_outputs) + q * LG)
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
-                        w[i][q][0] = v.x; w[i][q][1] = v.y; w[i][q][2] = v.z; w[i][q][3] = v.w;
-                    } else {
-                        w[i][q][0] = (active[q] && d < nvalid) ? __ldg(Wc + ((size_t)(tb + d) * table_rows + li) * n_outputs + q * LG) : 0.f;
-                    }
-                }
+                for (int q = 0; q < J; q++)
+                    w[i][q] = (active[q] && d < nvalid) ? __ldg(Wc + ((size_t)(tb + d) * table_rows + li) * n_outputs + q * LG) : 0.f;
             }
 #pragma unroll
             for (int i = 0; i < BATCH; i++)
 #pragma unroll
-                for (int q = 0; q < J; q++)
-#pragma unroll
-                    for (int e = 0; e < VEC; e++) part[q][e] += w[i][q][e];
+                for (int q = 0; q < J; q++) part[q] += w[i][q];
         }
 #pragma unroll
-        for (int q = 0; q < J; q++)
-#pragma unroll
-            for (int e = 0; e < VEC; e++) acc[q][e] += (double)part[q][e];
+        for (int q = 0; q < J; q++) acc[q] += (double)part[q];
     }
 #pragma unroll
     for (int m = LG; m < 32; m <<= 1) {
 #pragma unroll
-        for (int q = 0; q < J; q++)
-#pragma unroll
-            for (int e = 0; e < VEC; e++) acc[q][e] += __shfl_xor_sync(0xffffffffu, acc[q][e], m);
+        for (int q = 0; q < J; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], m);
     }
     if (g != 0) return;
 #pragma unroll
-    for (int q = 0; q < J; q++) {
-        if (!active[q]) continue;
-        float *out = y + b * n_outputs + col + q * LG * VEC;
-        if constexpr (VEC == 4) {
-            float4 cur = *reinterpret_cast<float4 *>(out);
-            cur.x += (float)acc[q][0]; cur.y += (float)acc[q][1]; cur.z += (float)acc[q][2]; cur.w += (float)acc[q][3];
-            *reinterpret_cast<float4 *>(out) = cur;
-        } else {
-            *out += (float)acc[q][0];
-        }
-    }
+    for (int q = 0; q < J; q++)
+        if (active[q]) y[b * n_outputs + col + q * LG] += (float)acc[q];
 }
 
 static int pow2_ceil(int v) {
@@ -517,8 +547,10 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
         const int t1 = (int)min((int64_t)n_detectors, t0 + per_range);
         KernelScope scope(K_FC_GATHER_FORWARD, stream);
         if (!int_mode) {
-            // columns of a lane: two where one pass of the warp leaves a remainder (scalar rows of 33 to 64 outputs)
-            const int cols = !vec4 && vpr > 32 && vpr <= 64 ? 2 : 1;
+            // columns of a lane: two where one pass of the warp leaves a remainder (scalar rows of 33 to 64 outputs), four for
+            // wider scalar rows once that gives every SM six warps (and where a grid has no room for a chunk per 32 columns)
+            const bool wide = !vec4 && vpr > 64 && (batch * ((vpr + 127) / 128) >= 6 * (int64_t)device_info().sm_count || vpr > 65535 * 32);
+            const int cols = wide ? 4 : !vec4 && vpr > 32 && vpr <= 64 ? 2 : 1;
             const dim3 vgrid((unsigned)blocks, (unsigned)((vpr + lanes * cols - 1) / (lanes * cols)));
             LUTB_REQUIRE(vgrid.y <= 65535, LUTB_ERR_SHAPE, "grid too large");
             auto launch = [&](auto kern) {
@@ -526,23 +558,25 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
             };
             if (vec4) {
                 switch (lanes) {
-                    case 32: launch(fc_gather_forward_vec_kernel<32, 4, 1>); break;
-                    case 16: launch(fc_gather_forward_vec_kernel<16, 4, 1>); break;
-                    case 8: launch(fc_gather_forward_vec_kernel<8, 4, 1>); break;
-                    case 4: launch(fc_gather_forward_vec_kernel<4, 4, 1>); break;
-                    case 2: launch(fc_gather_forward_vec_kernel<2, 4, 1>); break;
-                    default: launch(fc_gather_forward_vec_kernel<1, 4, 1>); break;
+                    case 32: launch(fc_gather_forward_vec_kernel<32>); break;
+                    case 16: launch(fc_gather_forward_vec_kernel<16>); break;
+                    case 8: launch(fc_gather_forward_vec_kernel<8>); break;
+                    case 4: launch(fc_gather_forward_vec_kernel<4>); break;
+                    case 2: launch(fc_gather_forward_vec_kernel<2>); break;
+                    default: launch(fc_gather_forward_vec_kernel<1>); break;
                 }
+            } else if (cols == 4) {
+                launch(fc_gather_forward_scalar_kernel<32, 4>);
             } else if (cols == 2) {
-                launch(fc_gather_forward_vec_kernel<32, 1, 2>);
+                launch(fc_gather_forward_scalar_kernel<32, 2>);
             } else {
                 switch (lanes) {
-                    case 32: launch(fc_gather_forward_vec_kernel<32, 1, 1>); break;
-                    case 16: launch(fc_gather_forward_vec_kernel<16, 1, 1>); break;
-                    case 8: launch(fc_gather_forward_vec_kernel<8, 1, 1>); break;
-                    case 4: launch(fc_gather_forward_vec_kernel<4, 1, 1>); break;
-                    case 2: launch(fc_gather_forward_vec_kernel<2, 1, 1>); break;
-                    default: launch(fc_gather_forward_vec_kernel<1, 1, 1>); break;
+                    case 32: launch(fc_gather_forward_scalar_kernel<32, 1>); break;
+                    case 16: launch(fc_gather_forward_scalar_kernel<16, 1>); break;
+                    case 8: launch(fc_gather_forward_scalar_kernel<8, 1>); break;
+                    case 4: launch(fc_gather_forward_scalar_kernel<4, 1>); break;
+                    case 2: launch(fc_gather_forward_scalar_kernel<2, 1>); break;
+                    default: launch(fc_gather_forward_scalar_kernel<1, 1>); break;
                 }
             }
         } else if (vec4) {

@@ -274,13 +274,14 @@ def test_input_gradient_kernel_splits(B, I, Nt, Nc, O):
             golden_util.assert_close(gW.cpu().numpy(), dW.reshape(-1), 1e-5, "dW")
 
 
-@pytest.mark.parametrize("O", [1, 2, 3, 7, 10, 17, 31, 33, 45, 63, 65, 130, 4, 36, 132])
-def test_forward_gather_widths(O):
-    """Rows of every lane group, one and two columns a lane, several column chunks, aligned and not; detectors that end
+@pytest.mark.parametrize("B,O", [(21, O) for O in (1, 2, 3, 7, 10, 17, 31, 33, 45, 63, 65, 130, 4, 36, 132)] +
+                         [(900, 65), (900, 127), (900, 131), (5, 16385)])
+def test_forward_gather_widths(B, O):
+    """Rows of every lane group, one, two and four columns a lane, several column chunks, aligned and not; detectors that end
     inside a group of 32."""
     from spiky_b200.lut_data_manager import LUTDataManagerF
 
-    B, I, Nt, Nc = 21, 40, 37, 4
+    I, Nt, Nc = 40, 37, 4
     x = synth.normal(980, (B, I))
     anchors = synth.anchor_pairs(981, Nt, Nc, I)
     W = synth.normal(982, (Nt * (1 << Nc) * O,), 0.0, 0.05)
@@ -295,3 +296,20 @@ def test_forward_gather_widths(O):
                     torch.from_numpy(anchors).reshape(-1).cuda(), y, ti)
     assert np.array_equal(ti.cpu().numpy(), idx.reshape(-1))
     golden_util.assert_close(y.cpu().numpy().reshape(B, O), want, 1e-5, "y")
+
+
+def test_forward_gather_of_very_wide_scalar_rows():
+    """More columns than a grid has chunks of 32 for: two samples, one detector, 2.1 M outputs that are no multiple of four."""
+    from spiky_b200.lut_data_manager import LUTDataManagerF
+
+    O = 65535 * 32 + 5
+    dm = LUTDataManagerF(4, O, 1, 1, 1, 0, 0, 32, 32)
+    dm.register_synapse_meta(1.0, -1.0, 1.0, 0.0, 0.0)
+    dm.initialize_neurons(True)
+    dm.to_device(0)
+    W = torch.randn(2 * O, device="cuda")
+    x = torch.tensor([1.0, 0.0, 0.0, 0.0, -1.0, 0.0, 0.0, 0.0], device="cuda")
+    y, idx = torch.zeros(2 * O, device="cuda"), torch.empty(2, dtype=torch.int32, device="cuda")
+    dm.forward_step(W, 2, x, torch.tensor([0, 1], dtype=torch.int32, device="cuda"), y, idx)
+    assert idx.tolist() == [1, 0]
+    assert torch.equal(y.view(2, O), W.view(2, O).flip(0))
