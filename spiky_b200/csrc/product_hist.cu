@@ -929,22 +929,32 @@ static int plan(const ProductCall &c, bool backward, bool allow_tc, void *worksp
     return LUTB_OK;
 }
 
-// Queries of one block of the pair kernels: the most, up to 128, that still give every SM a dozen blocks, 32 at least.  Routing,
-// 64 detectors, 32 / 64 / 128 queries: 1 x 128 tokens 37 / 63 / 117 us, 8 x 128 86 / 91 / 136, 4 x 256 117 / 121 / 139, 64 x 128
-// 529 / 467 / 458, 1 x 1024 453 / 413 / 410 (with every query of a key range in one block 851).
+// Queries of one block of the pair kernels: the most, up to 128, that still give every SM a dozen blocks.
+// Routing (`resident`: blocks an SM holds): below 32, down to 8, only while all blocks are resident at once: a block walks its
+// queries eight at a time, each step waits for the one before, so that short or few sequences take as long as their longest
+// block.  With positional anchors, 8 / 16 / 32 / 64 / 128 queries, us: 1 x 33 tokens, 16 detectors of 128 rows 19 / 27 / 39 (with a
+// warp per query 21); 64 detectors of 256 rows: 1 x 64 tokens 19 / 27 / 43, 1 x 128 27 / 31 / 46 / 63 / 117, 4 x 128 65 / 64 / 59,
+// 8 x 128 - / - / 86 / 91 / 136, 4 x 256 - / - / 117 / 121 / 139, 64 x 128 - / - / 529 / 467 / 458; 1 x 1024 tokens, 1024 rows
+// - / - / 453 / 413 / 410 (with every query of a key range in one block 851).
 // key_range: keys of one block (a block has the queries above its first key); 0: all of them, as the histogram kernel has it: its
 // blocks stage every key below their queries first, so that long sequences keep 128 queries (1 x 1024 tokens 187 us with 128
 // queries, 352 with 32; 1 x 500 tokens 64 and 42 us; 1 x 128 tokens 26 and 14 us).
-static int queries_per_block(int S, int64_t detectors_times_sequences, int key_range) {
-    const int least = key_range == 0 && S > 512 ? 128 : 32;
-    for (int q = 128; q > least; q /= 2) {
-        int64_t blocks = 0;
-        if (key_range == 0) blocks = (S + q - 1) / q;
+static int queries_per_block(int S, int64_t detectors_times_sequences, int key_range, int resident) {
+    const int64_t sm = device_info().sm_count;
+    auto blocks = [&](int q) {
+        int64_t n = 0;
+        if (key_range == 0) n = (S + q - 1) / q;
         else
-            for (int k0 = 0; k0 < S - 1; k0 += key_range) blocks += (S - 1 - k0 + q - 1) / q;
-        if (blocks * detectors_times_sequences >= 12 * (int64_t)device_info().sm_count) return q;
-    }
-    return least;
+            for (int k0 = 0; k0 < S - 1; k0 += key_range) n += (S - 1 - k0 + q - 1) / q;
+        return n * detectors_times_sequences;
+    };
+    const int least = key_range == 0 && S > 512 ? 128 : 32;
+    for (int q = 128; q > least; q /= 2)
+        if (blocks(q) >= 12 * sm) return q;
+    int q = least;
+    if (key_range != 0)
+        while (q > kTileQ && blocks(q / 2) <= resident * sm) q /= 2;
+    return q;
 }
 
 static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int64_t n, cudaStream_t stream) {
@@ -958,7 +968,7 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     const bool packed = T > 512;
     // warps per block: what puts the most warps on an SM (a wide table's counters leave room for one block only, which then
     // has to bring them all); very long sequences leave the positional operands in global memory
-    h.queries = queries_per_block(c.S, (int64_t)cfg->n_detectors * n, 0);
+    h.queries = queries_per_block(c.S, (int64_t)cfg->n_detectors * n, 0, 0);
     const int tiles = ((c.S < h.queries ? c.S : h.queries) + kHistTile - 1) / kHistTile;
     int warps = 0;
     for (int cap = staged_pe_anchors(cfg);; cap = 0) {
@@ -1109,7 +1119,9 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             ra.n_detectors = Nt; ra.n_anchors = cfg->n_anchors; ra.sliced = cfg->sliced_product; ra.cmp_eps = cfg->cmp_eps;
             ra.pe_cap = pe_cap; ra.pe_cells = pe_cells;
             // (no block for the last key range when its first key is the last token: it has no query)
-            ra.queries = queries_per_block(c.S, (int64_t)Nt * n, kRouteKeys);
+            const int most = cfg->n_anchors <= 8 ? 8 : 7;   // (the launch bounds of the kernel)
+            const int resident = (int)((size_t)kMaxSmemPerBlock / (route_smem + 2048));
+            ra.queries = queries_per_block(c.S, (int64_t)Nt * n, kRouteKeys, resident < most ? resident : most);
             const int ranges = (c.S - 1 + kRouteKeys - 1) / kRouteKeys, segs = (c.S - 1 + ra.queries - 1) / ra.queries;
             LUTB_REQUIRE((int64_t)ranges * segs <= 65535, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
             dim3 grid((unsigned)Nt, (unsigned)(ranges * segs), (unsigned)n);

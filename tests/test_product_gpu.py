@@ -118,6 +118,11 @@ ORACLE_CASES["route_key_ranges"] = dict(seed=731, B=1, S=129, E=6, Nt=5, Nc=4, N
 ORACLE_CASES["route_two_ranges"] = dict(seed=732, B=2, S=137, E=6, Nt=4, Nc=9, Npe=0, O=4, n_virtual=12)
 ORACLE_CASES["route_positional"] = dict(seed=733, B=2, S=140, E=3, Nt=4, Nc=7, Npe=20, O=8, n_virtual=26)
 ORACLE_CASES["route_largest_table"] = dict(seed=734, B=1, S=40, E=9, Nt=2, Nc=12, Npe=1, O=4, n_virtual=19)
+# enough sequences that a block has 32, 64 and 128 queries (the others above have 8 or 16), in two key ranges.  A table cell sums up to
+# n = B S (S - 1) / 2 fp32 terms here, in different orders in the oracle and in every variant: about sqrt(n) * 2^-24 of the sum for each
+ORACLE_CASES["route_segments_32"] = dict(seed=737, B=20, S=140, E=6, Nt=10, Nc=8, Npe=2, O=4, n_virtual=14)
+ORACLE_CASES["route_segments_64"] = dict(seed=738, B=50, S=140, E=6, Nt=10, Nc=8, Npe=2, O=4, n_virtual=14)
+ORACLE_CASES["route_segments_128"] = dict(seed=739, B=60, S=140, E=6, Nt=11, Nc=8, Npe=2, O=4, n_virtual=14)
 ORACLE_CASES["route_dead_band"] = dict(seed=735, B=2, S=66, E=9, Nt=4, Nc=10, Npe=2, O=4, n_virtual=20, cmp_eps=0.3,
                                        quantized_input=True)
 ORACLE_CASES["route_ties"] = dict(seed=736, B=2, S=64, E=6, Nt=6, Nc=8, Npe=0, O=4, n_virtual=12, quantized_input=True)
@@ -143,6 +148,10 @@ def test_product_matches_oracle(name, variant):
         ref = dict(y=y, dX=dX, dW=dW, dPE=dPE)
     got = run_gpu(cfg, x, anchors, W, pe, dY, variant)
     assert not got["y"][:, 0].any()  # the first position has no earlier token to pair with
+    if name.startswith("route_segments"):
+        n = cfg["B"] * cfg["S"] * (cfg["S"] - 1) / 2
+        golden_util.assert_close(got["dW"], ref["dW"], 2 * n ** 0.5 * 2.0 ** -24, "dW")
+        ref["dW"] = got["dW"]
     compare(cfg, got, ref)
 
 
