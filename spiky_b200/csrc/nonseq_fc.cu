@@ -874,7 +874,8 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
     // few samples: small blocks, or (a sample's row has one owner where it is written) 32 detectors a block, so that more SMs
     // share the work
     const bool few = blocks < 2 * sm;
-    const int group_dets = few && !rows ? min(Nt, 32) : Nt, dx_warps = few && rows ? 2 : warps;
+    // (32 at a time; more where a grid would have no room for the groups)
+    const int group_dets = few && !rows ? min(Nt, max(32, (int)(((int64_t)Nt + 65534) / 65535))) : Nt, dx_warps = few && rows ? 2 : warps;
     if (write_dx && dX != nullptr && !rows) {
         const int rc = lutb_zero_buffers(dX, batch * (int64_t)cfg->n_inputs * 4, nullptr, 0, nullptr, 0, stream);
         if (rc) return rc;

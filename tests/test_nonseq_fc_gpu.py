@@ -313,3 +313,35 @@ def test_forward_gather_of_very_wide_scalar_rows():
     dm.forward_step(W, 2, x, torch.tensor([0, 1], dtype=torch.int32, device="cuda"), y, idx)
     assert idx.tolist() == [1, 0]
     assert torch.equal(y.view(2, O), W.view(2, O).flip(0))
+
+
+def test_input_gradient_of_very_many_detectors():
+    """More groups of 32 detectors than a grid has rows (few samples): 2.1 M detectors of two rows."""
+    import ctypes
+    from spiky_b200 import _native
+
+    B, I, Nt = 2, 5000, 65535 * 32 + 33
+    g = torch.Generator(device="cuda").manual_seed(3)
+    W = torch.randn(Nt, 2, 4, device="cuda", generator=g)
+    dY = torch.randn(B, 4, device="cuda", generator=g)
+    first = torch.randint(0, I, (Nt,), device="cuda", generator=g)
+    anchors = torch.stack([first, (first + 1) % I], 1).int().contiguous()
+    idx = torch.randint(0, 2, (B, Nt), device="cuda", generator=g, dtype=torch.int32)
+    md = torch.randn(B, Nt, device="cuda", generator=g)
+    mk = torch.zeros(B, Nt, dtype=torch.int32, device="cuda")
+    dX = torch.zeros(B, I, device="cuda")
+    cfg = _native.LayerCfg(n_inputs=I, n_outputs=4, n_detectors=Nt, n_anchors=1, seq_len=1, pos_dim=0, forward_group=32,
+                           backward_group=32, int_mode=0, sliced_product=0, cmp_eps=0.0, reserved0=0.0, int_rescaler=1.0,
+                           lr_meta=1.0)
+    _native.check(_native.lib().lutb_nonseq_fc_backward(
+        ctypes.byref(cfg), B, W.data_ptr(), dY.data_ptr(), anchors.data_ptr(), idx.data_ptr(), md.data_ptr(), mk.data_ptr(),
+        dX.data_ptr(), None, _native.SKIP_TABLE_GRADIENT, 0, None, 0, torch.cuda.current_stream().cuda_stream))
+    sign = 2.0 * idx.double() - 1.0
+    dot = sign * torch.einsum("bo,to->bt", dY.double(), (W[:, 1] - W[:, 0]).double())
+    du = torch.where(md > 0, 0.5, -0.5) / (1.0 + md.double().abs()) ** 2 * dot
+    want = torch.zeros(B, I, dtype=torch.float64, device="cuda")
+    for b in range(B):
+        want[b].index_add_(0, anchors[:, 0].long(), du[b])
+        want[b].index_add_(0, anchors[:, 1].long(), -du[b])
+    # a cell sums about 840 fp32 terms
+    golden_util.assert_close(dX.cpu().numpy(), want.cpu().numpy(), 1e-5, "dX")
