@@ -920,7 +920,9 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
                 case 32: launch_rc = launch(fc_input_grad_kernel<32, 1, false>, fc_input_grad_kernel<32, 1, true>); break;
                 case 16: launch_rc = launch(fc_input_grad_kernel<16, 1, false>, fc_input_grad_kernel<16, 1, true>); break;
                 case 8: launch_rc = launch(fc_input_grad_kernel<8, 1, false>, fc_input_grad_kernel<8, 1, true>); break;
-                default: launch_rc = launch(fc_input_grad_kernel<4, 1, false>, fc_input_grad_kernel<4, 1, true>); break;
+                case 4: launch_rc = launch(fc_input_grad_kernel<4, 1, false>, fc_input_grad_kernel<4, 1, true>); break;
+                case 2: launch_rc = launch(fc_input_grad_kernel<2, 1, false>, fc_input_grad_kernel<2, 1, true>); break;
+                default: launch_rc = launch(fc_input_grad_kernel<1, 1, false>, fc_input_grad_kernel<1, 1, true>); break;
             }
         }
         if (launch_rc) return launch_rc;

@@ -241,7 +241,8 @@ def test_check_detectors_row_and_detector_splits(rows, I, Nt, Nc):
 
 @pytest.mark.parametrize("B,I,Nt,Nc,O", [(1, 7, 1, 1, 1), (9, 33, 5, 4, 4), (70, 100, 33, 6, 12), (600, 50, 70, 5, 33),
                                          (2400, 64, 64, 6, 32), (2403, 37, 16, 8, 64), (2500, 2052, 20, 3, 132),
-                                         (2400, 63, 40, 4, 5), (19000, 24, 9, 4, 8)])
+                                         (2400, 63, 40, 4, 5), (19000, 24, 9, 4, 8), (2500, 40, 40, 4, 1), (33, 40, 40, 4, 2),
+                                         (2500, 60, 35, 4, 2), (2500, 60, 35, 4, 3)])
 def test_input_gradient_kernel_splits(B, I, Nt, Nc, O):
     """Lane groups of every width, rows of several steps, few samples (32 detectors a block) and many; the input gradient
     added to what is there and written over what is there (with rows that fit shared memory and longer ones)."""
