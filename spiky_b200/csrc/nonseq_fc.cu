@@ -606,8 +606,10 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
 // --------------------------------------------------------------------------------------------
 // WRITE: dX is written instead of added to (and need not be cleared): the warp sums its sample's row in shared memory and
 // writes it out once.
+// Blocks an SM: 8 lanes a group with vector loads need 80 registers for two detectors in flight (at 64 they spilled: 65536 samples,
+// 64 detectors of 64 rows x 32 outputs 187 -> 165 us, 5000 samples 23 -> 19).
 template <int LG, int VEC, bool WRITE>
-__global__ void __launch_bounds__(256, LG >= 16 ? 2 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
+__global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                            const int2 *__restrict__ anchors,
                                                            const int32_t *__restrict__ idx,
                                                            const float *__restrict__ min_delta,
@@ -892,7 +894,8 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
             cfg->n_anchors, T, cfg->forward_group, cfg->int_rescaler);
     } else {
         const int groups = (Nt + group_dets - 1) / group_dets;
-        int64_t per_block = (batch * groups / ((int64_t)sm * 16) + dx_warps - 1) / dx_warps * dx_warps;
+        // (many short blocks: the last wave of 16 blocks an SM was a fifth empty, 60000 samples x 4000 inputs 216 -> 195 us)
+        int64_t per_block = (batch * groups / ((int64_t)sm * 32) + dx_warps - 1) / dx_warps * dx_warps;
         if (per_block < dx_warps) per_block = dx_warps;
         if (per_block > 4096) per_block = 4096;
         const dim3 grid((unsigned)((batch + per_block - 1) / per_block), (unsigned)groups);
