@@ -241,7 +241,7 @@ constexpr size_t kCheckBudget = 100 * 1024;   // staged rows of a block: two res
 // detectors, 2 to 13 anchors, training and evaluation; figures in us, two lanes / one lane a detector:
 //  - rows that leave room for one block of 1024 threads (the other side: 4 rows): many anchors and detectors, and row tiles for
 //    most of the SMs: 4096 rows x 4096 inputs, 4096 detectors of 8 anchors 0.78 of the time; 8192 x 4000, 16 detectors 291 / 109,
-//    1000 detectors of 2 anchors 60 / 56, 64 rows, 1000 of 8 10.4 / 6.3
+//    1000 detectors of 2 anchors 60 / 56, 64 rows, 1000 of 8 10.4 / 6.3; 100 x 6000, 4096 of 8 10.8 / 15.0; 20000 x 7000, 500 of 8 0.8
 //  - few detectors: one lane each leaves an SM short of threads, the sooner the more shared memory their rows take: 32768 x 784,
 //    64 detectors 0.87, 32768 x 3000, 64 detectors 0.6, 128 detectors 0.74; 100000 x 32, 64 detectors of 4 47 / 39
 //  - long rows: 32768 x 3000, 256 detectors of 6 0.9; x 1500 to 2048 0.93 to 0.97, of 2 anchors in evaluation 1.1
@@ -252,9 +252,12 @@ static bool two_lanes(int64_t rows, int n_inputs, int n_detectors, int n_anchors
     const int64_t tiles = (rows + 7) / 8;
     const int sm = device_info().sm_count;
     if (rows < 8 || staged > (size_t)kMaxSmemPerBlock - 1024) return false;
-    if (staged > kCheckBudget)
-        return n_anchors >= 6 && n_detectors >= 768 && tiles * ((n_detectors + 511) / 512) >= sm - sm / 8 &&
-               (rows <= 16384 || n_detectors >= 2048 || n_anchors >= 8);
+    if (staged > kCheckBudget) {
+        const int64_t items = tiles * ((n_detectors + 511) / 512);
+        if (n_anchors < 6) return false;
+        if (staged_bytes(4, n_inputs) > kCheckBudget) return n_detectors >= 448 && items >= sm / 3;   // (the other side: 2 rows)
+        return n_detectors >= 768 && items >= 2 * sm / 3 && (rows <= 16384 || n_detectors >= 2048 || n_anchors >= 8);
+    }
     if (n_detectors <= 32) return staged < 22 * 1024;
     if (n_detectors <= 128 && staged >= 22 * 1024) return true;
     if (n_detectors <= 64 && rows <= 8192) return true;

@@ -205,7 +205,7 @@ def test_sorted_variant_rejects_missing_workspace():
 @pytest.mark.parametrize("rows,I,Nt,Nc", [(1, 5, 1, 1), (8, 64, 33, 6), (9, 63, 257, 7), (700, 100, 300, 2), (2403, 30, 390, 6),
                                           (2500, 40, 24, 3), (8, 3200, 40, 4), (17, 3201, 40, 5), (19, 4096, 600, 8),
                                           (520, 4096, 770, 6), (523, 7232, 769, 7), (523, 7233, 769, 7), (17, 6400, 40, 5),
-                                          (17, 6401, 40, 3), (5, 9000, 31, 8)])
+                                          (17, 6401, 40, 3), (400, 6401, 450, 6), (5, 9000, 31, 8)])
 def test_check_detectors_row_and_detector_splits(rows, I, Nt, Nc):
     """Eight rows with one or two threads a detector (in one or two blocks per SM; 3200 and 7232 inputs are the longest that
     leave room for two and for one), fewer rows for longer inputs, anchor lists read two at a time or one by one, unused
