@@ -405,8 +405,9 @@ int lutb_infer_int8_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const i
                                void *stream);
 /*
  * The same with a workspace, and the fp32 counterpart (lutb_nonseq_fc_forward in its evaluation form): large layers
- * gather from tables staged in shared memory.  The workspace functions return the bytes a call can use, 0 where the
- * plain gather is the better one (workspace NULL selects it); alignment 256 bytes.  y / acc are accumulated into.
+ * gather from tables staged in shared memory.  The workspace functions return the bytes a call can use, about 800 MB at most
+ * (larger batches run in passes), 0 where the plain gather is the better one or not even a pass of 1024 samples fits
+ * (workspace NULL selects it); alignment 256 bytes.  y / acc are accumulated into.
  */
 size_t lutb_infer_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch, int dequant);
 int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t batch, const int8_t *q_tables, const float *scales,
@@ -416,7 +417,10 @@ size_t lutb_infer_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch);
 int lutb_infer_fp32_accumulate(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const float *x,
                                const int32_t *anchors, float *y, int32_t *idx, void *workspace, size_t workspace_bytes,
                                void *stream);
-/* Clears up to three buffers in one launch (sizes in bytes, multiples of 4; 4-byte aligned; size 0: none). */
+/*
+ * Clears up to three buffers (sizes in bytes, multiples of 4; 4-byte aligned; size 0: none): those below 1 MB in one launch,
+ * each larger one by a memset of its own.
+ */
 int lutb_zero_buffers(void *a, int64_t a_bytes, void *b, int64_t b_bytes, void *c, int64_t c_bytes, void *stream);
 int lutb_fixed_to_float(float *buffer, int64_t n, double int_rescaler, void *stream);
 

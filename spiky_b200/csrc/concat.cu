@@ -671,7 +671,8 @@ static int launch_concat_pairs_backward(const lutb_layer_cfg *cfg, int64_t batch
     double lr = cfg->lr_meta;
     if (external_lr >= 0.0) lr *= -(double)(float)external_lr;
     const int2 *an = reinterpret_cast<const int2 *>(anchors);
-    // the bound of the entry point: token state plus eight rows of dY
+    // the bound of the entry point, token state plus eight rows of dY, is an older kernel's and more than the launches below take:
+    // what was refused stays refused
     LUTB_REQUIRE(((size_t)((6 * S + 3) & ~3) + (size_t)8 * ((O + 3) & ~3)) * 4 <= (size_t)kMaxSmemPerBlock - 1024, LUTB_ERR_SHAPE,
                  "sequence too long for the sequence kernels");
     const int64_t per = samples_per_launch(Nt);

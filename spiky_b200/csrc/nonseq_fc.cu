@@ -601,16 +601,16 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
 // to a double per lane; the lanes of a group transpose-reduce their detectors' sums in double (one shuffle step per halving
 // of the detectors instead of a full reduction each), so that every lane ends with one detector's dot product and the
 // surrogate derivative (a double division) and the two reductions into dX run on 32 lanes.
-// Bound: load/store wavefronts (75 % of their peak at 65536 samples x 64 detectors of 64 rows x 32 outputs), latency where
-// samples are few.  Measured (one detector a group in flight, a full reduction per detector before), with the clearing of dX:
+// Bound: the latency of the row reads and load/store wavefronts (half of their peak at 65536 samples x 64 detectors of 64 rows x 32
+// outputs).  Measured (one detector a group in flight, a full reduction per detector before), with the clearing of dX:
 // 256 samples 10.9 -> 8.6 us; 1111 samples, 50 detectors, 33 outputs 32.0 -> 14.8 us; 512 samples, 64 detectors, 10 outputs
-// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.9 us; 65536 samples 187 -> 187 us.
+// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.5 us; 65536 samples 187 -> 167 us.
 // (Walking groups of detectors whose tables fit L1 measured 220 us there: the groups leave lanes idle.)
 // --------------------------------------------------------------------------------------------
 // WRITE: dX is written instead of added to (and need not be cleared): the warp sums its sample's row in shared memory and
 // writes it out once.
 // Blocks an SM: 8 lanes a group with vector loads need 80 registers for two detectors in flight (at 64 they spilled: 65536 samples,
-// 64 detectors of 64 rows x 32 outputs 187 -> 165 us, 5000 samples 23 -> 19).
+// 64 detectors of 64 rows x 32 outputs 187 -> 167 us, 5000 samples 23 -> 19).
 template <int LG, int VEC, bool WRITE>
 __global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                            const int2 *__restrict__ anchors,

@@ -835,8 +835,9 @@ static int launch_contract(KernelId id, GemmArgs g, int batches, cudaStream_t st
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// Shared memory the routing kernel of the direct staging (product_pairs.cuh) would take: the bound on the sequence length
-// of this path.
+// The bound on the sequence length of this path: the shared memory that a routing kernel staging whole sequences as the direct
+// kernels do (product_pairs.cuh) would take.  What is launched takes less: the histogram kernel without staged positional operands
+// (n_anchors + 1) floats a token, the routing kernel at most 181 KB whatever the length.
 static size_t stage_bytes(const ProductCall &c, size_t per_warp_floats) {
     return (pair_stage_floats(c.S, c.cfg->n_anchors, c.cfg->pos_dim) + (size_t)8 * per_warp_floats) * 4;
 }

@@ -91,7 +91,7 @@ def test_state_dict_round_trip():
 
 @pytest.mark.parametrize("sizes", [(1, 0, 0), (0, 5, 1023), (1024, 1025, 0), (3, 300001, 7), (0, 0, 0)])
 def test_zeroed_buffers(sizes):
-    """One launch clears up to three buffers: pieces of 4 KB, ragged ends, sizes of zero, unaligned starts."""
+    """One call clears up to three buffers: pieces of 4 KB, a memset from 1 MB on, ragged ends, sizes of zero, unaligned starts."""
     from spiky_b200 import _native
     from spiky_b200.lut_layer import _zeros
 
