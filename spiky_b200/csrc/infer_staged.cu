@@ -344,7 +344,8 @@ constexpr int64_t kPassSamples = 16384, kPassBytes = 800ll << 20;
 // here while the plain gather's chains get short, and more exact: they stay there; 36 outputs (two slices, the second nearly
 // empty) 46 / 93 at 1 sample, 134 / 146 at 4096 with 1024 detectors.  Wide rows, few samples: 1024 detectors x 256 rows x 1024
 // outputs, 1 sample 245 / 204, 64 samples 254 / 338; 512 detectors x 4096 outputs 435 / 107 at 1 sample, 452 / 370 at 256;
-// 256 outputs 64 / 58 and 64 / 97 at 1 and 256 samples with 512 detectors, 93 / 107 at 1 sample with 1024.  Tables in L2: 512
+// 256 outputs 64 / 58 and 64 / 97 at 1 and 256 samples with 512 detectors, 93 / 107 at 1 sample with 1024; 4096 detectors x 64 rows x
+// 512 outputs, 8 samples 431 / 594.  Tables in L2: 512
 // detectors x 16 rows x 512 outputs 71 / 58 at 256 samples.  A little more than one wave of work items is as slow as two: 512
 // detectors x 36 outputs x 4096 samples 91 / 81.
 // int8, from 1024 detectors on: 4096 detectors x 64 outputs 56 / 245, 183 / 318, 540 / 812, 1857 / 2440; 1024 detectors 50 / 68,
@@ -357,7 +358,7 @@ static bool staged_fp32_pays(int64_t batch, int Nt, int T, int O) {
     const int64_t items = (int64_t)((Nt + kDetBlock - 1) / kDetBlock) * ((batch + kTile - 1) / kTile) * ((O + kRow - 1) / kRow);
     if (Nt < 1024 && batch > kTile && items > sm && 2 * items < 3 * sm) return false;
     if (batch >= 512 || O <= (Nt < 1024 ? 128 : 256)) return true;
-    return O <= 1024 && batch >= (Nt < 1024 ? 128 : 32) && (int64_t)Nt * T >= 65536;
+    return O <= 1024 && batch * Nt >= (Nt < 1024 && O <= 512 ? 65536 : 32768) && (int64_t)Nt * T >= 65536;
 }
 static bool staged_int8_pays(int64_t batch, int O) { return O <= 512 || batch >= 256 || (O <= 1024 && batch >= 8); }
 

@@ -179,9 +179,12 @@ __global__ void __launch_bounds__(D == 2 ? 1024 : 256) check_detectors_kernel(co
             // (the bytes of rows past the end lie in the row's padding)
             uint8_t *dst = packed + (size_t)t * packed_pitch + row0 + half * RT;
             if constexpr (RT % 4 == 0) {
+                uint32_t four[RT / 4];
 #pragma unroll
                 for (int r = 0; r < RT; r += 4)
-                    *reinterpret_cast<uint32_t *>(dst + r) = (uint32_t)li[r] | (uint32_t)li[r + 1] << 8 | (uint32_t)li[r + 2] << 16 | (uint32_t)li[r + 3] << 24;
+                    four[r / 4] = (uint32_t)li[r] | (uint32_t)li[r + 1] << 8 | (uint32_t)li[r + 2] << 16 | (uint32_t)li[r + 3] << 24;
+                if constexpr (RT == 8) *reinterpret_cast<uint2 *>(dst) = make_uint2(four[0], four[1]);
+                else *reinterpret_cast<uint32_t *>(dst) = four[0];
             } else {
 #pragma unroll
                 for (int r = 0; r < RT; r++) dst[r] = (uint8_t)li[r];
@@ -246,8 +249,9 @@ constexpr size_t kCheckBudget = 100 * 1024;   // staged rows of a block: two res
 //    64 detectors 0.87, 32768 x 3000, 64 detectors 0.6, 128 detectors 0.74; 100000 x 32, 64 detectors of 4 47 / 39
 //  - long rows: 32768 x 3000, 256 detectors of 6 0.9; x 1500 to 2048 0.93 to 0.97, of 2 anchors in evaluation 1.1
 //  - a few row tiles per SM, which are all there is to fill it: 4096 x 300, 1024 detectors of 7 29 / 39; 32768 rows 1.1 to 1.2
+//  - indices that also leave as bytes (`packed`: 8 or 4 bytes a thread, `pitch` apart): 4096 x 512, 2048 detectors of 4 38 / 48
 //  - many anchors and detectors: 32768 x 784, 768 detectors of 8 anchors 0.95; 100000 x 32, 300 of 3 222 / 149
-static bool two_lanes(int64_t rows, int n_inputs, int n_detectors, int n_anchors) {
+static bool two_lanes(int64_t rows, int n_inputs, int n_detectors, int n_anchors, bool packed) {
     const size_t staged = staged_bytes(8, n_inputs);
     const int64_t tiles = (rows + 7) / 8;
     const int sm = device_info().sm_count;
@@ -258,6 +262,7 @@ static bool two_lanes(int64_t rows, int n_inputs, int n_detectors, int n_anchors
         if (staged_bytes(4, n_inputs) > kCheckBudget) return n_detectors >= 448 && items >= sm / 3;   // (the other side: 2 rows)
         return n_detectors >= 768 && items >= 2 * sm / 3 && (rows <= 16384 || n_detectors >= 2048 || n_anchors >= 8);
     }
+    if (packed && tiles >= sm) return true;
     if (n_detectors <= 32) return staged < 22 * 1024;
     if (n_detectors <= 128 && staged >= 22 * 1024) return true;
     if (n_detectors <= 64 && rows <= 8192) return true;
@@ -274,7 +279,7 @@ int launch_check_detectors(const float *x, int64_t rows, int n_inputs, const int
     // rows per group: 8 while two blocks fit an SM (each anchor pair is fetched once per 8 rows), or one block of twice the threads
     // where that pays; fewer for few or longer rows
     const size_t row_bytes = (size_t)n_inputs * sizeof(float);
-    const int D = two_lanes(rows, n_inputs, n_detectors, n_anchors) ? 2 : 1;
+    const int D = two_lanes(rows, n_inputs, n_detectors, n_anchors, packed != nullptr) ? 2 : 1;
     int R = 8;
     while (R > 1 && (rows < R || (D == 1 && staged_bytes(R, n_inputs) > kCheckBudget))) R >>= 1;
     // threads per row group: D per detector, rounded to warps; at most 256 detectors, or 512 where the rows leave room for one block
