@@ -638,7 +638,7 @@ static int launch_concat_pairs_forward(const lutb_layer_cfg *cfg, int64_t batch,
     KernelScope scope(K_CONCAT_FORWARD, st);
     if (cfg->int_mode) {
         dim3 grid((unsigned)Nt, (unsigned)batch);
-        if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(concat_forward_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(concat_forward_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         concat_forward_fixed_kernel<<<grid, 256, smem, st>>>(weights, idx, pos_idx, y, S, O, Nt, Nc, npe, cfg->int_rescaler, j_begin, j_end);
         LUTB_LAUNCH_CHECK();
         return LUTB_OK;
@@ -650,7 +650,7 @@ static int launch_concat_pairs_forward(const lutb_layer_cfg *cfg, int64_t batch,
         const int n = (int)min(per, batch - b0);
         const int rc = dispatch_pair_kernel(vec4, O, [&](auto lg, auto vec) -> int {
             auto kern = concat_forward_kernel<lg.value, vec.value>;
-            if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             kern<<<(unsigned)((int64_t)Nt * n), threads, smem, st>>>(weights, idx + b0 * S * Nt, pos_idx, y + b0 * S * O, n, S, O, Nt, Nc,
                                                                    npe, j_begin, j_end);
             return LUTB_OK;
@@ -689,7 +689,7 @@ static int launch_concat_pairs_backward(const lutb_layer_cfg *cfg, int64_t batch
             const int64_t tok = b0 * S;
             const int rc = dispatch_pair_kernel(vec4, O, [&](auto lg, auto vec) -> int {
                 auto kern = concat_backward_kernel<lg.value, vec.value, DX, DWF>;
-                if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 kern<<<(unsigned)((int64_t)Nt * n), threads, smem, st>>>(
                     weights, dY + tok * O, an, idx + tok * Nt, min_delta + tok * Nt, min_k + tok * Nt, pos_idx, pos_min_delta, pos_min_k,
                     dX + tok * cfg->n_inputs, dPE, target, n, S, cfg->n_inputs, O, Nt, Nc, npe, lr, j_begin, j_end, smem_dx);

@@ -123,7 +123,7 @@ int launch_fc_dw_sorted(const float *dY, const int32_t *idx, float *target, int6
     dw_sort_scan_kernel<<<(unsigned)n_detectors, 1024, 0, stream>>>(counts, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const size_t smem = (size_t)table_rows * sizeof(int32_t);
-    if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const int64_t segs = (int64_t)n_detectors * table_rows;
@@ -269,7 +269,7 @@ int launch_fc_dw_rows(const float *dY, const int32_t *idx, int64_t batch, int n_
     dw_sort_scan_kernel<<<(unsigned)n_detectors, 1024, 0, stream>>>(counts, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const size_t smem = (size_t)table_rows * sizeof(int32_t);
-    if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const int64_t n_seg = (int64_t)n_detectors * table_rows;

@@ -18,6 +18,9 @@ constexpr float kEpsF = 1e-17f;
 constexpr int32_t kNoAnchor = -1;                      // 0xFFFFFFFF marks an unused anchor pair
 
 constexpr int kMaxSmemPerBlock = 227 * 1024;  // opt-in dynamic shared memory limit on sm_100
+// Dynamic shared memory a launch takes without opting in.  (48 KB is the limit for dynamic and static arrays together: a histogram block of
+// 47.75 KB beside 0.7 KB of static arrays was refused.)
+constexpr size_t kPlainSmem = 40 * 1024;
 
 void set_error(const char *fmt, ...);
 

@@ -230,7 +230,7 @@ static int launch_check_detectors_r(const float *x, int64_t rows, int n_inputs, 
     LUTB_REQUIRE(blocks <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "batch too large for one launch");
     const bool train = min_delta != nullptr;
     auto kern = train ? check_detectors_kernel<R, D, true> : check_detectors_kernel<R, D, false>;
-    if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     KernelScope scope(K_CHECK_DETECTORS, stream);
     kern<<<(unsigned)blocks, tpg * groups, smem, stream>>>(x, rows, n_inputs, reinterpret_cast<const int2 *>(anchors),
                                                           n_detectors, n_anchors, cmp_eps, tpg, idx, min_delta, min_k, packed, packed_pitch);
@@ -912,7 +912,7 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
         auto launch = [&](auto add, auto write) -> int {
             const size_t smem = rows ? dx_warps * row_bytes : 0;
             auto kern = rows ? write : add;
-            if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             kern<<<grid, dx_warps * 32, smem, stream>>>(W, dY, reinterpret_cast<const int2 *>(anchors), idx, min_delta, min_k, dX, batch,
                                                   cfg->n_inputs, O, Nt, cfg->n_anchors, T, group_dets, (int)per_block);
             return LUTB_OK;

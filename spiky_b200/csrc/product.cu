@@ -368,10 +368,10 @@ extern "C" int lutb_product_forward(const lutb_layer_cfg *cfg, int64_t batch, in
         dim3 grid((unsigned)cfg->n_detectors, (unsigned)batch);
         KernelScope scope(K_PRODUCT_FORWARD, st);
         if (cfg->int_mode) {
-            if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(product_forward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(product_forward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             product_forward_kernel<true><<<grid, warps * 32, smem, st>>>(weights, x1, x2, pos_embeddings, anchors, y, seq_len, n_inputs_1, n_inputs_2, cfg->pos_dim, cfg->n_outputs, cfg->n_detectors, cfg->n_anchors, cfg->sliced_product, cfg->cmp_eps, cfg->int_rescaler);
         } else {
-            if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(product_forward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(product_forward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             product_forward_kernel<false><<<grid, warps * 32, smem, st>>>(weights, x1, x2, pos_embeddings, anchors, y, seq_len, n_inputs_1, n_inputs_2, cfg->pos_dim, cfg->n_outputs, cfg->n_detectors, cfg->n_anchors, cfg->sliced_product, cfg->cmp_eps, cfg->int_rescaler);
         }
         LUTB_LAUNCH_CHECK();
@@ -419,7 +419,7 @@ extern "C" int lutb_product_backward(const lutb_layer_cfg *cfg, int64_t batch, i
             dim3 grid((unsigned)Nt, (unsigned)batch);
 #define LUTB_PROD_BWD(DX, DWF, TARGET)                                                                                   \
     do {                                                                                                                 \
-        if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(product_backward_kernel<DX, DWF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(product_backward_kernel<DX, DWF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         product_backward_kernel<DX, DWF><<<grid, warps * 32, smem, st>>>(weights, x1, x2, pos_embeddings, anchors, dY, dX1, dX2, dPE, TARGET, seq_len, n_inputs_1, n_inputs_2, npe, O, Nt, Nc, cfg->sliced_product, cfg->cmp_eps, lr); \
     } while (0)
             if (external_lr >= 0.0) {

@@ -987,7 +987,7 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     dim3 grid((unsigned)cfg->n_detectors, (unsigned)((c.S + h.queries - 1) / h.queries), (unsigned)n);
     KernelScope scope(K_PRODUCT_HIST, stream);
     auto launch = [&](auto kern) -> int {
-        if (smem > 48 * 1024) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<grid, warps * 32, smem, stream>>>(h);
         return LUTB_OK;
     };
@@ -1128,7 +1128,7 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             dim3 grid((unsigned)Nt, (unsigned)(ranges * segs), (unsigned)n);
             KernelScope scope(K_PRODUCT_ROUTE, stream);
             auto launch = [&](auto kern) -> int {
-                if (route_smem > 48 * 1024)
+                if (route_smem > kPlainSmem)
                     LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_smem));
                 kern<<<grid, 32 * kRouteWarps, route_smem, stream>>>(ra);
                 return LUTB_OK;

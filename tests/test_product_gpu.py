@@ -1,4 +1,8 @@
 """CUDA path of product-mode sequence (attention) layers against the reference's golden vectors and the oracle."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -216,6 +220,29 @@ def test_product_histogram_rejects_unsupported():
     x, anchors, W, pe, dY = inputs_for(cfg)
     with pytest.raises(ValueError, match="histogram variant"):
         run_gpu(cfg, x, anchors, W, pe, dY, 2)
+
+
+@pytest.mark.parametrize("S,Npe", [(176, 2), (300, 0)])
+def test_histogram_blocks_just_below_48_kb(S, Npe):
+    """Dynamic shared memory that leaves no room for the kernel's static arrays in the 48 KB a launch has without opting in.
+    In a process of its own: an earlier, larger launch of the same kernel would have opted in for it."""
+    code = (
+        "import torch\n"
+        "from spiky_b200.lut_layer import LUTLayer, SynapseMeta\n"
+        f"layer = LUTLayer(16, 8, 3, 8, sequence_length={S}, concatenation_product=False, positional_dim={Npe}, random_seed=1,\n"
+        "                 synapse_meta=SynapseMeta(min_weight=-1.0, max_weight=1.0), device='cuda:0')\n"
+        "with torch.no_grad():\n"
+        "    layer._weights.normal_()\n"
+        f"x, out = torch.randn(1, {S}, 16, device='cuda'), []\n"
+        "for variant in (2, 3, 1):\n"
+        "    layer._product_variant = variant\n"
+        "    out.append(layer(x).detach())\n"
+        "for y in out[:2]:\n"
+        "    assert (y - out[2]).abs().max() <= 1e-5 * out[2].abs().max()\n"
+    )
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 def test_product_autograd_unified_pe():
