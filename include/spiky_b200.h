@@ -268,15 +268,14 @@ int lutb_product_forward(const lutb_layer_cfg *cfg, int64_t batch, int32_t seq_l
  *   DIRECT  one table row per (pair, detector) is gathered (forward) or gathered twice and scatter-added
  *           (backward) through L2; needs no workspace.
  *   HIST    per (query, detector) the selected rows are counted into a histogram first and the pass becomes dense
- *           contractions with the tables (see spiky_b200/csrc/product_hist.cuh): on the tensor cores when the library
- *           was built with them (lutb_fp32_gemm_available) and the workspace holds one sequence in their operand
- *           layout, else as register-tiled fp32 FMA contractions; fp32 accumulators only, 4 <= Nc <= 12, O % 4 == 0,
+ *           contractions with the tables (see spiky_b200/csrc/product_hist.cuh): on the tensor cores when the
+ *           workspace holds one sequence and their operand copies and S <= 2048, else as register-tiled fp32 FMA contractions; fp32 accumulators only, 4 <= Nc <= 12, O % 4 == 0,
  *           16-byte aligned tensors, and a caller workspace of at least lutb_product_workspace(cfg, 1, S, backward)
  *           bytes (the batch is processed in chunks of as many sequences as fit); LUTB_ERR_WORKSPACE / LUTB_ERR_MODE
  *           when asked for and not possible.
  *   HIST_FMA  HIST with the fp32 FMA contractions forced.
  *   AUTO    HIST when it is possible, a workspace is supplied and the sequence is long enough against the
- *           table (4 * S >= 2^Nc; forward without tensor cores: S >= 2^Nc), else DIRECT.
+ *           table (4 * S >= 2^Nc), else DIRECT.
  * lutb_product_workspace returns the bytes that let `batch` sequences go through in one chunk.
  */
 #define LUTB_PRODUCT_AUTO 0
@@ -444,19 +443,17 @@ int lutb_dense_to_sparse_32(void *source, int64_t n, int64_t *indices, void *val
 /*
  * fp32 GEMM on the sm_100a tensor cores with fp32-class accuracy (no reference counterpart; the reference has no
  * dense contraction): C [m x n] row-major = alpha * op(A) . op(B) + beta * C.  Default route: every operand is written
- * once as hi (x rounded to TF32) and lo = x - hi, and hi.hi + hi.lo + lo.hi is formed by TF32 GEMMs on concatenated
- * copies (tcgen05.mma, fp32 accumulators in tensor memory, operands staged by TMA); with
+ * once as hi (x rounded to TF32) and lo = x - hi, and hi.hi + hi.lo + lo.hi is formed by TF32 GEMMs on the copies (tcgen05.mma, fp32 accumulators in tensor memory, operands staged by TMA); with
  * LUTB_GEMM_FAST_FP32 or'ed into `kind` a single GEMM splits the operands into BF16 terms inside its mainloop
  * instead (no scratch copies, about half the speed).  Either way results agree with an fp32 FMA contraction to about
- * 1e-6 relative.  The long-sequence (histogram) path of the product-mode layer runs its three contractions through the
- * default route.
+ * 1e-6 relative.  (The histogram path of the product-mode layer has contractions of its own.)
  *   kind  LUTB_GEMM_A_ROWS_B_ROWS_OF_N: A [m x k] row-major, B stored as [n x k] row-major (C = A . B^T)
  *         LUTB_GEMM_A_ROWS_B_ROWS_OF_K: A [m x k] row-major, B stored as [k x n] row-major (C = A . B)
  *         LUTB_GEMM_A_COLS_B_ROWS_OF_K: A stored as [k x m] row-major, B as [k x n] row-major (C = A^T . B)
  * Pointers 16-byte aligned, leading dimensions and row lengths multiples of 4; workspace of
  * lutb_fp32_gemm_workspace(m, n, k) bytes (it holds the hi / lo copies).
  * lutb_fp32_gemm_available() is 0 when the library was built without a CUTLASS header tree (the call then fails with
- * LUTB_ERR_MODE and the histogram path keeps its fp32 FMA contractions).
+ * LUTB_ERR_MODE).
  */
 #define LUTB_GEMM_A_ROWS_B_ROWS_OF_N 0
 #define LUTB_GEMM_A_ROWS_B_ROWS_OF_K 1

@@ -1,16 +1,15 @@
-// fp32 GEMMs on the sm_100a tensor cores for the contractions of the product-mode histogram path.
+// General fp32 GEMMs on the sm_100a tensor cores (lutb_fp32_gemm; the histogram path of the product-mode layer has kernels of
+// its own, hist_gemm_sm100.cu).
 //
-// The contractions (product_hist.cuh) multiply exact small integers (row counts) or fp32 tables / gradients and must
-// keep fp32 accuracy (parity bar 1e-5), so plain TF32 or BF16 inputs are not an option.  Two routes, both CUTLASS 3
+// Results keep fp32 accuracy (1e-5), so plain TF32 or BF16 inputs are not an option.  Two routes, both CUTLASS 3
 // collectives instantiated for sm_100a (operands arrive in shared memory by TMA - a cluster of one block or one pair: plain copies of this
 // GPU's own memory -, tcgen05.mma accumulates in fp32 in tensor memory, the epilogue reads the accumulators back with
 // tcgen05.ld and applies alpha / beta):
 //
 //   split TF32 (default)  every fp32 operand x is written once as hi = x rounded to TF32 and lo = x - hi (exact)
 //                         rounded to TF32, and the product is formed as hi.hi + hi.lo + lo.hi; concatenated copies
-//                         make that ONE TF32 GEMM wherever the layouts allow.  An operand that holds integers below
-//                         2048 (row counts) is exact in TF32 and needs no split.  The dropped lo.lo term and the
-//                         rounding of lo are each below 2^-22 relative.
+//                         make that ONE TF32 GEMM where the layouts allow.  The dropped lo.lo term and the rounding of lo are each
+//                         below 2^-22 relative.
 //   fast fp32             one GEMM whose mainloop splits the operands into three BF16 terms on the fly (CUTLASS'
 //                         "FastF32" schedule); simpler, no scratch, but bound by the conversion work: 80-90 TFLOP/s on
 //                         the contraction shapes against 2-3 times that for the split TF32 route.
@@ -20,13 +19,13 @@
 #include "fp32_gemm_sm100.cuh"
 
 #ifdef LUTB_NO_CUTLASS
-// built without a CUTLASS header tree: the callers keep their fp32 FMA contractions
+// built without a CUTLASS header tree
 namespace lutb {
 bool tc_gemm_available() { return false; }
-size_t tc_gemm_workspace(TcGemmKind, int, int, int, bool) { return 0; }
+size_t tc_gemm_workspace(TcGemmKind, int, int, int) { return 0; }
 size_t tc_gemm_fast_workspace(int, int, int) { return 0; }
-int tc_gemm(TcGemmKind, int, int, int, const float *, int64_t, const float *, int64_t, float *, int64_t, float, float, bool,
-            void *, size_t, cudaStream_t) {
+int tc_gemm(TcGemmKind, int, int, int, const float *, int64_t, const float *, int64_t, float *, int64_t, float, float, void *, size_t,
+            cudaStream_t) {
     set_error("the library was built without the tensor-core contractions (no CUTLASS headers at build time)");
     return LUTB_ERR_MODE;
 }
@@ -103,29 +102,21 @@ static size_t workspace_of(int M, int N, int K) {
     return Cfg::Gemm::get_workspace_size(args);
 }
 
-// `batches` independent GEMMs of the same shape in one launch; operand b of batch l starts batch_b * l elements
-// after the first (and so on); one batch by default.
-struct Batches {
-    int count = 1;
-    int64_t a = 0, b = 0, c = 0;
-};
-
 template <class Cfg>
 static int run(int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,
-               float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream,
-               Batches batches = Batches{}) {
+               float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
     typename Cfg::StrideA sa;
     typename Cfg::StrideB sb;
     typename Cfg::StrideC sc;
     // the dynamic (non unit) mode of every stride is the leading dimension
-    if constexpr (cute::is_same_v<decltype(get<1>(sa)), cute::Int<1>>) sa = make_stride(lda, Int<1>{}, batches.a);
-    else sa = make_stride(Int<1>{}, lda, batches.a);
-    if constexpr (cute::is_same_v<decltype(get<1>(sb)), cute::Int<1>>) sb = make_stride(ldb, Int<1>{}, batches.b);
-    else sb = make_stride(Int<1>{}, ldb, batches.b);
-    sc = make_stride(ldc, Int<1>{}, batches.c);
+    if constexpr (cute::is_same_v<decltype(get<1>(sa)), cute::Int<1>>) sa = make_stride(lda, Int<1>{}, int64_t(0));
+    else sa = make_stride(Int<1>{}, lda, int64_t(0));
+    if constexpr (cute::is_same_v<decltype(get<1>(sb)), cute::Int<1>>) sb = make_stride(ldb, Int<1>{}, int64_t(0));
+    else sb = make_stride(Int<1>{}, ldb, int64_t(0));
+    sc = make_stride(ldc, Int<1>{}, int64_t(0));
     using ElementAB = typename Cfg::Element;
     typename Cfg::Gemm::Arguments args{cutlass::gemm::GemmUniversalMode::kGemm,
-                                       {M, N, K, batches.count},
+                                       {M, N, K, 1},
                                        {reinterpret_cast<const ElementAB *>(A), sa, reinterpret_cast<const ElementAB *>(B), sb},
                                        {{alpha, beta}, C, sc, C, sc}};
     typename Cfg::Gemm gemm;
@@ -195,57 +186,27 @@ static int split(const float *x, int64_t rows, int64_t cols, int64_t ld, float *
     return LUTB_OK;
 }
 
-// C = alpha * sum over the slices s of (P_s[:, 0:N] + P_s[:, N:2N]) + beta * C, P_s = P + s * M * 2N; the lo halves are
-// summed first (the smaller terms), then the hi halves, in rounded fp32.
-__global__ void combine_halves_kernel(const float *__restrict__ P, float *__restrict__ C, int64_t M, int64_t N, int64_t ldc,
-                                      float alpha, float beta, int slices) {
-    const int64_t n4 = M * (N / 4);
-    const int64_t slice = M * 2 * N;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / (N / 4), c = (i - r * (N / 4)) * 4;
-        float4 lo = *reinterpret_cast<const float4 *>(P + r * 2 * N + N + c);
-        for (int s_ = 1; s_ < slices; s_++) {
-            const float4 t = *reinterpret_cast<const float4 *>(P + s_ * slice + r * 2 * N + N + c);
-            lo.x += t.x; lo.y += t.y; lo.z += t.z; lo.w += t.w;
-        }
-        float4 hi = *reinterpret_cast<const float4 *>(P + r * 2 * N + c);
-        for (int s_ = 1; s_ < slices; s_++) {
-            const float4 t = *reinterpret_cast<const float4 *>(P + s_ * slice + r * 2 * N + c);
-            hi.x += t.x; hi.y += t.y; hi.z += t.z; hi.w += t.w;
-        }
-        float4 *dst = reinterpret_cast<float4 *>(C + r * ldc + c);
-        float4 v = make_float4(alpha * (lo.x + hi.x), alpha * (lo.y + hi.y), alpha * (lo.z + hi.z), alpha * (lo.w + hi.w));
-        if (beta != 0.f) {
-            const float4 o = *dst;
-            v.x += beta * o.x; v.y += beta * o.y; v.z += beta * o.z; v.w += beta * o.w;
-        }
-        *dst = v;
-    }
-}
-
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // A pair of SMs per 256 x 256 tile or one SM per 128 x 128 tile: whichever takes less time by waves of tiles.  A wave is what
 // the SMs hold at once; a pair's tile is four times the work on twice the SMs and takes 1.6 times as long (a byte from shared
 // memory feeds twice the multiply-adds).  Padding counts: a half empty 256-row tile takes as long as a full one.  Measured on the
-// contractions of the histogram path with their operand copies, one SM / pair, us:
-// pair: 8192 x 512 x 16384 214 / 176, 16384 x 512 x 8192 (A^T . B) 214 / 166, 8192 x 16384 x 768 318 / 258; 1024 x 2048 x 65536
-//   in 8 slices 423 / 341, 65536 x 2048 x 1024 384 / 337, 1024 x 65536 x 3072 592 / 488; 512 x 16384 x 768 50 / 46
-// one SM: 128 x 16384 x 768 34 / 39, 384 x 16384 x 768 45 / 48; A^T . B 16384 x 128 x 128 20 / 22, 10240 x 320 x 800 35 / 40
+// shapes of one deep GEMM with its operand copies, one SM / pair, us:
+// pair: 8192 x 16384 x 768 318 / 258, 1024 x 65536 x 3072 592 / 488, 512 x 16384 x 768 50 / 46
+// one SM: 128 x 16384 x 768 34 / 39, 384 x 16384 x 768 45 / 48
 // even: 160 to 256 x 16384 x 768 38 / 38, 640 x 16384 x 768 55 / 55; 1024 x 4096 x 768 takes the pair at 30 / 33
-static bool pair_tiles(int M, int N, int batches) {
+static bool pair_tiles(int M, int N) {
     const int64_t sm = device_info().sm_count > 1 ? device_info().sm_count : 2;
-    const int64_t pairs = (int64_t)((M + 255) / 256) * ((N + 255) / 256) * batches, singles = (int64_t)((M + 127) / 128) * ((N + 127) / 128) * batches;
+    const int64_t pairs = (int64_t)((M + 255) / 256) * ((N + 255) / 256), singles = (int64_t)((M + 127) / 128) * ((N + 127) / 128);
     const int64_t pair_waves = (pairs + sm / 2 - 1) / (sm / 2), single_waves = (singles + sm - 1) / sm;
     return 8 * pair_waves < 5 * single_waves;
 }
 template <class Cfg>
 static int run_tiles(int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,
-                     float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream,
-                     Batches batches = Batches{}) {
-    if (pair_tiles(M, N, batches.count))
-        return run<typename PairOf<Cfg>::type>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream, batches);
-    return run<Cfg>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream, batches);
+                     float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+    if (pair_tiles(M, N))
+        return run<typename PairOf<Cfg>::type>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream);
+    return run<Cfg>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, workspace, workspace_bytes, stream);
 }
 template <class Cfg>
 static size_t workspace_of_tiles(int M, int N, int K) {
@@ -253,69 +214,32 @@ static size_t workspace_of_tiles(int M, int N, int K) {
     return a > b ? a : b;
 }
 
-// Plan of one call.  TN (both operands contraction-major): one GEMM of depth 3K on concatenated copies.  NN / TT with an
-// exact A: one GEMM of width 2N on B = [hi | lo], halves added in the epilogue pass.  Anything else: the generic
-// sequence of two or three GEMMs on separate hi / lo copies.
+// Plan of one call.  TN (both operands contraction-major): one GEMM of depth 3K on concatenated copies.  Anything else: three
+// GEMMs on separate hi / lo copies.
 struct SplitPlan {
-    int mode;            // 0: deep TN, 1: wide (exact A), 2: generic
-    int slices, kc;      // mode 1: the contraction index is cut into `slices` pieces of kc (see mode1_slices)
-    size_t gemm_ws, a_bytes, b_bytes, p_bytes;
+    bool deep;
+    size_t gemm_ws, a_bytes, b_bytes;
 };
 
-// How the wide plan cuts its contraction index.  Inside a slice the tensor core accumulates, truncating its fp32
-// accumulator after every step (a bias that grows with the length of the chain); the slices' results are added in
-// rounded fp32.  A . B with A [M x K] row-major (few output tiles, deep contraction: the forward pass of the histogram
-// path): the slices are the batches of ONE launch, each into its own partial result, which also gives the launch
-// K / kc times as many blocks.  A^T . B: the slices run one after the other and accumulate through the epilogue.  kc is
-// at least 8 N, which keeps the traffic of the partial results below half of the slice's operand traffic.
-static void mode1_slices(TcGemmKind kind, int N, int K, int *slices, int *kc) {
-    int want = ((8 * N + 255) / 256) * 256;
-    const int floor_ = kind == TC_A_ROWS_B_ROWS_OF_K ? 2048 : 8192;
-    if (want < floor_) want = floor_;
-    *slices = 1;
-    *kc = K;
-    if (kind == TC_A_ROWS_B_ROWS_OF_K) {
-        // equal slices (one batched launch): the largest count of pieces of at least `want` that divides K evenly
-        for (int l = K / want; l > 1; l--)
-            if (K % l == 0 && (K / l) % 4 == 0) {
-                *slices = l;
-                *kc = K / l;
-                break;
-            }
-    } else if (K > want) {
-        *kc = want;
-        *slices = (K + want - 1) / want;
-    }
-}
-
-static SplitPlan split_plan(TcGemmKind kind, int M, int N, int K, bool a_exact) {
+static SplitPlan split_plan(TcGemmKind kind, int M, int N, int K) {
     SplitPlan p{};
-    if (kind == TC_A_ROWS_B_ROWS_OF_N && !a_exact) {
-        p.mode = 0;
+    p.deep = kind == TC_A_ROWS_B_ROWS_OF_N;
+    if (p.deep) {
         p.gemm_ws = align256(workspace_of_tiles<Tf32TN>(M, N, 3 * K));
         p.a_bytes = align256((size_t)M * 3 * K * 4);
         p.b_bytes = align256((size_t)N * 3 * K * 4);
-    } else if (kind != TC_A_ROWS_B_ROWS_OF_N && a_exact && N % 4 == 0) {
-        p.mode = 1;
-        mode1_slices(kind, N, K, &p.slices, &p.kc);
-        p.gemm_ws = align256(kind == TC_A_ROWS_B_ROWS_OF_K ? workspace_of_tiles<Tf32NN>(M, 2 * N, K) : workspace_of_tiles<Tf32TT>(M, 2 * N, K));
-        p.b_bytes = align256((size_t)K * 2 * N * 4);
-        p.p_bytes = align256((size_t)M * 2 * N * 4 * (kind == TC_A_ROWS_B_ROWS_OF_K ? p.slices : 1));
     } else {
-        p.mode = 2;
-        size_t w = workspace_of_tiles<Tf32TN>(M, N, K);
-        const size_t w2 = workspace_of_tiles<Tf32NN>(M, N, K), w3 = workspace_of_tiles<Tf32TT>(M, N, K);
-        w = w > w2 ? w : w2;
-        p.gemm_ws = align256(w > w3 ? w : w3);
-        p.a_bytes = a_exact ? 0 : align256((size_t)M * K * 4 * 2);
+        const size_t w2 = workspace_of<Tf32NN>(M, N, K), w3 = workspace_of<Tf32TT>(M, N, K);
+        p.gemm_ws = align256(w2 > w3 ? w2 : w3);
+        p.a_bytes = align256((size_t)M * K * 4 * 2);
         p.b_bytes = align256((size_t)N * K * 4 * 2);
     }
     return p;
 }
 
-size_t tc_gemm_workspace(TcGemmKind kind, int M, int N, int K, bool a_exact) {
-    const SplitPlan p = split_plan(kind, M, N, K, a_exact);
-    return p.gemm_ws + p.a_bytes + p.b_bytes + p.p_bytes + 512;
+size_t tc_gemm_workspace(TcGemmKind kind, int M, int N, int K) {
+    const SplitPlan p = split_plan(kind, M, N, K);
+    return p.gemm_ws + p.a_bytes + p.b_bytes + 512;
 }
 
 template <class Cfg>
@@ -324,32 +248,28 @@ static int run3(int M, int N, int K, const float *Ah, const float *Al, int64_t l
     // small terms first, so that they are added to each other before they meet the large one
     int rc = run<Cfg>(M, N, K, Ah, lda, Bl, ldb, C, ldc, alpha, beta, ws, ws_bytes, stream);
     if (rc) return rc;
-    if (Al != nullptr) {
-        rc = run<Cfg>(M, N, K, Al, lda, Bh, ldb, C, ldc, alpha, 1.f, ws, ws_bytes, stream);
-        if (rc) return rc;
-    }
+    rc = run<Cfg>(M, N, K, Al, lda, Bh, ldb, C, ldc, alpha, 1.f, ws, ws_bytes, stream);
+    if (rc) return rc;
     return run<Cfg>(M, N, K, Ah, lda, Bh, ldb, C, ldc, alpha, 1.f, ws, ws_bytes, stream);
 }
 
 int tc_gemm(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C,
-            int64_t ldc, float alpha, float beta, bool a_exact, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
-    const size_t need = tc_gemm_workspace(kind, M, N, K, a_exact);
+            int64_t ldc, float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+    const size_t need = tc_gemm_workspace(kind, M, N, K);
     LUTB_REQUIRE(workspace_bytes >= need, LUTB_ERR_WORKSPACE, "tensor-core contraction needs %zu bytes of workspace", need);
     // stored extents of the operands: A is [ar x ac], B is [br x bc] (row-major, contiguous in the second)
     const int64_t ar = kind == TC_A_COLS_B_ROWS_OF_K ? K : M, ac = kind == TC_A_COLS_B_ROWS_OF_K ? M : K;
     const int64_t br = kind == TC_A_ROWS_B_ROWS_OF_N ? N : K, bc = kind == TC_A_ROWS_B_ROWS_OF_N ? K : N;
     LUTB_REQUIRE(ac % 4 == 0 && bc % 4 == 0, LUTB_ERR_ALIGN, "tensor-core contraction: row lengths must be multiples of 4");
-    const SplitPlan plan = split_plan(kind, M, N, K, a_exact);
+    const SplitPlan plan = split_plan(kind, M, N, K);
     unsigned char *p = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255);
     void *gw = p;
     p += plan.gemm_ws;
     float *Bs = reinterpret_cast<float *>(p);
     p += plan.b_bytes;
     float *As = reinterpret_cast<float *>(p);
-    p += plan.a_bytes;
-    float *P = reinterpret_cast<float *>(p);
     int rc;
-    if (plan.mode == 0) {
+    if (plan.deep) {
         // A' = [hi | lo | hi], B' = [lo | hi | hi] along the contraction index: one GEMM of depth 3K.  The mainloop
         // walks the contraction index upwards and the tensor core truncates its fp32 accumulator after every step, an
         // error proportional to the accumulator's size: the two small products go first, while it is small.
@@ -359,53 +279,13 @@ int tc_gemm(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, c
         if (rc) return rc;
         return run_tiles<Tf32TN>(M, N, 3 * K, As, 3 * (int64_t)K, Bs, 3 * (int64_t)K, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
     }
-    if (plan.mode == 1) {
-        // B' = [hi | lo] along the free index: one GEMM of width 2N into P, then C = alpha * (P_hi + P_lo) + beta * C
-        rc = split(B, K, N, ldb, Bs, 2, 0b10u, stream);
-        if (rc) return rc;
-        int p_slices = 1;
-        if (kind == TC_A_ROWS_B_ROWS_OF_K) {
-            // the slices of the contraction index as the batches of one launch, each into its own partial result
-            Batches bt;
-            bt.count = p_slices = plan.slices;
-            bt.a = plan.kc;
-            bt.b = (int64_t)plan.kc * 2 * N;
-            bt.c = (int64_t)M * 2 * N;
-            rc = run_tiles<Tf32NN>(M, 2 * N, plan.kc, A, lda, Bs, 2 * (int64_t)N, P, 2 * (int64_t)N, 1.f, 0.f, gw, plan.gemm_ws, stream, bt);
-            if (rc) return rc;
-        } else {
-            for (int k0 = 0; k0 < K; k0 += plan.kc) {
-                const int kn = K - k0 < plan.kc ? K - k0 : plan.kc;
-                rc = run_tiles<Tf32TT>(M, 2 * N, kn, A + (int64_t)k0 * lda, lda, Bs + (int64_t)k0 * 2 * N, 2 * (int64_t)N, P,
-                                 2 * (int64_t)N, 1.f, k0 == 0 ? 0.f : 1.f, gw, plan.gemm_ws, stream);
-                if (rc) return rc;
-            }
-        }
-        const int64_t n4 = (int64_t)M * (N / 4);
-        int64_t blocks = (n4 + 255) / 256;
-        const int64_t cap = (int64_t)device_info().sm_count * 16;
-        if (blocks > cap) blocks = cap;
-        combine_halves_kernel<<<(unsigned)blocks, 256, 0, stream>>>(P, C, M, N, ldc, alpha, beta, p_slices);
-        LUTB_LAUNCH_CHECK();
-        return LUTB_OK;
-    }
-    // generic: separate hi / lo copies (one matrix with two parts each), two or three GEMMs
+    // separate hi / lo copies (one matrix with two parts each)
     rc = split(B, br, bc, ldb, Bs, 2, 0b10u, stream);
+    if (!rc) rc = split(A, ar, ac, lda, As, 2, 0b10u, stream);
     if (rc) return rc;
-    const float *Ah = A, *Al = nullptr;
-    int64_t lda_s = lda;
-    if (!a_exact) {
-        rc = split(A, ar, ac, lda, As, 2, 0b10u, stream);
-        if (rc) return rc;
-        Ah = As; Al = As + ac; lda_s = 2 * ac;
-    }
-    const float *Bh = Bs, *Bl = Bs + bc;
-    const int64_t ldb_s = 2 * bc;
-    switch (kind) {
-        case TC_A_ROWS_B_ROWS_OF_N: return run3<Tf32TN>(M, N, K, Ah, Al, lda_s, Bh, Bl, ldb_s, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
-        case TC_A_ROWS_B_ROWS_OF_K: return run3<Tf32NN>(M, N, K, Ah, Al, lda_s, Bh, Bl, ldb_s, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
-        default: return run3<Tf32TT>(M, N, K, Ah, Al, lda_s, Bh, Bl, ldb_s, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
-    }
+    const float *Al = As + ac, *Bl = Bs + bc;
+    if (kind == TC_A_ROWS_B_ROWS_OF_K) return run3<Tf32NN>(M, N, K, As, Al, 2 * ac, Bs, Bl, 2 * bc, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
+    return run3<Tf32TT>(M, N, K, As, Al, 2 * ac, Bs, Bl, 2 * bc, C, ldc, alpha, beta, gw, plan.gemm_ws, stream);
 }
 
 size_t tc_gemm_fast_workspace(int M, int N, int K) {
@@ -435,7 +315,7 @@ extern "C" size_t lutb_fp32_gemm_workspace(int32_t m, int32_t n, int32_t k) {
     if (!(m > 0 && n > 0 && k > 0)) return 0;
     size_t a = 0;
     for (int kind = 0; kind < 3; kind++) {
-        const size_t w = lutb::tc_gemm_workspace(static_cast<lutb::TcGemmKind>(kind), m, n, k, false);
+        const size_t w = lutb::tc_gemm_workspace(static_cast<lutb::TcGemmKind>(kind), m, n, k);
         a = w > a ? w : a;
     }
     const size_t b = lutb::tc_gemm_fast_workspace(m, n, k);
@@ -458,7 +338,7 @@ extern "C" int lutb_fp32_gemm(int kind, int32_t m, int32_t n, int32_t k, const f
     if (fast)
         return tc_gemm_fast(static_cast<TcGemmKind>(kind), m, n, k, a, lda, b, ldb, c, ldc, alpha, beta, workspace,
                             workspace_bytes, static_cast<cudaStream_t>(stream));
-    return tc_gemm(static_cast<TcGemmKind>(kind), m, n, k, a, lda, b, ldb, c, ldc, alpha, beta, false, workspace, workspace_bytes,
+    return tc_gemm(static_cast<TcGemmKind>(kind), m, n, k, a, lda, b, ldb, c, ldc, alpha, beta, workspace, workspace_bytes,
                    static_cast<cudaStream_t>(stream));
 }
 

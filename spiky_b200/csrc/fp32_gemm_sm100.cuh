@@ -1,4 +1,4 @@
-// fp32 GEMMs on the tensor cores (tcgen05) for the histogram path of the product-mode layer; see fp32_gemm_sm100.cu.
+// General fp32 GEMMs on the tensor cores (tcgen05); see fp32_gemm_sm100.cu.
 #pragma once
 
 #include "lutb_common.cuh"
@@ -15,11 +15,10 @@ enum TcGemmKind {
 bool tc_gemm_available();
 // C [M x N] row-major = alpha * op(A) . op(B) + beta * C; all pointers 16-byte aligned, lda / ldb / ldc multiples of 4.
 // Split-TF32 route: hi / lo copies of the operands in the workspace, concatenated so that one TF32 GEMM forms all the
-// cross products wherever the layouts allow (else two or three GEMMs accumulate into C).
-// a_exact: A holds integers below 2048 (row counts), which TF32 represents exactly: A is used as it is, two GEMMs.
-size_t tc_gemm_workspace(TcGemmKind kind, int M, int N, int K, bool a_exact);
+// cross products where the layouts allow (else three GEMMs accumulate into C).
+size_t tc_gemm_workspace(TcGemmKind kind, int M, int N, int K);
 int tc_gemm(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C,
-            int64_t ldc, float alpha, float beta, bool a_exact, void *workspace, size_t workspace_bytes, cudaStream_t stream);
+            int64_t ldc, float alpha, float beta, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 // Single-GEMM route: the mainloop splits the fp32 operands into BF16 terms on the fly.
 size_t tc_gemm_fast_workspace(int M, int N, int K);
 int tc_gemm_fast(TcGemmKind kind, int M, int N, int K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C,

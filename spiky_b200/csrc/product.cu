@@ -7,7 +7,6 @@
 // Reference: calculate_product_lookup_index[_backprop] (lut_runtime_kernels_logic.proto:32-198),
 // fill_outputs_product_cpu_logic (:2148-2264), propagate_backward_product_cpu_logic (:2396-2628),
 // gather_w_gradients_internal_product_cpu_logic (:2630-2744).
-#include "fp32_gemm_sm100.cuh"
 #include "product_hist.cuh"
 #include "product_pairs.cuh"
 
@@ -312,11 +311,9 @@ static int choose_variant(const ProductCall &c, int variant, bool backward, cons
         return LUTB_OK;
     }
     // The contractions cost rows-per-table multiply-adds per (query, detector, output), the direct kernels one table
-    // row through L2 per key: with the FMA contraction the histogram path pays once a query has about a quarter
-    // (backward) or all (forward) of the table's rows as keys; on the tensor cores the contraction is several times
-    // cheaper and the forward threshold drops to a quarter as well.
+    // row through L2 per key: the histogram path pays once a query has about a quarter of the table's rows as keys.
     const int64_t rows = (int64_t)1 << c.cfg->n_anchors;
-    const bool long_enough = (backward || tc_gemm_available()) ? 4 * (int64_t)c.S >= rows : (int64_t)c.S >= rows;
+    const bool long_enough = 4 * (int64_t)c.S >= rows;
     hist = possible && long_enough && workspace != nullptr &&
            workspace_bytes >= product_hist_workspace_bytes(c.cfg, 1, c.S, backward);
     return LUTB_OK;

@@ -5,7 +5,7 @@
 #include <type_traits>
 
 #include "product_hist.cuh"
-#include "fp32_gemm_sm100.cuh"
+#include "hist_gemm_sm100.cuh"
 #include "product_pairs.cuh"
 
 namespace lutb {
@@ -101,9 +101,9 @@ __device__ __forceinline__ void positional_ends(const AnchorLists &al, const flo
 // key ends of 32 keys are in registers while the warp walks its queries, whose operands (two anchors' query ends and
 // bits per 16-byte load) are the same for all lanes; a key-query anchor then costs a compare and a predicated OR.  The
 // loop over the anchors is unrolled for their number (NKQ), so that the four queries overlap.
-// F32_ROWS: the counters are written as fp32 in the layout [row of the chunk = local sequence * S + j][detector][T], the
-// operand layout of the tensor-core contractions (one plain GEMM over all detectors per pass); otherwise as uint16 in
-// the layout [detector][row of the chunk][T].
+// HALF_ROWS: the counters are written as fp16 (exact: counts are below 2048 there) in the layout [row of the chunk = local
+// sequence * S + j][detector][T], the operand layout of the tensor-core contractions (one plain GEMM over all detectors per
+// pass); otherwise as uint16 in the layout [detector][row of the chunk][T].
 // PACKED: two 16-bit counters per word (a count is at most S - 1 < 65536), which keeps 16 warps per block up to
 // 1024-row tables.
 // Bound: instruction issue, and at 256-row tables the 537 MB of counters it writes.  Measured (before: lanes over the keys
@@ -136,6 +136,12 @@ template <bool PACKED>
 __device__ __forceinline__ void count_row(uint32_t *hist, uint32_t li) {
     if (PACKED) atomicAdd(hist + (li >> 1), 1u << ((li & 1u) * 16u));
     else atomicAdd(hist + li, 1u);
+}
+
+// two 16-bit counts as fp16
+__device__ __forceinline__ uint32_t half_counts(uint32_t c) {
+    const __half2 h = __halves2half2(__ushort2half_rn((unsigned short)(c & 0xffffu)), __ushort2half_rn((unsigned short)(c >> 16)));
+    return *reinterpret_cast<const uint32_t *>(&h);
 }
 
 struct HistTile {
@@ -183,7 +189,7 @@ __device__ __forceinline__ void count_tile(const HistArgs &p, const AnchorLists 
     }
 }
 
-template <int MAXKQ, bool EPS, bool F32_ROWS, bool PACKED>
+template <int MAXKQ, bool EPS, bool HALF_ROWS, bool PACKED>
 __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
@@ -281,23 +287,23 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
         else count_tile<MAXKQ, false, EPS, PACKED>(p, al, h, qbits);
         __syncwarp();
         // write out and clear
-        float *out_f = static_cast<float *>(p.H) + ((size_t)(bl * S + j0) * p.n_detectors + t) * T;
+        __half *out_f = static_cast<__half *>(p.H) + ((size_t)(bl * S + j0) * p.n_detectors + t) * T;
         uint16_t *out_h = static_cast<uint16_t *>(p.H) + ((size_t)t * p.chunk_rows + bl * S + j0) * T;
-        for (int w = lane; w < nq * (T / 4); w += 32) {
-            const int q = w >> (Nc - 2), r = w & (T / 4 - 1);
-            uint4 c;
+        for (int w = lane; w < nq * (T / 8); w += 32) {
+            const int q = w >> (Nc - 3), r = w & (T / 8 - 1);
+            uint4 c;   // eight 16-bit counts
             if (PACKED) {
-                uint2 *cell = reinterpret_cast<uint2 *>(hist) + w;
-                const uint2 v = *cell;
-                *cell = make_uint2(0u, 0u);
-                c = make_uint4(v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16);
-            } else {
                 uint4 *cell = reinterpret_cast<uint4 *>(hist) + w;
                 c = *cell;
                 *cell = make_uint4(0u, 0u, 0u, 0u);
+            } else {
+                uint4 *cell = reinterpret_cast<uint4 *>(hist) + 2 * w;
+                const uint4 u = cell[0], v = cell[1];
+                cell[0] = cell[1] = make_uint4(0u, 0u, 0u, 0u);
+                c = make_uint4(u.x | u.y << 16, u.z | u.w << 16, v.x | v.y << 16, v.z | v.w << 16);
             }
-            if (F32_ROWS) *reinterpret_cast<float4 *>(out_f + (size_t)q * p.n_detectors * T + r * 4) = make_float4((float)c.x, (float)c.y, (float)c.z, (float)c.w);
-            else *reinterpret_cast<uint2 *>(out_h + (size_t)w * 4) = make_uint2(c.x | (c.y << 16), c.z | (c.w << 16));
+            if (HALF_ROWS) *reinterpret_cast<uint4 *>(out_f + (size_t)q * p.n_detectors * T + r * 8) = make_uint4(half_counts(c.x), half_counts(c.y), half_counts(c.z), half_counts(c.w));
+            else *reinterpret_cast<uint4 *>(out_h + (size_t)w * 8) = c;
         }
         __syncwarp();
     }
@@ -860,35 +866,32 @@ bool product_hist_supported(const ProductCall &c, const void *weights, const voi
     return stage_bytes(c, T + 64 * cfg->n_anchors) <= (size_t)kMaxSmemPerBlock - 1024;
 }
 
-static size_t bytes_per_sequence(const lutb_layer_cfg *cfg, int S, bool backward, bool tc) {
+static size_t bytes_per_sequence(const lutb_layer_cfg *cfg, int S, bool backward) {
     const size_t cells = (size_t)cfg->n_detectors * S * ((size_t)1 << cfg->n_anchors);
-    return align256(cells * (tc ? 4 : 2)) + (backward ? align256(cells * 4) : 0) + 512;
+    return align256(cells * 2) + (backward ? align256(cells * 4) : 0) + 512;
 }
 
-// Scratch of the tensor-core GEMMs of one pass over `rows` query rows: their own workspace plus the hi / lo copies of
-// the operands (the tables, and the output gradients in the backward pass); the largest of the calls the pass makes.
+// Scratch of the tensor-core contractions of one pass over `rows` query rows (operand copies: the tables, and the output
+// gradients in the backward pass); the largest of the calls the pass makes.
 static size_t tc_scratch_bytes(const lutb_layer_cfg *cfg, int64_t rows, bool backward) {
     const int KT = cfg->n_detectors << cfg->n_anchors, O = cfg->n_outputs;
-    const size_t fwd = tc_gemm_workspace(TC_A_ROWS_B_ROWS_OF_K, (int)rows, O, KT, true);
+    const size_t fwd = hist_gemm_workspace(HG_FORWARD, (int)rows, KT, O);
     if (!backward) return align256(fwd);
     // (the forward contraction's scratch counts here too: a forward pass that leaves its histogram for the backward
     // pass lays the workspace out as the backward pass does)
-    const size_t dw = tc_gemm_workspace(TC_A_COLS_B_ROWS_OF_K, KT, O, (int)rows, true),
-                 q = tc_gemm_workspace(TC_A_ROWS_B_ROWS_OF_N, (int)rows, KT, O, false);
+    const size_t dw = hist_gemm_workspace(HG_TABLE_GRAD, (int)rows, KT, O), q = hist_gemm_workspace(HG_ROW_DOTS, (int)rows, KT, O);
     const size_t m = dw > q ? dw : q;
     return align256(m > fwd ? m : fwd);
 }
 
 size_t product_hist_workspace_bytes(const lutb_layer_cfg *cfg, int64_t batch, int S, bool backward) {
-    // what lets `batch` sequences through in one pass with either contraction: fp32 counters and operand copies for the
-    // tensor cores, uint16 counters for the FMA kernel
-    const bool tc = tc_gemm_available();
-    return (tc ? tc_scratch_bytes(cfg, batch * S, backward) : 0) + (size_t)batch * bytes_per_sequence(cfg, S, backward, tc) + 256;
+    // what lets `batch` sequences through in one pass with either contraction
+    return tc_scratch_bytes(cfg, batch * S, backward) + (size_t)batch * bytes_per_sequence(cfg, S, backward) + 256;
 }
 
 struct HistPlan {
     int64_t chunk;  // sequences per pass
-    bool tc;        // tensor-core contractions: H is fp32 [row][detector][T], Q fp32 [row][detector][T]
+    bool tc;        // tensor-core contractions: H is fp16 [row][detector][T], Q fp32 [row][detector][T]
     void *H;
     float *Q;
     void *gemm_ws;
@@ -900,11 +903,11 @@ static int plan(const ProductCall &c, bool backward, bool allow_tc, void *worksp
     const uintptr_t base0 = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
     const size_t slack = base0 - reinterpret_cast<uintptr_t>(workspace);
     const size_t T = (size_t)1 << c.cfg->n_anchors;
-    // tensor cores when the library has them, the workspace holds at least one sequence in their layout, the GEMM
-    // extents fit 32-bit sizes and the row counts (at most S - 1) are exact in TF32
-    p.tc = allow_tc && tc_gemm_available() && c.S <= 2048 && (size_t)c.cfg->n_detectors * T < ((size_t)1 << 30) &&
-           bytes >= slack + tc_scratch_bytes(c.cfg, c.S, backward) + bytes_per_sequence(c.cfg, c.S, backward, true);
-    const size_t per_seq = bytes_per_sequence(c.cfg, c.S, backward, p.tc);
+    // tensor cores when the workspace holds at least one sequence and the operand copies, the extents fit 32-bit sizes and
+    // the row counts (at most S - 1) are exact in fp16
+    const size_t per_seq = bytes_per_sequence(c.cfg, c.S, backward);
+    p.tc = allow_tc && c.S <= 2048 && (size_t)c.cfg->n_detectors * T < ((size_t)1 << 30) &&
+           bytes >= slack + tc_scratch_bytes(c.cfg, c.S, backward) + per_seq;
     LUTB_REQUIRE(bytes >= slack + per_seq, LUTB_ERR_WORKSPACE,
                  "product histogram path: workspace of %zu bytes is smaller than the %zu bytes one sequence needs", bytes,
                  per_seq + 256);
@@ -926,7 +929,7 @@ static int plan(const ProductCall &c, bool backward, bool allow_tc, void *worksp
     p.gemm_ws_bytes = head;
     base += head;
     p.H = reinterpret_cast<void *>(base);
-    p.Q = backward ? reinterpret_cast<float *>(base + align256(cells * (p.tc ? 4 : 2))) : nullptr;
+    p.Q = backward ? reinterpret_cast<float *>(base + align256(cells * 2)) : nullptr;
     return LUTB_OK;
 }
 
@@ -1029,8 +1032,7 @@ int launch_product_hist_forward(const ProductCall &c, const float *weights, floa
         if (p.tc) {
             // y[rows, O] += H[rows, Nt*T] . W[Nt*T, O]
             KernelScope scope(K_PRODUCT_HIST_FORWARD, stream);
-            rc = tc_gemm(TC_A_ROWS_B_ROWS_OF_K, (int)rows, O, Nt * T, static_cast<const float *>(p.H), (int64_t)Nt * T, weights, O,
-                         y + b0 * c.S * O, O, 1.f, 1.f, /*a_exact=*/true, p.gemm_ws, p.gemm_ws_bytes, stream);
+            rc = hist_gemm_forward((int)rows, Nt * T, O, static_cast<const __half *>(p.H), weights, y + b0 * c.S * O, p.gemm_ws, p.gemm_ws_bytes, stream);
             if (rc) return rc;
             continue;
         }
@@ -1068,8 +1070,7 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
         if (p.tc) {
             // target[Nt*T, O] += lr * H^T . dY  (H stored [rows, Nt*T])
             KernelScope scope(K_PRODUCT_HIST_WEIGHT_GRAD, stream);
-            return tc_gemm(TC_A_COLS_B_ROWS_OF_K, Nt * T, O, (int)rows, static_cast<const float *>(p.H), (int64_t)Nt * T,
-                           dY + b0 * c.S * O, O, target, O, (float)lr, 1.f, /*a_exact=*/true, p.gemm_ws, p.gemm_ws_bytes, stream);
+            return hist_gemm_table_grad((int)rows, Nt * T, O, static_cast<const __half *>(p.H), dY + b0 * c.S * O, target, (float)lr, p.gemm_ws, p.gemm_ws_bytes, stream);
         }
         GemmArgs g{};
         g.A = p.H; g.B = dY + b0 * c.S * O; g.C = target;
@@ -1095,8 +1096,7 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
         if (p.tc) {
             // Q[rows, Nt*T] = dY[rows, O] . W^T  (W stored [Nt*T, O])
             KernelScope scope(K_PRODUCT_ROW_DOTS, stream);
-            rc = tc_gemm(TC_A_ROWS_B_ROWS_OF_N, (int)rows, Nt * T, O, dY + b0 * c.S * O, O, weights, O, p.Q, (int64_t)Nt * T, 1.f,
-                         0.f, /*a_exact=*/false, p.gemm_ws, p.gemm_ws_bytes, stream);
+            rc = hist_gemm_row_dots((int)rows, Nt * T, O, dY + b0 * c.S * O, weights, p.Q, p.gemm_ws, p.gemm_ws_bytes, stream);
             if (rc) return rc;
         } else {
             GemmArgs g{};

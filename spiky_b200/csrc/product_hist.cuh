@@ -6,7 +6,7 @@
 //     table gradient dW_t          += lr * H_t^T . dY                            (T x rows) . (rows x O)
 //     input gradient g(i,j,t)       = Q_t[(b,j), idx] - Q_t[(b,j), alt],  Q_t = dY . W_t^T   (rows x O) . (O x T)
 // so the row gathers and scatter-adds of the direct kernels (one table row per pair through L2) become dense
-// contractions: fp32-accurate GEMMs on the tensor cores (fp32_gemm_sm100.cuh; the counters are then kept as fp32 in
+// contractions: fp32-accurate GEMMs on the tensor cores (hist_gemm_sm100.cuh; the counters are then kept as fp16 in
 // the layout [row][detector][T], so that each of the three sums is ONE GEMM over all detectors), or, without them,
 // register-tiled fp32 FMA contractions whose table traffic is amortised over 128 query rows.  Worth it once a query
 // has about as many keys as the table has rows.
@@ -30,8 +30,8 @@ bool product_hist_supported(const ProductCall &c, const void *weights, const voi
 // sequences as the workspace holds).
 size_t product_hist_workspace_bytes(const lutb_layer_cfg *cfg, int64_t batch, int S, bool backward);
 
-// allow_tc: run the contractions on the tensor cores (fp32_gemm_sm100.cuh) when the library has them and the workspace
-// holds at least one sequence in their operand layout; otherwise, and when false, the fp32 FMA contraction runs.
+// allow_tc: run the contractions on the tensor cores (hist_gemm_sm100.cuh) when the workspace holds at least one
+// sequence and the operand copies; otherwise, and when false, the fp32 FMA contraction runs.
 // keep: leave the row histogram in the workspace where launch_product_hist_backward(..., reuse = true) finds it
 // (product_hist_keeps tells whether a workspace of that size allows it: the whole batch must be one pass).
 bool product_hist_keeps(const ProductCall &c, bool allow_tc, void *workspace, size_t workspace_bytes);

@@ -544,8 +544,7 @@ class _LUTDataManager:
         rows = 1 << self._n_anchors
         L = _native.lib()
         # the library's own rule for AUTO (include/spiky_b200.h): no workspace is needed when it will pick DIRECT
-        quarter = backward or bool(L.lutb_fp32_gemm_available())
-        if variant == _native.PRODUCT_AUTO and not ((4 * S >= rows) if quarter else (S >= rows)):
+        if variant == _native.PRODUCT_AUTO and 4 * S < rows:
             return None, 0
         one = L.lutb_product_workspace(ctypes.byref(cfg), 1, S, int(backward))
         want = min(L.lutb_product_workspace(ctypes.byref(cfg), B, S, int(backward)),
