@@ -152,6 +152,39 @@ def lib():
     return _lib
 
 
+_layer_calls = None
+LAYER_CALLS_PATH = os.path.join(_HERE, "lib", "_layer_calls.so")
+
+
+def layer_calls():
+    """The extension module of the native host side of layer calls (host/layer_calls.cpp), set up; raises RuntimeError when
+    it is missing."""
+    global _layer_calls
+    if _layer_calls is None:
+        if not os.path.exists(LAYER_CALLS_PATH):
+            raise RuntimeError(f"{LAYER_CALLS_PATH} is missing: build it with `python -m spiky_b200.build`")
+        import importlib.util
+
+        from .lut_data_manager import LUTDataManagerF, _LUTDataManager
+        from .lut_layer import GradientType, LUTLayerBasic
+        spec = importlib.util.spec_from_file_location("_layer_calls", LAYER_CALLS_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        handle = lib()
+        module.setup(
+            {name: ctypes.cast(getattr(handle, name), _vp).value for name in SIGNATURES},
+            LUTLayerBasic, LUTDataManagerF, _LUTDataManager, GradientType.Dense, GradientType.Internal, check,
+            ["forward_step", "backward_step", "forward_step_concat", "backward_step_concat", "forward_step_product",
+             "backward_step_product", "_check_input", "_prepare_positional_embeddings", "_process_gradients",
+             "_fresh_gradients", "_weight_grad_target", "_external_lr", "LUTForwardFN"],
+            ["_lookup_indices_callback", "_table_forward_hook", "_table_update_hook", "_table_gradient_sink"],
+            ["forward_step", "backward_backprop", "forward_step_concat", "backward_backprop_concat",
+             "forward_step_product", "backward_backprop_product", "_cfg", "_stream", "_require_cuda", "_expect",
+             "_sparse_forward", "_sparse_backward", "_product_workspace", "_histogram_key", "get_weights_dimension"])
+        _layer_calls = module
+    return _layer_calls
+
+
 class LutbError(RuntimeError):
     pass
 

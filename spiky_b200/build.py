@@ -1,4 +1,5 @@
-"""Builds libspiky_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libspiky_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _layer_calls.so (the native host side of
+layer calls, host/layer_calls.cpp, against the installed torch) with the host compiler.
 
     python -m spiky_b200.build [--force] [--verbose]
 
@@ -64,6 +65,32 @@ def _extra_flags(src):
     return flags
 
 
+HOST_SRC = os.path.join(HERE, "host", "layer_calls.cpp")
+HOST_LIB = os.path.join(LIBDIR, "_layer_calls.so")
+
+
+def _build_host(force):
+    """The extension module; rebuilt when its source, the C ABI's header or torch itself is newer."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    header = os.path.join(HERE, "..", "include", "spiky_b200.h")
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= _newest(
+            [HOST_SRC, header, os.path.join(root, "version.py")]):
+        return
+    gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), cuda,
+              sysconfig.get_paths()["include"]):
+        cmd += ["-isystem", d]
+    cmd += [HOST_SRC, "-o", HOST_LIB, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("host compiler failed for %s:\n%s\n%s" % (HOST_SRC, p.stdout, p.stderr))
+
+
 def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
 
@@ -73,10 +100,11 @@ def build(force=False, verbose=False):
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     if not sources:
         raise RuntimeError("no CUDA sources found under " + CSRC)
-    if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest(sources + headers):
-        return LIB
     objdir = os.path.join(LIBDIR, "obj")
     os.makedirs(objdir, exist_ok=True)
+    if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest(sources + headers):
+        _build_host(force)
+        return LIB
     nvcc = _nvcc()
     hdr_time = _newest(headers) if headers else 0.0
 
@@ -90,8 +118,10 @@ def build(force=False, verbose=False):
             raise RuntimeError("nvcc failed for %s:\n%s\n%s" % (src, p.stdout, p.stderr))
         return obj, "== %s\n%s%s" % (os.path.basename(src), p.stdout, p.stderr)
 
-    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(sources))) as ex:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(sources)) + 1) as ex:
+        host = ex.submit(_build_host, force)
         results = list(ex.map(compile_one, sources))
+        host.result()
     objs = [r[0] for r in results]
     log = "".join(r[1] for r in results)
     if log:

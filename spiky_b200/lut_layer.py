@@ -182,6 +182,13 @@ class _LUTFunction(torch.autograd.Function):
         return dx, dw, dpe, None
 
 
+def _layer_call(x, layer):
+    """First call of the process: load the native host side, which takes this function's place."""
+    global _layer_call
+    _layer_call = _native.layer_calls().apply
+    return _layer_call(x, layer)
+
+
 class LUTLayerBasic(nn.Module):
     """Common machinery of all LUT layers (reference: LUTLayerBasic, LUTLayer.py:197-1242)."""
 
@@ -734,6 +741,11 @@ class LUTLayerBasic(nn.Module):
         return self
 
     def forward(self, x):
+        # the ordinary cases in native code (host/layer_calls.cpp); what it leaves (None) goes the Python way below
+        if isinstance(x, torch.Tensor) and x.is_cuda and not torch.compiler.is_compiling():
+            y = _layer_call(x, self)
+            if y is not None:
+                return y
         if self._sequence_length == 1:
             return _LUTFunction.apply(x, self._weights, None, self)
         return _LUTFunction.apply(x, self._weights, self._prepare_positional_embeddings(), self)
