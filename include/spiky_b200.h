@@ -441,6 +441,18 @@ int lutb_dense_to_sparse_32(void *source, int64_t n, int64_t *indices, void *val
                             int64_t *count_out, int erase_input, void *workspace, size_t workspace_bytes, void *stream);
 
 /*
+ * The cells of a row list (lutb_nonseq_fc_table_grad_rows), without its count on the host: the non-zero words of the first
+ * min(*row_count, capacity) rows of `values`, row_words each, as (row_ids[r] * row_words + column, value) in list order.
+ * _count writes how many there are to count_out (device memory) and leaves its prefix sums in the workspace for _scatter,
+ * which writes the first `room` of them.  Workspace: lutb_dense_to_sparse_workspace(capacity * row_words) bytes.
+ */
+int lutb_row_cells_count(const float *values, const int64_t *row_count, int64_t capacity, int32_t row_words, int64_t *count_out,
+                         void *workspace, size_t workspace_bytes, void *stream);
+int lutb_row_cells_scatter(const float *values, const int64_t *row_ids, const int64_t *row_count, int64_t capacity,
+                           int32_t row_words, int64_t *cells, float *cell_values, int64_t room, void *workspace,
+                           size_t workspace_bytes, void *stream);
+
+/*
  * fp32 GEMM on the sm_100a tensor cores with fp32-class accuracy (no reference counterpart; the reference has no
  * dense contraction): C [m x n] row-major = alpha * op(A) . op(B) + beta * C.  Default route: every operand is written
  * once as hi (x rounded to TF32) and lo = x - hi, and hi.hi + hi.lo + lo.hi is formed by TF32 GEMMs on the copies (tcgen05.mma, fp32 accumulators in tensor memory, operands staged by TMA); with

@@ -111,6 +111,8 @@ SIGNATURES = {
     "lutb_dense_to_sparse_workspace": (_size, [_i64]),
     "lutb_count_nonzero_32": (_int, [_vp, _i64, _vp, _vp, _size, _vp]),
     "lutb_dense_to_sparse_32": (_int, [_vp, _i64, _vp, _vp, _i64, _vp, _int, _vp, _size, _vp]),
+    "lutb_row_cells_count": (_int, [_vp, _vp, _i64, ctypes.c_int32, _vp, _vp, _size, _vp]),
+    "lutb_row_cells_scatter": (_int, [_vp, _vp, _vp, _i64, ctypes.c_int32, _vp, _vp, _i64, _vp, _size, _vp]),
     "lutb_sparse_kernel_select": (_int, [_int, _int]),
     "lutb_device_wait_errors": (_int, [ctypes.POINTER(_int)]),
     "lutb_fp32_gemm_available": (_int, []),
@@ -173,14 +175,14 @@ def layer_calls():
         handle = lib()
         module.setup(
             {name: ctypes.cast(getattr(handle, name), _vp).value for name in SIGNATURES},
-            LUTLayerBasic, LUTDataManagerF, _LUTDataManager, GradientType.Dense, GradientType.Internal, check,
+            LUTLayerBasic, LUTDataManagerF, _LUTDataManager, GradientType.Dense, GradientType.Internal, GradientType.Sparse, check,
             ["forward_step", "backward_step", "forward_step_concat", "backward_step_concat", "forward_step_product",
              "backward_step_product", "_check_input", "_prepare_positional_embeddings", "_process_gradients",
-             "_fresh_gradients", "_weight_grad_target", "_external_lr", "LUTForwardFN"],
+             "_fresh_gradients", "_weight_grad_target", "_external_lr", "_backward_step_sparse_rows", "LUTForwardFN"],
             ["_lookup_indices_callback", "_table_forward_hook", "_table_update_hook", "_table_gradient_sink"],
             ["forward_step", "backward_backprop", "forward_step_concat", "backward_backprop_concat",
              "forward_step_product", "backward_backprop_product", "_cfg", "_stream", "_require_cuda", "_expect",
-             "_sparse_forward", "_sparse_backward", "_product_workspace", "_histogram_key", "get_weights_dimension"])
+             "_sparse_forward", "_sparse_backward", "table_gradient_rows", "table_gradient_cells", "_product_workspace", "_histogram_key", "get_weights_dimension"])
         _layer_calls = module
     return _layer_calls
 

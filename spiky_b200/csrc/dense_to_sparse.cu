@@ -117,6 +117,50 @@ __global__ void __launch_bounds__(kTileThreads) d2s_scatter_kernel(uint32_t *__r
     }
 }
 
+// The same over the rows of a table gradient (`values`: *row_count rows of `row_words`, at most `capacity`; `row_ids`: where in the
+// table each belongs), the count of which is still on the device: word c of list row r becomes cell row_ids[r] * row_words + c.
+__global__ void __launch_bounds__(kTileThreads) cells_tile_count_kernel(const uint32_t *__restrict__ values, const int64_t *__restrict__ row_count,
+                                                                        int64_t capacity, int row_words, bool vec,
+                                                                        int32_t *__restrict__ tile_counts) {
+    const int64_t n = min(__ldg(row_count), capacity) * row_words;
+    int total = 0;
+    if ((int64_t)blockIdx.x * kTileWords < n) {
+        uint32_t w[8];
+        load_tile_words(values, n, blockIdx.x, vec, w);
+        block_exclusive(count_words(w), &total);
+    }
+    if (threadIdx.x == 0) tile_counts[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kTileThreads) cells_scatter_kernel(const uint32_t *__restrict__ values, const int64_t *__restrict__ row_ids,
+                                                                     const int64_t *__restrict__ row_count, int64_t capacity, int row_words,
+                                                                     bool vec, const int64_t *__restrict__ tile_starts,
+                                                                     int64_t *__restrict__ cells, uint32_t *__restrict__ out, int64_t room) {
+    const int64_t n = min(__ldg(row_count), capacity) * row_words;
+    if ((int64_t)blockIdx.x * kTileWords >= n) return;
+    uint32_t w[8];
+    load_tile_words(values, n, blockIdx.x, vec, w);
+    const int mine = count_words(w);
+    int total;
+    int64_t pos = tile_starts[blockIdx.x] + block_exclusive(mine, &total);
+    if (mine == 0) return;
+    const int64_t first = (int64_t)blockIdx.x * kTileWords + (int64_t)threadIdx.x * 8;
+    int64_t row = first / row_words;
+    int col = (int)(first - row * row_words);
+    int64_t at = __ldg(row_ids + row) * row_words;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        if (w[e] != 0u) {
+            if (pos < room) { cells[pos] = at + col; out[pos] = w[e]; }
+            pos++;
+        }
+        if (++col == row_words && first + e + 1 < n) {
+            col = 0;
+            at = __ldg(row_ids + ++row) * row_words;
+        }
+    }
+}
+
 static int64_t tiles_of(int64_t n) { return (n + kTileWords - 1) / kTileWords; }
 
 }  // namespace lutb
@@ -178,6 +222,62 @@ extern "C" int lutb_dense_to_sparse_32(void *source, int64_t n, int64_t *indices
     KernelScope scope(K_DENSE_TO_SPARSE, st);
     d2s_scatter_kernel<<<(unsigned)tiles_of(n), kTileThreads, 0, st>>>(src, n, vec, starts, indices,
                                                                        static_cast<uint32_t *>(values), capacity, erase_input);
+    LUTB_LAUNCH_CHECK();
+    return LUTB_OK;
+}
+
+static int cells_checks(const float *values, const int64_t *row_count, int64_t capacity, int32_t row_words, void *workspace,
+                        size_t workspace_bytes, int32_t **counts, int64_t **starts) {
+    LUTB_REQUIRE(values && row_count, LUTB_ERR_NULL, "a required pointer is NULL");
+    LUTB_REQUIRE(capacity > 0 && row_words > 0, LUTB_ERR_SHAPE, "empty row list");
+    const int64_t n = capacity * row_words, t = tiles_of(n);
+    LUTB_REQUIRE(t <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "row list too large");
+    LUTB_REQUIRE(workspace && workspace_bytes >= lutb_dense_to_sparse_workspace(n), LUTB_ERR_WORKSPACE,
+                 "the cells of a row list need %zu bytes of workspace", lutb_dense_to_sparse_workspace(n));
+    const uintptr_t base = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
+    *counts = reinterpret_cast<int32_t *>(base);
+    *starts = reinterpret_cast<int64_t *>(base + (((size_t)t * 4 + 255) & ~(size_t)255));
+    return LUTB_OK;
+}
+
+extern "C" int lutb_row_cells_count(const float *values, const int64_t *row_count, int64_t capacity, int32_t row_words,
+                                    int64_t *count_out, void *workspace, size_t workspace_bytes, void *stream) {
+    int32_t *counts = nullptr;
+    int64_t *starts = nullptr;
+    const int rc = cells_checks(values, row_count, capacity, row_words, workspace, workspace_bytes, &counts, &starts);
+    if (rc) return rc;
+    LUTB_REQUIRE(count_out, LUTB_ERR_NULL, "a required pointer is NULL");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t t = tiles_of(capacity * row_words);
+    const bool vec = (reinterpret_cast<uintptr_t>(values) & 15) == 0;
+    {
+        KernelScope scope(K_DENSE_TO_SPARSE, st);
+        cells_tile_count_kernel<<<(unsigned)t, kTileThreads, 0, st>>>(reinterpret_cast<const uint32_t *>(values), row_count, capacity, row_words, vec, counts);
+    }
+    LUTB_LAUNCH_CHECK();
+    {
+        KernelScope scope(K_DENSE_TO_SPARSE, st);
+        d2s_scan_tiles_kernel<<<1, kTileThreads, 0, st>>>(counts, t, starts, count_out);
+    }
+    LUTB_LAUNCH_CHECK();
+    return LUTB_OK;
+}
+
+extern "C" int lutb_row_cells_scatter(const float *values, const int64_t *row_ids, const int64_t *row_count, int64_t capacity,
+                                      int32_t row_words, int64_t *cells, float *cell_values, int64_t room, void *workspace,
+                                      size_t workspace_bytes, void *stream) {
+    int32_t *counts = nullptr;
+    int64_t *starts = nullptr;
+    const int rc = cells_checks(values, row_count, capacity, row_words, workspace, workspace_bytes, &counts, &starts);
+    if (rc) return rc;
+    LUTB_REQUIRE(row_ids && cells && cell_values, LUTB_ERR_NULL, "a required pointer is NULL");
+    LUTB_REQUIRE(room >= 0, LUTB_ERR_SHAPE, "negative room");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool vec = (reinterpret_cast<uintptr_t>(values) & 15) == 0;
+    KernelScope scope(K_DENSE_TO_SPARSE, st);
+    cells_scatter_kernel<<<(unsigned)tiles_of(capacity * row_words), kTileThreads, 0, st>>>(
+        reinterpret_cast<const uint32_t *>(values), row_ids, row_count, capacity, row_words, vec, starts, cells,
+        reinterpret_cast<uint32_t *>(cell_values), room);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
 }

@@ -12,13 +12,19 @@
 
 namespace lutb {
 
-constexpr int kSortBlock = 1024;  // samples per (detector, block) histogram slice
+// Samples per (detector, block) histogram slice; a warp walks one slice in order.  The row list takes short ones while a detector's
+// counters are few enough for two steps of the scan over them (1111 samples, 50 detectors of 128 rows: a slice of 1024 is 32 dependent
+// steps, 16.6 us; of 128 4.0, the scan 3.5 -> 5.1).
+constexpr int kSortBlock = 1024, kRowsSortBlock = 128;
+static int rows_sort_block(int64_t batch, int table_rows) {
+    return table_rows * ((batch + kRowsSortBlock - 1) / kRowsSortBlock) <= 2048 ? kRowsSortBlock : kSortBlock;
+}
 
 // counts[t][row][k] = number of samples of block k that selected `row` in detector t
 __global__ void dw_sort_count_kernel(const int32_t *__restrict__ idx, int32_t *__restrict__ counts, int64_t batch,
-                                     int n_detectors, int table_rows, int nblk) {
+                                     int n_detectors, int table_rows, int nblk, int sort_block) {
     const int t = blockIdx.x, k = blockIdx.y;
-    const int64_t b0 = (int64_t)k * kSortBlock, b1 = min(batch, b0 + kSortBlock);
+    const int64_t b0 = (int64_t)k * sort_block, b1 = min(batch, b0 + sort_block);
     for (int64_t b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
         const int32_t r = __ldg(idx + b * n_detectors + t);
         atomicAdd(counts + ((size_t)t * table_rows + r) * nblk + k, 1);
@@ -54,12 +60,12 @@ __global__ void dw_sort_scan_kernel(int32_t *__restrict__ counts, int table_rows
 // stable scatter: one warp per (detector, block) walks its samples in order, 32 at a time
 __global__ void dw_sort_scatter_kernel(const int32_t *__restrict__ idx, const int32_t *__restrict__ offsets,
                                        int32_t *__restrict__ perm, int64_t batch, int n_detectors, int table_rows,
-                                       int nblk) {
+                                       int nblk, int sort_block) {
     extern __shared__ int32_t cursor[];  // [table_rows] next free slot of each row for this (detector, block)
     const int t = blockIdx.x, k = blockIdx.y, lane = threadIdx.x;
     for (int r = lane; r < table_rows; r += 32) cursor[r] = __ldg(offsets + ((size_t)t * table_rows + r) * nblk + k);
     __syncwarp();
-    const int64_t b0 = (int64_t)k * kSortBlock, b1 = min(batch, b0 + kSortBlock);
+    const int64_t b0 = (int64_t)k * sort_block, b1 = min(batch, b0 + sort_block);
     int32_t *out = perm + (size_t)t * batch;
     for (int64_t base = b0; base < b1; base += 32) {
         const int64_t b = base + lane;
@@ -100,9 +106,12 @@ __global__ void __launch_bounds__(256) dw_sort_reduce_kernel(const float *__rest
     }
 }
 
-size_t fc_dw_sorted_workspace(int64_t batch, int n_detectors, int table_rows) {
-    const int64_t nblk = (batch + kSortBlock - 1) / kSortBlock;
+static size_t sorted_workspace(int64_t batch, int n_detectors, int table_rows, int sort_block) {
+    const int64_t nblk = (batch + sort_block - 1) / sort_block;
     return ((size_t)n_detectors * table_rows * nblk + (size_t)n_detectors * batch) * sizeof(int32_t);
+}
+size_t fc_dw_sorted_workspace(int64_t batch, int n_detectors, int table_rows) {
+    return sorted_workspace(batch, n_detectors, table_rows, kSortBlock);
 }
 
 int launch_fc_dw_sorted(const float *dY, const int32_t *idx, float *target, int64_t batch, int n_outputs,
@@ -118,13 +127,13 @@ int launch_fc_dw_sorted(const float *dY, const int32_t *idx, float *target, int6
     if (clear_with_memset) LUTB_CUDA(cudaMemsetAsync(counts, 0, count_bytes, stream));
     dim3 grid((unsigned)n_detectors, (unsigned)nblk);
     KernelScope scope(K_FC_WEIGHT_GRAD, stream);
-    dw_sort_count_kernel<<<grid, 256, 0, stream>>>(idx, counts, batch, n_detectors, table_rows, nblk);
+    dw_sort_count_kernel<<<grid, 256, 0, stream>>>(idx, counts, batch, n_detectors, table_rows, nblk, kSortBlock);
     LUTB_LAUNCH_CHECK();
     dw_sort_scan_kernel<<<(unsigned)n_detectors, 1024, 0, stream>>>(counts, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const size_t smem = (size_t)table_rows * sizeof(int32_t);
     if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk);
+    dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk, kSortBlock);
     LUTB_LAUNCH_CHECK();
     const int64_t segs = (int64_t)n_detectors * table_rows;
     dw_sort_reduce_kernel<<<(unsigned)((segs + 7) / 8), 256, 0, stream>>>(dY, counts, perm, target, batch, n_outputs,
@@ -143,9 +152,9 @@ int launch_fc_dw_sorted(const float *dY, const int32_t *idx, float *target, int6
 // The reduction is a chain of dependent loads (sample number, then its gradient), so it wants many warps with few
 // segments each and several samples' loads in flight: blocks of 1024 segments gave a 6400-row layer 7 blocks and 32
 // segments a warp; 64 segments and 8 warps, four samples and two columns at a time, measured 90 -> 28 us there (1111
-// samples, 33 outputs).
+// samples, 33 outputs), 32 segments and 16 warps 28 -> 11 us.
 // ------------------------------------------------------------------------------------------
-constexpr int kRowsBlock = 64, kRowsThreads = 256;   // (two warps of segments: the scan in the emit kernel counts on it)
+constexpr int kRowsBlock = 32, kRowsThreads = 512;   // (one warp of segments: the scan in the emit kernel counts on it)
 
 __device__ __forceinline__ bool segment_touched(const int32_t *offsets, int64_t seg, int table_rows, int nblk, int64_t batch,
                                                 int32_t *begin, int32_t *end) {
@@ -197,18 +206,13 @@ __global__ void __launch_bounds__(kRowsThreads) dw_rows_emit_kernel(const float 
                                                                  double lr, int64_t capacity, int64_t *__restrict__ row_ids,
                                                                  float *__restrict__ values) {
     __shared__ int32_t position[kRowsBlock];   // list position of a touched segment, -1 otherwise
-    __shared__ int32_t first_sum;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t seg0 = (int64_t)blockIdx.x * kRowsBlock;
     int32_t b, e;
-    const bool mine = threadIdx.x < kRowsBlock;   // two warps look, all of them reduce
-    const bool touched = mine && seg0 + threadIdx.x < n_seg && segment_touched(offsets, seg0 + threadIdx.x, table_rows, nblk, batch, &b, &e);
-    const unsigned mask = __ballot_sync(0xffffffffu, touched);
-    if (threadIdx.x == 0) first_sum = __popc(mask);
-    __syncthreads();
-    if (mine) {
-        const int32_t before = __ldg(block_base + blockIdx.x) + (warp == 1 ? first_sum : 0);
-        position[threadIdx.x] = touched ? before + __popc(mask & ((1u << lane) - 1u)) : -1;
+    if (warp == 0) {   // one warp looks, all of them reduce
+        const bool touched = seg0 + lane < n_seg && segment_touched(offsets, seg0 + lane, table_rows, nblk, batch, &b, &e);
+        const unsigned mask = __ballot_sync(0xffffffffu, touched);
+        position[lane] = touched ? __ldg(block_base + blockIdx.x) + __popc(mask & ((1u << lane) - 1u)) : -1;
     }
     __syncthreads();
     for (int i = warp; i < kRowsBlock; i += kRowsThreads / 32) {
@@ -246,31 +250,32 @@ __global__ void __launch_bounds__(kRowsThreads) dw_rows_emit_kernel(const float 
 
 size_t fc_dw_rows_workspace(int64_t batch, int n_detectors, int table_rows) {
     const int64_t n_blocks = ((int64_t)n_detectors * table_rows + kRowsBlock - 1) / kRowsBlock;
-    const size_t sorted = (fc_dw_sorted_workspace(batch, n_detectors, table_rows) + 15) & ~(size_t)15;
+    const size_t sorted = (sorted_workspace(batch, n_detectors, table_rows, rows_sort_block(batch, table_rows)) + 15) & ~(size_t)15;
     return sorted + (size_t)n_blocks * sizeof(int32_t);
 }
 
 int launch_fc_dw_rows(const float *dY, const int32_t *idx, int64_t batch, int n_outputs, int n_detectors, int table_rows,
                       double lr, int64_t *row_ids, float *values, int64_t capacity, int64_t *count_out, void *workspace,
                       cudaStream_t stream) {
-    const int64_t nblk64 = (batch + kSortBlock - 1) / kSortBlock;
+    const int sort_block = rows_sort_block(batch, table_rows);
+    const int64_t nblk64 = (batch + sort_block - 1) / sort_block;
     LUTB_REQUIRE(nblk64 <= 65535, LUTB_ERR_SHAPE, "batch too large for the sorted table-gradient variant");
     LUTB_REQUIRE((size_t)table_rows * 4 <= 200 * 1024, LUTB_ERR_SHAPE, "table too large for the sorted table-gradient variant");
     const int nblk = (int)nblk64;
     int32_t *counts = static_cast<int32_t *>(workspace);
     int32_t *perm = counts + (size_t)n_detectors * table_rows * nblk;
-    const size_t sorted = (fc_dw_sorted_workspace(batch, n_detectors, table_rows) + 15) & ~(size_t)15;
+    const size_t sorted = (sorted_workspace(batch, n_detectors, table_rows, rows_sort_block(batch, table_rows)) + 15) & ~(size_t)15;
     int32_t *block_sums = reinterpret_cast<int32_t *>(static_cast<unsigned char *>(workspace) + sorted);
     LUTB_CUDA(cudaMemsetAsync(counts, 0, (size_t)n_detectors * table_rows * nblk * sizeof(int32_t), stream));
     dim3 grid((unsigned)n_detectors, (unsigned)nblk);
     KernelScope scope(K_FC_WEIGHT_GRAD, stream);
-    dw_sort_count_kernel<<<grid, 256, 0, stream>>>(idx, counts, batch, n_detectors, table_rows, nblk);
+    dw_sort_count_kernel<<<grid, 256, 0, stream>>>(idx, counts, batch, n_detectors, table_rows, nblk, sort_block);
     LUTB_LAUNCH_CHECK();
     dw_sort_scan_kernel<<<(unsigned)n_detectors, 1024, 0, stream>>>(counts, table_rows, nblk);
     LUTB_LAUNCH_CHECK();
     const size_t smem = (size_t)table_rows * sizeof(int32_t);
     if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(dw_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk);
+    dw_sort_scatter_kernel<<<grid, 32, smem, stream>>>(idx, counts, perm, batch, n_detectors, table_rows, nblk, sort_block);
     LUTB_LAUNCH_CHECK();
     const int64_t n_seg = (int64_t)n_detectors * table_rows;
     const int64_t n_blocks = (n_seg + kRowsBlock - 1) / kRowsBlock;

@@ -42,6 +42,11 @@ struct Library {
     decltype(&lutb_product_workspace) product_workspace;
     decltype(&lutb_product_keeps_histogram) product_keeps_histogram;
     decltype(&lutb_zero_buffers) zero_buffers;
+    decltype(&lutb_nonseq_fc_table_grad_rows) rows;
+    decltype(&lutb_nonseq_fc_table_grad_rows_workspace) rows_workspace;
+    decltype(&lutb_dense_to_sparse_workspace) cells_workspace;
+    decltype(&lutb_row_cells_count) cells_count;
+    decltype(&lutb_row_cells_scatter) cells_scatter;
 };
 Library lib;
 
@@ -49,12 +54,12 @@ Library lib;
 struct Names {
     PyObject *dict_parameters, *dict_buffers, *weights, *anchors, *positional, *training, *dm, *shared_context, *cmp_eps, *device, *policy,
         *type, *normalized, *sequence_length, *concatenation, *sliced, *positional_dim, *unified, *fully_connected, *dw_variant,
-        *product_variant, *dm_device, *dm_fully_connected, *dm_sparse, *dm_seq_len, *dm_forward_seen, *dm_kept, *n_weights,
+        *product_variant, *sparse_rows_direct, *dm_device, *dm_fully_connected, *dm_sparse, *dm_seq_len, *dm_forward_seen, *dm_kept, *n_weights,
         *rows_per_detector, *cfg, *c_struct, *input_shape, *output_shape, *prepare_positional, *external_lr, *scratch, *scratch_limit, *keep_limit,
         *product_ws;
 };
 Names names;
-PyObject *manager_class, *manager_base, *tensor_class, *parameter_class, *policy_dense, *policy_internal, *check_status, *layer_class;
+PyObject *manager_class, *manager_base, *tensor_class, *parameter_class, *policy_dense, *policy_internal, *policy_sparse, *check_status, *layer_class;
 // methods whose replacement, on an instance or by a subclass, sends a call to the Python route
 std::vector<std::pair<PyObject *, PyObject *>> layer_methods, manager_methods;   // (name, original)
 std::vector<PyObject *> layer_hooks;
@@ -339,6 +344,36 @@ variable_list python_backward(LayerNode &node, const std::vector<Tensor> &saved,
     raise_current();   // (the engine hands Python's own exception on to the caller of backward)
 }
 
+// The Sparse policy's list straight from the table-gradient pass: fully connected non-sequence layers, unless switched off.
+bool rows_direct(const Call &c) {
+    return c.mode == NONSEQ && c.fully_connected && item(c.dict, names.sparse_rows_direct) == nullptr &&
+           _PyType_Lookup(Py_TYPE(c.layer), names.sparse_rows_direct) == Py_True;
+}
+
+// What the manager's table_gradient_cells does, as a sparse tensor; undefined where no cell is touched.
+Tensor sparse_table_gradient(const Call &c, int64_t B, const Tensor &dy, const Tensor &idx) {
+    const int64_t O = c.cfg.n_outputs, capacity = std::min<int64_t>(B, (int64_t)1 << c.cfg.n_anchors) * c.cfg.n_detectors;
+    const auto on = at::TensorOptions().device(at::kCUDA, c.device);
+    auto bytes = [&](size_t n) { return at::empty({(int64_t)n}, on.dtype(at::kByte)); };
+    const size_t rows_need = lib.rows_workspace(&c.cfg, B), cells_need = lib.cells_workspace(capacity * O);
+    const Tensor ws = bytes(rows_need), ws2 = bytes(cells_need), ids = at::empty({capacity}, on.dtype(at::kLong)),
+                 values = new_f32({capacity * O}, c), counts = at::empty({2}, on.dtype(at::kLong));
+    int64_t *ids_p = static_cast<int64_t *>(ids.data_ptr()), *count = static_cast<int64_t *>(counts.data_ptr()), *total = count + 1;
+    check(lib.rows(&c.cfg, B, f32(dy), i32(idx), ids_p, f32(values), capacity, count, ws.data_ptr(), rows_need, stream_of(c)));
+    check(lib.cells_count(f32(values), count, capacity, (int32_t)O, total, ws2.data_ptr(), cells_need, stream_of(c)));
+    int64_t n;
+    {
+        pybind11::gil_scoped_release others;
+        n = counts.select(0, 1).item<int64_t>();
+    }
+    if (n == 0) return Tensor();
+    const Tensor cells = at::empty({1, n}, on.dtype(at::kLong)), out = new_f32({n}, c);
+    check(lib.cells_scatter(f32(values), ids_p, count, capacity, (int32_t)O, static_cast<int64_t *>(cells.data_ptr()), f32(out), n, ws2.data_ptr(),
+                            cells_need, stream_of(c)));
+    return at::_sparse_coo_tensor_unsafe(cells, out, c.weights.sizes(), at::TensorOptions().dtype(at::kFloat).layout(at::kSparse).device(at::kCUDA, c.device),
+                                         true);
+}
+
 variable_list LayerNode::apply(variable_list &&grads) {
     std::vector<Tensor> s;
     {
@@ -358,7 +393,7 @@ variable_list LayerNode::apply(variable_list &&grads) {
     const bool readable = ordinary_context() && read_layer(layer, c, true);
     if (!readable) PyErr_Clear();
     bool native = readable && c.mode == mode && !c.normalized &&
-                  (c.policy_type == policy_dense || c.policy_type == policy_internal) && is_true(item(c.dm_dict, names.dm_forward_seen));
+                  (c.policy_type == policy_dense || c.policy_type == policy_internal || (c.policy_type == policy_sparse && rows_direct(c))) && is_true(item(c.dm_dict, names.dm_forward_seen));
     for (size_t i = 0; native && i < s.size(); i++) {
         const bool ints = mode != PRODUCT && (i == 1 || i == 3 || i == 4 || i == 6);
         native = plain_cuda(s[i], ints ? at::kInt : at::kFloat, c.device);
@@ -371,7 +406,7 @@ variable_list LayerNode::apply(variable_list &&grads) {
     c10::cuda::CUDAGuard guard(c.device);
     const Tensor xc = x.contiguous(), dyc = dy.contiguous();
     const int64_t B = x.dim() > 0 ? x.size(0) : 0;
-    const bool internal = c.policy_type == policy_internal;
+    const bool internal = c.policy_type == policy_internal, listed = c.policy_type == policy_sparse;
     // shapes: the saved tensors could come from a hook, the gradient from anywhere
     const int64_t Nt = c.cfg.n_detectors, tokens = B * c.S;
     bool fits = B > 0 && dy.numel() == tokens * c.cfg.n_outputs && x.dim() >= 2 && x.size(1) == c.S;
@@ -394,18 +429,21 @@ variable_list LayerNode::apply(variable_list &&grads) {
         if (lr == -1.0 && PyErr_Occurred()) raise_current();
     }
     Tensor dx, dw, dpe;
-    if (!internal) dw = new_f32(c.weights.sizes(), c);
+    if (listed) lr = LUTB_SKIP_TABLE_GRADIENT;   // (the list has its own pass)
+    else if (!internal) dw = new_f32(c.weights.sizes(), c);
     float *target = f32(dw);
     if (mode == NONSEQ) {
         if (need_dx) dx = new_f32(x.sizes(), c);
         if (c.fully_connected) {
             if (need_dx) dw_variant |= LUTB_DX_WRITE;   // (written, not added to)
             if (dw.defined()) clear(c, dw);
+            if (listed && !need_dx) return {dx, sparse_table_gradient(c, B, dyc, s[1])};
             const size_t need = lib.fc_backward_workspace(&c.cfg, B, (int)dw_variant);
             Tensor ws;
             if (need) ws = at::empty({(int64_t)need}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, c.device));
             check(lib.fc_backward(&c.cfg, B, f32(c.weights), f32(dyc), i32(c.anchors), i32(s[1]), f32(s[2]), i32(s[3]), f32(dx), target, lr,
                                   (int)dw_variant, need ? ws.data_ptr() : nullptr, need, stream_of(c)));
+            if (listed) dw = sparse_table_gradient(c, B, dyc, s[1]);
         } else {
             clear(c, dx, dw);
             check(lib.sparse_backward(&c.cfg, &c.sparse, B, f32(c.weights), f32(dyc), i32(c.anchors), i32(s[1]), f32(s[2]), i32(s[3]), f32(dx),
@@ -582,7 +620,7 @@ PyObject *apply_entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::object manager_cls, pybind11::object base_cls, pybind11::object dense,
-           pybind11::object internal, pybind11::object check_fn, pybind11::list layer_names, pybind11::list hook_names, pybind11::list manager_names) {
+           pybind11::object internal, pybind11::object sparse, pybind11::object check_fn, pybind11::list layer_names, pybind11::list hook_names, pybind11::list manager_names) {
     auto take = [&](const char *name, auto &fn) { fn = reinterpret_cast<std::decay_t<decltype(fn)>>(addresses[name].cast<uintptr_t>()); };
     take("lutb_nonseq_fc_forward", lib.fc_forward);
     take("lutb_nonseq_fc_backward", lib.fc_backward);
@@ -596,12 +634,18 @@ void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::objec
     take("lutb_product_workspace", lib.product_workspace);
     take("lutb_product_keeps_histogram", lib.product_keeps_histogram);
     take("lutb_zero_buffers", lib.zero_buffers);
+    take("lutb_nonseq_fc_table_grad_rows", lib.rows);
+    take("lutb_nonseq_fc_table_grad_rows_workspace", lib.rows_workspace);
+    take("lutb_dense_to_sparse_workspace", lib.cells_workspace);
+    take("lutb_row_cells_count", lib.cells_count);
+    take("lutb_row_cells_scatter", lib.cells_scatter);
     auto keep = [](pybind11::object o) { return o.release().ptr(); };   // for the life of the process
     layer_class = keep(layer_cls);
     manager_class = keep(manager_cls);
     manager_base = keep(base_cls);
     policy_dense = keep(dense);
     policy_internal = keep(internal);
+    policy_sparse = keep(sparse);
     check_status = keep(check_fn);
     tensor_class = keep(pybind11::module_::import("torch").attr("Tensor"));
     parameter_class = keep(pybind11::module_::import("torch.nn").attr("Parameter"));
@@ -609,7 +653,7 @@ void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::objec
     names = Names{in("_parameters"), in("_buffers"), in("_weights"), in("_detector_anchors"), in("_positional_embeddings"), in("training"), in("_lut_dm"),
                   in("_shared_context"), in("_cmp_eps"), in("device"), in("_weights_gradient_policy"), in("type"), in("normalized"), in("_sequence_length"),
                   in("_concatenation_product"), in("_sliced_product_mode"), in("_positional_dim"), in("_unified_positional_embeddings"),
-                  in("_is_fully_connected"), in("_dw_variant"), in("_product_variant"), in("_device"),
+                  in("_is_fully_connected"), in("_dw_variant"), in("_product_variant"), in("_sparse_rows_direct"), in("_device"),
                   in("_fully_connected"), in("_sparse"), in("_seq_len"), in("_forward_seen"), in("_kept_histogram"), in("n_weights"),
                   in("_rows_per_detector"), in("_cfg"), in("c_struct"), in("input_shape"), in("output_shape"), in("_prepare_positional_embeddings"),
                   in("_external_lr"), in("_product_scratch"), in("product_scratch_limit"), in("product_keep_limit"), in("_product_workspace")};

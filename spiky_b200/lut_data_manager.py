@@ -359,11 +359,8 @@ class _LUTDataManager:
                                            w_input_gradients, external_lr, w_weights_gradients)
         _native.check(rc)
 
-    def table_gradient_rows(self, batch_size, r_output_gradients, r_lookup_indices):
-        """Table gradient of a fully connected non-sequence layer as a list of touched rows (not part of the
-        reference's class, which forms the dense gradient and compacts it): returns ``(row_ids int64 [n],
-        values fp32 [n, n_outputs])`` with ``row_ids = detector * 2^Nc + row`` ascending.  fp32 accumulators only.
-        Reads the number of touched rows back from the device (like the reference's converter does)."""
+    def _row_list(self, batch_size, r_output_gradients, r_lookup_indices):
+        """Launches the row-list table gradient; (row ids, values, count on the device, capacity in rows)."""
         self._require_cuda()
         if not self._fully_connected or self._seq_len != 1:
             raise ValueError("the row-list table gradient exists for fully connected non-sequence layers")
@@ -379,13 +376,41 @@ class _LUTDataManager:
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
             row_ids = torch.empty(capacity, dtype=torch.int64, device=dev)
             values = torch.empty(capacity * O, dtype=torch.float32, device=dev)
-            count = torch.zeros(1, dtype=torch.int64, device=dev)
+            count = torch.empty(1, dtype=torch.int64, device=dev)
             rc = L.lutb_nonseq_fc_table_grad_rows(ctypes.byref(cfg), B, _ptr(r_output_gradients), _ptr(r_lookup_indices),
                                                   _ptr(row_ids), _ptr(values), capacity, _ptr(count), _ptr(ws), ws_bytes,
                                                   self._stream())
         _native.check(rc)
+        return row_ids, values, count, capacity
+
+    def table_gradient_rows(self, batch_size, r_output_gradients, r_lookup_indices):
+        """Table gradient of a fully connected non-sequence layer as a list of touched rows (not part of the
+        reference's class, which forms the dense gradient and compacts it): returns ``(row_ids int64 [n],
+        values fp32 [n, n_outputs])`` with ``row_ids = detector * 2^Nc + row`` ascending.  fp32 accumulators only.
+        Reads the number of touched rows back from the device (like the reference's converter does)."""
+        row_ids, values, count, _ = self._row_list(batch_size, r_output_gradients, r_lookup_indices)
         n = int(count.item())
-        return row_ids[:n], values[:n * O].view(n, O)
+        return row_ids[:n], values[:n * self._n_outputs].view(n, self._n_outputs)
+
+    def table_gradient_cells(self, batch_size, r_output_gradients, r_lookup_indices):
+        """The same as (cell int64 [n], value fp32 [n]) lists, cells ascending and without zeros, or (None, None) when there
+        are none; one count is read back from the device, that of the cells."""
+        row_ids, values, count, capacity = self._row_list(batch_size, r_output_gradients, r_lookup_indices)
+        O, dev = self._n_outputs, values.device
+        L = _native.lib()
+        with torch.cuda.device(self._device):
+            need = L.lutb_dense_to_sparse_workspace(capacity * O)
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)
+            total = torch.empty(1, dtype=torch.int64, device=dev)
+            _native.check(L.lutb_row_cells_count(_ptr(values), _ptr(count), capacity, O, _ptr(total), _ptr(ws), need, self._stream()))
+            n = int(total.item())
+            if n == 0:
+                return None, None
+            cells = torch.empty(n, dtype=torch.int64, device=dev)
+            out = torch.empty(n, dtype=torch.float32, device=dev)
+            _native.check(L.lutb_row_cells_scatter(_ptr(values), _ptr(row_ids), _ptr(count), capacity, O, _ptr(cells), _ptr(out), n,
+                                                   _ptr(ws), need, self._stream()))
+        return cells, out
 
     def table_gradient(self, batch_size, r_output_gradients, r_lookup_indices, w_target, scale, chunk_begin=0,
                        chunk_end=None):

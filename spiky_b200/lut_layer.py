@@ -515,19 +515,10 @@ class LUTLayerBasic(nn.Module):
                                  min_anchor_deltas.reshape(-1), min_anchor_delta_indices.reshape(-1), x_grad.view(-1),
                                  SKIP_TABLE_GRADIENT, None, None, dw_variant=dw_variant)
         dx = None if x_grad is None else x_grad.view(x.shape)
-        rows, values = dm.table_gradient_rows(batch_size, grad_flat, idx_flat)
-        if rows.numel() == 0:
-            return dx, None
-        O = values.shape[1]
         # zero cells (an output gradient that is exactly zero or below the threshold) are not part of the list
-        flat = values.reshape(-1)
-        pad = (-flat.numel()) % 4
-        if pad:
-            flat = torch.cat([flat, flat.new_zeros(pad)])
-        nz, vals = self._shared_context.get_dense_to_sparse_converter(self._multi_id).dense_to_sparse_32(flat)
-        if nz is None:
+        cells, vals = dm.table_gradient_cells(batch_size, grad_flat, idx_flat)
+        if cells is None:
             return dx, None
-        cells = rows[nz // O] * O + nz % O
         if self._weights_gradient_policy.normalized:
             vals /= vals.abs().max().clip(1e-16)
         return dx, torch.sparse_coo_tensor(cells.unsqueeze(0), vals, size=self._weights.shape, device=self.device,

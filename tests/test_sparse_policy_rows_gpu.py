@@ -89,3 +89,29 @@ def test_row_list_entry_point_counts_rows_beyond_the_capacity():
     rc = L.lutb_nonseq_fc_table_grad_rows(ctypes.byref(cfg), B, ptr(dY), ptr(idx.reshape(-1).contiguous()), ptr(rows), ptr(vals),
                                           cap, ptr(count), ptr(ws), need - 1, stream)
     assert rc == -4
+
+
+@pytest.mark.parametrize("shape", [(1, 5, 1, 1, 1), (130, 16, 3, 4, 1), (257, 20, 7, 3, 13), (2049, 16, 9, 7, 33), (1024, 12, 33, 1, 8)])
+@pytest.mark.parametrize("zeros", ["none", "columns", "all"])
+def test_cells_of_the_row_list(shape, zeros):
+    """The (cell, value) list from the count that stays on the device: row lists that end inside and at a tile of 2048 words, rows
+    shorter and longer than a thread's eight words, both slice lengths of the sort."""
+    B, I, Nt, Nc, O = shape
+    layer = make_layer(I, Nc, Nt, O, seed=60 + B)
+    x = torch.from_numpy(synth.uniform(3, (B, 1, I))).cuda()
+    dY = synth.normal(4, (B, O))
+    if zeros == "columns":
+        dY[:, ::2] = 0.0
+    if zeros == "all":
+        dY[:] = 0.0
+    dYt = torch.from_numpy(dY).cuda()
+    _, idx, _, _ = layer.forward_step(x)
+    dm = layer._lut_dm
+    rows, values = dm.table_gradient_rows(B, dYt.view(-1), idx.reshape(-1))
+    cells, got = dm.table_gradient_cells(B, dYt.view(-1), idx.reshape(-1))
+    flat = values.reshape(-1)
+    at = flat.nonzero().view(-1)
+    if at.numel() == 0:
+        assert cells is None and got is None
+        return
+    assert torch.equal(cells, rows[at // O] * O + at % O) and torch.equal(got, flat[at])
