@@ -27,9 +27,8 @@
 // the result added by a kernel of their own): see the table at launch_contraction.
 #include "hist_gemm_sm100.cuh"
 
-#include <cuda.h>
-
 #include "mbarrier.cuh"
+#include "tensor_map.cuh"
 
 namespace lutb {
 
@@ -129,15 +128,17 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
     }
 }
 
-// Largest magnitude of every column (bits cleared by the caller): blocks of 64 threads by 4 rows, 4 columns a thread.
-__global__ void __launch_bounds__(256) column_max_kernel(const float *__restrict__ x, int64_t rows, int cols, uint32_t *__restrict__ bits) {
-    __shared__ uint4 part[4][64];
-    const int c4 = blockIdx.x * 64 + (threadIdx.x & 63), ty = threadIdx.x >> 6;
+// Largest magnitude of every column (bits cleared before): 4 columns a thread, 64 threads by 16 rows a block, one block an SM so
+// that few of them meet in the atomics (16384 x 256: 6.9 us; 9.7 with 444 blocks of 256 threads, 33 with 1024).
+constexpr int kMaxRows = 16;
+__global__ void __launch_bounds__(64 * kMaxRows) column_max_kernel(const float *__restrict__ x, int64_t rows, int cols, uint32_t *__restrict__ bits) {
+    __shared__ uint4 part[kMaxRows][64];
+    const int tx = threadIdx.x & 63, c4 = blockIdx.x * 64 + tx, ty = threadIdx.x >> 6;
     const bool live = c4 < (cols >> 2);
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
     if (live) {
 #pragma unroll 8
-        for (int64_t r = (int64_t)blockIdx.y * 4 + ty; r < rows; r += (int64_t)gridDim.y * 4) {
+        for (int64_t r = (int64_t)blockIdx.y * kMaxRows + ty; r < rows; r += (int64_t)gridDim.y * kMaxRows) {
             const float4 v = __ldg(reinterpret_cast<const float4 *>(x + r * cols) + c4);
             m.x = max(m.x, __float_as_uint(v.x) & 0x7fffffffu);
             m.y = max(m.y, __float_as_uint(v.y) & 0x7fffffffu);
@@ -145,20 +146,15 @@ __global__ void __launch_bounds__(256) column_max_kernel(const float *__restrict
             m.w = max(m.w, __float_as_uint(v.w) & 0x7fffffffu);
         }
     }
-    part[ty][threadIdx.x & 63] = m;
+    part[ty][tx] = m;
     __syncthreads();
-    if (ty == 0 && live) {
+    // a thread per column
+    const int col = blockIdx.x * 256 + threadIdx.x;
+    if (threadIdx.x < 256 && col < cols) {
+        uint32_t most = 0u;
 #pragma unroll
-        for (int k = 1; k < 4; k++) {
-            const uint4 o = part[k][threadIdx.x];
-            m.x = max(m.x, o.x); m.y = max(m.y, o.y); m.z = max(m.z, o.z); m.w = max(m.w, o.w);
-        }
-        // (most blocks find a larger one there: an atomic each on a few hundred addresses took 33 us for 16384 x 256)
-        const uint4 seen = __ldcg(reinterpret_cast<const uint4 *>(bits) + c4);
-        if (m.x > seen.x) atomicMax(bits + 4 * c4, m.x);
-        if (m.y > seen.y) atomicMax(bits + 4 * c4 + 1, m.y);
-        if (m.z > seen.z) atomicMax(bits + 4 * c4 + 2, m.z);
-        if (m.w > seen.w) atomicMax(bits + 4 * c4 + 3, m.w);
+        for (int k = 0; k < kMaxRows; k++) most = max(most, reinterpret_cast<const uint32_t *>(part[k])[threadIdx.x]);
+        if (most > __ldcg(bits + col)) atomicMax(bits + col, most);   // (later blocks mostly find a larger one there)
     }
 }
 
@@ -184,10 +180,13 @@ __global__ void __launch_bounds__(kAddThreads) add_parts_kernel(const float *__r
     const int64_t n4 = M * (N / 4);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         double s[4] = {0., 0., 0., 0.};
-#pragma unroll 8
-        for (int k = 0; k < parts; k++) {
-            const float4 t = __ldcs(reinterpret_cast<const float4 *>(P + k * part_stride) + i);
-            s[0] += t.x; s[1] += t.y; s[2] += t.z; s[3] += t.w;
+        for (int k0 = 0; k0 < parts; k0 += 16) {
+            float4 t[16];   // (all loads in flight: they are one latency each otherwise)
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                t[k] = k0 + k < parts ? __ldcs(reinterpret_cast<const float4 *>(P + (k0 + k) * part_stride) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 16; k++) { s[0] += t[k].x; s[1] += t[k].y; s[2] += t[k].z; s[3] += t[k].w; }
         }
         float4 *dst = reinterpret_cast<float4 *>(C) + i;
         float4 o = *dst;
@@ -514,35 +513,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (kEpilogueWarps
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-    static const EncodeTiled fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-            found != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiled>(p);
-    }();
-    return fn;
-}
-
 // A row-major matrix [rows x cols] read in boxes of box_rows x 64 (fp16) or written in boxes of 32 x 16 (fp32), swizzled.
 int tensor_map(CUtensorMap *map, bool half, const void *p, int64_t rows, int64_t cols, int64_t pitch_bytes, int box_rows) {
-    const int box_cols = half ? 64 : 16;
-    const EncodeTiled encode = encode_tiled();
-    LUTB_REQUIRE(encode != nullptr, LUTB_ERR_MODE, "the driver offers no tensor maps");
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, ones[2] = {1, 1};
-    const CUresult rc = encode(map, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(p), dims, strides,
-                               box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, half ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    LUTB_REQUIRE(rc == CUDA_SUCCESS, LUTB_ERR_SHAPE, "tensor map of %lld x %lld (pitch %lld bytes) refused: %d", (long long)rows,
-                 (long long)cols, (long long)pitch_bytes, (int)rc);
-    return LUTB_OK;
+    return tensor_map_2d(map, half ? 2 : 4, p, rows, cols, pitch_bytes, box_rows, half ? 64 : 16, half ? 128 : 64);
 }
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -587,10 +560,11 @@ int copy_by_row(const float *x, int64_t rows, int cols, const Copy &c, cudaStrea
 
 int copy_by_column(const float *x, int64_t rows, int cols, const Copy &c, cudaStream_t stream) {
     const int gx = (cols / 4 + 63) / 64;
-    const int64_t want = (rows + 15) / 16, cap = ((int64_t)device_info().sm_count * 8 + gx - 1) / gx, cap_max = ((int64_t)device_info().sm_count * 3 + gx - 1) / gx;
+    const int64_t sm = device_info().sm_count;
+    const int64_t want = (rows + 15) / 16, cap = (sm * 8 + gx - 1) / gx, cap_max = ((rows > 65536 ? 2 * sm : sm) + gx - 1) / gx;
     const dim3 grid((unsigned)gx, (unsigned)(want < cap ? want : cap)), grid_max((unsigned)gx, (unsigned)(want < cap_max ? want : cap_max));
     LUTB_CUDA(cudaMemsetAsync(c.bits, 0, (size_t)cols * 4, stream));
-    column_max_kernel<<<grid_max, 256, 0, stream>>>(x, rows, cols, c.bits);
+    column_max_kernel<<<grid_max, 64 * kMaxRows, 0, stream>>>(x, rows, cols, c.bits);
     LUTB_LAUNCH_CHECK();
     split_columns_kernel<<<grid, 256, 0, stream>>>(x, rows, cols, c.hi, c.lo, c.pitch, c.bits);
     LUTB_LAUNCH_CHECK();

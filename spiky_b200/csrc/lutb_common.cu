@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "lutb_common.cuh"
+#include "tensor_map.cuh"
 
 namespace lutb {
 
@@ -32,6 +33,38 @@ DeviceInfo device_info() {
     if (d.device < 64) sm_counts[d.device] = n;
     d.sm_count = n;
     return d;
+}
+
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+
+int tensor_map_2d(CUtensorMap *map, int element_bytes, const void *p, int64_t rows, int64_t cols, int64_t pitch_bytes, int box_rows, int box_cols,
+                  int swizzle_bytes) {
+    const EncodeTiled encode = encode_tiled();
+    LUTB_REQUIRE(encode != nullptr, LUTB_ERR_MODE, "the driver offers no tensor maps");
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, ones[2] = {1, 1};
+    const CUtensorMapDataType type = element_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : element_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    const CUtensorMapSwizzle swizzle = swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE;
+    const CUresult rc = encode(map, type, 2, const_cast<void *>(p), dims, strides,
+                               box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    LUTB_REQUIRE(rc == CUDA_SUCCESS, LUTB_ERR_SHAPE, "tensor map of %lld x %lld (pitch %lld bytes) refused: %d", (long long)rows,
+                 (long long)cols, (long long)pitch_bytes, (int)rc);
+    return LUTB_OK;
 }
 
 int validate_cfg(const lutb_layer_cfg *cfg) {
