@@ -174,12 +174,13 @@ extern "C" int lutb_infer_int8_accumulate_ws(const lutb_layer_cfg *cfg, int64_t 
     const int64_t pass = infer_staged_pass(cfg, batch, true);
     uint8_t *packed = static_cast<uint8_t *>(workspace);
     void *plan = packed + packed_index_bytes(cfg, pass);
+    uint32_t *anchor_plan = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(workspace) + need - anchor_plan_bytes(cfg));
     rc = launch_int8_scale_plan(cfg, scales, plan, st);
     if (rc) return rc;
     for (int64_t b0 = 0; b0 < batch; b0 += pass) {
         const int64_t n = batch - b0 < pass ? batch - b0 : pass;
         rc = launch_check_detectors(x + b0 * cfg->n_inputs, n, cfg->n_inputs, anchors, cfg->n_detectors, cfg->n_anchors, cfg->cmp_eps,
-                                    idx + b0 * cfg->n_detectors, nullptr, nullptr, st, packed, packed_index_pitch(n));
+                                    idx + b0 * cfg->n_detectors, nullptr, nullptr, st, packed, packed_index_pitch(n), anchor_plan);
         if (rc) return rc;
         rc = launch_infer_staged_int8(cfg, n, q_tables, scales, plan, packed, acc + b0 * cfg->n_outputs, st);
         if (rc) return rc;

@@ -2,11 +2,14 @@
 //
 // Gathering rows from L2 is limited by the number of row requests (about 37 G rows a second whether a row is 64 or 256
 // bytes), and a large batch asks for every row many times.  Here a block owns a tile of samples, keeps its sums in
-// registers and streams the tables of a run of detectors through a three-slot shared-memory ring (cp.async, two
+// registers and streams the tables of a run of detectors through a three-slot shared-memory ring (two
 // or four detectors a slot), so that a row costs one conflict-free shared-memory wavefront: the 8 lanes that add a row read its
 // 128 bytes side by side.  What a block loads is the whole table once per tile, so tiles are as large as the register
 // file allows; a small batch reads the tables once, in order, instead of by random rows.
 #include "infer_staged.cuh"
+
+#include "mbarrier.cuh"
+#include "tensor_map.cuh"
 
 namespace lutb {
 
@@ -42,87 +45,130 @@ struct StagedFp32 {
     int O, Nt, T, n_tiles, n_slices, n_items;
 };
 
-__global__ void __launch_bounds__(kStagedThreads, 1) infer_staged_fp32_kernel(const StagedFp32 p) {
-    extern __shared__ __align__(16) unsigned char sbuf[];
+// A warp of its own brings the tables in by TMA (a column slice of a whole table is one box) and the samples' indices by bulk
+// copies, and waits for a slot's readers one by one; the 16 warps that add wait for a slot to fill and say when they have read it, so
+// that none of them waits for the slowest (with cp.async and a block barrier per two detectors, 1024 samples a step: 834 -> 600 us
+// for 16384 samples, 4096 detectors of 256 rows x 64 outputs, the rate of the shared-memory wavefronts: 480 us of row reads and
+// 120 of tables coming in).
+__device__ int g_staged_wait_errors = 0;
+
+int staged_wait_errors(int *count_out) {
+    LUTB_CUDA(cudaMemcpyFromSymbol(count_out, g_staged_wait_errors, sizeof(int)));
+    return LUTB_OK;
+}
+
+// After a wait that ran out: tell the block's others, and leave only after a time in which every copy in flight has landed.
+__device__ __noinline__ void leave_late(volatile int *gave_up) {
+    if (*gave_up == 0) atomicAdd(&g_staged_wait_errors, 1);
+    *gave_up = 1;
+    const long long t0 = clock64();
+    while (clock64() - t0 < kWaitLimitCycles / 16) {
+    }
+}
+
+__device__ __forceinline__ void tma_load_box(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"(map), "r"(bar), "r"(x), "r"(y)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(kStagedThreads + 32, 1) infer_staged_fp32_kernel(const __grid_constant__ CUtensorMap tables, const StagedFp32 p) {
+    extern __shared__ __align__(128) unsigned char sbuf[];
     const int stage_floats = 2 * p.T * kRow;
     float *ring = reinterpret_cast<float *>(sbuf);                             // [kStages][2][T][kRow]
     uint8_t *ibuf = sbuf + (size_t)kStages * stage_floats * 4;                 // [kStages][2][kTile]
+    const uint32_t full0 = smem_addr(ibuf + (size_t)kStages * 2 * kTile), empty0 = full0 + 8 * kStages;
+    volatile int *gave_up = reinterpret_cast<volatile int *>(ibuf + (size_t)kStages * 2 * kTile + 16 * kStages);
     const int tid = threadIdx.x, g = tid / kLanes, l = tid % kLanes;
     const uint32_t mask = (uint32_t)p.T - 1u;   // (samples past the batch hold any byte)
-    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-        // detector blocks outermost: the blocks that run together read the same tables
-        const int per = p.n_tiles * p.n_slices;
-        const int db = item / per, ts = item - db * per;
-        const int tile = ts / p.n_slices, slice = ts - tile * p.n_slices;
-        const int t0 = db * kDetBlock, nd = min(kDetBlock, p.Nt - t0), np = (nd + 1) / 2;
-        const int64_t b0 = (int64_t)tile * kTile;
-        const int c0 = slice * kRow, width = min(kRow, p.O - c0);
-        auto load_stage = [&](int pr) {
-            if (pr < np) {
-                const int slot = pr % kStages;
-                const uint32_t dst = smem_addr(ring + (size_t)slot * stage_floats);
-                const int dets = min(2, nd - 2 * pr);
-                const float *src = p.W + (size_t)(t0 + 2 * pr) * p.T * p.O + c0;   // the two tables are neighbours
-                if (l * 4 < width)
-                    for (int r = g; r < dets * p.T; r += kGroups)
-                        async_copy<16>(dst + (uint32_t)(r * kRow + l * 4) * 4u, src + (size_t)r * p.O + l * 4);
-                // row indices of the tile (the packed rows are padded to whole tiles)
-                const uint32_t idst = smem_addr(ibuf + (size_t)slot * 2 * kTile);
-                if (tid < dets * (kTile / 16)) {
-                    const int d = tid / (kTile / 16), q = tid % (kTile / 16);
-                    async_copy<16>(idst + (uint32_t)(d * kTile + q * 16), p.packed + (size_t)(t0 + 2 * pr + d) * p.pitch + b0 + q * 16);
-                }
-            }
-            async_commit();
-        };
-        float2 acc[kSlots][2];
-#pragma unroll
-        for (int s = 0; s < kSlots; s++) acc[s][0] = acc[s][1] = make_float2(0.f, 0.f);
-        load_stage(0);
-        load_stage(1);
-        for (int pr = 0; pr < np; pr++) {
-            async_wait<1>();
-            __syncthreads();          // stage pr has landed; stage pr - 1 is free
-            load_stage(pr + 2);
-            const int slot = pr % kStages;
-            const char *tab = reinterpret_cast<const char *>(ring + (size_t)slot * stage_floats) + l * 16;
-            const uint8_t *ib = ibuf + (size_t)slot * 2 * kTile + g * kSlots;
-            const uint4 ia = *reinterpret_cast<const uint4 *>(ib);
-            const uint32_t wa[4] = {ia.x, ia.y, ia.z, ia.w};
-            if (2 * pr + 1 < nd) {
-                const uint4 ic = *reinterpret_cast<const uint4 *>(ib + kTile);
-                const uint32_t wb[4] = {ic.x, ic.y, ic.z, ic.w};
-                const char *tab2 = tab + (size_t)p.T * kRow * 4;
-#pragma unroll
-                for (int s = 0; s < kSlots; s++) {
-                    const uint32_t ra = (wa[s / 4] >> (8 * (s % 4))) & mask, rb = (wb[s / 4] >> (8 * (s % 4))) & mask;
-                    const float4 a = *reinterpret_cast<const float4 *>(tab + ra * (kRow * 4));
-                    const float4 b = *reinterpret_cast<const float4 *>(tab2 + rb * (kRow * 4));
-                    acc[s][0] = __fadd2_rn(acc[s][0], __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y)));
-                    acc[s][1] = __fadd2_rn(acc[s][1], __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w)));
-                }
-            } else {
-#pragma unroll
-                for (int s = 0; s < kSlots; s++) {
-                    const uint32_t ra = (wa[s / 4] >> (8 * (s % 4))) & mask;
-                    const float4 a = *reinterpret_cast<const float4 *>(tab + ra * (kRow * 4));
-                    acc[s][0] = __fadd2_rn(acc[s][0], make_float2(a.x, a.y));
-                    acc[s][1] = __fadd2_rn(acc[s][1], make_float2(a.z, a.w));
-                }
-            }
+    if (tid == 0) {
+        for (int s = 0; s < kStages; s++) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, kStagedThreads / 32);
         }
-        if (l * 4 < width) {
-            float *out = p.out + (size_t)db * p.batch * p.O + c0 + l * 4;
-#pragma unroll
-            for (int s = 0; s < kSlots; s++) {
-                const int64_t b = b0 + g * kSlots + s;
-                if (b < p.batch)
-                    *reinterpret_cast<float4 *>(out + (size_t)b * p.O) = make_float4(acc[s][0].x, acc[s][0].y, acc[s][1].x, acc[s][1].y);
-            }
-        }
-        async_wait<0>();
-        __syncthreads();   // the ring is free for the next item
+        *gave_up = 0;
+        fence_barrier_init();
     }
+    __syncthreads();
+    // detector blocks outermost: the blocks that run together read the same tables
+    const int per = p.n_tiles * p.n_slices;
+    int slot = 0;
+    uint32_t phase = 0u;
+    bool ok = true;
+    if (tid >= kStagedThreads) {
+        if (tid == kStagedThreads) {
+            for (int item = blockIdx.x; item < p.n_items && ok; item += gridDim.x) {
+                const int db = item / per, ts = item - db * per;
+                const int tile = ts / p.n_slices, slice = ts - tile * p.n_slices;
+                const int t0 = db * kDetBlock, nd = min(kDetBlock, p.Nt - t0);
+                for (int t = t0; t < t0 + nd; t += 2) {
+                    ok = mbar_wait(empty0 + 8 * slot, phase ^ 1u) && *gave_up == 0;
+                    if (!ok) break;
+                    const int dets = min(2, t0 + nd - t);
+                    const uint32_t bar = full0 + 8 * slot, dst = smem_addr(ring + (size_t)slot * stage_floats), idst = smem_addr(ibuf + (size_t)slot * 2 * kTile);
+                    mbar_arrive_expect_tx(bar, (uint32_t)dets * (uint32_t)(p.T * kRow * 4 + kTile));
+                    for (int d = 0; d < dets; d++) {
+                        tma_load_box(dst + (uint32_t)(d * p.T * kRow * 4), &tables, slice * kRow, (t + d) * p.T, bar);
+                        bulk_copy_g2s(idst + (uint32_t)(d * kTile), p.packed + (size_t)(t + d) * p.pitch + (size_t)tile * kTile, kTile, bar);
+                    }
+                    if (++slot == kStages) { slot = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else {
+        for (int item = blockIdx.x; item < p.n_items && ok; item += gridDim.x) {
+            const int db = item / per, ts = item - db * per;
+            const int tile = ts / p.n_slices, slice = ts - tile * p.n_slices;
+            const int t0 = db * kDetBlock, nd = min(kDetBlock, p.Nt - t0), np = (nd + 1) / 2;
+            const int64_t b0 = (int64_t)tile * kTile;
+            const int c0 = slice * kRow, width = min(kRow, p.O - c0);
+            float2 acc[kSlots][2];
+#pragma unroll
+            for (int s = 0; s < kSlots; s++) acc[s][0] = acc[s][1] = make_float2(0.f, 0.f);
+            for (int pr = 0; pr < np; pr++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, phase) && *gave_up == 0);
+                if (!ok) break;
+                const char *tab = reinterpret_cast<const char *>(ring + (size_t)slot * stage_floats) + l * 16;
+                const uint8_t *ib = ibuf + (size_t)slot * 2 * kTile + g * kSlots;
+                const uint4 ia = *reinterpret_cast<const uint4 *>(ib);
+                const uint32_t wa[4] = {ia.x, ia.y, ia.z, ia.w};
+                if (2 * pr + 1 < nd) {
+                    const uint4 ic = *reinterpret_cast<const uint4 *>(ib + kTile);
+                    const uint32_t wb[4] = {ic.x, ic.y, ic.z, ic.w};
+                    const char *tab2 = tab + (size_t)p.T * kRow * 4;
+#pragma unroll
+                    for (int s = 0; s < kSlots; s++) {
+                        const uint32_t ra = (wa[s / 4] >> (8 * (s % 4))) & mask, rb = (wb[s / 4] >> (8 * (s % 4))) & mask;
+                        const float4 a = *reinterpret_cast<const float4 *>(tab + ra * (kRow * 4));
+                        const float4 b = *reinterpret_cast<const float4 *>(tab2 + rb * (kRow * 4));
+                        acc[s][0] = __fadd2_rn(acc[s][0], __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y)));
+                        acc[s][1] = __fadd2_rn(acc[s][1], __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w)));
+                    }
+                } else {
+#pragma unroll
+                    for (int s = 0; s < kSlots; s++) {
+                        const uint32_t ra = (wa[s / 4] >> (8 * (s % 4))) & mask;
+                        const float4 a = *reinterpret_cast<const float4 *>(tab + ra * (kRow * 4));
+                        acc[s][0] = __fadd2_rn(acc[s][0], make_float2(a.x, a.y));
+                        acc[s][1] = __fadd2_rn(acc[s][1], make_float2(a.z, a.w));
+                    }
+                }
+                __syncwarp();
+                if ((tid & 31) == 0) mbar_arrive(empty0 + 8 * slot);
+                if (++slot == kStages) { slot = 0; phase ^= 1u; }
+            }
+            if (ok && l * 4 < width) {
+                float *out = p.out + (size_t)db * p.batch * p.O + c0 + l * 4;
+#pragma unroll
+                for (int s = 0; s < kSlots; s++) {
+                    const int64_t b = b0 + g * kSlots + s;
+                    if (b < p.batch)
+                        *reinterpret_cast<float4 *>(out + (size_t)b * p.O) = make_float4(acc[s][0].x, acc[s][0].y, acc[s][1].x, acc[s][1].y);
+                }
+            }
+        }
+    }
+    if (!ok) leave_late(gave_up);
 }
 
 // y[i] += sum over the detector blocks, in double
@@ -150,6 +196,9 @@ __global__ void __launch_bounds__(256) add_partials_kernel(const float *__restri
 // block gives the same double as fp64 multiply-adds (the fp64 unit takes a sixteenth of a warp a cycle: a conversion and a
 // multiply-add per entry bound the kernel).  Blocks whose scales spread over more than 2^7, or are not finite, take the
 // fp64 route; its sums use the same registers.
+// Two detectors' entries are taken at a time (dp2a: two products of a 16-bit and an 8-bit number), which is 10 instructions for four
+// columns of both against 24 with a sign extension and a multiply-add for each; with that, no spilled registers and whole sectors in the
+// final additions: 4096 samples, 4096 detectors x 64 outputs 328 -> 203 us.
 // 8 lanes x 8 columns per row (rows of 64 bytes; wider rows in column slices), four samples per lane group.  A work item is
 // (run of whole truncation blocks, tile, column slice); its int32 sums are added to the result with integer reductions.
 // --------------------------------------------------------------------------------------------
@@ -206,27 +255,33 @@ struct StagedInt8 {
     double fixed_scale;
 };
 
-// sign-extended byte k of x
-template <int K>
-__device__ __forceinline__ int signed_byte(uint32_t x) {
-    int r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(x), "n"(((8 + K) << 12) | ((8 + K) << 8) | ((8 + K) << 4) | K));
-    return r;
-}
+// c plus the products of a's two 16-bit halves with bytes 0 and 1 (lo) or 2 and 3 (hi) of b, b's bytes signed; a's halves signed
+// (h) or unsigned (l)
+__device__ __forceinline__ int dot_h_lo(uint32_t a, uint32_t b, int c) { asm("dp2a.lo.s32.s32 %0, %1, %2, %0;" : "+r"(c) : "r"(a), "r"(b)); return c; }
+__device__ __forceinline__ int dot_h_hi(uint32_t a, uint32_t b, int c) { asm("dp2a.hi.s32.s32 %0, %1, %2, %0;" : "+r"(c) : "r"(a), "r"(b)); return c; }
+__device__ __forceinline__ int dot_l_lo(uint32_t a, uint32_t b, int c) { asm("dp2a.lo.u32.s32 %0, %1, %2, %0;" : "+r"(c) : "r"(a), "r"(b)); return c; }
+__device__ __forceinline__ int dot_l_hi(uint32_t a, uint32_t b, int c) { asm("dp2a.hi.u32.s32 %0, %1, %2, %0;" : "+r"(c) : "r"(a), "r"(b)); return c; }
 
+// FP64: the items with a truncation block whose scales do not share an exponent range, which the other instantiation leaves
+// (together they spilled registers); each passes over the other's items.
+// (The fp32 kernel's ring of bulk copies was slower here, 234 us against 203: its registers are the scarce ones.)
+template <bool FP64>
 __global__ void __launch_bounds__(kStagedThreads, 1) infer_staged_int8_kernel(const StagedInt8 p) {
-    extern __shared__ __align__(16) unsigned char sbuf[];
+    extern __shared__ __align__(128) unsigned char sbuf[];
     const int stage_bytes = kDets8 * p.T * kCols8;
     unsigned char *ring = sbuf;                                     // [kStages][kDets8][T][kCols8]
     uint8_t *ibuf = sbuf + (size_t)kStages * stage_bytes;           // [kStages][kDets8][kTile8]
     int2 *mbuf = reinterpret_cast<int2 *>(ibuf + kStages * kDets8 * kTile8);   // [kStages][kDets8] integer scales
     const int tid = threadIdx.x, g = tid / kLanes, l = tid % kLanes;
-    const uint32_t mask = (uint32_t)p.T - 1u;   // (samples past the batch hold any byte)
+    const uint32_t mask = (uint32_t)p.T - 1u, mask4 = mask * 0x01010101u;   // (samples past the batch hold any byte)
     for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
         const int per = p.n_tiles * p.n_slices;
         const int db = item / per, ts = item - db * per;
         const int tile = ts / p.n_slices, slice = ts - tile * p.n_slices;
         const int t0 = db * p.dets_per_item, nd = min(p.dets_per_item, p.Nt - t0), np = (nd + kDets8 - 1) / kDets8;
+        bool spread = false;
+        for (int k = t0 / p.det_block; k * p.det_block < t0 + nd; k++) spread |= __ldg(p.plan.unit + k) == 0.0;
+        if (spread != FP64) continue;
         const int64_t b0 = (int64_t)tile * kTile8;
         const int c0 = slice * kCols8, width = min(kCols8, p.O - c0);
         auto load_stage = [&](int pr) {
@@ -270,21 +325,46 @@ __global__ void __launch_bounds__(kStagedThreads, 1) infer_staged_int8_kernel(co
             __syncthreads();
             load_stage(pr + 2);
             const int slot = pr % kStages;
-            for (int d = 0; d < min(kDets8, nd - kDets8 * pr); d++) {
-                const int t = t0 + kDets8 * pr + d;
-                const unsigned char *tab = ring + (size_t)slot * stage_bytes + (size_t)d * p.T * kCols8 + l * 8;
-                const uint32_t rows = *reinterpret_cast<const uint32_t *>(ibuf + (size_t)slot * kDets8 * kTile8 + d * kTile8 + g * kSlots8);
-                if (unit != 0.0) {
-                    const int2 m = mbuf[slot * kDets8 + d];
+            const int here = min(kDets8, nd - kDets8 * pr);
+            const unsigned char *stage_tab = ring + (size_t)slot * stage_bytes + l * 8;
+            const uint8_t *stage_ib = ibuf + (size_t)slot * kDets8 * kTile8 + g * kSlots8;
+            // Four columns of two detectors' rows at a time.  (masked: samples past the batch hold any byte)
+            auto add_pair = [&](const unsigned char *tab, const unsigned char *tab2, uint32_t rows, uint32_t rows2, int2 m, int2 m2) {
+                const uint32_t mh = __byte_perm((uint32_t)m.x, (uint32_t)m2.x, 0x5410), ml = __byte_perm((uint32_t)m.y, (uint32_t)m2.y, 0x5410);
+                rows &= mask4;
+                rows2 &= mask4;
 #pragma unroll
-                    for (int k = 0; k < kSlots8; k++) {
-                        const uint2 w = *reinterpret_cast<const uint2 *>(tab + ((rows >> (8 * k)) & mask) * kCols8);
-                        const int q[8] = {signed_byte<0>(w.x), signed_byte<1>(w.x), signed_byte<2>(w.x), signed_byte<3>(w.x),
-                                          signed_byte<0>(w.y), signed_byte<1>(w.y), signed_byte<2>(w.y), signed_byte<3>(w.y)};
+                for (int k = 0; k < kSlots8; k++) {
+                    const uint2 u = *reinterpret_cast<const uint2 *>(tab + __byte_perm(rows, 0u, 0x4440 | k) * kCols8);
+                    const uint2 v = *reinterpret_cast<const uint2 *>(tab2 + __byte_perm(rows2, 0u, 0x4440 | k) * kCols8);
+                    // (entry e of the first, entry e of the second) in neighbouring bytes
+                    const uint32_t q[4] = {__byte_perm(u.x, v.x, 0x5140), __byte_perm(u.x, v.x, 0x7362), __byte_perm(u.y, v.y, 0x5140),
+                                           __byte_perm(u.y, v.y, 0x7362)};
 #pragma unroll
-                        for (int e = 0; e < 8; e++) { h[k][e] += m.x * q[e]; lw[k][e] += m.y * q[e]; }
+                    for (int e = 0; e < 4; e++) {
+                        h[k][2 * e] = dot_h_lo(mh, q[e], h[k][2 * e]);
+                        h[k][2 * e + 1] = dot_h_hi(mh, q[e], h[k][2 * e + 1]);
+                        lw[k][2 * e] = dot_l_lo(ml, q[e], lw[k][2 * e]);
+                        lw[k][2 * e + 1] = dot_l_hi(ml, q[e], lw[k][2 * e + 1]);
                     }
-                } else {
+                }
+            };
+            for (int d = 0, step; d < here; d += step) {
+                const int t = t0 + kDets8 * pr + d;
+                const unsigned char *tab = stage_tab + (size_t)d * p.T * kCols8;
+                const uint8_t *ib = stage_ib + d * kTile8;
+                const uint32_t rows = *reinterpret_cast<const uint32_t *>(ib);
+                if (!FP64 || unit != 0.0) {
+                    const int2 *ms = mbuf + slot * kDets8 + d;
+                    if (d + 1 < here && left > 1) {
+                        step = 2;
+                        add_pair(tab, tab + (size_t)p.T * kCols8, rows, *reinterpret_cast<const uint32_t *>(ib + kTile8), ms[0], ms[1]);
+                    } else {   // (the second with a scale of zero)
+                        step = 1;
+                        add_pair(tab, tab, rows, rows, ms[0], make_int2(0, 0));
+                    }
+                } else if constexpr (FP64) {
+                    step = 1;
                     const double sd = (double)__ldg(p.scales + t);
 #pragma unroll
                     for (int k = 0; k < kSlots8; k++) {
@@ -298,29 +378,43 @@ __global__ void __launch_bounds__(kStagedThreads, 1) infer_staged_int8_kernel(co
                         }
                     }
                 }
-                if (--left == 0 || t + 1 == t0 + nd) {
+                left -= step;
+                if (left == 0 || t + step == t0 + nd) {
 #pragma unroll
                     for (int k = 0; k < kSlots8; k++)
 #pragma unroll
                         for (int e = 0; e < 8; e++) {
-                            const double v = unit != 0.0 ? (double)((long long)h[k][e] * 65536ll + (long long)lw[k][e]) * unit
+                            const double v = !FP64 || unit != 0.0 ? (double)((long long)h[k][e] * 65536ll + (long long)lw[k][e]) * unit
                                                          : __hiloint2double(h[k][e], lw[k][e]);
                             iacc[k][e] += to_fixed(v, p.fixed_scale);
                             h[k][e] = lw[k][e] = 0;
                         }
                     left = p.det_block;
-                    if (t + 1 < t0 + nd) unit = __ldg(p.plan.unit + ++blk);
+                    if (t + step < t0 + nd) unit = __ldg(p.plan.unit + ++blk);
                 }
             }
         }
-        if (l * 8 < width) {
+        // A lane has eight neighbouring columns of four samples: the eight lanes of a group change places (three halving steps) so
+        // that they add to neighbouring columns, whole sectors, at a time.  (One column in eight a time took eight times the requests
+        // to L2, 16 M additions for 4096 samples.)
 #pragma unroll
-            for (int k = 0; k < kSlots8; k++) {
-                const int64_t b = b0 + g * kSlots8 + k;
-                if (b >= p.batch) continue;
-                int32_t *dst = p.acc + (size_t)b * p.O + c0 + l * 8;
+        for (int k = 0; k < kSlots8; k++) {
 #pragma unroll
-                for (int e = 0; e < 8; e++) atomicAdd(dst + e, iacc[k][e]);
+            for (int o = 4; o >= 1; o >>= 1)
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    if ((e & o) == 0) {
+                        const bool upper = (l & o) != 0;
+                        const int other = __shfl_xor_sync(0xffffffffu, upper ? iacc[k][e] : iacc[k][e + o], o);
+                        if (upper) iacc[k][e] = other;
+                        else iacc[k][e + o] = other;
+                    }
+            const int64_t b = b0 + g * kSlots8 + k;
+            if (b < p.batch) {
+                int32_t *dst = p.acc + (size_t)b * p.O + c0;
+#pragma unroll
+                for (int e = 0; e < 8; e++)   // (entry e is now column 8 e + l)
+                    if (8 * e + l < width) atomicAdd(dst + 8 * e + l, iacc[k][e]);
             }
         }
         async_wait<0>();
@@ -380,7 +474,7 @@ int64_t infer_staged_pass(const lutb_layer_cfg *cfg, int64_t batch, bool int8) {
 }
 size_t packed_index_bytes(const lutb_layer_cfg *cfg, int64_t pass) { return align256(packed_index_pitch(pass) * cfg->n_detectors); }
 
-static size_t smem_fp32(int T) { return (size_t)kStages * 2 * ((size_t)T * kRow * 4 + kTile); }
+static size_t smem_fp32(int T) { return (size_t)kStages * 2 * ((size_t)T * kRow * 4 + kTile) + 16 * kStages + 16; }
 static size_t smem_int8(int T) { return (size_t)kStages * kDets8 * ((size_t)T * kCols8 + kTile8 + 8); }
 
 bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *weights, const void *y) {
@@ -395,13 +489,15 @@ bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, int64_t batch, const v
     return cfg->n_detectors >= kMinDetectorsInt8 && staged_int8_pays(batch, cfg->n_outputs);
 }
 
+size_t anchor_plan_bytes(const lutb_layer_cfg *cfg) { return align256((size_t)cfg->n_detectors * 8 * sizeof(uint32_t)); }
+
 size_t infer_staged_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
     const int64_t pass = infer_staged_pass(cfg, batch, false);
-    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256((size_t)(pass * partial_bytes(cfg, false))) + 256;
+    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256((size_t)(pass * partial_bytes(cfg, false))) + 256 + anchor_plan_bytes(cfg);
 }
 size_t infer_staged_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch) {
     const int64_t pass = infer_staged_pass(cfg, batch, true);
-    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256(scale_plan_bytes(cfg->n_detectors, trunc_blocks(cfg))) + 256;
+    return pass == 0 ? 0 : packed_index_bytes(cfg, pass) + align256(scale_plan_bytes(cfg->n_detectors, trunc_blocks(cfg))) + 256 + anchor_plan_bytes(cfg);
 }
 
 int launch_infer_staged_fp32(const lutb_layer_cfg *cfg, int64_t batch, const float *weights, const uint8_t *packed, float *partial,
@@ -418,10 +514,13 @@ int launch_infer_staged_fp32(const lutb_layer_cfg *cfg, int64_t batch, const flo
     p.n_items = (int)items;
     const size_t smem = smem_fp32(T);
     const int blocks = p.n_items < device_info().sm_count ? p.n_items : device_info().sm_count;
+    CUtensorMap tables;
+    const int rc = tensor_map_2d(&tables, 4, weights, (int64_t)p.Nt * T, O, (int64_t)O * 4, T, kRow, 0);
+    if (rc) return rc;
     LUTB_CUDA(cudaFuncSetAttribute(infer_staged_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     {
         KernelScope scope(K_FC_GATHER_FORWARD, stream);
-        infer_staged_fp32_kernel<<<(unsigned)blocks, kStagedThreads, smem, stream>>>(p);
+        infer_staged_fp32_kernel<<<(unsigned)blocks, kStagedThreads + 32, smem, stream>>>(tables, p);
         LUTB_LAUNCH_CHECK();
     }
     const int64_t n4 = batch * O / 4;
@@ -464,10 +563,12 @@ int launch_infer_staged_int8(const lutb_layer_cfg *cfg, int64_t batch, const int
     p.n_items = (int)items;
     const size_t smem = smem_int8(p.T);
     const int blocks = p.n_items < device_info().sm_count ? p.n_items : device_info().sm_count;
-    LUTB_CUDA(cudaFuncSetAttribute(infer_staged_int8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    KernelScope scope(K_INT8_GATHER, stream);
-    infer_staged_int8_kernel<<<(unsigned)blocks, kStagedThreads, smem, stream>>>(p);
-    LUTB_LAUNCH_CHECK();
+    for (auto kern : {infer_staged_int8_kernel<false>, infer_staged_int8_kernel<true>}) {
+        LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KernelScope scope(K_INT8_GATHER, stream);
+        kern<<<(unsigned)blocks, kStagedThreads, smem, stream>>>(p);
+        LUTB_LAUNCH_CHECK();
+    }
     return LUTB_OK;
 }
 

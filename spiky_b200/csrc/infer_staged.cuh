@@ -13,9 +13,11 @@ bool infer_staged_fp32_applies(const lutb_layer_cfg *cfg, int64_t batch, const v
 bool infer_staged_int8_applies(const lutb_layer_cfg *cfg, int64_t batch, const void *q_tables);
 
 // Samples of one pass (0: the staged gather does not run) and the workspace of a call: packed indices of a pass first
-// (packed_index_bytes), then the partial sums of the detector blocks (fp32) or the integer form of the scales (int8).
+// (packed_index_bytes), then the partial sums of the detector blocks (fp32) or the integer form of the scales (int8), last the
+// ordered anchors of the comparison (anchor_plan_bytes).
 int64_t infer_staged_pass(const lutb_layer_cfg *cfg, int64_t batch, bool int8);
 size_t packed_index_bytes(const lutb_layer_cfg *cfg, int64_t pass);
+size_t anchor_plan_bytes(const lutb_layer_cfg *cfg);
 size_t infer_staged_fp32_workspace(const lutb_layer_cfg *cfg, int64_t batch);
 size_t infer_staged_int8_workspace(const lutb_layer_cfg *cfg, int64_t batch);
 

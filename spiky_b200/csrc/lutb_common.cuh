@@ -138,6 +138,8 @@ __device__ __forceinline__ int32_t to_fixed(double v, double scale) {
 int peer_wait_errors(int *count_out);
 // The same of the contraction kernels (hist_gemm_sm100.cu).
 int contract_wait_errors(int *count_out);
+// The same of the staged inference kernel (infer_staged.cu).
+int staged_wait_errors(int *count_out);
 
 // In-place conversion of int32 fixed-point accumulators to fp32
 // (reference: convert_integers_to_floats_logic, proto:200-213).
