@@ -1,10 +1,10 @@
 // Contractions of the histogram path on the sm_100a tensor cores: fp32 results from fp16 operands.
 //
 // Row counts are small integers (below 2049), exact in fp16.  An fp32 operand x (a table, an output gradient) is scaled
-// by a power of two that brings the largest element of its row - or column - to [2^14, 2^15), and kept as two fp16
-// values: hi = x * s rounded, lo = (x * s - hi) * 2^11 rounded.  x * s = hi + lo * 2^-11 to 2^-22 of x, as with the two
+// by a power of two that brings the largest element of its row - or of its column within 1024 rows - to [2^14, 2^15), and kept as
+// two fp16 values: hi = x * s rounded, lo = (x * s - hi) * 2^11 rounded.  x * s = hi + lo * 2^-11 to 2^-22 of x, as with the two
 // 11-bit halves of a TF32 split, for elements down to 2^-29 of the largest, and to 2^-51 of the largest below that.  The scale
-// always belongs to a free index of the contraction, so it comes out of the sum as a factor of the result.
+// belongs to a free index of the contraction (and to a slice of the contraction, see below), so it comes out of the sum as a factor.
 // The products hi.hi go into one accumulator in tensor memory, hi.lo and lo.hi into another (their sum counts 2^-11 times),
 // lo.lo (below 2^-22) is dropped; kind::f16 runs at twice the rate of kind::tf32.
 //
@@ -19,7 +19,8 @@
 // their epilogues ran under the next tile's MMAs.  Here both accumulators (2 x 256 columns) are all of tensor memory: the MMAs
 // wait while they are read into registers, not for the rest of the epilogue.
 // The tensor core truncates its fp32 accumulator after each step, an error that grows with the length of the chain: after
-// kSliceBlocks * 64 elements the epilogue takes the sum over into registers (rounded fp32 additions) and the MMAs start afresh.
+// kSliceBlocks * 64 elements the epilogue takes the sum over into registers (rounded fp32 additions, where a column has a scale per
+// slice with its factor) and the MMAs start afresh.
 // Few tiles and a long contraction (the forward pass of few tokens): work items are (part of the contraction, tile), each
 // part's result goes to scratch and a second kernel adds the parts in order.
 //
@@ -61,7 +62,8 @@ struct ContractArgs {
     int m_fast;                   // tiles of neighbouring work items differ in m (else in n)
     int m_padded;                 // rows of one part's result in scratch (splits > 1)
     int accumulate;               // add to what is there
-    const uint32_t *row_bits, *col_bits;   // bits of the largest magnitude of each row of A / column of the result, or null
+    // bits of the largest magnitude of each row of A (or null) and of each column of the result: [N], or, A exact, [slice][N]
+    const uint32_t *row_bits, *col_bits;
     float alpha;
 };
 
@@ -128,46 +130,56 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
     }
 }
 
-// Largest magnitude of every column (bits cleared before): 4 columns a thread, 64 threads by 16 rows a block, one block an SM so
-// that few of them meet in the atomics (16384 x 256: 6.9 us; 9.7 with 444 blocks of 256 threads, 33 with 1024).
-constexpr int kMaxRows = 16;
-__global__ void __launch_bounds__(64 * kMaxRows) column_max_kernel(const float *__restrict__ x, int64_t rows, int cols, uint32_t *__restrict__ bits) {
-    __shared__ uint4 part[kMaxRows][64];
-    const int tx = threadIdx.x & 63, c4 = blockIdx.x * 64 + tx, ty = threadIdx.x >> 6;
+// Scaled by column and slice of kSliceRows rows: a block takes 32 columns of a slice, which stay in its registers between the
+// maximum and the copy, so that the matrix is read once (a pass for the maxima of whole columns took 41 of the 123 us for 65536 x
+// 1024, and 7 + 5 us for 16384 x 256).  bits: [slice][cols].
+constexpr int kSliceRows = kSliceBlocks * kBlockK, kCopyRows = 128;
+__global__ void __launch_bounds__(8 * kCopyRows) split_columns_kernel(const float *__restrict__ x, int64_t rows, int cols, __half *__restrict__ hi,
+                                                                      __half *__restrict__ lo, int pitch, uint32_t *__restrict__ bits) {
+    __shared__ uint32_t part[kCopyRows / 4][32];
+    constexpr int KEEP = kSliceRows / kCopyRows;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, c4 = blockIdx.y * 8 + tx;
     const bool live = c4 < (cols >> 2);
+    const int64_t r0 = (int64_t)blockIdx.x * kSliceRows;
+    float4 v[KEEP];
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (live) {
-#pragma unroll 8
-        for (int64_t r = (int64_t)blockIdx.y * kMaxRows + ty; r < rows; r += (int64_t)gridDim.y * kMaxRows) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(x + r * cols) + c4);
-            m.x = max(m.x, __float_as_uint(v.x) & 0x7fffffffu);
-            m.y = max(m.y, __float_as_uint(v.y) & 0x7fffffffu);
-            m.z = max(m.z, __float_as_uint(v.z) & 0x7fffffffu);
-            m.w = max(m.w, __float_as_uint(v.w) & 0x7fffffffu);
-        }
+#pragma unroll
+    for (int k = 0; k < KEEP; k++) {
+        const int64_t r = r0 + k * kCopyRows + ty;
+        v[k] = live && r < rows ? __ldg(reinterpret_cast<const float4 *>(x + r * cols) + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    part[ty][tx] = m;
+#pragma unroll
+    for (int k = 0; k < KEEP; k++) {
+        m.x = max(m.x, __float_as_uint(v[k].x) & 0x7fffffffu);
+        m.y = max(m.y, __float_as_uint(v[k].y) & 0x7fffffffu);
+        m.z = max(m.z, __float_as_uint(v[k].z) & 0x7fffffffu);
+        m.w = max(m.w, __float_as_uint(v[k].w) & 0x7fffffffu);
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {   // a warp has four rows of the eight column quadruples
+        m.x = max(m.x, __shfl_xor_sync(0xffffffffu, m.x, o));
+        m.y = max(m.y, __shfl_xor_sync(0xffffffffu, m.y, o));
+        m.z = max(m.z, __shfl_xor_sync(0xffffffffu, m.z, o));
+        m.w = max(m.w, __shfl_xor_sync(0xffffffffu, m.w, o));
+    }
+    if ((threadIdx.x & 31) < 8) *reinterpret_cast<uint4 *>(&part[threadIdx.x >> 5][4 * tx]) = m;
     __syncthreads();
-    // a thread per column
-    const int col = blockIdx.x * 256 + threadIdx.x;
-    if (threadIdx.x < 256 && col < cols) {
+    if (threadIdx.x < 32) {
         uint32_t most = 0u;
 #pragma unroll
-        for (int k = 0; k < kMaxRows; k++) most = max(most, reinterpret_cast<const uint32_t *>(part[k])[threadIdx.x]);
-        if (most > __ldcg(bits + col)) atomicMax(bits + col, most);   // (later blocks mostly find a larger one there)
+        for (int k = 0; k < kCopyRows / 4; k++) most = max(most, part[k][threadIdx.x]);
+        part[0][threadIdx.x] = most;
+        if (blockIdx.y * 32 + threadIdx.x < cols) bits[(int64_t)blockIdx.x * cols + blockIdx.y * 32 + threadIdx.x] = most;
     }
-}
-
-// Scaled by column.
-__global__ void __launch_bounds__(256) split_columns_kernel(const float *__restrict__ x, int64_t rows, int cols, __half *__restrict__ hi,
-                                                            __half *__restrict__ lo, int pitch, const uint32_t *__restrict__ bits) {
-    const int c4 = blockIdx.x * 64 + (threadIdx.x & 63), ty = threadIdx.x >> 6;
-    if (c4 >= (cols >> 2)) return;
-    const uint4 b = *(reinterpret_cast<const uint4 *>(bits) + c4);
+    __syncthreads();
+    if (!live) return;
+    const uint4 b = *reinterpret_cast<const uint4 *>(&part[0][4 * tx]);
     const float sx = scale_of(b.x), sy = scale_of(b.y), sz = scale_of(b.z), sw = scale_of(b.w);
-#pragma unroll 4
-    for (int64_t r = (int64_t)blockIdx.y * 4 + ty; r < rows; r += (int64_t)gridDim.y * 4) {
-        const Halves q = split4(__ldg(reinterpret_cast<const float4 *>(x + r * cols) + c4), sx, sy, sz, sw);
+#pragma unroll
+    for (int k = 0; k < KEEP; k++) {
+        const int64_t r = r0 + k * kCopyRows + ty;
+        if (r >= rows) break;
+        const Halves q = split4(v[k], sx, sy, sz, sw);
         *(reinterpret_cast<uint2 *>(hi + r * pitch) + c4) = q.hi;
         *(reinterpret_cast<uint2 *>(lo + r * pitch) + c4) = q.lo;
     }
@@ -175,18 +187,19 @@ __global__ void __launch_bounds__(256) split_columns_kernel(const float *__restr
 
 // C += alpha * sum of the parts, in order and in double (up to 32 parts: fp32 additions were most of the result's error).
 constexpr int kAddThreads = 64;
+template <int AHEAD>   // parts whose loads are in flight (they are one latency each otherwise)
 __global__ void __launch_bounds__(kAddThreads) add_parts_kernel(const float *__restrict__ P, float *__restrict__ C, int64_t M, int N, int parts,
                                                         int64_t part_stride, float alpha) {
     const int64_t n4 = M * (N / 4);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         double s[4] = {0., 0., 0., 0.};
-        for (int k0 = 0; k0 < parts; k0 += 16) {
-            float4 t[16];   // (all loads in flight: they are one latency each otherwise)
+        for (int k0 = 0; k0 < parts; k0 += AHEAD) {
+            float4 t[AHEAD];
 #pragma unroll
-            for (int k = 0; k < 16; k++)
+            for (int k = 0; k < AHEAD; k++)
                 t[k] = k0 + k < parts ? __ldcs(reinterpret_cast<const float4 *>(P + (k0 + k) * part_stride) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < 16; k++) { s[0] += t[k].x; s[1] += t[k].y; s[2] += t[k].z; s[3] += t[k].w; }
+            for (int k = 0; k < AHEAD; k++) { s[0] += t[k].x; s[1] += t[k].y; s[2] += t[k].z; s[3] += t[k].w; }
         }
         float4 *dst = reinterpret_cast<float4 *>(C) + i;
         float4 o = *dst;
@@ -391,8 +404,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (kEpilogueWarps
         uint32_t phase = 0u, acc_phase = 1u;
         for (int i = cluster; i < items && ok; i += clusters) {
             const Item it = item_of(g, i);
-            for (int kb0 = it.kb0; kb0 < it.kb1 && ok; kb0 += kSliceBlocks) {
-                const int kb1 = min(it.kb1, kb0 + kSliceBlocks);
+            for (int kb0 = it.kb0, kb1; kb0 < it.kb1 && ok; kb0 = kb1) {
+                kb1 = min(it.kb1, (kb0 / kSliceBlocks + 1) * kSliceBlocks);
                 ok = wait_cluster(free0, acc_phase) && *gave_up == 0u;
                 if (!ok) break;
                 fence_after();
@@ -428,17 +441,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (kEpilogueWarps
         for (int i = cluster; i < items && ok; i += clusters) {
             const Item it = item_of(g, i);
             const int n0 = it.n_tile * kTileN + cols0, row0 = it.m_tile * kTileM + (int)rank * 128 + quarter * 32;
-            float factor[kWarpCols / 32];   // of columns c * 32 + lane
+            // factors of columns c * 32 + lane (of the slice, where a column has one for each)
+            float factor[kWarpCols / 32];
+            auto load_factors = [&](const uint32_t *bits) {
 #pragma unroll
-            for (int c = 0; c < kWarpCols / 32; c++) {
-                const int n = n0 + c * 32 + lane;
-                factor[c] = g.col_bits != nullptr && n < g.N ? inverse_scale(__ldg(g.col_bits + n)) : 1.f;
-            }
-            const float row_factor = g.row_bits != nullptr && row0 + lane < g.M ? inverse_scale(__ldg(g.row_bits + row0 + lane)) : 1.f;
+                for (int c = 0; c < kWarpCols / 32; c++) {
+                    const int n = n0 + c * 32 + lane;
+                    factor[c] = n < g.N ? inverse_scale(__ldg(bits + n)) : 1.f;
+                }
+            };
+            if (A_PARTS == 2) load_factors(g.col_bits);
+            const float row_factor = A_PARTS == 2 && row0 + lane < g.M ? inverse_scale(__ldg(g.row_bits + row0 + lane)) : 1.f;
             float sum[kWarpCols];
 #pragma unroll
             for (int n = 0; n < kWarpCols; n++) sum[n] = 0.f;
-            for (int kb0 = it.kb0; kb0 < it.kb1; kb0 += kSliceBlocks) {
+            for (int kb0 = it.kb0; kb0 < it.kb1; kb0 = (kb0 / kSliceBlocks + 1) * kSliceBlocks) {
+                if (A_PARTS == 1) {
+                    // through this warp's piece of shared memory, from which every lane reads four at a time (the last tile's
+                    // stores have left it)
+                    load_factors(g.col_bits + (int64_t)(kb0 / kSliceBlocks) * g.N);
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < kWarpCols / 32; c++) out_ptr[c * 32 + lane] = factor[c];
+                    __syncwarp();
+                }
                 ok = __all_sync(0xffffffffu, wait_cluster(done0, acc_phase) && *gave_up == 0u);
                 if (!ok) break;
                 fence_after();
@@ -453,7 +480,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (kEpilogueWarps
                     loaded(big);
                     loaded(small);
 #pragma unroll
-                    for (int n = 0; n < 16; n++) sum[c * 16 + n] += fmaf(__uint_as_float(small[n]), kLoScale, __uint_as_float(big[n]));
+                    for (int n4 = 0; n4 < 4; n4++) {
+                        const float4 f4 = A_PARTS == 1 ? *reinterpret_cast<const float4 *>(out_ptr + c * 16 + n4 * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+                        const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int n = n4 * 4 + e;
+                            const float v = fmaf(__uint_as_float(small[n]), kLoScale, __uint_as_float(big[n]));
+                            sum[c * 16 + n] = A_PARTS == 1 ? fmaf(v, f[e], sum[c * 16 + n]) : sum[c * 16 + n] + v;
+                        }
+                    }
                 }
                 fence_before();
                 __syncwarp();
@@ -461,17 +497,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * (kEpilogueWarps
             }
             if (!ok) break;
             // both factors within 2^+-60: any order will do; else the smaller one first, no overflow on the way to a finite result
-            bool near = fabsf(__log2f(row_factor)) < 60.f;
+            bool near = true;
+            if (A_PARTS == 2) {
+                near = fabsf(__log2f(row_factor)) < 60.f;
 #pragma unroll
-            for (int c = 0; c < kWarpCols / 32; c++) near = near && fabsf(__log2f(factor[c])) < 60.f;
-            near = __all_sync(0xffffffffu, near);
+                for (int c = 0; c < kWarpCols / 32; c++) near = near && fabsf(__log2f(factor[c])) < 60.f;
+                near = __all_sync(0xffffffffu, near);
+            } else {
+                __syncwarp();   // (the piece held the factors)
+            }
 #pragma unroll
             for (int c = 0; c < kWarpCols / 16; c++) {
                 float o[16];
 #pragma unroll
                 for (int n = 0; n < 16; n++) {
-                    const float f = __shfl_sync(0xffffffffu, factor[c / 2], (c & 1) * 16 + n);
                     o[n] = sum[c * 16 + n];
+                    if (A_PARTS == 1) {
+                        o[n] *= g.alpha;
+                        continue;
+                    }
+                    const float f = __shfl_sync(0xffffffffu, factor[c / 2], (c & 1) * 16 + n);
                     if (near) o[n] = g.alpha * (o[n] * row_factor * f);
                     else o[n] = g.alpha * (o[n] * fminf(row_factor, f) * fmaxf(row_factor, f));
                 }
@@ -558,15 +603,12 @@ int copy_by_row(const float *x, int64_t rows, int cols, const Copy &c, cudaStrea
     return LUTB_OK;
 }
 
+int64_t slices_of(int64_t rows) { return (rows + kSliceRows - 1) / kSliceRows; }
+
 int copy_by_column(const float *x, int64_t rows, int cols, const Copy &c, cudaStream_t stream) {
-    const int gx = (cols / 4 + 63) / 64;
-    const int64_t sm = device_info().sm_count;
-    const int64_t want = (rows + 15) / 16, cap = (sm * 8 + gx - 1) / gx, cap_max = ((rows > 65536 ? 2 * sm : sm) + gx - 1) / gx;
-    const dim3 grid((unsigned)gx, (unsigned)(want < cap ? want : cap)), grid_max((unsigned)gx, (unsigned)(want < cap_max ? want : cap_max));
-    LUTB_CUDA(cudaMemsetAsync(c.bits, 0, (size_t)cols * 4, stream));
-    column_max_kernel<<<grid_max, 64 * kMaxRows, 0, stream>>>(x, rows, cols, c.bits);
-    LUTB_LAUNCH_CHECK();
-    split_columns_kernel<<<grid, 256, 0, stream>>>(x, rows, cols, c.hi, c.lo, c.pitch, c.bits);
+    LUTB_REQUIRE((cols + 31) / 32 <= 65535, LUTB_ERR_SHAPE, "tensor-core contraction: too many columns");
+    const dim3 grid((unsigned)slices_of(rows), (unsigned)((cols + 31) / 32));
+    split_columns_kernel<<<grid, 8 * kCopyRows, 0, stream>>>(x, rows, cols, c.hi, c.lo, c.pitch, c.bits);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
 }
@@ -620,7 +662,8 @@ int launch_contraction(ContractArgs g, const CUtensorMap (&a)[2], const CUtensor
     LUTB_LAUNCH_CHECK();
     if (g.splits > 1) {
         const int64_t want = ((int64_t)g.M * (g.N / 4) + kAddThreads - 1) / kAddThreads, cap = (int64_t)device_info().sm_count * 16;
-        add_parts_kernel<<<(unsigned)(want < cap ? want : cap), kAddThreads, 0, stream>>>(parts, C, g.M, g.N, g.splits, (int64_t)g.m_padded * g.N, alpha);
+        auto add = g.splits > 4 ? add_parts_kernel<16> : g.splits > 2 ? add_parts_kernel<4> : add_parts_kernel<2>;
+        add<<<(unsigned)(want < cap ? want : cap), kAddThreads, 0, stream>>>(parts, C, g.M, g.N, g.splits, (int64_t)g.m_padded * g.N, alpha);
         LUTB_LAUNCH_CHECK();
     }
     return LUTB_OK;
@@ -634,8 +677,8 @@ int blocks_of(int k) { return (k + kBlockK - 1) / kBlockK; }
 }  // namespace
 
 size_t hist_gemm_workspace(HistGemmKind kind, int rows, int KT, int O) {
-    if (kind == HG_FORWARD) return copy_bytes(KT, O, O) + parts_bytes(rows, O, blocks_of(KT)) + 256;
-    if (kind == HG_TABLE_GRAD) return copy_bytes(rows, O, O) + parts_bytes(KT, O, blocks_of(rows)) + 256;
+    if (kind == HG_FORWARD) return copy_bytes(KT, O, slices_of(KT) * O) + parts_bytes(rows, O, blocks_of(KT)) + 256;
+    if (kind == HG_TABLE_GRAD) return copy_bytes(rows, O, slices_of(rows) * O) + parts_bytes(KT, O, blocks_of(rows)) + 256;
     return copy_bytes(rows, O, rows) + copy_bytes(KT, O, KT) + 256;
 }
 
@@ -647,7 +690,7 @@ int hist_gemm_forward(int rows, int KT, int O, const __half *H, const float *W, 
                       cudaStream_t stream) {
     LUTB_CONTRACT_WORKSPACE(HG_FORWARD);
     unsigned char *p = aligned_base(workspace);
-    const Copy w = take_copy(p, KT, O, O);
+    const Copy w = take_copy(p, KT, O, slices_of(KT) * O);
     float *parts = parts_bytes(rows, O, blocks_of(KT)) ? reinterpret_cast<float *>(p) : nullptr;
     int rc = copy_by_column(W, KT, O, w, stream);
     if (rc) return rc;
@@ -667,7 +710,7 @@ int hist_gemm_table_grad(int rows, int KT, int O, const __half *H, const float *
                          size_t workspace_bytes, cudaStream_t stream) {
     LUTB_CONTRACT_WORKSPACE(HG_TABLE_GRAD);
     unsigned char *p = aligned_base(workspace);
-    const Copy d = take_copy(p, rows, O, O);
+    const Copy d = take_copy(p, rows, O, slices_of(rows) * O);
     float *parts = parts_bytes(KT, O, blocks_of(rows)) ? reinterpret_cast<float *>(p) : nullptr;
     int rc = copy_by_column(dY, rows, O, d, stream);
     if (rc) return rc;
