@@ -6,6 +6,8 @@
 #include "fc_dw_sorted.cuh"
 #include "infer_staged.cuh"
 
+#include <type_traits>
+
 namespace lutb {
 
 // --------------------------------------------------------------------------------------------
@@ -521,7 +523,11 @@ __global__ void __launch_bounds__(256) fc_gather_forward_vec_kernel(const float 
     const int col = (blockIdx.y * LG + j) * 4;
     const bool active = col < n_outputs;
     const int32_t *idx_b = idx + b * n_detectors;
-    const float *Wc = W + col;
+    // addresses: this lane's columns of a table, tables NG apart, plus 32-bit row numbers times the row's bytes (a 64-bit product per
+    // row less: 65536 samples, 64 detectors of 64 rows x 32 outputs 46.8 -> 42.9 us; 8192 samples, 16 detectors, 256 outputs 17.3 -> 14.8)
+    const char *table = reinterpret_cast<const char *>(W + ((size_t)(t0 + g) * table_rows) * n_outputs + col);
+    const size_t group_bytes = (size_t)NG * table_rows * n_outputs * 4;
+    const uint32_t row_bytes = (uint32_t)n_outputs * 4u;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int tb = t0; tb < t1; tb += 32) {
         const int nvalid = min(32, t1 - tb);
@@ -534,9 +540,9 @@ __global__ void __launch_bounds__(256) fc_gather_forward_vec_kernel(const float 
             for (int i = 0; i < BATCH; i++) {
                 const int d = (i0 + i) * NG + g;
                 const int32_t li = __shfl_sync(0xffffffffu, mine, d);
-                w[i] = (active && d < nvalid)
-                           ? __ldg(reinterpret_cast<const float4 *>(Wc + ((size_t)(tb + d) * table_rows + li) * n_outputs))
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
+                w[i] = (active && d < nvalid) ? __ldg(reinterpret_cast<const float4 *>(table + (uint64_t)(uint32_t)li * row_bytes))
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                table += group_bytes;
             }
 #pragma unroll
             for (int i = 0; i < BATCH; i++) { part[0] += w[i].x; part[1] += w[i].y; part[2] += w[i].z; part[3] += w[i].w; }
@@ -706,14 +712,19 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
 // Bound: the latency of the row reads and load/store wavefronts (half of their peak at 65536 samples x 64 detectors of 64 rows x 32
 // outputs).  Measured (one detector a group in flight, a full reduction per detector before), with the clearing of dX:
 // 256 samples 10.9 -> 8.6 us; 1111 samples, 50 detectors, 33 outputs 32.0 -> 14.8 us; 512 samples, 64 detectors, 10 outputs
-// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.5 us; 65536 samples 187 -> 167 us.
+// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.5 us; 65536 samples 187 -> 167 us, and 117 as said at ONE below.
 // (Walking groups of detectors whose tables fit L1 measured 220 us there: the groups leave lanes idle.)
 // --------------------------------------------------------------------------------------------
 // WRITE: dX is written instead of added to (and need not be cleared): the warp sums its sample's row in shared memory and
 // writes it out once.
 // Blocks an SM: 8 lanes a group with vector loads need 80 registers for two detectors in flight (at 64 they spilled: 65536 samples,
 // 64 detectors of 64 rows x 32 outputs 187 -> 167 us, 5000 samples 23 -> 19).
-template <int LG, int VEC, bool WRITE>
+// ONE: rows of one step (n_outputs <= LG * VEC).  A lane then has one fp32 product sum per detector, which the first exchange
+// takes as it is; lanes without a column and detectors without an anchor to flip read the first column and one row twice (nobody
+// takes what comes out), so that the loads need no predicates and four detectors are in flight; addresses are row numbers times the
+// row's bytes.  65536 samples 167 -> 117 us, 256 samples 7.4 -> 5.2.  (The same for rows of several steps spilled registers and
+// gained nothing.)
+template <int LG, int VEC, bool WRITE, bool ONE>
 __global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                            const int2 *__restrict__ anchors,
                                                            const int32_t *__restrict__ idx,
@@ -721,12 +732,14 @@ __global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 
                                                            const int32_t *__restrict__ min_k, float *__restrict__ dX,
                                                            int64_t batch, int n_inputs, int n_outputs, int n_detectors,
                                                            int n_anchors, int table_rows, int group_dets, int block_samples) {
-    constexpr int NG = 32 / LG, CH = LG < 8 ? LG : 8, U = CH < (LG >= 16 ? 4 : 2) ? CH : (LG >= 16 ? 4 : 2);   // CH detectors a group at a time
+    constexpr int NG = 32 / LG, CH = LG < 8 ? LG : 8, UM = LG >= 16 || ONE ? 4 : 2, U = CH < UM ? CH : UM;   // CH detectors a group at a time
     const int lane = threadIdx.x & 31, g = lane / LG, j = lane - g * LG;
     const int my_s = j * NG + g;   // this lane's detector of every 32: iteration i of group g takes detector i * NG + g
     const int t_begin = blockIdx.y * group_dets, t_end = min(n_detectors, t_begin + group_dets);
     const int64_t b_end = min(batch, ((int64_t)blockIdx.x + 1) * block_samples);
     extern __shared__ __align__(16) float dx_rows[];
+    const uint32_t row_bytes = (uint32_t)n_outputs * 4u;
+    const size_t table_bytes = (size_t)table_rows * row_bytes;
     const int row_floats = (n_inputs + 3) & ~3;
     float *dx_s = dx_rows + (threadIdx.x >> 5) * row_floats;
     if (WRITE) {
@@ -753,14 +766,44 @@ __global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 
                 my_m = __ldg(min_delta + base + tb + my_s);
             }
             double dot = 0.0;
+            const int32_t own_row = my_k >= 0 ? my_idx : 0, own_alt = my_k >= 0 ? my_idx ^ (1 << my_k) : 0;
+            const bool in_row = j * VEC < n_outputs;
+            const char *tables = reinterpret_cast<const char *>(W + (size_t)tb * table_rows * n_outputs + (in_row ? j * VEC : 0));
 #pragma unroll 1
             for (int ch = 0; ch < LG && ch * NG < nvalid; ch += CH) {
-                double v[CH];
+                using Part = std::conditional_t<ONE, float, double>;
+                Part v[CH];
 #pragma unroll
                 for (int i0 = 0; i0 < CH; i0 += U) {
 #pragma unroll
-                    for (int u = 0; u < U; u++) v[i0 + u] = 0.0;
+                    for (int u = 0; u < U; u++) v[i0 + u] = 0;
                     if ((ch + i0) * NG >= nvalid) continue;   // warp uniform
+                    if constexpr (ONE) {
+                        const char *row[U], *alt[U];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const int i = ch + i0 + u, s = i * NG + g;
+                            const uint32_t li = (uint32_t)__shfl_sync(0xffffffffu, own_row, g * LG + i);
+                            const uint32_t la = (uint32_t)__shfl_sync(0xffffffffu, own_alt, g * LG + i);
+                            const char *tab = tables + (size_t)(uint32_t)(s < nvalid ? s : 0) * table_bytes;
+                            row[u] = tab + (uint64_t)li * row_bytes;
+                            alt[u] = tab + (uint64_t)la * row_bytes;
+                        }
+                        float a[U][VEC], c[U][VEC];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            Vec<VEC>::load(reinterpret_cast<const float *>(row[u]), a[u]);
+                            Vec<VEC>::load(reinterpret_cast<const float *>(alt[u]), c[u]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            float part = 0.f;
+#pragma unroll
+                            for (int e = 0; e < VEC; e++) part = fmaf(d0[e], a[u][e] - c[u][e], part);
+                            v[i0 + u] = in_row ? part : 0.f;
+                        }
+                        continue;
+                    }
                     const float *row[U], *alt[U];
                     bool on[U];
 #pragma unroll
@@ -803,19 +846,30 @@ __global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 
                     }
                 }
                 // lane j ends with the chunk's detector j % CH: halving steps over the detectors, then plain ones
+                double w[CH];
 #pragma unroll
-                for (int o = CH / 2; o >= 1; o >>= 1) {
-                    const bool upper = (j & o) != 0;
+                for (int i = 0; i < CH; i++) w[i] = (double)v[i];
+                if constexpr (ONE && CH > 1) {   // (the first step exchanges the fp32 sums as they are)
+                    const bool upper = (j & (CH / 2)) != 0;
 #pragma unroll
-                    for (int i = 0; i < o; i++) {
-                        const double send = upper ? v[i] : v[i + o];
-                        const double keep = upper ? v[i + o] : v[i];
-                        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    for (int i = 0; i < CH / 2; i++) {
+                        const Part send = upper ? v[i] : v[i + CH / 2], keep = upper ? v[i + CH / 2] : v[i];
+                        w[i] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, send, CH / 2);
                     }
                 }
 #pragma unroll
-                for (int o = CH; o < LG; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-                if (j / CH == ch / CH) dot = v[0];
+                for (int o = ONE ? CH / 4 : CH / 2; o >= 1; o >>= 1) {
+                    const bool upper = (j & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < o; i++) {
+                        const double send = upper ? w[i] : w[i + o];
+                        const double keep = upper ? w[i + o] : w[i];
+                        w[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+#pragma unroll
+                for (int o = CH; o < LG; o <<= 1) w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+                if (j / CH == ch / CH) dot = w[0];
             }
             if (my_s < nvalid && my_k >= 0) {
                 const double du = surrogate_up(my_m) * dot;
@@ -1014,25 +1068,24 @@ int launch_fc_backward(const lutb_layer_cfg *cfg, int64_t batch, float *W, const
                                                   cfg->n_inputs, O, Nt, cfg->n_anchors, T, group_dets, (int)per_block);
             return LUTB_OK;
         };
-        if (vec4) {
-            switch (lanes) {
-                case 32: launch_rc = launch(fc_input_grad_kernel<32, 4, false>, fc_input_grad_kernel<32, 4, true>); break;
-                case 16: launch_rc = launch(fc_input_grad_kernel<16, 4, false>, fc_input_grad_kernel<16, 4, true>); break;
-                case 8: launch_rc = launch(fc_input_grad_kernel<8, 4, false>, fc_input_grad_kernel<8, 4, true>); break;
-                case 4: launch_rc = launch(fc_input_grad_kernel<4, 4, false>, fc_input_grad_kernel<4, 4, true>); break;
-                case 2: launch_rc = launch(fc_input_grad_kernel<2, 4, false>, fc_input_grad_kernel<2, 4, true>); break;
-                default: launch_rc = launch(fc_input_grad_kernel<1, 4, false>, fc_input_grad_kernel<1, 4, true>); break;
+        auto pick = [&](auto lg, auto v) -> int {
+            constexpr int LG = decltype(lg)::value, V = decltype(v)::value;
+            if constexpr (LG == 32) {   // (the only groups whose rows can have more steps than one)
+                if (O > LG * V) return launch(fc_input_grad_kernel<LG, V, false, false>, fc_input_grad_kernel<LG, V, true, false>);
             }
-        } else {
+            return launch(fc_input_grad_kernel<LG, V, false, true>, fc_input_grad_kernel<LG, V, true, true>);
+        };
+        auto pick_lanes = [&](auto v) -> int {
             switch (lanes) {
-                case 32: launch_rc = launch(fc_input_grad_kernel<32, 1, false>, fc_input_grad_kernel<32, 1, true>); break;
-                case 16: launch_rc = launch(fc_input_grad_kernel<16, 1, false>, fc_input_grad_kernel<16, 1, true>); break;
-                case 8: launch_rc = launch(fc_input_grad_kernel<8, 1, false>, fc_input_grad_kernel<8, 1, true>); break;
-                case 4: launch_rc = launch(fc_input_grad_kernel<4, 1, false>, fc_input_grad_kernel<4, 1, true>); break;
-                case 2: launch_rc = launch(fc_input_grad_kernel<2, 1, false>, fc_input_grad_kernel<2, 1, true>); break;
-                default: launch_rc = launch(fc_input_grad_kernel<1, 1, false>, fc_input_grad_kernel<1, 1, true>); break;
+                case 32: return pick(std::integral_constant<int, 32>{}, v);
+                case 16: return pick(std::integral_constant<int, 16>{}, v);
+                case 8: return pick(std::integral_constant<int, 8>{}, v);
+                case 4: return pick(std::integral_constant<int, 4>{}, v);
+                case 2: return pick(std::integral_constant<int, 2>{}, v);
+                default: return pick(std::integral_constant<int, 1>{}, v);
             }
-        }
+        };
+        launch_rc = vec4 ? pick_lanes(std::integral_constant<int, 4>{}) : pick_lanes(std::integral_constant<int, 1>{});
         if (launch_rc) return launch_rc;
     }
     }
