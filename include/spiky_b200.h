@@ -183,7 +183,9 @@ typedef struct lutb_sparse_index {
     int32_t max_count;          /* max of det_count */
     int32_t max_table_slots;    /* largest "slots per detector table" of chunk_info; 0 = unknown (gather kernels only) */
     int32_t tables_aligned16;   /* 1 when every detector table starts at a multiple of 4 slots and spans a multiple of
-                                   4 slots, so that it can be bulk-copied with 16-byte granularity; 0 otherwise */
+                                   4 slots, so that it can be bulk-copied with 16-byte granularity; 0 otherwise.
+                                   + 2 (a hint) when most weights lie in rows of pairs: even number of synapses, even
+                                   stride, even table start, no forward group that ends inside a pair */
 } lutb_sparse_index;
 
 /*
@@ -193,10 +195,10 @@ typedef struct lutb_sparse_index {
  *   GATHER  one warp per (detector chunk, few samples); the selected rows are fetched through L2.  Any layer.
  *   STAGED  a block owns a range of detectors for 512 samples at a time; whole tables are streamed through a
  *           shared-memory ring (cp.async.bulk + mbarrier) and the samples' rows are read from there.  fp32 accumulators,
- *           rows of at most 32 synapses, tables_aligned16, three tables must fit 227 KB; LUTB_ERR_MODE when forced and
+ *           rows of at most 32 synapses, tables_aligned16 & 1, three tables must fit 227 KB; LUTB_ERR_MODE when forced and
  *           not possible.
- *   AUTO    forward: STAGED when possible, 2 * batch >= rows per table and the layer has at least 4 detectors per SM,
- *           else GATHER; input gradient: GATHER (the staged variant measured slower on B200).
+ *   AUTO    forward: STAGED when possible, tables_aligned16 without the hint of pairs, 2 * batch >= rows per table and
+ *           the layer has at least 4 detectors per SM, else GATHER; input gradient: GATHER (the staged variant measured slower on B200).
  * lutb_device_wait_errors: every device-side wait (the staged kernels' and lutb_peer_barrier's) is bounded (about a
  * second); a wait that runs out makes its block leave early (results are then incomplete) and is counted here.  Reads the counter of the current
  * device and synchronises it; 0 in a healthy run.

@@ -13,7 +13,7 @@
 
 namespace lutb {
 
-// The training kernels give one warp to a (chunk, run of kSampleRun samples) pair.  A chunk is a run of
+// The training kernels give one warp to a (chunk, run of samples) pair.  A chunk is a run of
 // up to 32 consecutive detectors that share one target list (the detectors of one group) and whose
 // tables lie back to back.  Work is ordered chunk-major: warps that run at the same time work on the
 // same few chunks for different samples, so a chunk's tables (a few hundred KB) are fetched from HBM
@@ -22,16 +22,32 @@ namespace lutb {
 // sample ahead so that it overlaps the row reads of the current sample) and turns it into the offset
 // of the selected row from the chunk's first table; offsets are broadcast with shuffles while the lanes
 // cover the synapses of a row, so every row access is one contiguous segment and all row reads of a
-// sample are in flight together.  Rows of up to LG synapses use LG-lane groups (NG = 32 / LG groups
-// take detectors round-robin).
-constexpr int kSampleRun = 4;
+// sample are in flight together.  Rows of up to LG * VEC synapses use LG-lane groups (NG = 32 / LG groups
+// take detectors round-robin); VEC = 2 where every row of the chunk is made of aligned pairs (rows_of_pairs):
+// half of the loads and broadcasts.
+// Bound: requests of 64 to 100 byte rows to L2, about 6 TB/s of the sectors they touch.  Measured, 256-row tables, tables from
+// HBM, one synapse a lane and 4 samples a run before.  Forward, 8192 detectors x 16 synapses: 100 samples 59 -> 30 us, 512 109 -> 62 (the
+// staged kernel, sparse_staged.cu: 70 and 75), 4096 288 (staged 544); 4608 detectors, 512 samples 57 -> 36 (53).  Input gradient,
+// 6400 + 8192 detectors, 512 samples: 236 -> 216 us; 8192 detectors, 4096 samples with 4 and 16 a run 727 -> 638.  Table gradient
+// (two-element reductions): no change at 512 samples, 16384 samples with 4 and 16 a run 1957 -> 1793.
 
-// With 512 samples over 256-row tables every row is touched about twice per step, so half of the row gathers are
-// compulsory DRAM misses at random addresses.  Each warp therefore asks L2 for its share of the tables of the
+// Samples of a run: a longer one shares the chunk's description, targets and the first index read among more samples, as long
+// as the runs are enough warps to fill the GPU several times over.  warps_per_sm: what a pass needs (forward 192, input
+// gradient 64, table gradient 128; measured at 1 to 16384 samples x 4608, 6400 and 8192 detectors: within 5 % of the best run
+// of 1, 2, 4, 8 and 16).  Forward, 8192 detectors, runs of 1 / 4 / 16: 4 samples 13 / 39 us, 512 92 / 62 / 127, 4096 351 (4) / 288.
+static int sample_run(int64_t batch, int64_t n_chunks, int warps_per_sm) {
+    const int64_t wanted = (int64_t)warps_per_sm * device_info().sm_count;
+    int run = 1;
+    while (run < 16 && (batch + 2 * run - 1) / (2 * run) * n_chunks >= wanted) run *= 2;
+    return run;
+}
+
+// Rows read one synapse at a time: with 512 samples over 256-row tables every row is touched about twice per step, so half of the
+// row gathers are compulsory DRAM misses at random addresses.  Each warp therefore asks L2 for its share of the tables of the
 // chunk that will be processed kPrefetchAhead chunks later (about the chunks in flight on the whole GPU), turning
-// those misses into a sequential stream that is resident when the gathers arrive.  Forward only: it runs 4 % faster
-// for 20 % more DRAM reads (rows no sample selects are fetched too); the fused backward gained nothing from prefetching
-// the table rows and lost time when its gradient rows were prefetched as well.
+// those misses into a sequential stream that is resident when the gathers arrive.  Forward only, and only where the batch selects
+// most rows of a table: 512 samples 116 -> 111 us, 16 samples 41 -> 50 without that condition.  Rows read in pairs gain nothing (62 -> 66);
+// the fused backward gained nothing from prefetching the table rows and lost time when its gradient rows were prefetched as well.
 constexpr int kPrefetchAhead = 40;
 
 __device__ __forceinline__ void prefetch_chunk(const SparseView &sp, const float *base, int64_t c, int64_t r, int64_t runs,
@@ -51,45 +67,74 @@ __device__ __forceinline__ void prefetch_chunk(const SparseView &sp, const float
 // The chunk's detectors are summed in registers, so the shared output cells see one reduction per
 // (sample, chunk, target) instead of one per synapse.
 // --------------------------------------------------------------------------------------------
-template <int LG, bool INT_MODE>
+template <int VEC>
+__device__ __forceinline__ void load_row(const float *p, float (&v)[VEC]) {
+    if constexpr (VEC == 2) {
+        const float2 f = __ldg(reinterpret_cast<const float2 *>(p));
+        v[0] = f.x; v[1] = f.y;
+    } else {
+        v[0] = __ldg(p);
+    }
+}
+
+// Rows of pairs: every row of the chunk starts on 8 bytes and no pair of synapses has a hole inside (base: the tables' array)
+__device__ __forceinline__ bool rows_of_pairs(const SparseView &sp, const ChunkStatic &cs, const float *base) {
+    return ((cs.P | cs.stride | cs.table | (int)cs.wbase0) & 1) == 0 && ((sp.group & 1) == 0 || cs.P <= sp.group) &&
+           (reinterpret_cast<uintptr_t>(base) & 7) == 0;
+}
+
+template <int LG, int VEC, bool INT_MODE>
 __device__ __forceinline__ void chunk_forward(const SparseView &sp, const ChunkStatic &cs, const float *__restrict__ W,
                                               const int32_t *__restrict__ idx, float *__restrict__ y, int64_t b0,
                                               int64_t b1, int n_outputs, int n_detectors, int lane,
                                               double fixed_scale) {
     constexpr int NG = 32 / LG;
-    const int g = lane / LG, j = lane - g * LG;
-    const bool valid = j < cs.P;
+    const int g = lane / LG, j = lane - g * LG, p = j * VEC;
+    const bool valid = p < cs.P;
     const bool has_det = lane < cs.ndet;
-    const float *Wb = W + cs.wbase0 + j + hole_offset(j, sp);
-    const int target = (valid && g == 0) ? __ldg(sp.syn_target + cs.toff + j) : 0;
+    const float *Wb = W + cs.wbase0 + p + hole_offset(p, sp);
+    int target[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; e++) target[e] = (valid && g == 0) ? __ldg(sp.syn_target + cs.toff + p + e) : 0;
     const int32_t *idx_l = idx + cs.det0 + lane;
     int32_t li_next = has_det ? __ldg(idx_l + b0 * n_detectors) : 0;
     for (int64_t b = b0; b < b1; b++) {
         const int32_t row_off = has_det ? lane * cs.table + li_next * cs.stride : 0;
         if (b + 1 < b1 && has_det) li_next = __ldg(idx_l + (b + 1) * n_detectors);
-        float w[LG];
+        float w[LG][VEC];
 #pragma unroll
         for (int i = 0; i < LG; i++) {
             const int d = i * NG + g;
             const int32_t off = __shfl_sync(0xffffffffu, row_off, d);
-            w[i] = (valid && d < cs.ndet) ? __ldg(Wb + off) : 0.f;
+#pragma unroll
+            for (int e = 0; e < VEC; e++) w[i][e] = 0.f;
+            if (valid && d < cs.ndet) load_row<VEC>(Wb + off, w[i]);
         }
-        float acc = 0.f;
-        int32_t iacc = 0;
+        float acc[VEC] = {};
+        int32_t iacc[VEC] = {};
 #pragma unroll
         for (int i = 0; i < LG; i++) {
             // beyond the chunk w is exactly 0 and truncates to 0
-            if (INT_MODE) iacc += to_fixed((double)w[i], fixed_scale);
-            else acc += w[i];
+#pragma unroll
+            for (int e = 0; e < VEC; e++) {
+                if (INT_MODE) iacc[e] += to_fixed((double)w[i][e], fixed_scale);
+                else acc[e] += w[i][e];
+            }
         }
 #pragma unroll
         for (int m = LG; m < 32; m <<= 1) {
-            if (INT_MODE) iacc += __shfl_xor_sync(0xffffffffu, iacc, m);
-            else acc += __shfl_xor_sync(0xffffffffu, acc, m);
+#pragma unroll
+            for (int e = 0; e < VEC; e++) {
+                if (INT_MODE) iacc[e] += __shfl_xor_sync(0xffffffffu, iacc[e], m);
+                else acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], m);
+            }
         }
         if (valid && g == 0) {
-            if (INT_MODE) atomicAdd(reinterpret_cast<int32_t *>(y) + b * n_outputs + target, iacc);
-            else atomicAdd(y + b * n_outputs + target, acc);
+#pragma unroll
+            for (int e = 0; e < VEC; e++) {
+                if (INT_MODE) atomicAdd(reinterpret_cast<int32_t *>(y) + b * n_outputs + target[e], iacc[e]);
+                else atomicAdd(y + b * n_outputs + target[e], acc[e]);
+            }
         }
     }
 }
@@ -98,19 +143,24 @@ template <bool INT_MODE>
 __global__ void __launch_bounds__(256, 4) sparse_forward_kernel(SparseView sp, const float *__restrict__ W,
                                                             const int32_t *__restrict__ idx, float *__restrict__ y,
                                                             int64_t batch, int n_outputs, int n_detectors,
-                                                            double fixed_scale) {
+                                                            double fixed_scale, int run, bool prefetch) {
     const int lane = threadIdx.x & 31;
-    const int64_t runs = (batch + kSampleRun - 1) / kSampleRun;
+    const int64_t runs = (batch + run - 1) / run;
     const int64_t work = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (work >= runs * sp.n_chunks) return;
     const int64_t c = work / runs;
-    const int64_t b0 = (work - c * runs) * kSampleRun;
-    const int64_t b1 = min(batch, b0 + kSampleRun);
-    prefetch_chunk(sp, W, c + kPrefetchAhead, work - c * runs, runs, lane);
+    const int64_t b0 = (work - c * runs) * run;
+    const int64_t b1 = min(batch, b0 + run);
     const ChunkStatic cs = load_chunk(sp, c);
-    if (cs.P <= 8) chunk_forward<8, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
-    else if (cs.P <= 16) chunk_forward<16, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
-    else if (cs.P <= 32) chunk_forward<32, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+    const bool pairs = !INT_MODE && cs.P <= 32 && rows_of_pairs(sp, cs, W);
+    if (prefetch && !pairs) prefetch_chunk(sp, W, c + kPrefetchAhead, work - c * runs, runs, lane);
+    if (pairs) {
+        if (cs.P <= 8) chunk_forward<4, 2, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+        else if (cs.P <= 16) chunk_forward<8, 2, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+        else chunk_forward<16, 2, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+    } else if (cs.P <= 8) chunk_forward<8, 1, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+    else if (cs.P <= 16) chunk_forward<16, 1, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
+    else if (cs.P <= 32) chunk_forward<32, 1, INT_MODE>(sp, cs, W, idx, y, b0, b1, n_outputs, n_detectors, lane, fixed_scale);
     else {
         // rows longer than a warp: plain loop, one detector at a time
         const float *Wb = W + cs.wbase0;
@@ -154,7 +204,7 @@ __global__ void __launch_bounds__(256, 4) sparse_forward_kernel(SparseView sp, c
 // measured faster than one fused pass, and required by the internal (in-place SGD) policy, where the
 // table gradient modifies the very weights other samples still have to read.
 // --------------------------------------------------------------------------------------------
-template <int LG, bool DO_DX, bool DO_DW, bool INT_DW>
+template <int LG, int VEC, bool DO_DX, bool DO_DW, bool INT_DW>
 __device__ __forceinline__ void chunk_backward(const SparseView &sp, const ChunkStatic &cs, const float *__restrict__ W,
                                                const float *__restrict__ dY, const int2 *__restrict__ anchors,
                                                const int32_t *__restrict__ idx, const float *__restrict__ min_delta,
@@ -163,11 +213,13 @@ __device__ __forceinline__ void chunk_backward(const SparseView &sp, const Chunk
                                                int n_outputs, int n_detectors, int n_anchors, int lane, double lr,
                                                double fixed_scale) {
     constexpr int NG = 32 / LG;
-    const int g = lane / LG, j = lane - g * LG;
-    const bool valid = j < cs.P;
+    const int g = lane / LG, j = lane - g * LG, p = j * VEC;
+    const bool valid = p < cs.P;
     const bool has_det = lane < cs.ndet;
-    const int q = j + hole_offset(j, sp);
-    const int my_target = valid ? __ldg(sp.syn_target + cs.toff + j) : 0;
+    const int q = p + hole_offset(p, sp);
+    int my_target[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; e++) my_target[e] = valid ? __ldg(sp.syn_target + cs.toff + p + e) : 0;
     const float *Wb = W + cs.wbase0 + q;
     float *Tb = DO_DW ? target_arr + cs.wbase0 + q : nullptr;
     // lane (g, j) ends up owning detector j * NG + g of the chunk
@@ -175,32 +227,41 @@ __device__ __forceinline__ void chunk_backward(const SparseView &sp, const Chunk
     const int64_t det_l = cs.det0 + lane;
     // per-sample inputs are fetched one sample ahead
     int32_t li_n = 0, k_n = 0;
-    float m_n = 0.f, gp_n = 0.f;
+    float m_n = 0.f, gp_n[VEC] = {};
     if (has_det) {
         li_n = __ldg(idx + b0 * n_detectors + det_l);
         if (DO_DX) { k_n = __ldg(min_k + b0 * n_detectors + det_l); m_n = __ldg(min_delta + b0 * n_detectors + det_l); }
     }
-    if (valid) gp_n = __ldg(dY + b0 * n_outputs + my_target);
+#pragma unroll
+    for (int e = 0; e < VEC; e++) if (valid) gp_n[e] = __ldg(dY + b0 * n_outputs + my_target[e]);
     for (int64_t b = b0; b < b1; b++) {
         const int32_t li = li_n, my_k = k_n;
-        const float my_m = m_n, gp = gp_n;
+        const float my_m = m_n;
+        float gp[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; e++) gp[e] = gp_n[e];
         if (b + 1 < b1) {
             if (has_det) {
                 li_n = __ldg(idx + (b + 1) * n_detectors + det_l);
                 if (DO_DX) { k_n = __ldg(min_k + (b + 1) * n_detectors + det_l); m_n = __ldg(min_delta + (b + 1) * n_detectors + det_l); }
             }
-            if (valid) gp_n = __ldg(dY + (b + 1) * n_outputs + my_target);
+#pragma unroll
+            for (int e = 0; e < VEC; e++) if (valid) gp_n[e] = __ldg(dY + (b + 1) * n_outputs + my_target[e]);
         }
         const int32_t row_off = has_det ? lane * cs.table + li * cs.stride : 0;
         // alternative row: minimum-margin bit flipped
         const int32_t alt_off = (DO_DX && has_det) ? row_off + ((li ^ (1 << my_k)) - li) * cs.stride : 0;
-        float val = 0.f;
-        int32_t ival = 0;
+        float val[VEC] = {};
+        int32_t ival[VEC] = {};
         bool active = false;
-        if (DO_DW && valid && fabsf(gp) > kEpsF) {
-            active = true;
-            if (INT_DW) ival = to_fixed((double)gp * lr, fixed_scale);
-            else val = lr == 1.0 ? gp : (float)((double)gp * lr);   // the product with 1.0 is gp itself
+        if (DO_DW && valid) {
+#pragma unroll
+            for (int e = 0; e < VEC; e++) {
+                if (!(fabsf(gp[e]) > kEpsF)) continue;   // (nothing to add; both are added as they are where the other one counts)
+                active = true;
+                if (INT_DW) ival[e] = to_fixed((double)gp[e] * lr, fixed_scale);
+                else val[e] = lr == 1.0 ? gp[e] : (float)((double)gp[e] * lr);   // the product with 1.0 is gp itself
+            }
         }
         float v[LG];
 #pragma unroll
@@ -210,11 +271,22 @@ __device__ __forceinline__ void chunk_backward(const SparseView &sp, const Chunk
             if (DO_DX) {
                 const int32_t ao = __shfl_sync(0xffffffffu, alt_off, d);
                 // detectors beyond the chunk have ro == ao == 0: the difference is exactly zero
-                v[i] = valid ? gp * (__ldg(Wb + ro) - __ldg(Wb + ao)) : 0.f;
+                float a[VEC] = {}, c[VEC] = {};
+                if (valid) {
+                    load_row<VEC>(Wb + ro, a);
+                    load_row<VEC>(Wb + ao, c);
+                }
+                v[i] = 0.f;
+#pragma unroll
+                for (int e = 0; e < VEC; e++) v[i] = fmaf(gp[e], a[e] - c[e], v[i]);
             }
             if (DO_DW && active && d < cs.ndet) {
-                if (INT_DW) atomicAdd(reinterpret_cast<int32_t *>(Tb) + ro, ival);
-                else atomicAdd(Tb + ro, val);
+                if constexpr (VEC == 2) {
+                    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(Tb + ro), "f"(val[0]), "f"(val[1]) : "memory");
+                } else {
+                    if (INT_DW) atomicAdd(reinterpret_cast<int32_t *>(Tb) + ro, ival[0]);
+                    else atomicAdd(Tb + ro, val[0]);
+                }
             }
         }
         if (!DO_DX) continue;
@@ -254,21 +326,22 @@ __global__ void __launch_bounds__(256, DO_DX ? 3 : 4) sparse_backward_kernel(Spa
                                                              float *__restrict__ dX, float *__restrict__ target_arr,
                                                              int64_t batch, int n_inputs, int n_outputs,
                                                              int n_detectors, int n_anchors, double lr,
-                                                             double fixed_scale) {
+                                                             double fixed_scale, int run) {
     const int lane = threadIdx.x & 31;
-    const int64_t runs = (batch + kSampleRun - 1) / kSampleRun;
+    const int64_t runs = (batch + run - 1) / run;
     const int64_t work = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (work >= runs * sp.n_chunks) return;
     const int64_t c = work / runs;
-    const int64_t b0 = (work - c * runs) * kSampleRun;
-    const int64_t b1 = min(batch, b0 + kSampleRun);
+    const int64_t b0 = (work - c * runs) * run;
+    const int64_t b1 = min(batch, b0 + run);
     const ChunkStatic cs = load_chunk(sp, c);
-    if (cs.P <= 8)
-        chunk_backward<8, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
-    else if (cs.P <= 16)
-        chunk_backward<16, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
-    else
-        chunk_backward<32, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+    if (!INT_DW && rows_of_pairs(sp, cs, DO_DX ? W : target_arr)) {
+        if (cs.P <= 8) chunk_backward<4, 2, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+        else if (cs.P <= 16) chunk_backward<8, 2, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+        else chunk_backward<16, 2, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+    } else if (cs.P <= 8) chunk_backward<8, 1, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+    else if (cs.P <= 16) chunk_backward<16, 1, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
+    else chunk_backward<32, 1, DO_DX, DO_DW, INT_DW>(sp, cs, W, dY, anchors, idx, min_delta, min_k, dX, target_arr, b0, b1, n_inputs, n_outputs, n_detectors, n_anchors, lane, lr, fixed_scale);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -317,14 +390,14 @@ __global__ void __launch_bounds__(256, 4) sparse_table_grad_range_kernel(SparseV
                                                                      const IdxT *__restrict__ idx,
                                                                      float *__restrict__ target_arr, int64_t batch,
                                                                      int n_outputs, int n_detectors, double lr,
-                                                                     int64_t chunk_begin, int64_t n_range) {
+                                                                     int64_t chunk_begin, int64_t n_range, int run) {
     const int lane = threadIdx.x & 31;
-    const int64_t runs = (batch + kSampleRun - 1) / kSampleRun;
+    const int64_t runs = (batch + run - 1) / run;
     const int64_t work = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (work >= runs * n_range) return;
     const int64_t c = work / runs;
-    const int64_t b0 = (work - c * runs) * kSampleRun;
-    const int64_t b1 = min(batch, b0 + kSampleRun);
+    const int64_t b0 = (work - c * runs) * run;
+    const int64_t b1 = min(batch, b0 + run);
     const ChunkStatic cs = load_chunk(sp, chunk_begin + c);
     if (cs.P <= 8) chunk_table_grad<8, IdxT>(sp, cs, dY, idx, target_arr, b0, b1, n_outputs, n_detectors, lane, lr);
     else if (cs.P <= 16) chunk_table_grad<16, IdxT>(sp, cs, dY, idx, target_arr, b0, b1, n_outputs, n_detectors, lane, lr);
@@ -514,14 +587,16 @@ extern "C" int lutb_nonseq_sparse_forward(const lutb_layer_cfg *cfg, const lutb_
     if (staged) return launch_sparse_forward_staged(cfg, sp, batch, weights, idx, y, st);
     SparseView v = make_view(sp);
     unsigned blocks;
-    rc = chunk_grid(((batch + kSampleRun - 1) / kSampleRun) * sp->n_chunks, &blocks);
+    const int run = sample_run(batch, sp->n_chunks, 192);
+    rc = chunk_grid(((batch + run - 1) / run) * sp->n_chunks, &blocks);
     if (rc) return rc;
+    const bool prefetch = 2 * batch >= (int64_t)1 << cfg->n_anchors;
     {
         KernelScope scope(K_SPARSE_FORWARD, st);
         if (cfg->int_mode)
-            sparse_forward_kernel<true><<<blocks, 256, 0, st>>>(v, weights, idx, y, batch, cfg->n_outputs, cfg->n_detectors, cfg->int_rescaler);
+            sparse_forward_kernel<true><<<blocks, 256, 0, st>>>(v, weights, idx, y, batch, cfg->n_outputs, cfg->n_detectors, cfg->int_rescaler, run, prefetch);
         else
-            sparse_forward_kernel<false><<<blocks, 256, 0, st>>>(v, weights, idx, y, batch, cfg->n_outputs, cfg->n_detectors, cfg->int_rescaler);
+            sparse_forward_kernel<false><<<blocks, 256, 0, st>>>(v, weights, idx, y, batch, cfg->n_outputs, cfg->n_detectors, cfg->int_rescaler, run, prefetch);
     }
     LUTB_LAUNCH_CHECK();
     if (cfg->int_mode) return launch_fixed_to_float(y, batch * (int64_t)cfg->n_outputs, cfg->int_rescaler, st);
@@ -554,15 +629,19 @@ extern "C" int lutb_nonseq_sparse_backward(const lutb_layer_cfg *cfg, const lutb
     if (external_lr >= 0.0) lr *= -(double)(float)external_lr;
     float *target = external_lr >= 0.0 ? weights : dW;
     const bool long_rows = sp->max_count > 32;
-    unsigned blocks;
-    rc = chunk_grid(long_rows ? batch * (int64_t)Nt : ((batch + kSampleRun - 1) / kSampleRun) * sp->n_chunks, &blocks);
+    const int dx_run = sample_run(batch, sp->n_chunks, 64), dw_run = sample_run(batch, sp->n_chunks, 128);
+    unsigned dx_blocks, dw_blocks;
+    rc = chunk_grid(long_rows ? batch * (int64_t)Nt : ((batch + dx_run - 1) / dx_run) * sp->n_chunks, &dx_blocks);
+    if (rc) return rc;
+    rc = chunk_grid(long_rows ? batch * (int64_t)Nt : ((batch + dw_run - 1) / dw_run) * sp->n_chunks, &dw_blocks);
     if (rc) return rc;
 #define LUTB_SPARSE_BWD(DX, DWF, INTF)                                                                              \
     do {                                                                                                            \
+        const unsigned blocks = DX ? dx_blocks : dw_blocks;                                                          \
         if (long_rows)                                                                                              \
             sparse_backward_long_kernel<DX, DWF, INTF><<<blocks, 256, 0, st>>>(v, weights, dY, an, idx, min_delta, min_k, dX, target, batch, cfg->n_inputs, O, Nt, cfg->n_anchors, lr, cfg->int_rescaler); \
         else                                                                                                        \
-            sparse_backward_kernel<DX, DWF, INTF><<<blocks, 256, 0, st>>>(v, weights, dY, an, idx, min_delta, min_k, dX, target, batch, cfg->n_inputs, O, Nt, cfg->n_anchors, lr, cfg->int_rescaler); \
+            sparse_backward_kernel<DX, DWF, INTF><<<blocks, 256, 0, st>>>(v, weights, dY, an, idx, min_delta, min_k, dX, target, batch, cfg->n_inputs, O, Nt, cfg->n_anchors, lr, cfg->int_rescaler, DX ? dx_run : dw_run); \
     } while (0)
     // Two passes.  The input gradient (row gathers, dX updates) and the table gradient (fire-and-forget reductions into
     // the selected rows) run faster one after the other than fused into one kernel (0.33 + 0.19 ms against 0.70 ms for the
@@ -624,17 +703,18 @@ extern "C" int lutb_nonseq_sparse_table_grad(const lutb_layer_cfg *cfg, const lu
     SparseView v = make_view(sp);
     const int64_t n_range = chunk_end - chunk_begin;
     unsigned blocks;
-    rc = chunk_grid(((batch + kSampleRun - 1) / kSampleRun) * n_range, &blocks);
+    const int run = sample_run(batch, n_range, 128);
+    rc = chunk_grid(((batch + run - 1) / run) * n_range, &blocks);
     if (rc) return rc;
     const double lr = cfg->lr_meta * scale;
     const int O = cfg->n_outputs, Nt = cfg->n_detectors;
     KernelScope scope(K_SPARSE_WEIGHT_GRAD, st);
     if (idx_bytes == 1)
-        sparse_table_grad_range_kernel<uint8_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const uint8_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range);
+        sparse_table_grad_range_kernel<uint8_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const uint8_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range, run);
     else if (idx_bytes == 2)
-        sparse_table_grad_range_kernel<uint16_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const uint16_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range);
+        sparse_table_grad_range_kernel<uint16_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const uint16_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range, run);
     else
-        sparse_table_grad_range_kernel<int32_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const int32_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range);
+        sparse_table_grad_range_kernel<int32_t><<<blocks, 256, 0, st>>>(v, dY, static_cast<const int32_t *>(idx), target, batch, O, Nt, lr, chunk_begin, n_range, run);
     LUTB_LAUNCH_CHECK();
     return LUTB_OK;
 }

@@ -552,7 +552,7 @@ static int stages_of(const lutb_sparse_index *sp) {
 
 bool sparse_staged_possible(const lutb_layer_cfg *cfg, const lutb_sparse_index *sp, const float *weights) {
     if (cfg->int_mode != 0 || cfg->seq_len != 1) return false;
-    if (sp->max_count > 32 || sp->max_table_slots <= 0 || sp->max_table_slots > 65535 || !sp->tables_aligned16) return false;
+    if (sp->max_count > 32 || sp->max_table_slots <= 0 || sp->max_table_slots > 65535 || !(sp->tables_aligned16 & 1)) return false;
     if ((reinterpret_cast<uintptr_t>(weights) & 15) != 0) return false;
     return stages_of(sp) >= kMinStages;
 }
@@ -565,6 +565,10 @@ bool sparse_staged_preferred(int pass, const lutb_layer_cfg *cfg, const lutb_spa
     // in shared memory collide on its banks about as often as they would miss in L1), so it is never the
     // library's choice.
     if (pass != 0) return false;
+    // Most rows made of pairs: the gather kernel reads them with half of the loads, 512 samples 36 / 71 / 62 us against 53 / 68 / 75 for
+    // 4608 / 6400 / 8192 detectors, 4096 samples 156 / 315 / 288 against 325 / 425 / 544.  One synapse at a time it takes 57 / 111 / 105
+    // at 512 samples.
+    if (sp->tables_aligned16 & 2) return false;
     const int64_t rows = (int64_t)1 << cfg->n_anchors;
     return 2 * batch >= rows && cfg->n_detectors >= 4 * device_info().sm_count;
 }

@@ -226,8 +226,12 @@ class SparseIndex:
             wbase0 = (ci[:, 6] & 0xFFFFFFFF) | (ci[:, 7] << 32)
             self.max_table_slots = int(ci[:, 5].max().item())
             self.tables_aligned16 = int(bool(((wbase0 % 4 == 0) & (ci[:, 5] % 4 == 0)).all().item()))
+            # rows that the gather kernels read two synapses at a time: whether they hold at least 3/4 of the weights
+            pairs = ((wbase0 | ci[:, 3] | ci[:, 4] | ci[:, 5]) % 2 == 0) & ((self.group_size % 2 == 0) | (ci[:, 3] <= self.group_size))
+            size = ci[:, 1] * ci[:, 3]
+            self.pair_rows = int(4 * int((size * pairs).sum()) >= 3 * int(size.sum()))
         else:
-            self.max_table_slots, self.tables_aligned16 = 0, 0
+            self.max_table_slots, self.tables_aligned16, self.pair_rows = 0, 0, 0
 
     CHUNK = 32  # detectors per chunk = lanes of a warp
 
@@ -409,7 +413,8 @@ class SparseIndex:
             det_count=self.det_count.data_ptr(), det_sstart=self.det_sstart.data_ptr(),
             syn_det=self.syn_det.data_ptr(), syn_target=self.syn_target.data_ptr(),
             chunk_info=self.chunk_info.data_ptr(), n_chunks=self.n_chunks, n_syn_per_sample=self.n_syn_per_sample, n_weights=self.n_weights, group_size=self.group_size,
-            max_count=self.max_count, max_table_slots=self.max_table_slots, tables_aligned16=self.tables_aligned16)
+            max_count=self.max_count, max_table_slots=self.max_table_slots,
+            tables_aligned16=self.tables_aligned16 | 2 * getattr(self, "pair_rows", 0))
 
     def nbytes(self):
         return sum(getattr(self, n).numel() * getattr(self, n).element_size() for n in self._TENSORS)
