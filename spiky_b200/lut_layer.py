@@ -516,9 +516,23 @@ class LUTLayerBasic(nn.Module):
                                  SKIP_TABLE_GRADIENT, None, None, dw_variant=dw_variant)
         dx = None if x_grad is None else x_grad.view(x.shape)
         # zero cells (an output gradient that is exactly zero or below the threshold) are not part of the list
-        cells, vals = dm.table_gradient_cells(batch_size, grad_flat, idx_flat)
-        if cells is None:
-            return dx, None
+        if getattr(dm.table_gradient_rows, "__func__", None) is LUTDataManagerF.table_gradient_rows:
+            cells, vals = dm.table_gradient_cells(batch_size, grad_flat, idx_flat)
+            if cells is None:
+                return dx, None
+        else:   # a data manager with row lists of its own: its rows are compacted here
+            rows, values = dm.table_gradient_rows(batch_size, grad_flat, idx_flat)
+            if rows.numel() == 0:
+                return dx, None
+            O = values.shape[1]
+            flat = values.reshape(-1)
+            pad = (-flat.numel()) % 4
+            if pad:
+                flat = torch.cat([flat, flat.new_zeros(pad)])
+            nz, vals = self._shared_context.get_dense_to_sparse_converter(self._multi_id).dense_to_sparse_32(flat)
+            if nz is None:
+                return dx, None
+            cells = rows[nz // O] * O + nz % O
         if self._weights_gradient_policy.normalized:
             vals /= vals.abs().max().clip(1e-16)
         return dx, torch.sparse_coo_tensor(cells.unsqueeze(0), vals, size=self._weights.shape, device=self.device,
