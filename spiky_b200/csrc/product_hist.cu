@@ -108,11 +108,13 @@ __device__ __forceinline__ void positional_ends(const AnchorLists &al, const flo
 // 1024-row tables.
 // Bound: instruction issue, and at 256-row tables the 537 MB of counters it writes.  Measured (before: lanes over the keys
 // of one query, the anchors' operands read from shared memory for every pair): 64 sequences x 128 tokens, 64 detectors of
-// 256 rows 271 -> 182 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 187 us.
+// 256 rows 271 -> 195 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 173 us.  Blocks of one detector run together, as in
+// product_route_kernel: 195 -> 190 us.
 // --------------------------------------------------------------------------------------------
 constexpr int kHistTile = 4;
 
 struct HistArgs {
+    int sequences;   // of the chunk
     const float *x1, *x2, *pe;
     const int32_t *anchors;
     void *H;
@@ -193,9 +195,10 @@ template <int MAXKQ, bool EPS, bool HALF_ROWS, bool PACKED>
 __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
-    const int t = blockIdx.x;
+    // blocks of one detector run together, see product_route_kernel
+    const int t = blockIdx.x / p.sequences;
     const int j_begin = (gridDim.y - 1 - blockIdx.y) * p.queries;   // the ranges with the most keys first
-    const int64_t bl = blockIdx.z, b = p.b0 + bl;
+    const int64_t bl = blockIdx.x - t * p.sequences, b = p.b0 + bl;
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc, Sp = (S + 31) & ~31;
     const int j_end = min(S, j_begin + p.queries);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -328,14 +331,19 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
 // eight queries.
 // Measured (before: a warp per query, about 600 instructions per 32 pairs): 64 sequences x 128 tokens, 64 detectors of 256
 // rows 862 -> 490 us; 1 x 1024 tokens, 64 detectors of 1024 rows 1910 -> 435 us (851 before a block's queries were limited).
-// The rounded reciprocal of the surrogate is 6 % of that (460 and 413 us with a refined hardware approximation, which gave
-// the same bits on what was tried).  Two barriers per eight queries instead of four
+// Since then the pairs of two queries are interleaved (475 -> 438 us and 446 -> 409; four at a time 540 and 416) and the blocks
+// numbered detector by detector instead of sequence by sequence (438 -> 396 and 409 -> 361: fewer blocks add to the dX of one
+// sequence at a time, and fewer of the loops for different numbers of anchors run side by side; which weighs more was not
+// isolated).  Slower: asking for the next tile's rows before the query cells are added up (447 -> 457), a loop for every number
+// of anchors instead of every other one (438 -> 480), blocks of one detector on one SM (396 -> 421).  The rounded reciprocal of the
+// surrogate takes 8 %.  Two barriers per eight queries instead of four
 // gave 8 % at 128 tokens; a per-warp window of distances for dPE instead of an add per pair cost 20 % there.
 // --------------------------------------------------------------------------------------------
 constexpr int kRouteWarps = 4, kRouteKeys = 32 * kRouteWarps, kTileQ = 8, kRouteWindow = kRouteKeys + kTileQ;
 constexpr int kExLd = 33;          // leading dimension of the (query, key) exchange tile
 
 struct RouteArgs {
+    int sequences, parts;   // sequences of the chunk; blocks per (detector, sequence)
     const float *x1, *x2, *pe;
     const int32_t *anchors;
     const float *Q;
@@ -401,69 +409,97 @@ __device__ __forceinline__ void route_tile(const RouteArgs &p, const AnchorLists
         step1 = b.w ? kHistAnchors : b.z;
         pe_bit = 1u << al.pe_k[0];
     }
-#pragma unroll 2
-    for (int q = 0; q < kTileQ; q++) {
-        const int j = r.j0 + q;
-        uint32_t li = r.kbits | __shfl_sync(0xffffffffu, r.qbits, q);
-        unsigned long long best = margin_key(__shfl_sync(0xffffffffu, r.qmd, q), __shfl_sync(0xffffffffu, r.qlow, q));
-        best = r.kmin < best ? r.kmin : best;
-        if (NKQ > 0) {
-            // anchor numbers ascend: strictly smaller is enough inside this group
-            float md = kFltMax;
-            uint32_t low = 0u;
-            const float4 *qv4 = reinterpret_cast<const float4 *>(r.qv + q * kHistAnchors);
+    // Two queries at a time, in three phases: both table rows' entries are asked for before the first reciprocal, and both key
+    // cells are read before either is written (the compiler may not move a load across a store of shared memory itself).
+    constexpr int U = 2;
+#pragma unroll 1
+    for (int q0 = 0; q0 < kTileQ; q0 += U) {
+        float dus[U], slopes[U], halves[U];
+        int offs[U];
 #pragma unroll
-            for (int m = 0; m < NKQ; m += 2) {
-                const float4 f = qv4[m / 2];
-                const float da = __fsub_rn(kv[m], f.x), db = __fsub_rn(kv[m + 1], f.z);
-                const uint32_t ba = __float_as_uint(f.y), bb = __float_as_uint(f.w);
-                if (EPS ? greater_than_zero(da, p.cmp_eps) : da > 0.f) li |= ba;
-                if (fabsf(da) < md) { md = fabsf(da); low = margin_low<EPS>(ba, da); }
-                if (EPS ? greater_than_zero(db, p.cmp_eps) : db > 0.f) li |= bb;
-                if (fabsf(db) < md) { md = fabsf(db); low = margin_low<EPS>(bb, db); }
+        for (int u = 0; u < U; u++) {
+            const int q = q0 + u, j = r.j0 + q;
+            uint32_t li = r.kbits | __shfl_sync(0xffffffffu, r.qbits, q);
+            unsigned long long best = margin_key(__shfl_sync(0xffffffffu, r.qmd, q), __shfl_sync(0xffffffffu, r.qlow, q));
+            best = r.kmin < best ? r.kmin : best;
+            if (NKQ > 0) {
+                // anchor numbers ascend: strictly smaller is enough inside this group
+                float md = kFltMax;
+                uint32_t low = 0u;
+                const float4 *qv4 = reinterpret_cast<const float4 *>(r.qv + q * kHistAnchors);
+#pragma unroll
+                for (int m = 0; m < NKQ; m += 2) {
+                    const float4 f = qv4[m / 2];
+                    const float da = __fsub_rn(kv[m], f.x), db = __fsub_rn(kv[m + 1], f.z);
+                    const uint32_t ba = __float_as_uint(f.y), bb = __float_as_uint(f.w);
+                    if (EPS ? greater_than_zero(da, p.cmp_eps) : da > 0.f) li |= ba;
+                    if (fabsf(da) < md) { md = fabsf(da); low = margin_low<EPS>(ba, da); }
+                    if (EPS ? greater_than_zero(db, p.cmp_eps) : db > 0.f) li |= bb;
+                    if (fabsf(db) < md) { md = fabsf(db); low = margin_low<EPS>(bb, db); }
+                }
+                const unsigned long long mixed = margin_key(md, low);
+                best = mixed < best ? mixed : best;
             }
-            const unsigned long long mixed = margin_key(md, low);
-            best = mixed < best ? mixed : best;
+            const bool pair = r.i < j && j < r.j_end;
+            const int dist = max(0, min(j, p.S - 1) - r.i - 1);
+            if (PE && r.n_pe > 0) {
+                {
+                    const float d = __fsub_rn(end0[q * step0], end1[q * step1]);
+                    if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= pe_bit;
+                    const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(pe_bit, d));
+                    best = c < best ? c : best;
+                }
+                for (int m = 1; m < r.n_pe; m++) {
+                    float v0, v1;
+                    positional_ends(al, r.smem, r.qd + q * kHistAnchors, m, m < p.pe_cap, r.ikey, q, r.xk,
+                                    r.x2b + (size_t)min(j, p.S - 1) * p.e2, r.pe_t + (size_t)dist * r.pe_stride, v0, v1);
+                    const uint32_t bit = 1u << al.pe_k[m];
+                    const float d = __fsub_rn(v0, v1);
+                    if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= bit;
+                    const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(bit, d));
+                    best = c < best ? c : best;
+                }
+            }
+            const float md = __uint_as_float((uint32_t)(best >> 32));
+            const uint32_t low = (uint32_t)best, bit = EPS ? low >> 1 : low;
+            const bool positive = EPS ? (low & 1u) != 0u : (li & bit) != 0u;
+            // up(d) * (Q[row] - Q[flipped row]) in fp32: Q is an fp32 contraction already (the direct kernels and the
+            // fixed-point mode keep the double-precision reciprocal of the reference's formula)
+            const float *qrow = r.Qs + q * T;
+            slopes[u] = 1.0f + md;
+            dus[u] = qrow[li] - qrow[li ^ bit];
+            halves[u] = pair && bit != 0u ? (positive ? 0.5f : -0.5f) : 0.f;
+            offs[u] = bit ? (31 - __clz(bit)) * 32 : 0;
         }
-        const bool pair = r.i < j && j < r.j_end;
-        const int dist = max(0, min(j, p.S - 1) - r.i - 1);
-        if (PE && r.n_pe > 0) {
-            {
-                const float d = __fsub_rn(end0[q * step0], end1[q * step1]);
-                if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= pe_bit;
-                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(pe_bit, d));
-                best = c < best ? c : best;
-            }
-            for (int m = 1; m < r.n_pe; m++) {
-                float v0, v1;
-                positional_ends(al, r.smem, r.qd + q * kHistAnchors, m, m < p.pe_cap, r.ikey, q, r.xk,
-                                r.x2b + (size_t)min(j, p.S - 1) * p.e2, r.pe_t + (size_t)dist * r.pe_stride, v0, v1);
-                const uint32_t bit = 1u << al.pe_k[m];
-                const float d = __fsub_rn(v0, v1);
-                if (EPS ? greater_than_zero(d, p.cmp_eps) : d > 0.f) li |= bit;
-                const unsigned long long c = margin_key(fabsf(d), margin_low<EPS>(bit, d));
-                best = c < best ? c : best;
-            }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const float rc = __frcp_rn(slopes[u]);
+            const float du = halves[u] * rc * rc * dus[u];
+            dus[u] = halves[u] != 0.f && fabsf(du) > kEpsF ? du : 0.f;
         }
-        const float md = __uint_as_float((uint32_t)(best >> 32));
-        const uint32_t low = (uint32_t)best, bit = EPS ? low >> 1 : low;
-        const bool positive = EPS ? (low & 1u) != 0u : (li & bit) != 0u;
-        // up(d) * (Q[row] - Q[flipped row]) in fp32: Q is an fp32 contraction already (the direct kernels and the
-        // fixed-point mode keep the double-precision reciprocal of the reference's formula)
-        const float rc = __frcp_rn(1.0f + md);
-        const float *qrow = r.Qs + q * T;
-        float du = (positive ? 0.5f : -0.5f) * rc * rc * (qrow[li] - qrow[li ^ bit]);
-        du = pair && bit != 0u && fabsf(du) > kEpsF ? du : 0.f;
-        const int off = bit ? (31 - __clz(bit)) * 32 : 0;
-        r.kcol[off + lane] += du;
-        r.ex[q * kExLd + lane] = make_float2(du, __int_as_float(off));
-        if (PE && r.n_pe > 0) {
-            if ((bit & r.pe_mask) && du != 0.f) {
+        static_assert(U == 2);
+        {   // both cells are read before either is written
+            float c0 = r.kcol[offs[0] + lane], c1 = r.kcol[offs[1] + lane];
+            c0 += dus[0];
+            c1 = (offs[1] == offs[0] ? c0 : c1) + dus[1];
+            r.kcol[offs[0] + lane] = c0;
+            r.kcol[offs[1] + lane] = c1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int q = q0 + u, off = offs[u];
+            const float du = dus[u];
+            r.ex[q * kExLd + lane] = make_float2(du, __int_as_float(off));
+            if (PE && r.n_pe > 0) {
+                // (du is zero where there is no pair or no anchor)
                 const int k = off / 32;
+                if (((r.pe_mask >> k) & 1u) && du != 0.f) {
+                    const int dist = max(0, min(r.j0 + q, p.S - 1) - r.i - 1);
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    if (al.comp[2 * k + e] == 2)
-                        add_positional(p, r.pacc, dist, r.t, al.elem[2 * k + e], e == 0 ? du : -du);
+                    for (int e = 0; e < 2; e++) {
+                        if (al.comp[2 * k + e] == 2)
+                            add_positional(p, r.pacc, dist, r.t, al.elem[2 * k + e], e == 0 ? du : -du);
+                    }
                 }
             }
         }
@@ -474,13 +510,13 @@ template <int MAXKQ, bool EPS>
 __global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_route_kernel(const RouteArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
-    const int t = blockIdx.x;
-    // blockIdx.y: (segment of p.queries queries, key range); the later key ranges have fewer segments
+    const int place = blockIdx.x / p.sequences, t = place / p.parts, part = place - t * p.parts;
+    // a part: (segment of p.queries queries, key range); the later key ranges have fewer segments
     const int n_ranges = (p.S - 1 + kRouteKeys - 1) / kRouteKeys;
-    const int seg = blockIdx.y / n_ranges, k0 = (blockIdx.y - seg * n_ranges) * kRouteKeys;
+    const int seg = part / n_ranges, k0 = (part - seg * n_ranges) * kRouteKeys;
     const int j_begin = k0 + 1 + seg * p.queries, j_end = min(p.S, j_begin + p.queries);
     if (j_begin >= p.S) return;
-    const int64_t bl = blockIdx.z, b = p.b0 + bl;
+    const int64_t bl = blockIdx.x - place * p.sequences, b = p.b0 + bl;
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float *Qs = smem;                                             // [kTileQ][T]
@@ -592,17 +628,21 @@ __global__ void __launch_bounds__(32 * kRouteWarps, MAXKQ <= 8 ? 8 : 7) product_
             if (EPS || n_pe > 0) {
                 if (MAXKQ > 8 && !EPS && n_kq <= 6) route_tile<6, true, EPS, MAXKQ>(p, al, r, kv);
                 else route_tile<MAXKQ, true, EPS, MAXKQ>(p, al, r, kv);
-            } else if (n_kq <= 2) route_tile<2, false, EPS, MAXKQ>(p, al, r, kv);
-            else if (n_kq <= 4) route_tile<4, false, EPS, MAXKQ>(p, al, r, kv);
+            } else if (n_kq <= 4) route_tile<4, false, EPS, MAXKQ>(p, al, r, kv);
             else if (n_kq <= 6) route_tile<6, false, EPS, MAXKQ>(p, al, r, kv);
             else route_tile<MAXKQ, false, EPS, MAXKQ>(p, al, r, kv);
             __syncwarp();
             // lanes over (query, quarter of the keys)
             const float2 *mine = ex + (lane & (kTileQ - 1)) * kExLd + (lane / kTileQ) * kTileQ;
 #pragma unroll
-            for (int n = 0; n < 8; n++) {
-                const float2 v = mine[n];
-                qcol[__float_as_int(v.y) + lane] += v.x;
+            for (int n = 0; n < 8; n += 2) {
+                const float2 v = mine[n], w = mine[n + 1];
+                const int o0 = __float_as_int(v.y) + lane, o1 = __float_as_int(w.y) + lane;
+                float c0 = qcol[o0], c1 = qcol[o1];
+                c0 += v.x;
+                c1 = (o1 == o0 ? c0 : c1) + w.x;
+                qcol[o0] = c0;
+                qcol[o1] = c1;
             }
         }
         __syncthreads();
@@ -987,7 +1027,9 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     }
     LUTB_REQUIRE(warps > 0, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
     const size_t smem = hist_floats(T, packed, warps, cfg->n_anchors, h.pe_cap, c.S) * 4;
-    dim3 grid((unsigned)cfg->n_detectors, (unsigned)((c.S + h.queries - 1) / h.queries), (unsigned)n);
+    h.sequences = (int)n;
+    LUTB_REQUIRE(cfg->n_detectors * n <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "product histogram path: too many blocks for one launch");
+    const dim3 grid((unsigned)(cfg->n_detectors * n), (unsigned)((c.S + h.queries - 1) / h.queries));
     KernelScope scope(K_PRODUCT_HIST, stream);
     auto launch = [&](auto kern) -> int {
         if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1125,12 +1167,15 @@ int launch_product_hist_backward(const ProductCall &c, const float *weights, con
             ra.queries = queries_per_block(c.S, (int64_t)Nt * n, kRouteKeys, resident < most ? resident : most);
             const int ranges = (c.S - 1 + kRouteKeys - 1) / kRouteKeys, segs = (c.S - 1 + ra.queries - 1) / ra.queries;
             LUTB_REQUIRE((int64_t)ranges * segs <= 65535, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
-            dim3 grid((unsigned)Nt, (unsigned)(ranges * segs), (unsigned)n);
+            ra.sequences = (int)n;
+            ra.parts = ranges * segs;
+            const int64_t grid = (int64_t)Nt * ra.parts * n;
+            LUTB_REQUIRE(grid <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "product histogram path: too many blocks for one launch");
             KernelScope scope(K_PRODUCT_ROUTE, stream);
             auto launch = [&](auto kern) -> int {
                 if (route_smem > kPlainSmem)
                     LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_smem));
-                kern<<<grid, 32 * kRouteWarps, route_smem, stream>>>(ra);
+                kern<<<(unsigned)grid, 32 * kRouteWarps, route_smem, stream>>>(ra);
                 return LUTB_OK;
             };
             const bool eps = cfg->cmp_eps != 0.f;
