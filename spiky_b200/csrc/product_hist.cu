@@ -104,12 +104,13 @@ __device__ __forceinline__ void positional_ends(const AnchorLists &al, const flo
 // HALF_ROWS: the counters are written as fp16 (exact: counts are below 2048 there) in the layout [row of the chunk = local
 // sequence * S + j][detector][T], the operand layout of the tensor-core contractions (one plain GEMM over all detectors per
 // pass); otherwise as uint16 in the layout [detector][row of the chunk][T].
-// PACKED: two 16-bit counters per word (a count is at most S - 1 < 65536), which keeps 16 warps per block up to
-// 1024-row tables.
-// Bound: instruction issue, and at 256-row tables the 537 MB of counters it writes.  Measured (before: lanes over the keys
-// of one query, the anchors' operands read from shared memory for every pair): 64 sequences x 128 tokens, 64 detectors of
-// 256 rows 271 -> 195 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 173 us.  Blocks of one detector run together, as in
-// product_route_kernel: 195 -> 190 us.
+// PER: counters per 32-bit word, four for sequences of at most 256 tokens (a count is at most S - 1), else two.
+// Bound: load/store wavefronts and issue, and at 256-row tables the 537 MB of counters it writes.  Measured (before: lanes over the
+// keys of one query, the anchors' operands read from shared memory for every pair): 64 sequences x 128 tokens, 64 detectors of
+// 256 rows 271 -> 195 us; 1 x 1024 tokens, 64 detectors of 1024 rows 844 -> 173 us.  Then, with bytes or pairs of counters instead of
+// words, fp16 without conversion instructions, blocks of one detector together (as in product_route_kernel) and more blocks of fewer
+// warps: 195 -> 174 us; 4 x 256 tokens, 64 detectors of 1024 rows 100 -> 65; 4 x 200, 40 of 512 rows 51 -> 30; 2 x 512, 64 of 256
+// rows 90 -> 79; 1 x 1024 172.
 // --------------------------------------------------------------------------------------------
 constexpr int kHistTile = 4;
 
@@ -126,23 +127,27 @@ struct HistArgs {
 };
 
 // dynamic shared memory of one block, in floats: per warp counters and query operands | key ends | key bits | positional operands
-__host__ __device__ inline size_t hist_warp_floats(int T, bool packed) {
-    return (size_t)kHistTile * T / (packed ? 2 : 1) + kHistTile * kHistAnchors * 3;
+__host__ __device__ inline size_t hist_warp_floats(int T, int per_word) {
+    return (size_t)kHistTile * T / per_word + kHistTile * kHistAnchors * 3;
 }
-__host__ __device__ inline size_t hist_floats(int T, bool packed, int warps, int n_anchors, int pe_cap, int S) {
+__host__ __device__ inline size_t hist_floats(int T, int per_word, int warps, int n_anchors, int pe_cap, int S) {
     const int Sp = (S + 31) & ~31;
-    return warps * hist_warp_floats(T, packed) + (size_t)(n_anchors + 1 + 3 * pe_cap) * Sp;
+    return warps * hist_warp_floats(T, per_word) + (size_t)(n_anchors + 1 + 3 * pe_cap) * Sp;
 }
 
-template <bool PACKED>
+template <int PER>
 __device__ __forceinline__ void count_row(uint32_t *hist, uint32_t li) {
-    if (PACKED) atomicAdd(hist + (li >> 1), 1u << ((li & 1u) * 16u));
-    else atomicAdd(hist + li, 1u);
+    if (PER == 4) atomicAdd(hist + (li >> 2), 1u << ((li & 3u) * 8u));
+    else atomicAdd(hist + (li >> 1), 1u << ((li & 1u) * 16u));
 }
 
-// two 16-bit counts as fp16
+// Two counts below 2048 in the halves of c, as fp16: 1024 + the lower ten bits is 0x6400 with these bits behind it, bit 10 is worth
+// 1024 = 0x6400 = 25 * 0x400 itself; exact.  (A conversion instruction takes eight times as long as these.)
+template <bool TEN_BITS>
 __device__ __forceinline__ uint32_t half_counts(uint32_t c) {
-    const __half2 h = __halves2half2(__ushort2half_rn((unsigned short)(c & 0xffffu)), __ushort2half_rn((unsigned short)(c >> 16)));
+    const uint32_t lower = TEN_BITS ? c | 0x64006400u : (c & 0x03ff03ffu) | 0x64006400u, upper = (c & 0x04000400u) * 25u;
+    __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&lower), __half2half2(__ushort_as_half((unsigned short)0x6400)));
+    if (!TEN_BITS) h = __hadd2(h, *reinterpret_cast<const __half2 *>(&upper));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
@@ -155,10 +160,10 @@ struct HistTile {
 };
 
 // counts the keys of queries j0 .. j0 + nq - 1
-template <int NKQ, bool PE, bool EPS, bool PACKED>
+template <int NKQ, bool PE, bool EPS, int PER>
 __device__ __forceinline__ void count_tile(const HistArgs &p, const AnchorLists &al, const HistTile &h, uint32_t qbits) {
     const int lane = threadIdx.x & 31;
-    const int T = 1 << p.n_anchors, words = PACKED ? T / 2 : T;
+    const int T = 1 << p.n_anchors, words = T / PER;
     for (int i0 = 0; i0 < h.j0 + h.nq - 1; i0 += 32) {
         const int i = i0 + lane;
         float kv[NKQ > 0 ? NKQ : 1];
@@ -185,13 +190,13 @@ __device__ __forceinline__ void count_tile(const HistArgs &p, const AnchorLists 
                         if (above<EPS>(v0, v1, p.cmp_eps)) li |= 1u << al.pe_k[m];
                     }
                 }
-                count_row<PACKED>(h.hist + q * words, li);
+                count_row<PER>(h.hist + q * words, li);
             }
         }
     }
 }
 
-template <int MAXKQ, bool EPS, bool HALF_ROWS, bool PACKED>
+template <int MAXKQ, bool EPS, bool HALF_ROWS, int PER>
 __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ AnchorLists al;
@@ -202,8 +207,8 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
     const int S = p.S, Nc = p.n_anchors, T = 1 << Nc, Sp = (S + 31) & ~31;
     const int j_end = min(S, j_begin + p.queries);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int words = PACKED ? T / 2 : T;
-    const size_t per_warp = hist_warp_floats(T, PACKED);
+    const int words = T / PER;
+    const size_t per_warp = hist_warp_floats(T, PER);
     uint32_t *hist = reinterpret_cast<uint32_t *>(smem + warp * per_warp);          // [kHistTile][words]
     float2 *qv = reinterpret_cast<float2 *>(hist + kHistTile * words);             // [kHistTile][kHistAnchors] (query end, bit)
     float *qd = reinterpret_cast<float *>(qv + kHistTile * kHistAnchors);          // [kHistTile][kHistAnchors]
@@ -282,12 +287,12 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
             }
         }
         h.j0 = j0; h.nq = nq;
-        if (EPS || n_pe > 0) count_tile<MAXKQ, true, EPS, PACKED>(p, al, h, qbits);
-        else if (n_kq <= 2) count_tile<2, false, EPS, PACKED>(p, al, h, qbits);
-        else if (n_kq <= 4) count_tile<4, false, EPS, PACKED>(p, al, h, qbits);
-        else if (n_kq <= 6) count_tile<6, false, EPS, PACKED>(p, al, h, qbits);
-        else if (MAXKQ == 8 || n_kq <= 8) count_tile<8, false, EPS, PACKED>(p, al, h, qbits);
-        else count_tile<MAXKQ, false, EPS, PACKED>(p, al, h, qbits);
+        if (EPS || n_pe > 0) count_tile<MAXKQ, true, EPS, PER>(p, al, h, qbits);
+        else if (n_kq <= 2) count_tile<2, false, EPS, PER>(p, al, h, qbits);
+        else if (n_kq <= 4) count_tile<4, false, EPS, PER>(p, al, h, qbits);
+        else if (n_kq <= 6) count_tile<6, false, EPS, PER>(p, al, h, qbits);
+        else if (MAXKQ == 8 || n_kq <= 8) count_tile<8, false, EPS, PER>(p, al, h, qbits);
+        else count_tile<MAXKQ, false, EPS, PER>(p, al, h, qbits);
         __syncwarp();
         // write out and clear
         __half *out_f = static_cast<__half *>(p.H) + ((size_t)(bl * S + j0) * p.n_detectors + t) * T;
@@ -295,17 +300,18 @@ __global__ void __launch_bounds__(512, 2) product_hist_kernel(const HistArgs p) 
         for (int w = lane; w < nq * (T / 8); w += 32) {
             const int q = w >> (Nc - 3), r = w & (T / 8 - 1);
             uint4 c;   // eight 16-bit counts
-            if (PACKED) {
+            if (PER == 4) {
+                uint2 *cell = reinterpret_cast<uint2 *>(hist) + w;
+                const uint2 u = *cell;
+                *cell = make_uint2(0u, 0u);
+                c = make_uint4(__byte_perm(u.x, 0u, 0x4140), __byte_perm(u.x, 0u, 0x4342), __byte_perm(u.y, 0u, 0x4140), __byte_perm(u.y, 0u, 0x4342));
+            } else {
                 uint4 *cell = reinterpret_cast<uint4 *>(hist) + w;
                 c = *cell;
                 *cell = make_uint4(0u, 0u, 0u, 0u);
-            } else {
-                uint4 *cell = reinterpret_cast<uint4 *>(hist) + 2 * w;
-                const uint4 u = cell[0], v = cell[1];
-                cell[0] = cell[1] = make_uint4(0u, 0u, 0u, 0u);
-                c = make_uint4(u.x | u.y << 16, u.z | u.w << 16, v.x | v.y << 16, v.z | v.w << 16);
             }
-            if (HALF_ROWS) *reinterpret_cast<uint4 *>(out_f + (size_t)q * p.n_detectors * T + r * 8) = make_uint4(half_counts(c.x), half_counts(c.y), half_counts(c.z), half_counts(c.w));
+            constexpr bool kTen = PER == 4;
+            if (HALF_ROWS) *reinterpret_cast<uint4 *>(out_f + (size_t)q * p.n_detectors * T + r * 8) = make_uint4(half_counts<kTen>(c.x), half_counts<kTen>(c.y), half_counts<kTen>(c.z), half_counts<kTen>(c.w));
             else *reinterpret_cast<uint4 *>(out_h + (size_t)w * 8) = c;
         }
         __syncwarp();
@@ -1009,24 +1015,27 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     h.b0 = b0; h.chunk_rows = n * c.S;
     h.S = c.S; h.e1 = c.e1; h.e2 = c.e2; h.npe = cfg->pos_dim;
     h.n_detectors = cfg->n_detectors; h.n_anchors = cfg->n_anchors; h.sliced = cfg->sliced_product; h.cmp_eps = cfg->cmp_eps;
-    const bool packed = T > 512;
-    // warps per block: what puts the most warps on an SM (a wide table's counters leave room for one block only, which then
-    // has to bring them all); very long sequences leave the positional operands in global memory
+    const int per_word = c.S <= 256 ? 4 : 2;
+    // warps per block: what puts the most warps on an SM, of 32 at most (a wide table's counters leave room for one block only, which
+    // then has to bring them all), and with many blocks rather four of 8 warps than two of 16, whose starts overlap less (64
+    // sequences x 128 tokens, 64 detectors of 256 rows 196 -> 174 us; one of 700 tokens, 512 rows, the other way round 164 / 107);
+    // very long sequences leave the positional operands in global memory
     h.queries = queries_per_block(c.S, (int64_t)cfg->n_detectors * n, 0, 0);
+    const bool many = (int64_t)cfg->n_detectors * n * ((c.S + h.queries - 1) / h.queries) * 8 >= 64ll * device_info().sm_count;
     const int tiles = ((c.S < h.queries ? c.S : h.queries) + kHistTile - 1) / kHistTile;
     int warps = 0;
     for (int cap = staged_pe_anchors(cfg);; cap = 0) {
         int most = 0;
         for (int w = 16; w >= 1; w /= 2) {
-            const size_t need = hist_floats(T, packed, w, cfg->n_anchors, cap, c.S) * 4 + 1024;
-            const int resident = w * (int)((size_t)kMaxSmemPerBlock / need);
-            if (resident > most && (w <= tiles || w == 1)) { most = resident; warps = w; }
+            const size_t need = hist_floats(T, per_word, w, cfg->n_anchors, cap, c.S) * 4 + 1024;
+            const int resident = min(32, w * (int)((size_t)kMaxSmemPerBlock / need));
+            if ((resident > most || (resident == most && many && w == 8)) && (w <= tiles || w == 1)) { most = resident; warps = w; }
         }
         h.pe_cap = cap;
         if (most >= 4 || cap == 0) break;
     }
     LUTB_REQUIRE(warps > 0, LUTB_ERR_SHAPE, "product histogram path: sequence too long");
-    const size_t smem = hist_floats(T, packed, warps, cfg->n_anchors, h.pe_cap, c.S) * 4;
+    const size_t smem = hist_floats(T, per_word, warps, cfg->n_anchors, h.pe_cap, c.S) * 4;
     h.sequences = (int)n;
     LUTB_REQUIRE(cfg->n_detectors * n <= 0x7FFFFFFF, LUTB_ERR_SHAPE, "product histogram path: too many blocks for one launch");
     const dim3 grid((unsigned)(cfg->n_detectors * n), (unsigned)((c.S + h.queries - 1) / h.queries));
@@ -1039,9 +1048,12 @@ static int launch_hist(const ProductCall &c, const HistPlan &p, int64_t b0, int6
     const bool eps = cfg->cmp_eps != 0.f;
     auto pick = [&](auto f32) -> int {
         constexpr bool F = decltype(f32)::value;
-        if (cfg->n_anchors <= 8) return eps ? launch(product_hist_kernel<8, true, F, false>) : launch(product_hist_kernel<8, false, F, false>);
-        if (!packed) return eps ? launch(product_hist_kernel<12, true, F, false>) : launch(product_hist_kernel<12, false, F, false>);
-        return eps ? launch(product_hist_kernel<12, true, F, true>) : launch(product_hist_kernel<12, false, F, true>);
+        auto width = [&](auto per) -> int {
+            constexpr int P = decltype(per)::value;
+            if (cfg->n_anchors <= 8) return eps ? launch(product_hist_kernel<8, true, F, P>) : launch(product_hist_kernel<8, false, F, P>);
+            return eps ? launch(product_hist_kernel<12, true, F, P>) : launch(product_hist_kernel<12, false, F, P>);
+        };
+        return per_word == 4 ? width(std::integral_constant<int, 4>{}) : width(std::integral_constant<int, 2>{});
     };
     const int rc = p.tc ? pick(std::true_type{}) : pick(std::false_type{});
     if (rc) return rc;
