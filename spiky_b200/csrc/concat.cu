@@ -192,8 +192,13 @@ __global__ void __launch_bounds__(256) concat_forward_fixed_kernel(const float *
 // reductions per touched cell at the end instead of two per pair (S * nc cells against S * (S - 1) / 2 pairs); without
 // it (sequences whose cells do not fit) every pair issues its own.
 // --------------------------------------------------------------------------------------------
-template <int LG, int VEC, bool DO_DX, bool DO_DW>
-__global__ void __launch_bounds__(256) concat_backward_kernel(const float *__restrict__ W, const float *__restrict__ dY,
+// ONE: rows of one step (n_outputs <= LG * VEC).  The two queries' rows of dY are then loaded once per pair of queries and chosen by
+// a bit, and the pairs whose positional margin is the smallest (about a quarter) have a loop of their own behind the others', which
+// leaves registers for three blocks an SM instead of two.  Bound: the latency and rate of random rows from HBM.  Measured with and
+// without: 32 x 32 tokens, 64 detectors of 65536 rows x 32 outputs, input gradient 97 -> 87 us, with the table gradient 149 -> 109;
+// 16 x 32 tokens, 32 detectors of 16384 rows x 64 outputs 67 -> 55; 8 x 33 tokens x 10 outputs 46 -> 31.
+template <int LG, int VEC, bool DO_DX, bool DO_DW, bool ONE>
+__global__ void __launch_bounds__(256, !ONE || LG == 32 ? 1 : LG == 16 ? 2 : 3) concat_backward_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                              const int2 *__restrict__ anchors,
                                                              const int32_t *__restrict__ idx,
                                                              const float *__restrict__ min_delta,
@@ -237,6 +242,24 @@ __global__ void __launch_bounds__(256) concat_backward_kernel(const float *__res
     for (int r = warp; 2 * r < j_end - j_begin; r += nwarps) {
         const int ja = j_end - 1 - r, jb = j_begin + r;
         const int count = ja + (jb != ja ? jb : 0);   // (the middle query of an odd number is alone)
+        float da[VEC], db[VEC], ua[VEC], ub[VEC];     // ONE: this lane's columns of dY of both queries; as the table gradient takes them
+        bool add_a = false, add_b = false;
+        if constexpr (ONE) {
+            load_row<VEC>(dYb + (size_t)ja * n_outputs + q * VEC, q * VEC < n_outputs, da);
+            load_row<VEC>(dYb + (size_t)jb * n_outputs + q * VEC, q * VEC < n_outputs, db);
+            if (DO_DW) {
+                auto scaled = [&](const float (&d)[VEC], float (&up)[VEC], bool &add) {
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) {
+                        up[e] = lr != 1.0 ? (float)((double)d[e] * lr) : d[e];   // lr == 1: dY itself
+                        up[e] = fabsf(d[e]) > kEpsF ? up[e] : 0.f;
+                    }
+                    add = q * VEC < n_outputs && (VEC == 4 || fabsf(d[0]) > kEpsF);
+                };
+                scaled(da, ua, add_a);
+                scaled(db, ub, add_b);
+            }
+        }
         for (int p0 = 0; p0 < count; p0 += 32) {
             // this lane's pair; my_j < 0: none
             int my_j = -1, my_i = 0, my_flip = 0, my_pos = 0;
@@ -263,58 +286,100 @@ __global__ void __launch_bounds__(256) concat_backward_kernel(const float *__res
             }
             const unsigned pe_mask = DO_DX ? __ballot_sync(0xffffffffu, my_pe) : 0u;
             float v[LG], vp[LG];
+            if constexpr (ONE) {
+                // pairs of the longer query come first, so that one number tells the query, and one whether there is a pair
+                const bool in_row = q * VEC < n_outputs;
+                const int col = q * VEC;
 #pragma unroll
-            for (int i0 = 0; i0 < LG; i0 += U) {
+                for (int i0 = 0; i0 < LG; i0 += U) {
 #pragma unroll
-                for (int u = 0; u < U; u++) { v[i0 + u] = 0.f; vp[i0 + u] = 0.f; }
-                if (p0 + i0 >= count) continue;   // (warp uniform; group 0 holds the first pairs)
-                uint32_t r0[U], r1[U], r2[U];
-                int jj[U];
-                bool pe[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int src = g * LG + i0 + u;
-                    r0[u] = __shfl_sync(0xffffffffu, my_row, src);
-                    jj[u] = __shfl_sync(0xffffffffu, my_j, src);
-                    pe[u] = (pe_mask >> src) & 1u;
-                    if (DO_DX) {
-                        r1[u] = __shfl_sync(0xffffffffu, my_alt, src);
-                        r2[u] = pe_mask ? __shfl_sync(0xffffffffu, my_palt, src) : 0u;
-                    }
-                }
-                for (int c0 = 0; c0 < n_outputs; c0 += LG * VEC) {
-                    const int col = c0 + q * VEC;
-                    float d[U][VEC], a[U][VEC], c[U][VEC], e2[U][VEC];
+                    for (int u = 0; u < U; u++) v[i0 + u] = 0.f;
+                    if (p0 + i0 >= count) continue;   // (warp uniform; group 0 holds the first pairs)
+                    uint32_t r0[U];
+                    float a[U][VEC], c[U][VEC];
 #pragma unroll
                     for (int u = 0; u < U; u++) {
-                        const bool on = jj[u] >= 0 && col < n_outputs;
-                        load_row<VEC>(dYb + (size_t)max(jj[u], 0) * n_outputs + col, on, d[u]);
+                        const int src = g * LG + i0 + u;
+                        r0[u] = __shfl_sync(0xffffffffu, my_row, src);
                         if (DO_DX) {
+                            const uint32_t r1 = __shfl_sync(0xffffffffu, my_alt, src);
+                            const bool on = in_row && p0 + src < count;
                             load_row<VEC>(Wt + (size_t)r0[u] * n_outputs + col, on, a[u]);
-                            load_row<VEC>(Wt + (size_t)r1[u] * n_outputs + col, on, c[u]);
-                            load_row<VEC>(Wt + (size_t)r2[u] * n_outputs + col, on && pe[u], e2[u]);
+                            load_row<VEC>(Wt + (size_t)r1 * n_outputs + col, on, c[u]);
                         }
                     }
 #pragma unroll
                     for (int u = 0; u < U; u++) {
+                        const int pair = p0 + g * LG + i0 + u;
+                        const bool first = pair < ja;
                         if (DO_DX) {
-                            float s0 = 0.f, s1 = 0.f;
+                            float s0 = 0.f;
 #pragma unroll
-                            for (int e = 0; e < VEC; e++) {
-                                s0 = fmaf(d[u][e], a[u][e] - c[u][e], s0);
-                                s1 = fmaf(d[u][e], a[u][e] - e2[u][e], s1);
-                            }
-                            v[i0 + u] += s0;
-                            vp[i0 + u] += s1;
+                            for (int e = 0; e < VEC; e++) s0 = fmaf(first ? da[e] : db[e], a[u][e] - c[u][e], s0);
+                            v[i0 + u] = s0;
                         }
-                        if (DO_DW && jj[u] >= 0 && col < n_outputs) {
+                        if (DO_DW && pair < count && (first ? add_a : add_b)) {
                             float up[VEC];
 #pragma unroll
-                            for (int e = 0; e < VEC; e++) {
-                                up[e] = lr != 1.0 ? (float)((double)d[u][e] * lr) : d[u][e];   // lr == 1: dY itself
-                                up[e] = fabsf(d[u][e]) > kEpsF ? up[e] : 0.f;
+                            for (int e = 0; e < VEC; e++) up[e] = first ? ua[e] : ub[e];
+                            red_row<VEC>(Tt + (size_t)r0[u] * n_outputs + col, up);
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i0 = 0; i0 < LG; i0 += U) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) { v[i0 + u] = 0.f; vp[i0 + u] = 0.f; }
+                    if (p0 + i0 >= count) continue;   // (warp uniform; group 0 holds the first pairs)
+                    uint32_t r0[U], r1[U], r2[U];
+                    int jj[U];
+                    bool pe[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int src = g * LG + i0 + u;
+                        r0[u] = __shfl_sync(0xffffffffu, my_row, src);
+                        jj[u] = __shfl_sync(0xffffffffu, my_j, src);
+                        pe[u] = (pe_mask >> src) & 1u;
+                        if (DO_DX) {
+                            r1[u] = __shfl_sync(0xffffffffu, my_alt, src);
+                            r2[u] = pe_mask ? __shfl_sync(0xffffffffu, my_palt, src) : 0u;
+                        }
+                    }
+                    for (int c0 = 0; c0 < n_outputs; c0 += LG * VEC) {
+                        const int col = c0 + q * VEC;
+                        float d[U][VEC], a[U][VEC], c[U][VEC], e2[U][VEC];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const bool on = jj[u] >= 0 && col < n_outputs;
+                            load_row<VEC>(dYb + (size_t)max(jj[u], 0) * n_outputs + col, on, d[u]);
+                            if (DO_DX) {
+                                load_row<VEC>(Wt + (size_t)r0[u] * n_outputs + col, on, a[u]);
+                                load_row<VEC>(Wt + (size_t)r1[u] * n_outputs + col, on, c[u]);
+                                load_row<VEC>(Wt + (size_t)r2[u] * n_outputs + col, on && pe[u], e2[u]);
                             }
-                            if (VEC == 4 || fabsf(d[u][0]) > kEpsF) red_row<VEC>(Tt + (size_t)r0[u] * n_outputs + col, up);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            if (DO_DX) {
+                                float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+                                for (int e = 0; e < VEC; e++) {
+                                    s0 = fmaf(d[u][e], a[u][e] - c[u][e], s0);
+                                    s1 = fmaf(d[u][e], a[u][e] - e2[u][e], s1);
+                                }
+                                v[i0 + u] += s0;
+                                vp[i0 + u] += s1;
+                            }
+                            if (DO_DW && jj[u] >= 0 && col < n_outputs) {
+                                float up[VEC];
+#pragma unroll
+                                for (int e = 0; e < VEC; e++) {
+                                    up[e] = lr != 1.0 ? (float)((double)d[u][e] * lr) : d[u][e];   // lr == 1: dY itself
+                                    up[e] = fabsf(d[u][e]) > kEpsF ? up[e] : 0.f;
+                                }
+                                if (VEC == 4 || fabsf(d[u][0]) > kEpsF) red_row<VEC>(Tt + (size_t)r0[u] * n_outputs + col, up);
+                            }
                         }
                     }
                 }
@@ -331,6 +396,29 @@ __global__ void __launch_bounds__(256) concat_backward_kernel(const float *__res
                 }
             }
             if (pe_mask) {
+                if constexpr (ONE) {
+#pragma unroll
+                    for (int i0 = 0; i0 < LG; i0 += U) {
+#pragma unroll
+                        for (int u = 0; u < U; u++) vp[i0 + u] = 0.f;
+                        if (p0 + i0 >= count) continue;
+                        float a[U][VEC], c[U][VEC];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const int src = g * LG + i0 + u;
+                            const uint32_t r0 = __shfl_sync(0xffffffffu, my_row, src), r2 = __shfl_sync(0xffffffffu, my_palt, src);
+                            const bool on = q * VEC < n_outputs && ((pe_mask >> src) & 1u);
+                            load_row<VEC>(Wt + (size_t)r0 * n_outputs + q * VEC, on, a[u]);
+                            load_row<VEC>(Wt + (size_t)r2 * n_outputs + q * VEC, on, c[u]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const bool first = p0 + g * LG + i0 + u < ja;
+#pragma unroll
+                            for (int e = 0; e < VEC; e++) vp[i0 + u] = fmaf(first ? da[e] : db[e], a[u][e] - c[u][e], vp[i0 + u]);
+                        }
+                    }
+                }
 #pragma unroll
                 for (int o = LG / 2; o >= 1; o >>= 1) {
                     const bool upper = (q & o) != 0;
@@ -688,7 +776,13 @@ static int launch_concat_pairs_backward(const lutb_layer_cfg *cfg, int64_t batch
             const int n = (int)min(per, batch - b0);
             const int64_t tok = b0 * S;
             const int rc = dispatch_pair_kernel(vec4, O, [&](auto lg, auto vec) -> int {
-                auto kern = concat_backward_kernel<lg.value, vec.value, DX, DWF>;
+                constexpr int L = decltype(lg)::value, V = decltype(vec)::value;
+                auto kern = concat_backward_kernel<L, V, DX, DWF, false>;
+                // (rows of one step; 32 lanes with vectors would spill: 128 outputs 74 us against 54.  Fewer blocks than SMs: the
+                // second loop's latency counts instead, 1 x 32 tokens 18 us against 13)
+                if constexpr (L <= 16 || V == 1) {
+                    if (O <= L * V && (int64_t)Nt * n >= device_info().sm_count) kern = concat_backward_kernel<L, V, DX, DWF, true>;
+                }
                 if (smem > kPlainSmem) LUTB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 kern<<<(unsigned)((int64_t)Nt * n), threads, smem, st>>>(
                     weights, dY + tok * O, an, idx + tok * Nt, min_delta + tok * Nt, min_k + tok * Nt, pos_idx, pos_min_delta, pos_min_k,
