@@ -712,20 +712,21 @@ int launch_fc_gather_forward(const float *W, const int32_t *idx, float *y, int64
 // Bound: the latency of the row reads and load/store wavefronts (half of their peak at 65536 samples x 64 detectors of 64 rows x 32
 // outputs).  Measured (one detector a group in flight, a full reduction per detector before), with the clearing of dX:
 // 256 samples 10.9 -> 8.6 us; 1111 samples, 50 detectors, 33 outputs 32.0 -> 14.8 us; 512 samples, 64 detectors, 10 outputs
-// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.5 us; 65536 samples 187 -> 167 us, and 117 as said at ONE below.
+// 18.8 -> 8.7 us; 8192 samples, 16 detectors, 256 outputs 33.4 -> 28.5 us; 65536 samples 187 -> 167 us, and 109 as said at ONE below.
 // (Walking groups of detectors whose tables fit L1 measured 220 us there: the groups leave lanes idle.)
 // --------------------------------------------------------------------------------------------
 // WRITE: dX is written instead of added to (and need not be cleared): the warp sums its sample's row in shared memory and
 // writes it out once.
-// Blocks an SM: 8 lanes a group with vector loads need 80 registers for two detectors in flight (at 64 they spilled: 65536 samples,
-// 64 detectors of 64 rows x 32 outputs 187 -> 167 us, 5000 samples 23 -> 19).
+// Blocks an SM: rows of one step four, from 16 lanes a group on three (115 us with three for the layer of 65536 samples above, 109 with
+// four, 5000 samples 12.8 and 13.2; 20000 samples, 50 detectors of 128 rows x 64 outputs 58 with two, 47 with three; 16384 samples x 128 outputs
+// 44 and 38), others two (8192 samples x 256 outputs 28 with two, 34 with three: spills).
 // ONE: rows of one step (n_outputs <= LG * VEC).  A lane then has one fp32 product sum per detector, which the first exchange
 // takes as it is; lanes without a column and detectors without an anchor to flip read the first column and one row twice (nobody
 // takes what comes out), so that the loads need no predicates and four detectors are in flight; addresses are row numbers times the
-// row's bytes.  65536 samples 167 -> 117 us, 256 samples 7.4 -> 5.2.  (The same for rows of several steps spilled registers and
+// row's bytes.  65536 samples 167 -> 109 us, 256 samples 7.4 -> 5.3.  (The same for rows of several steps spilled registers and
 // gained nothing.)
 template <int LG, int VEC, bool WRITE, bool ONE>
-__global__ void __launch_bounds__(256, LG >= 16 ? 2 : LG == 8 && VEC == 4 ? 3 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
+__global__ void __launch_bounds__(256, !ONE ? 2 : LG >= 16 ? 3 : 4) fc_input_grad_kernel(const float *__restrict__ W, const float *__restrict__ dY,
                                                            const int2 *__restrict__ anchors,
                                                            const int32_t *__restrict__ idx,
                                                            const float *__restrict__ min_delta,
