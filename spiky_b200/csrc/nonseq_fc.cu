@@ -508,8 +508,12 @@ __global__ void __launch_bounds__(256) fc_gather_forward_fixed_kernel(const floa
 // Forward gather for fp32 accumulators and 16-byte aligned rows: one warp per (sample, chunk of LG float4 columns); the row
 // loads of up to 16 detectors per lane are all issued before the first one is consumed, which is what hides the latency of the
 // (random) row reads.
+// Blocks an SM named for the groups of 4, 16 and 32 lanes: without it the compiler does not issue all row loads first (20000 samples, 50
+// detectors x 64 outputs 30 -> 19 us, x 16 11.5 -> 10.1; 16384 samples, 32 detectors x 128 outputs 17.8 -> 15.9; 256 samples, 64 detectors x 64 outputs
+// 7.6 -> 3.9; four or six instead of five are within 5 % there); the others are best left alone (65536 samples, 64 detectors x 32 outputs 41.3
+// against 42.2 to 46.8).
 template <int LG>
-__global__ void __launch_bounds__(256) fc_gather_forward_vec_kernel(const float *__restrict__ W,
+__global__ void __launch_bounds__(256, LG == 4 || LG >= 16 ? 5 : 0) fc_gather_forward_vec_kernel(const float *__restrict__ W,
                                                                    const int32_t *__restrict__ idx,
                                                                    float *__restrict__ y, int64_t batch, int n_outputs,
                                                                    int n_detectors, int table_rows, int t0, int t1) {
