@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(128) anchor_plan_kernel(const int2 *__restrict
 // PLAN (evaluation only): the anchors come from a list of one word each that anchor_plan_kernel has put in an order in which the
 // four detectors of a wavefront collide less (1.5 times instead of 2.1 with random anchors), four anchors a load instead of
 // two, and with the addresses worked out.  The order of the comparisons does not matter to the indices.  EPS: there is a dead band;
-// without one the sign of a difference is the answer.  16384 rows x 4096 inputs, 4096 detectors of 8 anchors:
+// without one the sign bit of minus the difference, which is never -0, is the answer.  16384 rows x 4096 inputs, 4096 detectors of 8 anchors:
 // 445 -> 319 us (list and collisions 445 -> 367, addresses and signs 367 -> 319).
 template <int R, int D, bool TRAIN, bool PLAN, bool EPS = true>
 __global__ void __launch_bounds__(D == 2 ? 1024 : 256) check_detectors_kernel(const float *__restrict__ x, int64_t rows, int n_inputs,
@@ -226,10 +226,11 @@ __global__ void __launch_bounds__(D == 2 ? 1024 : 256) check_detectors_kernel(co
                     const float4 b = *reinterpret_cast<const float4 *>(rows4 + (((e >> 10) & 0x3fff0u) ^ which));
                     const uint32_t bit = 1u << ((e >> 28) & 7u);
                     // minus the anchor's difference: second input less first, or the reverse where they are swapped (one rounding, as
-                    // a subtraction; a sum that is not a number has a clear sign bit)
+                    // a subtraction; a sum that is not a number has a clear sign bit).  The zero turns -0 into +0, so that a
+                    // difference of two zeros is +0 whatever their signs.
                     const float f = __uint_as_float((e & 0x80000000u) | 0x3f800000u);
-                    const float d[4] = {__fmaf_rn(-f, a.x, __fmul_rn(f, b.x)), __fmaf_rn(-f, a.y, __fmul_rn(f, b.y)),
-                                        __fmaf_rn(-f, a.z, __fmul_rn(f, b.z)), __fmaf_rn(-f, a.w, __fmul_rn(f, b.w))};
+                    const float d[4] = {__fmaf_rn(-f, a.x, __fmaf_rn(f, b.x, 0.f)), __fmaf_rn(-f, a.y, __fmaf_rn(f, b.y, 0.f)),
+                                        __fmaf_rn(-f, a.z, __fmaf_rn(f, b.z, 0.f)), __fmaf_rn(-f, a.w, __fmaf_rn(f, b.w, 0.f))};
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         if constexpr (EPS) {

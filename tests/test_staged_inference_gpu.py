@@ -52,6 +52,35 @@ def test_ordered_anchor_lists_give_the_same_indices(shape, eps):
     assert (y[rows] - want).abs().max() <= 16 * 2.0 ** -24 * want.abs().max() * 12
 
 
+# rows on both sides of where the lists start to be used
+@pytest.mark.parametrize("rows", [1000, 1184, 1301])
+@pytest.mark.parametrize("eps", [0.0, 0.4])
+@pytest.mark.parametrize("tables", ["fp32", "int8"])
+def test_zeros_of_both_signs_are_equal(tables, eps, rows):
+    """Anchors over inputs that are +0, -0 or a number on either end (the lists may swap the ends): a pair of zeros sets no bit,
+    and the same row has the same indices in any batch."""
+    from spiky_b200.inference import LUTInference
+
+    I, Nt, Nc, O = 48, 1030, 8, 40   # (int8 lists need rows of eight)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    values = torch.tensor([0.0, -0.0, 0.0, -0.0, 0.75, -0.75], device="cuda")
+    x = values[torch.randint(0, 6, (rows, I), device="cuda", generator=g)]
+    x[::7] = 0.0
+    x[::7, ::2] = -0.0
+    anchors = torch.randint(0, I, (Nt, Nc, 2), device="cuda", generator=g, dtype=torch.int32)
+    W = torch.randn(Nt * (1 << Nc) * O, device="cuda", generator=g)
+    if tables == "int8":
+        layer = LUTInference(I, O, Nt, Nc, anchors, (W * 40).clamp(-128, 127).to(torch.int8), torch.ones(Nt, device="cuda"), cmp_eps=eps)
+    else:
+        layer = LUTInference(I, O, Nt, Nc, anchors, W, cmp_eps=eps)
+    layer(x)
+    idx = layer.last_indices.clone()
+    assert torch.equal(idx, row_indices(x, anchors, Nc, np.float32(eps).item()))
+    assert not idx[::7].any()
+    layer(x[:300])
+    assert torch.equal(layer.last_indices, idx[:300])
+
+
 @pytest.mark.parametrize("block", [1, 2, 5, 32, 255, 1024])
 @pytest.mark.parametrize("spread", ["none", "some", "all"])
 def test_int8_sums_of_detector_pairs(block, spread):
