@@ -266,8 +266,17 @@ PyObject *ident(const Tensor &t) {
 }
 PyObject *histogram_key(const Call &c, int64_t B, const Tensor &x, const Tensor &pe, double eps, int variant) {
     Ref ix(ident(x)), ia(ident(c.anchors)), ip(ident(pe));
-    return Py_BuildValue("(LLOOOOLLOdi)", (long long)B, (long long)c.S, ix.get(), ix.get(), ia.get(), ip.get(), (long long)(x.numel() / (B * c.S)),
-                         (long long)(x.numel() / (B * c.S)), c.cfg.sliced_product ? Py_True : Py_False, eps, variant);
+    return Py_BuildValue("(LLOOOOLLOdiK)", (long long)B, (long long)c.S, ix.get(), ix.get(), ia.get(), ip.get(), (long long)(x.numel() / (B * c.S)),
+                         (long long)(x.numel() / (B * c.S)), c.cfg.sliced_product ? Py_True : Py_False, eps, variant,
+                         (unsigned long long)(uintptr_t)stream_of(c));
+}
+// What the manager's _kept_histogram holds: (workspace, key, what was counted).  The memory the key names stays taken as long as the
+// key can be found, so that no other call's inputs can lie there.
+PyObject *kept_entry(const Call &c, const Tensor &workspace, PyObject *key, const Tensor &x, const Tensor &pe) {
+    Ref t(THPVariable_Wrap(workspace)), tx(THPVariable_Wrap(x.detach())), ta(THPVariable_Wrap(c.anchors.detach())),
+        tp(pe.defined() ? THPVariable_Wrap(pe.detach()) : Py_NewRef(Py_None));
+    if (!t || !tx || !ta || !tp) return nullptr;
+    return Py_BuildValue("(OO(OOOO))", t.get(), key, tx.get(), tx.get(), ta.get(), tp.get());
 }
 double context_eps(const Call &c) {
     return PyFloat_AsDouble(item(instance_dict(item(c.dict, names.shared_context)), names.cmp_eps));
@@ -470,7 +479,7 @@ variable_list LayerNode::apply(variable_list &&grads) {
     PyDict_SetItem(c.dm_dict, names.dm_kept, Py_None);
     Tensor ws;
     int flags = 0;
-    if (kept && PyTuple_Check(kept.get()) && PyTuple_GET_SIZE(kept.get()) == 2) {
+    if (kept && PyTuple_Check(kept.get()) && PyTuple_GET_SIZE(kept.get()) == 3) {
         Ref key(histogram_key(c, B, xc, pe, context_eps(c), variant));
         const int same = key ? PyObject_RichCompareBool(PyTuple_GET_ITEM(kept.get(), 1), key.get(), Py_EQ) : -1;
         if (same < 0) raise_current();
@@ -581,10 +590,10 @@ PyObject *apply(PyObject *x_obj, PyObject *layer) {
                 if (want > 0 && (int64_t)want <= class_int(names.keep_limit)) {
                     const Tensor own = at::empty({(int64_t)want}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, c.device));
                     if (lib.product_keeps_histogram(&c.cfg, B, (int32_t)S, (int32_t)inputs, (int32_t)inputs, variant, own.data_ptr(), want)) {
-                        Ref key(histogram_key(c, B, xc, pe, context_eps(c), variant)), t(THPVariable_Wrap(own));
-                        Ref pair(key && t ? PyTuple_Pack(2, t.get(), key.get()) : nullptr);
-                        if (!pair) raise_current();
-                        PyDict_SetItem(c.dm_dict, names.dm_kept, pair.get());
+                        Ref key(histogram_key(c, B, xc, pe, context_eps(c), variant));
+                        Ref entry(key ? kept_entry(c, own, key.get(), xc, pe) : nullptr);
+                        if (!entry) raise_current();
+                        PyDict_SetItem(c.dm_dict, names.dm_kept, entry.get());
                         ws = own;
                         flags = LUTB_PRODUCT_KEEP_HIST;
                     }

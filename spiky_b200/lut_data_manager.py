@@ -491,9 +491,10 @@ class _LUTDataManager:
                     if L.lutb_product_keeps_histogram(ctypes.byref(cfg), B, S, int(n_inputs_1), int(n_inputs_2),
                                                       int(variant), _ptr(own), want):
                         ws, ws_bytes, flags = own, want, _native.PRODUCT_KEEP_HIST
+                        read = (r_input_1, r_input_2, r_detector_anchors, r_positional_embeddings)
                         self._kept_histogram = (own, self._histogram_key(
-                            B, S, r_input_1, r_input_2, r_detector_anchors, r_positional_embeddings, n_inputs_1,
-                            n_inputs_2, sliced_mode, cmp_eps, variant))
+                            B, S, *read, n_inputs_1, n_inputs_2, sliced_mode, cmp_eps, variant, self._stream()),
+                            tuple(None if t is None else t.detach() for t in read))
             rc = _native.lib().lutb_product_forward(
                 ctypes.byref(cfg), B, S, _ptr(r_weights), _ptr(r_input_1), _ptr(r_input_2), int(n_inputs_1),
                 int(n_inputs_2), _ptr(r_positional_embeddings), _ptr(r_detector_anchors), _ptr(w_output),
@@ -501,17 +502,21 @@ class _LUTDataManager:
         _native.check(rc)
         self._forward_seen = True
 
+    # (workspace, key, what was counted) of the last forward pass that left its histogram.  The key names the inputs by their
+    # address, so the entry keeps their memory (detached: the graph behind them is not kept): no other call's inputs, temporary
+    # copies of strided ones among them, can come to lie there meanwhile.
     _kept_histogram = None
     # largest workspace a forward pass may hold on to until its backward pass (per layer)
     product_keep_limit = 2 << 30
 
     @staticmethod
-    def _histogram_key(B, S, x1, x2, anchors, pe, e1, e2, sliced, cmp_eps, variant):
-        """What the row histogram depends on: the inputs (storage and version), anchors, embeddings and geometry."""
+    def _histogram_key(B, S, x1, x2, anchors, pe, e1, e2, sliced, cmp_eps, variant, stream):
+        """What the row histogram depends on: the inputs (storage and version), anchors, embeddings and geometry; and the
+        stream on which it was counted."""
         def ident(t):
             return None if t is None else (t.data_ptr(), t._version, t.numel())
         return (B, S, ident(x1), ident(x2), ident(anchors), ident(pe), int(e1), int(e2), bool(sliced), float(cmp_eps),
-                int(variant))
+                int(variant), int(stream))
 
     def backward_backprop_product(self, r_weights, batch_size, sequence_length, r_input_1, r_input_2,
                                   r_detector_anchors, r_output_gradients, w_input_gradients_1, w_input_gradients_2,
@@ -547,7 +552,7 @@ class _LUTDataManager:
             ws, ws_bytes = self._product_workspace(cfg, B, S, True, variant, r_weights.device)
             if kept is not None and kept[1] == self._histogram_key(
                     B, S, r_input_1, r_input_2, r_detector_anchors, r_positional_embeddings, n_inputs_1, n_inputs_2,
-                    sliced_mode, cmp_eps, variant):
+                    sliced_mode, cmp_eps, variant, self._stream()):
                 # the forward pass over these very inputs left its histogram in this workspace
                 ws, ws_bytes, variant = kept[0], kept[0].numel(), int(variant) | _native.PRODUCT_REUSE_HIST
             rc = _native.lib().lutb_product_backward(

@@ -1,5 +1,8 @@
 """The native host side of layer calls (host/layer_calls.cpp) against the Python route, which an instance attribute that
 replaces one of the layer's methods selects."""
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -162,3 +165,58 @@ def test_product_histogram_crosses_between_the_routes():
         want = want or got
         for u, v in zip(got, want):
             close(u, v)
+
+
+@pytest.mark.parametrize("route", [lambda layer: layer, python_route], ids=["native", "python"])
+@pytest.mark.parametrize("way", ["strided", "offloaded", "other_stream"])
+def test_a_kept_histogram_is_of_its_own_call(route, way):
+    """Two forward passes, then the backward pass of the first one: the histogram that the second left is of other inputs, also where
+    the inputs that a pass reads are copies whose memory is free again after it."""
+    xs = [make("product")[1], make("product", seed=4)[1]]
+    dy = torch.linspace(-1.0, 1.0, 3 * 9 * 12, device="cuda").view(3, 9, 12)
+
+    def graph(layer, x):
+        if way == "strided":
+            wide = torch.empty(3, 9, 40, device="cuda")
+            wide[..., ::2] = x
+            return layer(wide[..., ::2].requires_grad_())
+        if way == "offloaded":   # what comes back lies wherever there is room
+            with torch.autograd.graph.save_on_cpu():
+                return layer(x.clone().requires_grad_())
+        return layer(x.clone().requires_grad_())
+
+    want = route(make("product")[0])
+    graph(want, xs[0]).backward(dy)
+    layer = route(make("product")[0])
+    y = graph(layer, xs[0])
+    if way == "other_stream":
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            graph(layer, xs[0])
+        torch.cuda.current_stream().wait_stream(s)
+    else:
+        with torch.no_grad():
+            graph(layer, xs[1])
+    y.backward(dy)
+    close(layer._weights.grad, want._weights.grad)
+    close(layer._positional_embeddings.grad, want._positional_embeddings.grad)
+    assert layer._lut_dm._kept_histogram is None   # and nothing of the inputs is kept after it
+
+
+def test_a_kept_histogram_keeps_no_graph():
+    layer, x, gen = make("product")
+    for route in (layer, python_route(make("product")[0])):
+        class Mark(torch.autograd.Function):
+            @staticmethod
+            def forward(ctx, x, mark):
+                ctx.mark = mark
+                return x.clone()
+
+        mark = type("Mark", (), {})()
+        alive = weakref.ref(mark)
+        y = route(Mark.apply(x.clone().requires_grad_(), mark))
+        assert route._lut_dm._kept_histogram is not None
+        del y, mark
+        gc.collect()
+        assert alive() is None
