@@ -182,7 +182,8 @@ def layer_calls():
             ["_lookup_indices_callback", "_table_forward_hook", "_table_update_hook", "_table_gradient_sink"],
             ["forward_step", "backward_backprop", "forward_step_concat", "backward_backprop_concat",
              "forward_step_product", "backward_backprop_product", "_cfg", "_stream", "_require_cuda", "_expect",
-             "_sparse_forward", "_sparse_backward", "table_gradient_rows", "table_gradient_cells", "_product_workspace", "_histogram_key", "get_weights_dimension"])
+             "_sparse_forward", "_sparse_backward", "table_gradient_rows", "table_gradient_cells", "_product_workspace",
+             "_product_scratch_bytes", "_histogram_key", "get_weights_dimension"])
         _layer_calls = module
     return _layer_calls
 

@@ -55,8 +55,7 @@ struct Names {
     PyObject *dict_parameters, *dict_buffers, *weights, *anchors, *positional, *training, *dm, *shared_context, *cmp_eps, *device, *policy,
         *type, *normalized, *sequence_length, *concatenation, *sliced, *positional_dim, *unified, *fully_connected, *dw_variant,
         *product_variant, *sparse_rows_direct, *dm_device, *dm_fully_connected, *dm_sparse, *dm_seq_len, *dm_forward_seen, *dm_kept, *n_weights,
-        *rows_per_detector, *cfg, *c_struct, *input_shape, *output_shape, *prepare_positional, *external_lr, *scratch, *scratch_limit, *keep_limit,
-        *product_ws;
+        *rows_per_detector, *cfg, *c_struct, *input_shape, *output_shape, *prepare_positional, *external_lr, *scratch_limit, *keep_limit;
 };
 Names names;
 PyObject *manager_class, *manager_base, *tensor_class, *parameter_class, *policy_dense, *policy_internal, *policy_sparse, *check_status, *layer_class;
@@ -282,25 +281,15 @@ double context_eps(const Call &c) {
     return PyFloat_AsDouble(item(instance_dict(item(c.dict, names.shared_context)), names.cmp_eps));
 }
 
-// the manager's shared scratch (its _product_workspace, which is called where the buffer has to grow)
-Tensor product_scratch(const Call &c, int64_t B, bool backward, int variant) {
+// bytes of scratch of one call, as the manager's _product_scratch_bytes has them; 0: none
+size_t product_scratch_bytes(const Call &c, int64_t B, bool backward, int variant) {
     const int64_t rows = (int64_t)1 << c.cfg.n_anchors;
-    if (variant == LUTB_PRODUCT_DIRECT || c.S < 2 || (variant == LUTB_PRODUCT_AUTO && 4 * c.S < rows)) return Tensor();
+    if (variant == LUTB_PRODUCT_DIRECT || c.S < 2 || (variant == LUTB_PRODUCT_AUTO && 4 * c.S < rows)) return 0;
     const size_t one = lib.product_workspace(&c.cfg, 1, (int32_t)c.S, backward), all = lib.product_workspace(&c.cfg, B, (int32_t)c.S, backward);
-    const size_t most = std::max(one, (size_t)std::max<int64_t>(0, class_int(names.scratch_limit))), want = std::min(all, most);
-    Ref dict(PyObject_GetAttr(manager_base, names.scratch));
-    if (!dict) raise_current();
-    PyObject *dev = item(c.dict, names.device);
-    PyObject *buf = PyDict_Check(dict.get()) ? PyDict_GetItemWithError(dict.get(), dev) : nullptr;
-    if (exact_tensor(buf) && (size_t)THPVariable_Unpack(buf).numel() >= want) return THPVariable_Unpack(buf);
-    Ref cfg(PyObject_CallMethodObjArgs(c.dm, names.cfg, item(instance_dict(item(c.dict, names.shared_context)), names.cmp_eps),
-                                       item(c.dict, names.sliced), nullptr));
-    Ref b(PyLong_FromLongLong(B)), s(PyLong_FromLongLong(c.S)), v(PyLong_FromLong(variant));
-    if (!cfg) raise_current();
-    Ref r(PyObject_CallMethodObjArgs(c.dm, names.product_ws, cfg.get(), b.get(), s.get(), backward ? Py_True : Py_False, v.get(), dev, nullptr));
-    if (!r) raise_current();
-    PyObject *t = PyTuple_GET_ITEM(r.get(), 0);
-    return t == Py_None ? Tensor() : THPVariable_Unpack(t);
+    return std::min(all, std::max(one, (size_t)std::max<int64_t>(0, class_int(names.scratch_limit))));
+}
+Tensor new_bytes(size_t bytes, const Call &c) {
+    return bytes ? at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, c.device)) : Tensor();
 }
 
 int product_variant(const Call &c) {
@@ -489,7 +478,7 @@ variable_list LayerNode::apply(variable_list &&grads) {
             flags = LUTB_PRODUCT_REUSE_HIST;
         }
     }
-    if (!flags) ws = product_scratch(c, B, true, variant);
+    if (!flags) ws = new_bytes(product_scratch_bytes(c, B, true, variant), c);
     check(lib.product_backward(&c.cfg, B, (int32_t)c.S, f32(c.weights), f32(xc), f32(xc), (int32_t)e, (int32_t)e, f32(pe), i32(c.anchors),
                                f32(dyc), f32(dx), f32(dx), f32(dpe), target, lr, variant | flags, ws.defined() ? ws.data_ptr() : nullptr,
                                ws.defined() ? (size_t)ws.numel() : 0, stream_of(c)));
@@ -582,13 +571,14 @@ PyObject *apply(PyObject *x_obj, PyObject *layer) {
                                      f32(pmd), i32(pmk), stream_of(c)));
         } else {
             PyDict_SetItem(c.dm_dict, names.dm_kept, Py_None);
-            Tensor ws = product_scratch(c, B, false, variant);
+            Tensor ws;
+            const size_t scratch = product_scratch_bytes(c, B, false, variant);
             int flags = 0;
-            if (c.training && ws.defined()) {
+            if (c.training && scratch > 0) {
                 // training: the row histogram is left in a workspace of its own for the backward pass
                 const size_t want = lib.product_workspace(&c.cfg, B, (int32_t)S, 1);
                 if (want > 0 && (int64_t)want <= class_int(names.keep_limit)) {
-                    const Tensor own = at::empty({(int64_t)want}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, c.device));
+                    const Tensor own = new_bytes(want, c);
                     if (lib.product_keeps_histogram(&c.cfg, B, (int32_t)S, (int32_t)inputs, (int32_t)inputs, variant, own.data_ptr(), want)) {
                         Ref key(histogram_key(c, B, xc, pe, context_eps(c), variant));
                         Ref entry(key ? kept_entry(c, own, key.get(), xc, pe) : nullptr);
@@ -599,6 +589,7 @@ PyObject *apply(PyObject *x_obj, PyObject *layer) {
                     }
                 }
             }
+            if (!flags) ws = new_bytes(scratch, c);
             check(lib.product_forward(&c.cfg, B, (int32_t)S, f32(c.weights), f32(xc), f32(xc), (int32_t)inputs, (int32_t)inputs, f32(pe),
                                       i32(c.anchors), f32(out), variant | flags, ws.defined() ? ws.data_ptr() : nullptr,
                                       ws.defined() ? (size_t)ws.numel() : 0, stream_of(c)));
@@ -665,7 +656,7 @@ void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::objec
                   in("_is_fully_connected"), in("_dw_variant"), in("_product_variant"), in("_sparse_rows_direct"), in("_device"),
                   in("_fully_connected"), in("_sparse"), in("_seq_len"), in("_forward_seen"), in("_kept_histogram"), in("n_weights"),
                   in("_rows_per_detector"), in("_cfg"), in("c_struct"), in("input_shape"), in("output_shape"), in("_prepare_positional_embeddings"),
-                  in("_external_lr"), in("_product_scratch"), in("product_scratch_limit"), in("product_keep_limit"), in("_product_workspace")};
+                  in("_external_lr"), in("product_scratch_limit"), in("product_keep_limit")};
     auto originals = [&](PyObject *cls, pybind11::list list, std::vector<std::pair<PyObject *, PyObject *>> &out) {
         for (auto n : list) {
             PyObject *name = in(n.cast<std::string>().c_str());

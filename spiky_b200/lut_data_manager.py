@@ -481,9 +481,8 @@ class _LUTDataManager:
         cfg = self._cfg(cmp_eps, sliced=sliced_mode)
         self._kept_histogram = None
         with torch.cuda.device(dev):
-            ws, ws_bytes = self._product_workspace(cfg, B, S, False, variant, r_weights.device)
             flags = 0
-            if keep_histogram and ws is not None:
+            if keep_histogram and self._product_scratch_bytes(cfg, B, S, False, variant):
                 L = _native.lib()
                 want = L.lutb_product_workspace(ctypes.byref(cfg), B, S, 1)
                 if 0 < want <= _LUTDataManager.product_keep_limit:
@@ -495,6 +494,8 @@ class _LUTDataManager:
                         self._kept_histogram = (own, self._histogram_key(
                             B, S, *read, n_inputs_1, n_inputs_2, sliced_mode, cmp_eps, variant, self._stream()),
                             tuple(None if t is None else t.detach() for t in read))
+            if not flags:
+                ws, ws_bytes = self._product_workspace(cfg, B, S, False, variant, r_weights.device)
             rc = _native.lib().lutb_product_forward(
                 ctypes.byref(cfg), B, S, _ptr(r_weights), _ptr(r_input_1), _ptr(r_input_2), int(n_inputs_1),
                 int(n_inputs_2), _ptr(r_positional_embeddings), _ptr(r_detector_anchors), _ptr(w_output),
@@ -549,12 +550,14 @@ class _LUTDataManager:
         cfg = self._cfg(cmp_eps, sliced=sliced_mode)
         kept, self._kept_histogram = self._kept_histogram, None
         with torch.cuda.device(dev):
-            ws, ws_bytes = self._product_workspace(cfg, B, S, True, variant, r_weights.device)
             if kept is not None and kept[1] == self._histogram_key(
                     B, S, r_input_1, r_input_2, r_detector_anchors, r_positional_embeddings, n_inputs_1, n_inputs_2,
                     sliced_mode, cmp_eps, variant, self._stream()):
                 # the forward pass over these very inputs left its histogram in this workspace
                 ws, ws_bytes, variant = kept[0], kept[0].numel(), int(variant) | _native.PRODUCT_REUSE_HIST
+            else:
+                kept = None
+                ws, ws_bytes = self._product_workspace(cfg, B, S, True, variant, r_weights.device)
             rc = _native.lib().lutb_product_backward(
                 ctypes.byref(cfg), B, S, _ptr(r_weights), _ptr(r_input_1), _ptr(r_input_2), int(n_inputs_1),
                 int(n_inputs_2), _ptr(r_positional_embeddings), _ptr(r_detector_anchors), _ptr(r_output_gradients),
@@ -562,29 +565,29 @@ class _LUTDataManager:
                 _ptr(w_weights_gradients), float(external_lr), int(variant), _ptr(ws), ws_bytes, self._stream())
         _native.check(rc)
 
-    # scratch of the histogram variant of the product kernels: one buffer per device, shared by all layers
-    # (a call only uses it between its own launches on the current stream)
-    _product_scratch = {}
+    # most scratch of one call of the histogram variant of the product kernels (more than one sequence's; the batch goes through in
+    # as many passes as that takes).  Every call takes its own from torch's allocator, which orders a block's next use on the
+    # stream of the call: calls on several streams or threads, and under capture, share nothing.
     product_scratch_limit = 16 << 30
+    _product_scratch = {}   # (calls hold on to no scratch; the name is there for programs that clear it)
 
-    def _product_workspace(self, cfg, B, S, backward, variant, device):
-        """(tensor or None, bytes) handed to the product entry points; None lets AUTO fall back to DIRECT."""
+    def _product_scratch_bytes(self, cfg, B, S, backward, variant):
+        """Bytes of scratch the product entry points get; 0 lets AUTO fall back to DIRECT."""
         if variant == _native.PRODUCT_DIRECT or self._INT_MODE or S < 2:
-            return None, 0
+            return 0
         rows = 1 << self._n_anchors
         L = _native.lib()
         # the library's own rule for AUTO (include/spiky_b200.h): no workspace is needed when it will pick DIRECT
         if variant == _native.PRODUCT_AUTO and 4 * S < rows:
-            return None, 0
+            return 0
         one = L.lutb_product_workspace(ctypes.byref(cfg), 1, S, int(backward))
-        want = min(L.lutb_product_workspace(ctypes.byref(cfg), B, S, int(backward)),
+        return min(L.lutb_product_workspace(ctypes.byref(cfg), B, S, int(backward)),
                    max(one, _LUTDataManager.product_scratch_limit))
-        buf = _LUTDataManager._product_scratch.get(device)
-        if buf is None or buf.numel() < want:
-            _LUTDataManager._product_scratch[device] = None
-            buf = torch.empty(want, dtype=torch.uint8, device=device)
-            _LUTDataManager._product_scratch[device] = buf
-        return buf, buf.numel()
+
+    def _product_workspace(self, cfg, B, S, backward, variant, device):
+        """(tensor or None, bytes) handed to the product entry points."""
+        want = self._product_scratch_bytes(cfg, B, S, backward, variant)
+        return (torch.empty(want, dtype=torch.uint8, device=device) if want else None), want
 
     # ------------------------------------------------------------------ concatenation-mode sequence runtime
     def forward_step_concat(self, r_weights, batch_size, r_input, r_detector_anchors, w_output, w_lookup_indices,
