@@ -248,10 +248,12 @@ __global__ void __launch_bounds__(kRowsThreads) dw_rows_emit_kernel(const float 
     }
 }
 
+// A workspace for more samples does for fewer as well: the last batch with short slices needs more than those after it.
 size_t fc_dw_rows_workspace(int64_t batch, int n_detectors, int table_rows) {
-    const int64_t n_blocks = ((int64_t)n_detectors * table_rows + kRowsBlock - 1) / kRowsBlock;
-    const size_t sorted = (sorted_workspace(batch, n_detectors, table_rows, rows_sort_block(batch, table_rows)) + 15) & ~(size_t)15;
-    return sorted + (size_t)n_blocks * sizeof(int32_t);
+    const int64_t n_blocks = ((int64_t)n_detectors * table_rows + kRowsBlock - 1) / kRowsBlock, last_short = 2048 / table_rows * kRowsSortBlock;
+    size_t sorted = sorted_workspace(batch, n_detectors, table_rows, rows_sort_block(batch, table_rows));
+    if (batch > last_short && last_short > 0) sorted = max(sorted, sorted_workspace(last_short, n_detectors, table_rows, kRowsSortBlock));
+    return ((sorted + 15) & ~(size_t)15) + (size_t)n_blocks * sizeof(int32_t);
 }
 
 int launch_fc_dw_rows(const float *dY, const int32_t *idx, int64_t batch, int n_outputs, int n_detectors, int table_rows,
