@@ -159,19 +159,23 @@ LAYER_CALLS_PATH = os.path.join(_HERE, "lib", "_layer_calls.so")
 
 
 def layer_calls():
-    """The extension module of the native host side of layer calls (host/layer_calls.cpp), set up; raises RuntimeError when
-    it is missing."""
+    """The extension module of the native host side of layer calls (host/layer_calls.cpp), set up; raises RuntimeError or
+    ImportError when it is missing or was built against another torch."""
     global _layer_calls
     if _layer_calls is None:
         if not os.path.exists(LAYER_CALLS_PATH):
             raise RuntimeError(f"{LAYER_CALLS_PATH} is missing: build it with `python -m spiky_b200.build`")
         import importlib.util
 
+        import torch
+
         from .lut_data_manager import LUTDataManagerF, _LUTDataManager
         from .lut_layer import GradientType, LUTLayerBasic
         spec = importlib.util.spec_from_file_location("_layer_calls", LAYER_CALLS_PATH)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
+        if module.torch_version != torch.__version__.split("+")[0]:   # (it uses torch's own data structures)
+            raise RuntimeError(f"{LAYER_CALLS_PATH} was built against torch {module.torch_version}, this is {torch.__version__}")
         handle = lib()
         module.setup(
             {name: ctypes.cast(getattr(handle, name), _vp).value for name in SIGNATURES},

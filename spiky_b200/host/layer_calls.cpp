@@ -11,6 +11,7 @@
 // them are autograd's own for an empty function), projection layer 206 / 105, concatenation-mode layer 238 / 109; the logits of
 // a four-layer transformer 607 / 314.
 #include <torch/extension.h>
+#include <torch/version.h>
 
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -676,5 +677,6 @@ PyMethodDef methods[] = {{"apply", (PyCFunction)(void (*)(void))apply_entry, MET
 
 PYBIND11_MODULE(_layer_calls, m) {
     m.def("setup", &setup);
+    m.attr("torch_version") = TORCH_VERSION;
     PyModule_AddFunctions(m.ptr(), methods);
 }

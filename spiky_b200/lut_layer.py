@@ -14,6 +14,7 @@ synapse-growth engine, so freshly constructed layers draw different random ancho
 does for the same seed (inject ``_explicit_anchors`` or use ``load_structure`` to reproduce a
 reference-built layer); anchors are a persistent buffer, so ``state_dict()`` round-trips them.
 """
+import warnings
 from dataclasses import dataclass
 from enum import Enum
 from typing import List
@@ -182,11 +183,23 @@ class _LUTFunction(torch.autograd.Function):
         return dx, dw, dpe, None
 
 
-def _layer_call(x, layer):
-    """First call of the process: load the native host side, which takes this function's place."""
+def _first_layer_call(x, layer):
+    """First call of the process: load the native host side, which takes this function's place.  Without it the Python route has
+    every call (the kernels are the same)."""
     global _layer_call
-    _layer_call = _native.layer_calls().apply
+    try:
+        _layer_call = _native.layer_calls().apply
+    except (ImportError, RuntimeError) as e:
+        warnings.warn(f"layer calls take the Python route, at about twice the host time: {e}", RuntimeWarning, stacklevel=3)
+        _layer_call = _no_layer_call
     return _layer_call(x, layer)
+
+
+def _no_layer_call(x, layer):
+    return None
+
+
+_layer_call = _first_layer_call
 
 
 class LUTLayerBasic(nn.Module):
