@@ -114,7 +114,8 @@ bool plain_cuda(const Tensor &t, at::ScalarType type, c10::DeviceIndex device) {
 }
 bool ordinary_context() {
     return !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() &&
-           at::functorch::functorchTLSAccessor() == nullptr;
+           (at::functorch::functorchTLSAccessor() == nullptr ||   // (it stays after the first transform; a key is there while one is active)
+            !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode));
 }
 
 enum Mode { NONSEQ, CONCAT, PRODUCT };

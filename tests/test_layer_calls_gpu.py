@@ -220,3 +220,11 @@ def test_a_kept_histogram_keeps_no_graph():
         del y, mark
         gc.collect()
         assert alive() is None
+
+
+def test_native_route_after_a_transform():
+    layer, x, gen = make("fc")
+    torch.vmap(lambda t: t + 1)(x)
+    assert not isinstance(layer(x.requires_grad_()).grad_fn, torch.autograd.function.BackwardCFunction)   # (the Python route's node)
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: layer(t).sum())(x)   # as before any of it: the Python route's answer while one is active
