@@ -187,7 +187,12 @@ def layer_calls():
             ["forward_step", "backward_backprop", "forward_step_concat", "backward_backprop_concat",
              "forward_step_product", "backward_backprop_product", "_cfg", "_stream", "_require_cuda", "_expect",
              "_sparse_forward", "_sparse_backward", "table_gradient_rows", "table_gradient_cells", "_product_workspace",
-             "_product_scratch_bytes", "_histogram_key", "get_weights_dimension"])
+             "_product_scratch_bytes", "_histogram_key", "get_weights_dimension"],
+            # what a layer's backward pass reads of it, in Python or native
+            ["_parameters", "_buffers", "_modules", "training", "device", "_lut_dm", "_shared_context", "_weights_gradient_policy",
+             "_sequence_length", "_concatenation_product", "_sliced_product_mode", "_unified_positional_embeddings", "_positional_dim",
+             "_is_fully_connected", "_n_inputs", "_n_outputs", "_n_detectors", "_n_anchors_per_detector", "_n_lookup_neurons",
+             "_input_shape", "_output_shape", "_multi_id", "_dw_variant", "_product_variant", "_sparse_rows_direct", "_external_lr_hook"])
         _layer_calls = module
     return _layer_calls
 

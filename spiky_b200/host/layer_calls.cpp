@@ -5,7 +5,8 @@
 // stays the definition of every case: fixed-point layers, replaced methods and hooks, tensor subclasses, tracing and
 // torch's modes, functorch transforms, forward-mode differentiation, whatever a check refuses.  Nothing is kept from one call
 // for the next: every attribute is read from the layer each time.  The node's backward pass looks again, and calls the
-// layer's Python method where it finds anything out of the ordinary.
+// layer's Python method where it finds anything out of the ordinary.  It does not own the layer, which may own its output: see
+// LayerNode.
 //
 // Measured, host time of forward and backward (Python route / this one): fully connected layer of 256 samples 231 / 110 us (59 of
 // them are autograd's own for an empty function), projection layer 206 / 105, concatenation-mode layer 238 / 109; the logits of
@@ -19,6 +20,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
@@ -63,6 +65,7 @@ PyObject *manager_class, *manager_base, *tensor_class, *parameter_class, *policy
 // methods whose replacement, on an instance or by a subclass, sends a call to the Python route
 std::vector<std::pair<PyObject *, PyObject *>> layer_methods, manager_methods;   // (name, original)
 std::vector<PyObject *> layer_hooks;
+std::vector<PyObject *> layer_parts;   // names of what a layer's backward pass reads
 
 struct Ref {   // owned reference
     PyObject *p = nullptr;
@@ -302,30 +305,81 @@ int product_variant(const Call &c) {
 }
 
 // ------------------------------------------------------------------------------------------------ backward
+// Python's collector cannot look into a node in C++: one that owned its layer would keep a layer that holds on to its own output
+// for ever.  So it knows the layer weakly, and owns what a layer that looks the same is made of (the parameters, the manager, the
+// settings), for a backward pass that comes after the layer has gone.  (A node in Python, torch.autograd.Function's, costs 11 us a call.)
 struct LayerNode : public torch::autograd::Node {
-    PyObject *layer;   // owned
+    PyObject *layer_ref, *cls;       // owned: weak reference, class
+    std::vector<PyObject *> parts;   // owned, or null; by layer_parts
     Mode mode;
     std::vector<SavedVariable> saved;
 
-    LayerNode(PyObject *l, Mode m) : layer(Py_NewRef(l)), mode(m) {}
+    LayerNode(PyObject *layer, PyObject *ref, PyObject *dict, Mode m) : layer_ref(ref), cls(Py_NewRef((PyObject *)Py_TYPE(layer))), mode(m) {
+        parts.reserve(layer_parts.size());
+        for (PyObject *name : layer_parts) parts.push_back(Py_XNewRef(item(dict, name)));
+    }
     ~LayerNode() override {
         if (Py_IsInitialized()) {
             pybind11::gil_scoped_acquire gil;
-            Py_CLEAR(layer);
+            Py_CLEAR(layer_ref);
+            Py_CLEAR(cls);
+            for (PyObject *&p : parts) Py_CLEAR(p);
         }
+    }
+    // The layer, or one made of its parts (a new reference; null with an exception)
+    PyObject *layer() const {
+        PyObject *alive = PyWeakref_GetObject(layer_ref);   // (borrowed; None: gone)
+        if (alive == nullptr) return nullptr;
+        if (alive != Py_None) return Py_NewRef(alive);
+        Ref args(PyTuple_New(0)), dict(PyDict_New());
+        if (!args || !dict) return nullptr;
+        for (size_t i = 0; i < parts.size(); i++)
+            if (parts[i] != nullptr && PyDict_SetItem(dict.get(), layer_parts[i], parts[i]) != 0) return nullptr;
+        PyTypeObject *type = reinterpret_cast<PyTypeObject *>(cls);
+        Ref made(type->tp_new(type, args.get(), nullptr));
+        if (!made || PyObject_SetAttrString(made.get(), "__dict__", dict.get()) != 0) return nullptr;
+        return Py_NewRef(made.get());
     }
     std::string name() const override { return "_LUTFunctionBackward"; }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
         for (auto &s : saved) s.reset_data();
     }
+    std::vector<Tensor> unpack() {
+        std::vector<Tensor> s;
+        std::lock_guard<std::mutex> lock(mutex_);
+        s.reserve(saved.size());
+        for (auto &v : saved) s.push_back(v.unpack());
+        return s;
+    }
     variable_list apply(variable_list &&grads) override;
 };
 
+// y.grad_fn.saved_tensors
+PyObject *saved_tensors(PyObject *self, void *) {
+    HANDLE_TH_ERRORS
+    auto *node = dynamic_cast<LayerNode *>(reinterpret_cast<torch::autograd::THPCppFunction *>(self)->cdata.get());
+    TORCH_CHECK(node != nullptr, "not the node of a layer call");
+    const std::vector<Tensor> s = node->unpack();
+    Ref t(PyTuple_New((Py_ssize_t)s.size()));
+    if (!t) return nullptr;
+    for (size_t i = 0; i < s.size(); i++) PyTuple_SET_ITEM(t.get(), (Py_ssize_t)i, THPVariable_Wrap(s[i]));
+    return Py_NewRef(t.get());
+    END_HANDLE_TH_ERRORS
+}
+// y.grad_fn.layer
+PyObject *node_layer(PyObject *self, void *) {
+    HANDLE_TH_ERRORS
+    auto *node = dynamic_cast<LayerNode *>(reinterpret_cast<torch::autograd::THPCppFunction *>(self)->cdata.get());
+    TORCH_CHECK(node != nullptr, "not the node of a layer call");
+    return node->layer();
+    END_HANDLE_TH_ERRORS
+}
+
 // The layer's Python method, on the saved tensors: everything the native route does not take.
-variable_list python_backward(LayerNode &node, const std::vector<Tensor> &saved, const Tensor &dy, bool need_dx) try {
+variable_list python_backward(LayerNode &node, PyObject *layer_obj, const std::vector<Tensor> &saved, const Tensor &dy, bool need_dx) try {
     namespace py = pybind11;
-    py::object layer = py::reinterpret_borrow<py::object>(node.layer), none = py::none();
+    py::object layer = py::reinterpret_borrow<py::object>(layer_obj), none = py::none();
     auto obj = [&](size_t i) { return i < saved.size() ? py::cast(saved[i]) : none; };
     py::object r;
     if (node.mode == NONSEQ)
@@ -375,22 +429,19 @@ Tensor sparse_table_gradient(const Call &c, int64_t B, const Tensor &dy, const T
 }
 
 variable_list LayerNode::apply(variable_list &&grads) {
-    std::vector<Tensor> s;
-    {
-        std::lock_guard<std::mutex> lock(mutex_);
-        s.reserve(saved.size());
-        for (auto &v : saved) s.push_back(v.unpack());
-    }
+    std::vector<Tensor> s = unpack();
     const bool need_dx = task_should_compute_output(0);
     Tensor dy = grads[0];
     pybind11::gil_scoped_acquire gil;
+    Ref layer_obj(layer());
+    if (!layer_obj) raise_current();
     const Tensor &x = s[0];
     if (!dy.defined()) {   // an output nobody used: zeros, as torch hands them to a Python function
         const auto &m = input_metadata(0);
         dy = at::zeros_symint(m.shape_as_dim_vector(), m.options());
     }
     Call c;
-    const bool readable = ordinary_context() && read_layer(layer, c, true);
+    const bool readable = ordinary_context() && read_layer(layer_obj.get(), c, true);
     if (!readable) PyErr_Clear();
     bool native = readable && c.mode == mode && !c.normalized &&
                   (c.policy_type == policy_dense || c.policy_type == policy_internal || (c.policy_type == policy_sparse && rows_direct(c))) && is_true(item(c.dm_dict, names.dm_forward_seen));
@@ -401,7 +452,7 @@ variable_list LayerNode::apply(variable_list &&grads) {
     native = native && plain_cuda(dy, at::kFloat, c.device);
     int64_t dw_variant = 0;
     native = native && as_int(item(c.dict, names.dw_variant), dw_variant) && (mode != PRODUCT || product_variant(c) >= 0);
-    if (!native) return python_backward(*this, s, dy, need_dx);
+    if (!native) return python_backward(*this, layer_obj.get(), s, dy, need_dx);
     at::NoGradGuard no_grad;   // (results carry no graph either way: their values come from kernels)
     c10::cuda::CUDAGuard guard(c.device);
     const Tensor xc = x.contiguous(), dyc = dy.contiguous();
@@ -420,10 +471,10 @@ variable_list LayerNode::apply(variable_list &&grads) {
     } else {
         fits = fits && s.size() == (size_t)(c.npe > 0 ? 2 : 1) && (c.npe == 0 || s[1].numel() == (c.S - 1) * Nt * c.npe);
     }
-    if (!fits) return python_backward(*this, s, dy, need_dx);
+    if (!fits) return python_backward(*this, layer_obj.get(), s, dy, need_dx);
     double lr = -1.0;
     if (internal) {
-        Ref r(PyObject_CallMethodNoArgs(layer, names.external_lr));
+        Ref r(PyObject_CallMethodNoArgs(layer_obj.get(), names.external_lr));
         if (!r) raise_current();
         lr = PyFloat_AsDouble(r.get());
         if (lr == -1.0 && PyErr_Occurred()) raise_current();
@@ -605,7 +656,9 @@ PyObject *apply(PyObject *x_obj, PyObject *layer) {
         }
     }
     if (needs_grad) {
-        auto node = std::shared_ptr<LayerNode>(new LayerNode(layer, c.mode), torch::autograd::deleteNode);
+        PyObject *ref = PyWeakref_NewRef(layer, nullptr);
+        if (ref == nullptr) raise_current();
+        auto node = std::shared_ptr<LayerNode>(new LayerNode(layer, ref, c.dict, c.mode), torch::autograd::deleteNode);
         node->set_next_edges(pe_in.defined() ? torch::autograd::collect_next_edges(x, c.weights, pe_in)
                                              : torch::autograd::collect_next_edges(x, c.weights));
         for (const Tensor &t : saved) node->saved.emplace_back(t, false);
@@ -622,7 +675,8 @@ PyObject *apply_entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::object manager_cls, pybind11::object base_cls, pybind11::object dense,
-           pybind11::object internal, pybind11::object sparse, pybind11::object check_fn, pybind11::list layer_names, pybind11::list hook_names, pybind11::list manager_names) {
+           pybind11::object internal, pybind11::object sparse, pybind11::object check_fn, pybind11::list layer_names, pybind11::list hook_names, pybind11::list manager_names,
+           pybind11::list part_names) {
     auto take = [&](const char *name, auto &fn) { fn = reinterpret_cast<std::decay_t<decltype(fn)>>(addresses[name].cast<uintptr_t>()); };
     take("lutb_nonseq_fc_forward", lib.fc_forward);
     take("lutb_nonseq_fc_backward", lib.fc_backward);
@@ -670,6 +724,15 @@ void setup(pybind11::dict addresses, pybind11::object layer_cls, pybind11::objec
     originals(layer_class, layer_names, layer_methods);
     originals(manager_class, manager_names, manager_methods);
     for (auto n : hook_names) layer_hooks.push_back(in(n.cast<std::string>().c_str()));
+    for (auto n : part_names) layer_parts.push_back(in(n.cast<std::string>().c_str()));
+    using namespace torch::autograd;   // (as the macro wants it)
+    static PyGetSetDef properties[] = {THP_FUNCTION_DEFAULT_PROPERTIES,
+                                       {"saved_tensors", saved_tensors, nullptr, nullptr, nullptr},
+                                       {"layer", node_layer, nullptr, nullptr, nullptr},
+                                       {nullptr}};
+    static PyTypeObject node_type;
+    _initFunctionPyTypeObject(node_type, "_LUTFunctionBackward", properties, nullptr);
+    registerCppFunction(typeid(LayerNode), &node_type);
 }
 
 PyMethodDef methods[] = {{"apply", (PyCFunction)(void (*)(void))apply_entry, METH_FASTCALL, "output of layer(x), or None"}, {nullptr, nullptr, 0, nullptr}};

@@ -228,3 +228,43 @@ def test_native_route_after_a_transform():
     assert not isinstance(layer(x.requires_grad_()).grad_fn, torch.autograd.function.BackwardCFunction)   # (the Python route's node)
     with pytest.raises(RuntimeError):
         torch.func.grad(lambda t: layer(t).sum())(x)   # as before any of it: the Python route's answer while one is active
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_layer_that_keeps_its_output(kind):
+    """It is freed with it, and the node shows what it has saved, and the layer."""
+    layer, x, gen = make(kind)
+    x = x.requires_grad_()
+    other = python_route(make(kind)[0])
+    y = other(x)
+    shapes = [tuple(t.shape) for t in y.grad_fn.saved_tensors]
+    layer.last = layer(x)
+    node = layer.last.grad_fn
+    assert [tuple(t.shape) for t in node.saved_tensors] == shapes and node.saved_tensors[0] is x
+    assert node.layer is layer and node.name() == "_LUTFunctionBackward" and node.next_functions[0][0] is not None
+    alive = weakref.ref(layer)
+    del layer, node
+    gc.collect()
+    assert alive() is None
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("backward", ["native", "python"])
+def test_backward_after_the_layer_has_gone(kind, backward):
+    layer, x, gen = make(kind)
+    want, dy = passed(make(kind)[0], x, gen=gen)
+    x = x.detach().requires_grad_()
+    y = layer(x)
+    if backward == "python":   # a gradient that the native route leaves
+        class Sub(torch.Tensor):
+            pass
+        y.register_hook(lambda g: g.as_subclass(Sub))
+    parameters = list(layer.parameters())
+    alive = weakref.ref(layer)
+    del layer
+    gc.collect()
+    assert alive() is None
+    y.backward(dy)
+    got = [y.detach(), x.grad] + [None if p.grad is None else p.grad.to_dense() for p in parameters] + [p.detach() for p in parameters]
+    for u, v in zip(got, want):
+        close(u if u is None else u.as_subclass(torch.Tensor), v)
