@@ -307,8 +307,7 @@ int tc_gemm_fast(TcGemmKind kind, int M, int N, int K, const float *A, int64_t l
 }  // namespace lutb
 #endif  // LUTB_NO_CUTLASS
 
-// C-ABI face of the contraction (used by the tests and by callers that want the same fp32-accurate tensor-core GEMM
-// the histogram path uses).
+// C-ABI face, for callers that want an fp32-accurate tensor-core GEMM; nothing else in the library uses it.
 extern "C" int lutb_fp32_gemm_available(void) { return lutb::tc_gemm_available() ? 1 : 0; }
 
 extern "C" size_t lutb_fp32_gemm_workspace(int32_t m, int32_t n, int32_t k) {

@@ -79,7 +79,8 @@ __device__ __forceinline__ void stage_rows(float *xs, const float *__restrict__ 
 }
 
 // One word of a plan: the swizzled 16-byte slots of the two inputs (of the first four rows; the other four's differ in the lowest
-// bit) in the order in which they are read, the anchor's bit, and whether that order is the reverse of the anchor's.
+// bit) in the order in which they are read, the anchor's bit, and whether that order is the reverse of the anchor's.  (14 bits a slot
+// hold 8192 inputs; eight rows of more than 7232 do not fit shared memory, so that lists are made up to there, see two_lanes().)
 constexpr int kPlanInputs = 8192, kPlanAnchors = 8;
 __device__ __forceinline__ uint32_t plan_word(int first, int second, int k, int swapped) {
     return (uint32_t)swizzle_slot(2 * first) | (uint32_t)swizzle_slot(2 * second) << 14 | (uint32_t)k << 28 | (uint32_t)swapped << 31;

@@ -58,3 +58,16 @@ def test_runs_of_samples(batch):
     idx = want["idx"]
     most = max(np.bincount(idx[:, t], minlength=16).max() for t in range(idx.shape[1]))
     assert np.abs(got["dW"].astype(np.float64) - want["dW"]).max() <= 2 * 2.0 ** -24 * most * most * np.abs(dY).max()
+
+
+@pytest.mark.parametrize("batch", [1, 793, 1585, 3173, 6341, 12645])
+def test_table_gradient_of_runs_is_exact(batch):
+    """Output gradients on a grid of 2^-6 of which any sum of a batch is an fp32 number: a run of samples that is left out or counted
+    twice shows in every cell, whatever the order of the sums."""
+    layer, x, dY = make((4, 4), 32, 9, batch)
+    dY = np.round(np.clip(dY, -4, 4) * 64) / 64
+    dY = dY.astype(np.float32)
+    assert batch * 4 * 64 < 2 ** 24
+    got, want = run_layer(layer, x, dY), oracle_layer(layer, x, dY, 4)
+    assert np.array_equal(got["idx"], want["idx"])
+    assert np.abs(want["dW"]).max() > 0 and np.array_equal(got["dW"], want["dW"])

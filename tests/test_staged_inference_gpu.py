@@ -23,7 +23,8 @@ def row_indices(x, anchors, Nc, eps):
     return idx
 
 
-# a row tile per SM is where the lists start to be used: 8 * 148 rows; the longest rows they reach, and one past
+# a row tile per SM is where the lists start to be used: 8 * 148 rows; rows of 8192 inputs and one past take another kernel (eight of
+# them do not fit shared memory: see test_ordered_anchor_lists_of_long_rows)
 @pytest.mark.parametrize("shape", [(1184, 8192, 517, 8), (1190, 8193, 517, 8), (1187, 3200, 1030, 6), (2500, 40, 2047, 5), (1200, 33, 513, 1)])
 @pytest.mark.parametrize("eps", [0.0, 0.4])
 def test_ordered_anchor_lists_give_the_same_indices(shape, eps):
@@ -50,6 +51,12 @@ def test_ordered_anchor_lists_give_the_same_indices(shape, eps):
     want = torch.stack([W[torch.arange(Nt, device="cuda"), idx[b].long()].double().sum(0) for b in rows])
     # 12 rows of a run are added in fp32, the runs in double
     assert (y[rows] - want).abs().max() <= 16 * 2.0 ** -24 * want.abs().max() * 12
+
+
+# eight rows with their anchors' ends in one block of an SM from 3200 inputs on, up to the longest that fit its shared memory, and one past
+@pytest.mark.parametrize("inputs", [3201, 5000, 7231, 7232, 7233])
+def test_ordered_anchor_lists_of_long_rows(inputs):
+    test_ordered_anchor_lists_give_the_same_indices((1187, inputs, 1030, 8), 0.0)
 
 
 # rows on both sides of where the lists start to be used
