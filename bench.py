@@ -1522,6 +1522,8 @@ def run_ours(args):
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": (traffic / max(d["timed"] / args.steps, 1)) if traffic else None,
                          "traffic_source": traffic_note,
+                         "algorithmic_bytes_are": "what the kernel asks for, every sample's rows counted, most of which come "
+                                                  "from caches; traffic is what HBM moved",
                          "algorithmic_bytes_per_launch": alg[dom] * wl.units_per_step / max(d["timed"] / args.steps, 1),
                          "ms_per_launch": dom_ms, "launches_per_step": d["timed"] / args.steps},
             "kernels": per_kernel,

@@ -25,7 +25,8 @@ namespace lutb {
 // sample are in flight together.  Rows of up to LG * VEC synapses use LG-lane groups (NG = 32 / LG groups
 // take detectors round-robin); VEC = 2 where every row of the chunk is made of aligned pairs (rows_of_pairs):
 // half of the loads and broadcasts.
-// Bound: requests of 64 to 100 byte rows to L2, about 6 TB/s of the sectors they touch.  Measured, 256-row tables, tables from
+// Bound: the latency of the row loads, with too few of them in flight (34 to 46 % of the warps, their largest stall; L1 55 to 72 % busy, L2 40 to
+// 52 %, issue 38 to 59 %, DRAM 23 to 35 %: no unit is full).  Measured, 256-row tables, tables from
 // HBM, one synapse a lane and 4 samples a run before.  Forward, 8192 detectors x 16 synapses: 100 samples 59 -> 30 us, 512 109 -> 62 (the
 // staged kernel, sparse_staged.cu: 70 and 75), 4096 288 (staged 544); 4608 detectors, 512 samples 57 -> 36 (53).  Input gradient,
 // 6400 + 8192 detectors, 512 samples: 236 -> 216 us; 8192 detectors, 4096 samples with 4 and 16 a run 727 -> 638.  Table gradient

@@ -8,8 +8,10 @@
 // so the row gathers and scatter-adds of the direct kernels (one table row per pair through L2) become dense
 // contractions: fp32-accurate GEMMs on the tensor cores (hist_gemm_sm100.cuh; the counters are then kept as fp16 in
 // the layout [row][detector][T], so that each of the three sums is ONE GEMM over all detectors), or, without them,
-// register-tiled fp32 FMA contractions whose table traffic is amortised over 128 query rows.  Worth it once a query
-// has about as many keys as the table has rows.
+// register-tiled fp32 FMA contractions whose table traffic is amortised over 128 query rows.  On the tensor cores worth it once a
+// query has a quarter of the table's rows as keys: forward, 16 detectors x 256 outputs, direct / tensor cores / FMA, ms: 4 x 512 tokens, 2048 rows
+// 2.79 / 0.18 / 3.58, 8 x 256, 1024 rows 0.73 / 0.09 / 1.78, 32 x 64, 256 rows 0.069 / 0.045 / 0.46.  The FMA contractions are chosen for more than
+// 2048 tokens only, of which the direct kernels' shared memory does not hold a sequence.
 #pragma once
 
 #include "lutb_common.cuh"
