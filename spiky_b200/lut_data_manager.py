@@ -508,7 +508,7 @@ class _LUTDataManager:
     # copies of strided ones among them, can come to lie there meanwhile.
     _kept_histogram = None
     # largest workspace a forward pass may hold on to until its backward pass (per layer)
-    product_keep_limit = 2 << 30
+    product_keep_limit = (8 << 30) // 3   # (a third of it can be room for halves of small elements, hist_gemm_sm100.cu)
 
     @staticmethod
     def _histogram_key(B, S, x1, x2, anchors, pe, e1, e2, sliced, cmp_eps, variant, stream):
