@@ -836,8 +836,7 @@ __device__ __noinline__ void second_phase(uint32_t base, uint32_t full0, uint32_
         for (int i = cluster; i < items && ok; i += clusters) {
             const Item it = item_of(g, i);
             const int row0 = it.m_tile * kTileM + (int)rank * 128 + quarter * 32;
-            const Sides t = sides(it);
-            ok = each_second_turn<A_PARTS>(g, it, t, [&](int kb0, int turn, uint32_t) {
+            ok = each_second_turn<A_PARTS>(g, it, sides(it), [&](int kb0, int turn, uint32_t) {
                 if (!__all_sync(0xffffffffu, wait_cluster(done0, acc_phase) && *gave_up == 0u)) return false;
                 fence_after();
                 acc_phase ^= 1u;
@@ -847,7 +846,12 @@ __device__ __noinline__ void second_phase(uint32_t base, uint32_t full0, uint32_
                 if (lane == 0) arrive_in_cluster(free_first);
                 return true;
             });
-            if (ok && (t.a_single || t.b_single)) add_single_products(g, t, row0, it.n_tile * kTileN + cols0);
+        }
+        // (behind all turns: nobody waits for these, and they have no limit in time)
+        for (int i = cluster; i < items && ok && A_PARTS == 2; i += clusters) {
+            const Item it = item_of(g, i);
+            const Sides t = sides(it);
+            if (t.a_single || t.b_single) add_single_products(g, t, it.m_tile * kTileM + (int)rank * 128 + quarter * 32, it.n_tile * kTileN + cols0);
         }
     }
     if (!ok) give_up(gave_up);
